@@ -26,15 +26,23 @@ __device__ inline void fb_pair(const StepConst& c, const double* dx, double r2, 
 // at (xΔt½, ρΔt½, vΔt½, P(ρΔt½)) with the stage-1 ∇W and fbmolforce! at x.
 // The reference's terms,
 // src/gpukernels_sph.jl, in their algebraically equal pair-once forms:
-//  * ∇W = Δx d𝒲/r with d𝒲/r = dWr (1 - u)^3 -- no division by r;
+//  * ∇W = Δx d𝒲/r with d𝒲/r = dWr (1 - u)^3 -- no division by r; in stage 1
+//    then Δv·∇W = (Δv·Δx) d𝒲/r and Δx·∇W = r² d𝒲/r;
 //  * ∂ρ∂tDDT! (:542-631): both sides share DDTkh m₀ (-Δx·∇W)/(r² + η²);
 //  * ∂v∂t! (:740-776) and ∂v∂t_av! (:852-901) as one factor of ∇W,
-//    -m₀ (Pk + Pm)/(ρk ρm) + 2 α c₀ h m₀ (Δv·Δx)/((r² + η²)(ρk + ρm)).
+//    -m₀ (Pk + Pm)/(ρk ρm) + 2 α c₀ h m₀ (Δv·Δx)/((r² + η²)(ρk + ρm));
+//  * ∂v∂tpF! (:1373-1409) with the products s/m₀ and 1.5π/2h.
+// The FP64 pipe bounds the pass, so a pair runs only the terms its ptypes
+// allow:
+//  * no term at all (neither side real, ptypes not both negative: the wall's
+//    inner pairs): stage 1 writes zero slots, stage 2 leaves them;
+//  * one side real: fbmolforce! alone, and that only within r₀.
 template <int D, int STAGE>
 __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, const PairBuf& B, int64_t u) {
   const int4 q = B.pq[u];
   const int k = q.x, m = q.y, e = q.z;
   int me = q.w;
+  const int ptk = S.pt[k], ptm = S.pt[m];
   if (STAGE == 1 && me < 0) {
     // the partner's row was not staged when the pair list was written: k's
     // position in m's (ascending) row of the finished neighbour list
@@ -47,109 +55,104 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
     me = (int)lo;
     B.pq[u] = make_int4(k, m, e, me);
   }
-  const double* const* XP = STAGE == 1 ? S.x : S.xh;
-  const double* const* VP = STAGE == 1 ? S.v : S.vh;
-  const double* RP = STAGE == 1 ? S.rho : S.rhoh;
-  const double* PP = STAGE == 1 ? S.P1 : S.P2;
-  const double* IP = STAGE == 1 ? S.ir : S.irh;
-  double dx[D], dv[D], gw[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    dx[d] = XP[d][k] - XP[d][m];
-    dv[d] = VP[d][k] - VP[d][m];
-  }
-  const double r2 = dotD<D>(dx, dx);
-  const bool r2pos = dbits(r2) != 0;  // r2 is +0 or positive
-  const int ptk = S.pt[k], ptm = S.pt[m];
   const bool mixed = (ptk > 0) != (ptm > 0);
-  double r = 0.0;
-  if (STAGE == 1) {
-    if (r2pos) r = sqrt_nr(r2);
-    const double uu = r * c.Hinv;
-    double w = 0.0, dwr = 0.0;
-    if (dbits(uu) < ONE_BITS) {
-      const double t = 1.0 - uu;
-      const double t2 = t * t;
-      if (c.need_w) w = ((1.0 + 4.0 * uu) * (t2 * t2)) * c.nW;
-      dwr = (t2 * t) * c.dWr;
-    }
-    if (!r2pos) dwr = NAN;  // the reference's d𝒲(0)/0
-    if (c.need_w) {
-      // both rows' slots: xsphcorr! and cspmcorr! walk every row
-      S.We[e] = w;
-      S.We[me] = w;
-    }
-    // stage 2 reads ∇W from the pair's k-side slot only (the call's ∑∇W is
-    // recomputed from the positions at its end)
+  const bool both = ptk > 0 && ptm > 0;
+  const bool press = ptk * ptm > 0;
+  double dk = 0.0, dm = 0.0, f[3] = {0.0, 0.0, 0.0};
+  if (!(mixed || both || press)) {
+    if (STAGE == 2) return;  // the slots hold stage 1's zeros
+  } else if (mixed) {
+    double dx[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) dx[d] = S.x[d][k] - S.x[d][m];
+    const double r2 = dotD<D>(dx, dx);
+    if (!(dbits(r2) > dbits(c.fb_r2cut))) fb_pair<D>(c, dx, r2, dbits(r2) != 0 ? sqrt_nr(r2) : 0.0, f);
+  } else {
+    const double* const* XP = STAGE == 1 ? S.x : S.xh;
+    const double* const* VP = STAGE == 1 ? S.v : S.vh;
+    const double* RP = STAGE == 1 ? S.rho : S.rhoh;
+    const double* PP = STAGE == 1 ? S.P1 : S.P2;
+    const double* IP = STAGE == 1 ? S.ir : S.irh;
+    double dx[D], dv[D], gw[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      gw[d] = dx[d] * dwr;
-      S.gWe[d][e] = gw[d];
+      dx[d] = XP[d][k] - XP[d][m];
+      dv[d] = VP[d][k] - VP[d][m];
     }
-  } else {
-    if (c.use_pF && r2pos) r = sqrt_nr(r2);
-#pragma unroll
-    for (int d = 0; d < D; ++d) gw[d] = S.gWe[d][e];
-  }
-  const double rk = RP[k], rm = RP[m], irk = IP[k], irm = IP[m];
-  const bool both = ptk > 0 && ptm > 0;
-  double dk = 0.0, dm = 0.0;
-  double sg = ptk * ptm > 0 ? -c.m0 * ((PP[k] + PP[m]) * (irk * irm)) : 0.0;
-  double visc = 0.0;
-  if (both) {
-    const double inv = rcp_nr(r2 + c.eta2);
-    const double m0dot = c.m0 * dotD<D>(dv, gw);
-    dk = m0dot;
-    dm = m0dot;
-    if (ptk > 1 || ptm > 1) {
-      const double com = c.DDTkhm0 * (-dotD<D>(dx, gw)) * inv;
-      const double ez = c.DDTgz * dx[1];
-      const double drr = rm - rk;
-      if (ptk > 1) {
-        const double dp = c.rho0 * (1.0 + pf7m1_fast(ez, c.ginv, c.gamma)) - c.rho0;
-        dk += (drr - dp) * com * irm;
-      }
-      if (ptm > 1) {
-        const double dn = c.rho0 * (1.0 + pf7m1_fast(-ez, c.ginv, c.gamma)) - c.rho0;
-        dm += (-drr - dn) * com * irk;
-      }
-    }
+    const double r2 = dotD<D>(dx, dx);
     const double cond = dotD<D>(dv, dx);
-    const bool av = neg_int(cond);
-    if (av || c.use_visc) {
-      const double isum = rcp_nr(rk + rm);
-      if (av) sg += c.avK * cond * inv * isum;
-      if (c.use_visc) visc = 4.0 * c.nu * c.m0 * dotD<D>(dx, gw) * isum * inv;
-    }
-  }
-  double f[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) f[d] = c.use_visc ? fma(visc, dv[d], sg * gw[d]) : sg * gw[d];
-  if (mixed) {
+    const bool r2pos = dbits(r2) != 0;  // r2 is +0 or positive
+    double r = 0.0, dxgw, dvgw;
     if (STAGE == 1) {
-      fb_pair<D>(c, dx, r2, r, f);
-    } else {
-      double dxf[D];
+      if (r2pos) r = sqrt_nr(r2);
+      const double uu = r * c.Hinv;
+      double w = 0.0, dwr = 0.0;
+      if (dbits(uu) < ONE_BITS) {
+        const double t = 1.0 - uu;
+        const double t2 = t * t;
+        if (c.need_w) w = ((1.0 + 4.0 * uu) * (t2 * t2)) * c.nW;
+        dwr = (t2 * t) * c.dWr;
+      }
+      if (!r2pos) dwr = NAN;  // the reference's d𝒲(0)/0
+      if (c.need_w) {
+        // both rows' slots: xsphcorr! and cspmcorr! walk every row (and read
+        // the pairs of two real sides only)
+        S.We[e] = w;
+        S.We[me] = w;
+      }
+      // stage 2 reads ∇W by pair (the call's ∑∇W is recomputed from the
+      // positions at its end)
 #pragma unroll
-      for (int d = 0; d < D; ++d) dxf[d] = S.x[d][k] - S.x[d][m];
-      const double r2f = dotD<D>(dxf, dxf);
-      fb_pair<D>(c, dxf, r2f, dbits(r2f) != 0 ? sqrt_nr(r2f) : 0.0, f);
+      for (int d = 0; d < D; ++d) {
+        gw[d] = dx[d] * dwr;
+        S.gWe[d][u] = gw[d];
+      }
+      dxgw = r2 * dwr;
+      dvgw = cond * dwr;
+    } else {
+      if (c.use_pF && r2pos) r = sqrt_nr(r2);
+#pragma unroll
+      for (int d = 0; d < D; ++d) gw[d] = S.gWe[d][u];
+      dxgw = dotD<D>(dx, gw);
+      dvgw = dotD<D>(dv, gw);
+    }
+    const double rk = RP[k], rm = RP[m], irk = IP[k], irm = IP[m];
+    double sg = press ? -c.m0 * ((PP[k] + PP[m]) * (irk * irm)) : 0.0;
+    double visc = 0.0;
+    if (both) {
+      const double inv = rcp_nr(r2 + c.eta2);
+      dk = c.m0 * dvgw;
+      dm = dk;
+      if (ptk > 1 || ptm > 1) {
+        const double com = c.DDTkhm0 * (-dxgw) * inv;
+        const double ez = c.DDTgz * dx[1];
+        const double drr = rm - rk;
+        if (ptk > 1) {
+          const double dp = c.rho0 * (1.0 + pf7m1_fast(ez, c.ginv, c.gamma)) - c.rho0;
+          dk += (drr - dp) * com * irm;
+        }
+        if (ptm > 1) {
+          const double dn = c.rho0 * (1.0 + pf7m1_fast(-ez, c.ginv, c.gamma)) - c.rho0;
+          dm += (-drr - dn) * com * irk;
+        }
+      }
+      const bool av = neg_int(cond);
+      if (av || c.use_visc) {
+        const double ii = rcp_nr(rk + rm) * inv;
+        if (av) sg += c.avK * cond * ii;
+        if (c.use_visc) visc = c.visc4 * dxgw * ii;
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < D; ++d) f[d] = c.use_visc ? fma(visc, dv[d], sg * gw[d]) : sg * gw[d];
+    if (c.use_pF && both && dbits(r) < dbits(c.twoh)) {
+      const double scos = c.pfs * cos_fast(c.pfk * r) * rcp_nr(r + c.hp1);
+#pragma unroll
+      for (int d = 0; d < D; ++d) f[d] = fma(scos, dx[d], f[d]);
     }
   }
-  if (c.use_pF) {
-    Acc<D> A;
-    A.zero();
-    pf_term<D>(c, A, ptk, ptm, dx, r);
-#pragma unroll
-    for (int d = 0; d < D; ++d) f[d] += A.pf[d];
-  }
-  B.cd[e] = dk;
-  B.cd[me] = dm;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    B.ca[d][e] = f[d];
-    B.ca[d][me] = -f[d];
-  }
+  put_slot(B.ce + e, dk, f[0], f[1], f[2]);
+  put_slot(B.ce + me, dm, -f[0], -f[1], -f[2]);
 }
 
 // Pass A over all pairs in chunks of 32 consecutive pairs, one chunk per warp
@@ -181,24 +184,60 @@ __global__ void __launch_bounds__(PA_TPB, 1) k_pairA(StepConst c, SArr<D> S, Pai
 // update's divisions and EOS power would issue on the FP64 pipe with 32 / L
 // lanes of a warp active: GB300 issues 2 FP64 thread-instructions per cycle
 // per SM, so that costs the full warp's time for a few lanes' work.)
-template <int D>
 struct RowSums {
-  double drho[32];
-  double a[D][32];
+  double v[4][32];  // ∂ρ/∂t, then ∂v/∂t, of the block's particles
 };
 
+// The four sums of a row over its L lanes.  Each of the first two exchanges
+// halves the values a lane still carries instead of summing all four on every
+// lane: 2 + 1 adds and one per further level, where a butterfly of all four
+// takes 4 log2 L -- at 32 lanes the butterfly cost the FP64 pipe more than
+// the row's entries did.  Lane q < 4 ends with the value of index
+// 2 (q & 1) + (q >> 1); with L = 2, lane 0 with 0 and 1 and lane 1 with 2 and 3.
+template <int L>
+__device__ __forceinline__ void lanes_total4(const double* s, int lane, int g, unsigned gm, RowSums& R) {
+  const bool b0 = lane & 1, b1 = lane & 2;
+  double k0 = b0 ? s[2] : s[0], k1 = b0 ? s[3] : s[1];
+  k0 += __shfl_xor_sync(gm, b0 ? s[0] : s[2], 1);
+  k1 += __shfl_xor_sync(gm, b0 ? s[1] : s[3], 1);
+  if constexpr (L == 2) {
+    R.v[2 * lane][g] = k0;
+    R.v[2 * lane + 1][g] = k1;
+  } else {
+    double t = b1 ? k1 : k0;
+    t += __shfl_xor_sync(gm, b1 ? k0 : k1, 2);
+#pragma unroll
+    for (int o = 4; o < L; o <<= 1) t += __shfl_xor_sync(gm, t, o);
+    if (lane < 4) R.v[2 * (lane & 1) + (lane >> 1)][g] = t;
+  }
+}
+
 template <int D, int L>
-__device__ __forceinline__ void pairB_sums(const SArr<D>& S, const PairBuf& B, int64_t N, RowSums<D>& R) {
+__device__ __forceinline__ void pairB_sums(const SArr<D>& S, const PairBuf& B, int64_t N, RowSums& R) {
   const int g = threadIdx.x / L, lane = threadIdx.x % L;
   const int64_t k = (int64_t)blockIdx.x * 32 + g;
-  double drho = 0.0, a[D];
+  if (k < N) {  // whole groups take part
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    const int64_t e1 = S.rs[k + 1];
+    int64_t e = S.rs[k] + lane;
+    // four entries' loads in flight at a time; each lane adds its entries in
+    // row order
+    for (; e + 3 * L < e1; e += 4 * L) {
+      double v[4][4];
 #pragma unroll
-  for (int d = 0; d < D; ++d) a[d] = 0.0;
-  if (k < N) row_sums<D, L>(S, B, k, lane, group_mask<L>(), drho, a);  // whole groups take part
-  if (lane == 0) {
-    R.drho[g] = drho;
+      for (int j = 0; j < 4; ++j) get_slot(B.ce + e + j * L, v[j]);
 #pragma unroll
-    for (int d = 0; d < D; ++d) R.a[d][g] = a[d];
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int d = 0; d < 1 + D; ++d) s[d] += v[j][d];
+    }
+    for (; e < e1; e += L) {
+      double v[4];
+      get_slot(B.ce + e, v);
+#pragma unroll
+      for (int d = 0; d < 1 + D; ++d) s[d] += v[d];
+    }
+    lanes_total4<L>(s, lane, g, group_mask<L>(), R);
   }
   __syncthreads();
 }
@@ -208,7 +247,7 @@ template <int D, int L>
 __global__ void __launch_bounds__(32 * L) k_pairB1(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S,
                                                    PairBuf B) {
   if (*S.ovf) return;
-  __shared__ RowSums<D> R;
+  __shared__ RowSums R;
   // warp 0 updates the block's 32 particles: their state is loaded before the
   // row sums, so that these loads overlap them (the row sums read only the
   // entry slots)
@@ -230,8 +269,8 @@ __global__ void __launch_bounds__(32 * L) k_pairB1(StepConst c, const Scal* __re
   if (!mine) return;
   double a[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) a[d] = R.a[d][threadIdx.x];
-  const double drho = R.drho[threadIdx.x];
+  for (int d = 0; d < D; ++d) a[d] = R.v[1 + d][threadIdx.x];
+  const double drho = R.v[0][threadIdx.x];
   a[1] = a[1] - c.g;
   double rv = rh0 + drho * hdt;
   if (rv < c.rho0 && ptk < 0) rv = c.rho0;
@@ -253,7 +292,7 @@ template <int D, int L>
 __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict__ sc, int64_t N, SArr<D> S,
                                                    PairBuf B, NextBin nb) {
   if (*S.ovf) return;  // uniform over the grid, before the barriers below
-  __shared__ RowSums<D> R;
+  __shared__ RowSums R;
   const bool w0 = threadIdx.x < 32;
   const int64_t k = (int64_t)blockIdx.x * 32 + threadIdx.x;
   // warp 0's particles' state, loaded before the row sums so that these
@@ -280,8 +319,8 @@ __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict
   if (mine) {
     double a[D], xn[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) a[d] = R.a[d][threadIdx.x];
-    const double drho = R.drho[threadIdx.x];
+    for (int d = 0; d < D; ++d) a[d] = R.v[1 + d][threadIdx.x];
+    const double drho = R.v[0][threadIdx.x];
     a[1] = a[1] - c.g;
     S.drho[k] = drho;
     S.Plast[k] = p2;

@@ -24,64 +24,40 @@ namespace gcsph {
 // ---------------------------------------------------------------------------
 // stage 1 at (x, ρ, v) + predictors
 // ---------------------------------------------------------------------------
-template <int D, int L, bool FAST = (L > 1)>
+template <int D>
 __global__ void __launch_bounds__(STPB) k_stage1(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S) {
   if (*S.ovf) return;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t k = gt / L;
-  const int lane = (int)(gt % L);
-  if (k >= N) return;  // whole sub-group leaves together
-  const unsigned gm = group_mask<L>();
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= N) return;
   const double dt = sc->dt;
   double xk[D], vk[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) { xk[d] = S.x[d][k]; vk[d] = S.v[d][k]; }
   const double rk = S.rho[k], Pk = S.P1[k];
-  const double irk = FAST ? S.ir[k] : 0.0;
   const int ptk = S.pt[k];
   double drho = 0.0;
   Acc<D> A;
   A.zero();
   const int64_t e0 = S.rs[k], e1 = S.rs[k + 1];
-  for (int64_t e = e0 + lane; e < e1; e += L) {
+  for (int64_t e = e0; e < e1; ++e) {
     const int32_t m = S.nbr[e];
     double dx[D], dv[D], gw[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) { dx[d] = xk[d] - S.x[d][m]; dv[d] = vk[d] - S.v[d][m]; }
     const double r2 = dotD<D>(dx, dx);
-    double r, dwk_r;
-    if (FAST) {
-      const double ri = rsqrt(r2);
-      r = r2 > 0.0 ? r2 * ri : 0.0;
-      const double u = r * c.Hinv;
-      S.We[e] = wc2_w(u, c.nW);
-      dwk_r = wc2_dw(u, c.nDW) * ri;
-    } else {
-      r = sqrt(r2);
-      const double u = r * c.Hinv;
-      S.We[e] = wc2_w(u, c.nW);                     // sphW!, :84-100
-      dwk_r = wc2_dw(u, c.nDW) / r;                 // sph∇W!, :196-213
-    }
+    const double r = sqrt(r2);
+    const double u = r * c.Hinv;
+    S.We[e] = wc2_w(u, c.nW);                       // sphW!, :84-100
+    const double dwk_r = wc2_dw(u, c.nDW) / r;      // sph∇W!, :196-213
 #pragma unroll
     for (int d = 0; d < D; ++d) { gw[d] = dx[d] * dwk_r; S.gWe[d][e] = gw[d]; }
     const int ptm = S.pt[m];
     const double rm = S.rho[m];
-    if (FAST) {
-      const bool both = ptk > 0 && ptm > 0;
-      const double inv_r2eta = both ? 1.0 / (r2 + c.eta2) : 0.0;
-      const double irm = S.ir[m];
-      if (both) drho += ddt_term_fast<D>(c, ptk, dx, inv_r2eta, gw, dv, rk, rm, irm);
-      mom_terms_fast<D>(c, A, ptk, ptm, dx, inv_r2eta, gw, dv, rk, rm, irk, irm, Pk, S.P1[m]);
-    } else {
-      if (ptk > 0 && ptm > 0) drho += ddt_term<D>(c, ptk, ptm, dx, r2, gw, dv, rk, rm);
-      mom_terms<D>(c, A, ptk, ptm, dx, r2, gw, dv, rk, rm, Pk, S.P1[m]);
-    }
+    if (ptk > 0 && ptm > 0) drho += ddt_term<D>(c, ptk, ptm, dx, r2, gw, dv, rk, rm);
+    mom_terms<D>(c, A, ptk, ptm, dx, r2, gw, dv, rk, rm, Pk, S.P1[m]);
     fb_term<D>(c, A, ptk, ptm, dx, r2);
     if (c.use_pF) pf_term<D>(c, A, ptk, ptm, dx, r);
   }
-  drho = group_sum<L>(drho, gm);
-  group_sum_acc<D, L>(A, c, gm);
-  if (lane != 0) return;
   double a[D];
   finish_acc<D>(c, A, a);
   // update_ρp∂ρ∂tΔt!, update_vp∂v∂tΔt!, update_xpvΔt! (:1088-1169), Δt/2
@@ -103,27 +79,23 @@ __global__ void __launch_bounds__(STPB) k_stage1(StepConst c, const Scal* __rest
 // ---------------------------------------------------------------------------
 // stage 2 at (xΔt½, ρΔt½, vΔt½) with stage-1 ∇W, + symplectic_update!
 // ---------------------------------------------------------------------------
-template <int D, int L, bool FAST = (L > 1)>
+template <int D>
 __global__ void __launch_bounds__(STPB) k_stage2(StepConst c, Scal* __restrict__ sc, int64_t N, SArr<D> S) {
   if (*S.ovf) return;  // uniform over the grid, before the block reduction below
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t k = gt / L;
-  const int lane = (int)(gt % L);
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double mc = 0.0;
   if (k < N) {
-    const unsigned gm = group_mask<L>();
     const double dt = sc->dt;
     double xk[D], xhk[D], vhk[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) { xk[d] = S.x[d][k]; xhk[d] = S.xh[d][k]; vhk[d] = S.vh[d][k]; }
     const double rk = S.rhoh[k], Pk = S.P2[k];
-    const double irk = FAST ? S.irh[k] : 0.0;
     const int ptk = S.pt[k];
     double drho = 0.0;
     Acc<D> A;
     A.zero();
     const int64_t e0 = S.rs[k], e1 = S.rs[k + 1];
-    for (int64_t e = e0 + lane; e < e1; e += L) {
+    for (int64_t e = e0; e < e1; ++e) {
       const int32_t m = S.nbr[e];
       double dx[D], dv[D], gw[D], dxf[D];
 #pragma unroll
@@ -135,16 +107,8 @@ __global__ void __launch_bounds__(STPB) k_stage2(StepConst c, Scal* __restrict__
       const double r2 = dotD<D>(dx, dx);
       const int ptm = S.pt[m];
       const double rm = S.rhoh[m];
-      if (FAST) {
-        const bool both = ptk > 0 && ptm > 0;
-        const double inv_r2eta = both ? 1.0 / (r2 + c.eta2) : 0.0;
-        const double irm = S.irh[m];
-        if (both) drho += ddt_term_fast<D>(c, ptk, dx, inv_r2eta, gw, dv, rk, rm, irm);
-        mom_terms_fast<D>(c, A, ptk, ptm, dx, inv_r2eta, gw, dv, rk, rm, irk, irm, Pk, S.P2[m]);
-      } else {
-        if (ptk > 0 && ptm > 0) drho += ddt_term<D>(c, ptk, ptm, dx, r2, gw, dv, rk, rm);
-        mom_terms<D>(c, A, ptk, ptm, dx, r2, gw, dv, rk, rm, Pk, S.P2[m]);
-      }
+      if (ptk > 0 && ptm > 0) drho += ddt_term<D>(c, ptk, ptm, dx, r2, gw, dv, rk, rm);
+      mom_terms<D>(c, A, ptk, ptm, dx, r2, gw, dv, rk, rm, Pk, S.P2[m]);
       if ((ptk > 0) != (ptm > 0)) {
 #pragma unroll
         for (int d = 0; d < D; ++d) dxf[d] = xk[d] - S.x[d][m];
@@ -152,37 +116,33 @@ __global__ void __launch_bounds__(STPB) k_stage2(StepConst c, Scal* __restrict__
       }
       if (c.use_pF) pf_term<D>(c, A, ptk, ptm, dx, sqrt(r2));
     }
-    drho = group_sum<L>(drho, gm);
-    group_sum_acc<D, L>(A, c, gm);
-    if (lane == 0) {
-      double a[D];
-      finish_acc<D>(c, A, a);
-      S.drho[k] = drho;
-      S.Plast[k] = Pk;
-      // symplectic_update!, :1204-1245
-      const double epsi = -(drho / rk) * dt;
-      double rv = S.rho[k] * (2.0 - epsi) / (2.0 + epsi);
-      if (rv < c.rho0 && ptk <= 1) rv = c.rho0;
-      S.rho[k] = rv;
-      S.rhoho[k] = rv;
-      S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
-      S.ir[k] = 1.0 / rv;
-      const double ml = ptk > 1 ? 1.0 : 0.0;
+    double a[D];
+    finish_acc<D>(c, A, a);
+    S.drho[k] = drho;
+    S.Plast[k] = Pk;
+    // symplectic_update!, :1204-1245
+    const double epsi = -(drho / rk) * dt;
+    double rv = S.rho[k] * (2.0 - epsi) / (2.0 + epsi);
+    if (rv < c.rho0 && ptk <= 1) rv = c.rho0;
+    S.rho[k] = rv;
+    S.rhoho[k] = rv;
+    S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
+    S.ir[k] = 1.0 / rv;
+    const double ml = ptk > 1 ? 1.0 : 0.0;
 #pragma unroll
-      for (int d = 0; d < D; ++d) {
-        S.a[d][k] = a[d];
-        const double vv = S.v[d][k];
-        const double nv = vv + a[d] * dt * ml;
-        S.vho[d][k] = nv;
-        S.v[d][k] = nv;
-        const double ddx = (vv + nv) * 0.5 * dt;
-        const double cd = S.cdx[d][k] + ddx;
-        S.cdx[d][k] = cd;
-        mc = fmax(mc, fabs(cd));
-        const double xv = xk[d] + ddx;
-        S.xho[d][k] = xv;
-        S.xo[d][k] = xv;
-      }
+    for (int d = 0; d < D; ++d) {
+      S.a[d][k] = a[d];
+      const double vv = S.v[d][k];
+      const double nv = vv + a[d] * dt * ml;
+      S.vho[d][k] = nv;
+      S.v[d][k] = nv;
+      const double ddx = (vv + nv) * 0.5 * dt;
+      const double cd = S.cdx[d][k] + ddx;
+      S.cdx[d][k] = cd;
+      mc = fmax(mc, fabs(cd));
+      const double xv = xk[d] + ddx;
+      S.xho[d][k] = xv;
+      S.xo[d][k] = xv;
     }
   }
   // maximum(maximum.(abs, cΔx)), src/sphproblem.jl:325
@@ -703,7 +663,7 @@ struct sph_handle {
   DevBuf X[2][3], XH[2][3], V[2][3], VH[2][3], RHO[2], RHOH[2], P1, P2, PT, A[3], DRHO, CDX[3], BUF2[3], PLAST, We,
       GWe[3], IR, IRH;
   DevBuf PT_b, BUF2_b[3];  // spares for the in-loop re-sort
-  DevBuf CD, CA[3], PQ;     // pair-once passes: per-entry contributions, flat pair list
+  DevBuf CE, PQ;            // pair-once passes: per-entry contributions, flat pair list
   int ix = 0, ixh = 0, iv = 0, ivh = 0, irho = 0, irhoh = 0;
   int64_t we_cap = 0;
   int lanes = 0;  // lanes per particle in the pair passes; 0 = by mean row length
@@ -748,8 +708,11 @@ static StepConst make_const(const sph_handle* h) {
   c.dWr = -20.0 * c.nDW * c.Hinv;
   c.DDTkhm0 = c.DDTkh * p.m0;
   c.avK = 2.0 * p.alpha * p.c0 * p.h * p.m0;
+  c.visc4 = 4.0 * p.nu * p.m0;
   c.twoh = 2.0 * p.h;
   c.pfc = 1.5 * GCSPH_PI64;
+  c.pfk = 1.5 * GCSPH_PI64 / (2.0 * p.h);
+  c.pfs = p.s / p.m0;
   c.hp1 = 0.1 * p.h;
   c.use_visc = p.nu > 0;
   c.use_pF = p.s > 0;
@@ -831,12 +794,11 @@ static int grow_entry_arrays(sph_handle* h) {
   const int64_t want = core.nbr_cap;
   int rc;
   if ((rc = h->We.ensure(sizeof(double) * want, core.st))) return rc;
-  if ((rc = h->CD.ensure(sizeof(double) * want, core.st))) return rc;
+  if ((rc = h->CE.ensure(sizeof(PairOut) * want, core.st))) return rc;
   if (want / 2 + 1 > (int64_t)INT32_MAX) return fail(GCSPH_ECAPACITY, "neighbour entries past 2^31");
   if ((rc = h->PQ.ensure(sizeof(int4) * (want / 2 + 1), core.st))) return rc;
   for (int d = 0; d < D; ++d) {
     if ((rc = h->GWe[d].ensure(sizeof(double) * want, core.st))) return rc;
-    if ((rc = h->CA[d].ensure(sizeof(double) * want, core.st))) return rc;
   }
   h->we_cap = want;
   return GCSPH_OK;
@@ -845,8 +807,7 @@ static int grow_entry_arrays(sph_handle* h) {
 template <int D>
 static PairBuf make_pairbuf(sph_handle* h) {
   PairBuf B{};
-  B.cd = h->CD.as<double>();
-  for (int d = 0; d < D; ++d) B.ca[d] = h->CA[d].as<double>();
+  B.ce = h->CE.as<PairOut>();
   B.pq = h->PQ.as<int4>();
   B.npair = h->cl->core.rs_up.as<int64_t>() + h->N;
   return B;
@@ -1056,6 +1017,7 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
   c.fb_d = 0.4;
   c.fb_r0 = 2.0 * p.dx;
   c.fb_eta2 = 0.01 * (c.fb_r0 * c.fb_r0);
+  c.fb_r2cut = c.fb_r0 * c.fb_r0 * (1.0 + 1e-6);
   const int L = choose_lanes(h);
   const bool once = L > 1;  // pair-once passes; L = 1 keeps the serial gather (bit-identical to the oracle)
   // W of the pairs is read by xsphcorr! and by a CSPM step's cspmcorr! only
@@ -1073,13 +1035,14 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
     timer_end(T_ROWSUM, st);
   } else {
     timer_begin(T_STAGE1, st);
-    PAIR_LAUNCH(k_stage1, L, c, dsc, h->N, make_arr<D>(h));
+    k_stage1<D><<<nb, STPB, 0, st>>>(c, dsc, h->N, make_arr<D>(h));
     GC_LAUNCHED();
     timer_end(T_STAGE1, st);
   }
   c.fb_d = p.bound_D;
   c.fb_r0 = p.bound_l;
   c.fb_eta2 = 0.01 * (c.fb_r0 * c.fb_r0);
+  c.fb_r2cut = c.fb_r0 * c.fb_r0 * (1.0 + 1e-6);
   if (once) {
     timer_begin(T_STAGE2, st);
     PAIRA_LAUNCH(2, c, make_arr<D>(h), make_pairbuf<D>(h));
@@ -1105,7 +1068,7 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
     timer_end(T_ROWSUM, st);
   } else {
     timer_begin(T_STAGE2, st);
-    PAIR_LAUNCH(k_stage2, L, c, dsc, h->N, make_arr<D>(h));
+    k_stage2<D><<<nb, STPB, 0, st>>>(c, dsc, h->N, make_arr<D>(h));
     GC_LAUNCHED();
     timer_end(T_STAGE2, st);
   }
@@ -1542,10 +1505,9 @@ void sph_destroy(sph_handle* h) {
   DevBuf* one[] = {&h->rhoh_o, &h->P_o, &h->drho_o, &h->sumW_o, &h->P1, &h->P2, &h->PT, &h->DRHO, &h->PLAST,
                    &h->We, &h->IR, &h->IRH, &h->scal, &h->RHO[0], &h->RHO[1], &h->RHOH[0], &h->RHOH[1], &h->PT_b};
   for (DevBuf* b : one) b->release();
-  h->CD.release();
+  h->CE.release();
   h->PQ.release();
   for (int d = 0; d < 3; ++d) {
-    h->CA[d].release();
     h->BUF2_b[d].release();
     h->vown[d].release();
     h->vh_o[d].release();

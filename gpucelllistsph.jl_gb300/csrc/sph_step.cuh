@@ -14,10 +14,12 @@ static constexpr int STPB = 128;
 struct StepConst {
   double h, eta2, m0, rho0, ginv, DDTkh, DDTgz, P0, alpha, c0, nu, g, s, Hinv, nW, nDW;
   double fb_d, fb_r0, fb_eta2;  // fbmolforce constants of the stage being run
+  double fb_r2cut;              // r₀² (1 + 1e-6): past it √r² >= r₀ whatever the rounding
   // pair-once products of the constants: d𝒲/r = dWr (1 - u)^3 (u / r = H⁻¹),
-  // δ-SPH's DDTkh m₀, and ∂v∂t_av!'s 2 α c₀ h m₀
-  double dWr, DDTkhm0, avK;
+  // δ-SPH's DDTkh m₀, ∂v∂t_av!'s 2 α c₀ h m₀ and ∂v∂t_visc!'s 4 ν m₀
+  double dWr, DDTkhm0, avK, visc4;
   double twoh, pfc, hp1;        // 2h, 1.5*pi, 0.1h  (∂v∂tpF!)
+  double pfk, pfs;              // 1.5 pi / 2h and s / m₀ (∂v∂tpF! of the pair-once pass)
   double dpc_l0inv, dpc_nW, dpc_whinv, dpc_pmin, dpc_pmax, dpc_lambda, dpc_kernlim, dpc_eta2;
   double dpc_r2cut;  // l0² (1 + 1e-6): past it u = √r² / l0 >= 1 whatever the rounding
   double xsph_c;                // 2*m0*eps
@@ -60,10 +62,10 @@ struct SArr {
   double* vh[3];
   double* rhoh;
   double* P2;
-  double* ir;   // 1/ρ (FAST stage 1)
-  double* irh;  // 1/ρΔt½ (FAST stage 2)
+  double* ir;   // 1/ρ (pair-once stage 1)
+  double* irh;  // 1/ρΔt½ (pair-once stage 2)
   double* We;
-  double* gWe[3];
+  double* gWe[3];  // ∇W: per neighbour entry on serial rows, per pair of the flat list on split rows
   double* a[3];
   double* drho;
   double* cdx[3];
@@ -197,15 +199,9 @@ __device__ inline void pf_term(const StepConst& c, Acc<D>& A, int ptk, int ptm, 
   }
 }
 
-// ---------------------------------------------------------------------------
-// FAST variants (lanes > 1): the same terms with fewer FP64 divisions -- the
-// FP64 pipe issues 2 thread-instructions per cycle per SM on GB300 and an IEEE
-// division costs ~8 of them.  1/ρ per particle is precomputed, 1/(r²+η²) is
-// shared by ∂ρ∂tDDT!, ∂v∂t_av! and ∂v∂t_visc!, 1/(ρᵢ+ρⱼ) by av and visc, and
-// powfancy7th's Newton step t - t(t³ - x/t⁴)/(4t³ + 3x/t⁴) is evaluated in the
-// equal form t - t(t⁷ - x)/(4t⁷ + 3x) with one division.  Each change moves a
-// result by a few ulp, inside the spread the reference's own atomics give.
-// ---------------------------------------------------------------------------
+// powfancy7th's step t - t(t³ - x/t⁴)/(4t³ + 3x/t⁴) in the equal form
+// t - t(t⁷ - x)/(4t⁷ + 3x), with one division (the pair-once passes, outside
+// the range of the series below)
 __device__ inline double powfancy7th_1div(double x, double ginv, int gamma) {
   if (gamma != 7) return pow(x, ginv);
   const double ax = fabs(x);
@@ -220,49 +216,6 @@ __device__ inline double powfancy7th_1div(double x, double ginv, int gamma) {
     t = t - (t * (t7 - x)) / (4.0 * t7 + 3.0 * x);
   }
   return t;
-}
-
-template <int D>
-__device__ inline double ddt_term_fast(const StepConst& c, int ptk, const double* dx, double inv_r2eta,
-                                       const double* gw, const double* dv, double rk, double rm, double irm) {
-  double dot3 = -dotD<D>(dx, gw);
-  double s = c.m0 * dotD<D>(dv, gw);
-  if (ptk > 1) {
-    double drhopvp = c.rho0 * powfancy7th_1div(1.0 + c.DDTgz * dx[1], c.ginv, c.gamma) - c.rho0;
-    double visc_densi = c.DDTkh * ((rm - rk) - drhopvp) * inv_r2eta;
-    s += visc_densi * dot3 * c.m0 * irm;
-  }
-  return s;
-}
-
-template <int D>
-__device__ inline void mom_terms_fast(const StepConst& c, Acc<D>& A, int ptk, int ptm, const double* dx,
-                                      double inv_r2eta, const double* gw, const double* dv, double rk, double rm,
-                                      double irk, double irm, double Pk, double Pm) {
-  if (ptk * ptm > 0) {
-    const double sc = -c.m0 * ((Pk + Pm) * (irk * irm));
-#pragma unroll
-    for (int d = 0; d < D; ++d) A.p[d] += sc * gw[d];
-  }
-  if (ptk > 0 && ptm > 0) {
-    const double cond = dotD<D>(dv, dx);
-    const bool av = cond < 0.0;
-    if (av || c.use_visc) {
-      const double inv_sum = 1.0 / (rk + rm);
-      if (av) {
-        const double dmu = c.h * cond * inv_r2eta;
-        const double dPi = (-c.alpha * c.c0 * dmu) * (2.0 * inv_sum);
-        const double sc = -dPi * c.m0;
-#pragma unroll
-        for (int d = 0; d < D; ++d) A.av[d] += sc * gw[d];
-      }
-      if (c.use_visc) {
-        const double nuterm = 4.0 * c.nu * c.m0 * dotD<D>(dx, gw) * inv_sum * inv_r2eta;
-#pragma unroll
-        for (int d = 0; d < D; ++d) A.vi[d] += nuterm * dv[d];
-      }
-    }
-  }
 }
 
 // a = ((((p + av) + visc) - g) + fb) + pF
@@ -303,19 +256,6 @@ __device__ inline double group_sum(double v, unsigned gm) {
   for (int o = L / 2; o > 0; o >>= 1) v = v + __shfl_xor_sync(gm, v, o);
   return v;
 }
-template <int D, int L>
-__device__ inline void group_sum_acc(Acc<D>& A, const StepConst& c, unsigned gm) {
-  if constexpr (L > 1) {
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      A.p[d] = group_sum<L>(A.p[d], gm);
-      A.av[d] = group_sum<L>(A.av[d], gm);
-      if (c.use_visc) A.vi[d] = group_sum<L>(A.vi[d], gm);
-      A.fb[d] = group_sum<L>(A.fb[d], gm);
-      if (c.use_pF) A.pf[d] = group_sum<L>(A.pf[d], gm);
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Pair-once stage passes (lanes > 1, the default).  The gather above
@@ -326,11 +266,23 @@ __device__ inline void group_sum_acc(Acc<D>& A, const StepConst& c, unsigned gm)
 // per-entry slots: slot e in k's row and slot mirror(e) in m's row.  Pass B:
 // each particle sums its whole row (L lanes, fixed order -- deterministic, no
 // atomics) and runs the predictor or the corrector.  Cost: one write + one
-// read of (1+D) doubles per neighbour entry.
+// read of a 32-byte slot per neighbour entry.  A slot is one DRAM and L2
+// sector: the partner side's slots are scattered, and as separate arrays each
+// of their 1 + D doubles touched a sector of its own.
 // ---------------------------------------------------------------------------
+struct __align__(32) PairOut {
+  double rho, a[3];       // ∂ρ/∂t and ∂v/∂t (gravity not included); a[2] unused in 2-D
+};
+// a slot in one 32-byte access
+__device__ __forceinline__ void put_slot(PairOut* p, double r, double a0, double a1, double a2) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(r), "d"(a0), "d"(a1), "d"(a2) : "memory");
+}
+// (the slots are read by a later launch than the one that wrote them)
+__device__ __forceinline__ void get_slot(const PairOut* p, double* v) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
 struct PairBuf {
-  double* cd;             // ∂ρ/∂t contribution per neighbour entry
-  double* ca[3];          // ∂v/∂t contribution per neighbour entry (gravity not included)
+  PairOut* ce;            // per neighbour entry: the pair's contribution to that row's sums
   int4* pq;               // (k, m, e, mirror(e)) of every pair, k < m (mirror -1: stage 1 finds it)
   const int64_t* npair;   // number of pairs (device scalar)
 };
@@ -339,10 +291,9 @@ struct PairBuf {
 // Pair-once arithmetic.  The FP64 pipe is the bound of pass A (2 FP64
 // thread-instructions per cycle per SM on GB300), so its compares run on the
 // integer pipe over the bit patterns, and its reciprocals and its root are
-// Newton-Raphson iterations from the hardware's approximate reciprocal and
-// reciprocal square root (rcp.approx / rsqrt.approx .f64, about 2^-22
-// relative): two steps each, quadratic convergence, a result within a few
-// ulp -- fewer FP64 instructions than the IEEE-rounded sequences, inside the
+// polynomial corrections of the hardware's approximate reciprocal and
+// reciprocal square root (rcp.approx / rsqrt.approx .f64, about 2^-20
+// relative): one third-order step each, a result within a few ulp -- fewer FP64 instructions than the IEEE-rounded sequences, inside the
 // FP64 contract this path is held to.
 // ---------------------------------------------------------------------------
 __device__ inline long long dbits(double x) { return __double_as_longlong(x); }
@@ -352,27 +303,53 @@ __device__ inline bool neg_int(double x) {
   return (unsigned long long)dbits(x) - 0x8000000000000001ull < 0x7FF0000000000000ull;
 }
 
-// 1/x, x normal (Newton-Raphson: y <- y + y (1 - x y))
+// 1/x, x normal: one third-order (Halley) step from the hardware's
+// approximate reciprocal, y <- y (1 + e + e^2) with e = 1 - x y.  |e| is about
+// 2^-20, so e^3 lies below the rounding; three FP64 instructions, where two
+// Newton steps take four.
 __device__ inline double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
-// sqrt(x), x normal and positive (Newton-Raphson on 1/sqrt(x):
-// y <- y + y (1/2 - (x/2) y^2), then x y)
+// sqrt(x), x normal and positive: s = x y from the approximate reciprocal
+// root y, then s (1 + e/2 + 3e^2/8) with e = 1 - s y (third order again): five
+// FP64 instructions, where two Newton steps on the root and the product take
+// eight.
 __device__ inline double sqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double hx = 0.5 * x;
-  double e = fma(-hx, y * y, 0.5);
-  y = fma(y, e, y);
-  e = fma(-hx, y * y, 0.5);
-  y = fma(y, e, y);
-  return x * y;
+  const double s = x * y;
+  const double e = fma(-s, y, 1.0);
+  return fma(s, e * fma(0.375, e, 0.5), s);
+}
+
+// cos(t) for 0 <= t < 3π/2 (∂v∂tpF! inside 2h): reduction by the nearest
+// multiple of π/2 (head and tail in FMAs), then one Taylor series, cosine's or
+// sine's by the quadrant's parity -- the coefficients are selected on the
+// integer pipe, so the FP64 pipe runs one series rather than gc_cos's two.
+__device__ inline double cos_fast(double t) {
+  const double C[8] = {-0.5, 0.041666666666666664, -0.001388888888888889, 2.48015873015873e-05,
+                       -2.755731922398589e-07, 2.08767569878681e-09, -1.1470745597729725e-11, 4.779477332387385e-14};
+  const double S[8] = {-0.16666666666666666, 0.008333333333333333, -0.0001984126984126984, 2.7557319223985893e-06,
+                       -2.505210838544172e-08, 1.6059043836821613e-10, -7.647163731819816e-13, 2.8114572543455206e-15};
+  const double MAGIC = 6755399441055744.0;  // 1.5 * 2^52: the sum's low mantissa bits are the rounded integer
+  const double km = fma(t, 0.6366197723675814, MAGIC);
+  const int q = (int)dbits(km);
+  const double kd = km - MAGIC;
+  double r = fma(-kd, 1.5707963267948966, t);
+  r = fma(-kd, 6.123233995736766e-17, r);
+  const double z = r * r;
+  const bool odd = q & 1;
+  double p = odd ? S[7] : C[7];
+#pragma unroll
+  for (int i = 6; i >= 0; --i) p = fma(p, z, odd ? S[i] : C[i]);
+  const double zr = z * r;
+  const double v = fma(odd ? zr : z, p, odd ? r : 1.0);
+  // cos t = cos r, -sin r, -cos r, sin r in the quadrants 0 .. 3
+  return __longlong_as_double(dbits(v) ^ ((long long)((q + 1) & 2) << 62));
 }
 
 // powfancy7th(x) - 1 for x = 1 + eps, src/gpukernels_sph.jl:499-515.  Where
@@ -405,66 +382,6 @@ __device__ inline double pf7m1_fast(double eps_in, double ginv, int gamma) {
   }
   return powfancy7th_1div(x, ginv, gamma) - 1.0;
 }
-
-// all momentum terms of one pair (FAST expressions), summed into f
-template <int D>
-__device__ inline void pair_force_fast(const StepConst& c, int ptk, int ptm, const double* dx, double r2,
-                                       double inv_r2eta, const double* gw, const double* dv, double rk, double rm,
-                                       double irk, double irm, double Pk, double Pm, double* f) {
-  Acc<D> A;
-  A.zero();
-  mom_terms_fast<D>(c, A, ptk, ptm, dx, inv_r2eta, gw, dv, rk, rm, irk, irm, Pk, Pm);
-#pragma unroll
-  for (int d = 0; d < D; ++d) f[d] = (A.p[d] + A.av[d]) + (c.use_visc ? A.vi[d] : 0.0);
-}
-
-template <int D, int STAGE>
-__device__ inline void pair_tail_terms(const StepConst& c, int ptk, int ptm, const double* dxf, const double* dx,
-                                       double r, double* f) {
-  Acc<D> A;
-  A.zero();
-  fb_term<D>(c, A, ptk, ptm, dxf, dotD<D>(dxf, dxf));
-  if (c.use_pF) pf_term<D>(c, A, ptk, ptm, dx, r);
-#pragma unroll
-  for (int d = 0; d < D; ++d) f[d] = (f[d] + A.fb[d]) + (c.use_pF ? A.pf[d] : 0.0);
-}
-
-// row sums of the per-entry contributions of particle k, L lanes
-template <int D, int L>
-__device__ inline void row_sums(const SArr<D>& S, const PairBuf& B, int64_t k, int lane, unsigned gm, double& drho,
-                                double* a) {
-  drho = 0.0;
-#pragma unroll
-  for (int d = 0; d < D; ++d) a[d] = 0.0;
-  const int64_t e0 = S.rs[k], e1 = S.rs[k + 1];
-  int64_t e = e0 + lane;
-  // four entries' loads in flight at a time; each sum still adds its
-  // entries in row order
-  for (; e + 3 * L < e1; e += 4 * L) {
-    double cv[4], av[4][D];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      cv[j] = B.cd[e + j * L];
-#pragma unroll
-      for (int d = 0; d < D; ++d) av[j][d] = B.ca[d][e + j * L];
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      drho += cv[j];
-#pragma unroll
-      for (int d = 0; d < D; ++d) a[d] += av[j][d];
-    }
-  }
-  for (; e < e1; e += L) {
-    drho += B.cd[e];
-#pragma unroll
-    for (int d = 0; d < D; ++d) a[d] += B.ca[d][e];
-  }
-  drho = group_sum<L>(drho, gm);
-#pragma unroll
-  for (int d = 0; d < D; ++d) a[d] = group_sum<L>(a[d], gm);
-}
-
 
 // pair-once passes (sph_once.cu): pass A over the device-side pair count,
 // one block per SM; pass B (row sums + predictor / corrector) with L lanes

@@ -1,0 +1,40 @@
+"""The pair-once passes on split rows, where their pair classes and lane
+counts can go wrong: walls whose pairs add nothing, walls of negative ptype
+(pressure between two of them, no other term), mixed pairs within and beyond
+r₀, surface tension over the whole range of its cosine, and every lane count
+of the row sums.  Against the CPU oracle with the FP64 contract (1e-12
+normwise, or 16x the noise of the reference's own re-ordered sums)."""
+import numpy as np
+import pytest
+
+from test_sph_gpu import check, make_pair, run_both, well_conditioned_v
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(pkg, D, layers):
+    if D == 2:
+        case = pkg.workloads.dam_break_2d(dx=0.04, fluid=(0.6, 0.8), tank=(1.2, 1.0), layer_ptype=layers)
+    else:
+        case = pkg.workloads.dam_break_3d(dx=0.05, fluid=(0.3, 0.4, 0.2), tank=(0.6, 0.6, 0.3), layer_ptype=layers)
+    case.s = 0.05
+    case.extra = dict(nu=0.2, xsph_eps=0.5, cspmn=3)
+    # off the lattice, so that no separation sits at a cut
+    rng = np.random.default_rng(11)
+    fl = case.ptype > 1
+    case.x = case.x.copy()
+    case.x[:, fl] += rng.uniform(-0.05, 0.05, (D, int(fl.sum()))) * case.dx
+    case.rho = case.rho + rng.uniform(0.0, 2.0, case.rho.size)
+    return case
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("layers", [(1, 0, 0), (1, -1, -1), (0, -1, 1)])
+@pytest.mark.parametrize("lanes", [2, 4, 32])
+def test_pair_classes(gpu_pkg, orc, D, layers, lanes):
+    case = _case(gpu_pkg, D, layers)
+    v = well_conditioned_v(case)
+    prob, ref = make_pair(gpu_pkg, orc, case, lanes, v=v)
+    for _ in range(2):  # the second call replays the captured graph
+        run_both(prob, ref, 4)
+    check(orc, prob, ref, case, lanes, [(4, {}), (4, {})], v=v)
