@@ -705,10 +705,9 @@ static StepConst make_const(const sph_handle* h) {
     c.nW = wc2_norm_w<3>(c.Hinv);
     c.nDW = wc2_norm_dw<3>(c.Hinv);
   }
-  c.dWr = -20.0 * c.nDW * c.Hinv;
-  c.DDTkhm0 = c.DDTkh * p.m0;
-  c.avK = 2.0 * p.alpha * p.c0 * p.h * p.m0;
-  c.visc4 = 4.0 * p.nu * p.m0;
+  c.dWr = -20.0 * c.nDW * c.Hinv * p.m0;
+  c.avK = 2.0 * p.alpha * p.c0 * p.h;
+  c.visc4 = 4.0 * p.nu;
   c.twoh = 2.0 * p.h;
   c.pfc = 1.5 * GCSPH_PI64;
   c.pfk = 1.5 * GCSPH_PI64 / (2.0 * p.h);
@@ -1028,7 +1027,7 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
   // pass A as the stage and the two row-sum passes together
   if (once) {
     timer_begin(T_STAGE1, st);
-    PAIRA_LAUNCH(1, c, make_arr<D>(h), make_pairbuf<D>(h));
+    PAIRA_LAUNCH(1, c, make_arr<D>(h), make_pairbuf<D>(h), core.nfull_est / 2);
     timer_end(T_STAGE1, st);
     timer_begin(T_ROWSUM, st);
     PAIRB_LAUNCH(1, L, c, dsc, make_arr<D>(h), make_pairbuf<D>(h));
@@ -1045,7 +1044,7 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
   c.fb_r2cut = c.fb_r0 * c.fb_r0 * (1.0 + 1e-6);
   if (once) {
     timer_begin(T_STAGE2, st);
-    PAIRA_LAUNCH(2, c, make_arr<D>(h), make_pairbuf<D>(h));
+    PAIRA_LAUNCH(2, c, make_arr<D>(h), make_pairbuf<D>(h), core.nfull_est / 2);
     timer_end(T_STAGE2, st);
     timer_begin(T_ROWSUM, st);
     // without Δt_stepping nothing after pass B2 feeds the step's end: its

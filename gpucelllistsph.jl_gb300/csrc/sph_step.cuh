@@ -15,9 +15,9 @@ struct StepConst {
   double h, eta2, m0, rho0, ginv, DDTkh, DDTgz, P0, alpha, c0, nu, g, s, Hinv, nW, nDW;
   double fb_d, fb_r0, fb_eta2;  // fbmolforce constants of the stage being run
   double fb_r2cut;              // r₀² (1 + 1e-6): past it √r² >= r₀ whatever the rounding
-  // pair-once products of the constants: d𝒲/r = dWr (1 - u)^3 (u / r = H⁻¹),
-  // δ-SPH's DDTkh m₀, ∂v∂t_av!'s 2 α c₀ h m₀ and ∂v∂t_visc!'s 4 ν m₀
-  double dWr, DDTkhm0, avK, visc4;
+  // pair-once products of the constants: m₀ d𝒲/r = dWr (1 - u)^3 (u / r = H⁻¹),
+  // ∂v∂t_av!'s 2 α c₀ h and ∂v∂t_visc!'s 4 ν
+  double dWr, avK, visc4;
   double twoh, pfc, hp1;        // 2h, 1.5*pi, 0.1h  (∂v∂tpF!)
   double pfk, pfs;              // 1.5 pi / 2h and s / m₀ (∂v∂tpF! of the pair-once pass)
   double dpc_l0inv, dpc_nW, dpc_whinv, dpc_pmin, dpc_pmax, dpc_lambda, dpc_kernlim, dpc_eta2;
@@ -65,7 +65,7 @@ struct SArr {
   double* ir;   // 1/ρ (pair-once stage 1)
   double* irh;  // 1/ρΔt½ (pair-once stage 2)
   double* We;
-  double* gWe[3];  // ∇W: per neighbour entry on serial rows, per pair of the flat list on split rows
+  double* gWe[3];  // ∇W per neighbour entry on serial rows, m₀∇W per pair of the flat list on split rows
   double* a[3];
   double* drho;
   double* cdx[3];
@@ -387,7 +387,7 @@ __device__ inline double pf7m1_fast(double eps_in, double ginv, int gamma) {
 // one block per SM; pass B (row sums + predictor / corrector) with L lanes
 // per particle, 32 particles per block
 template <int D>
-int launch_pairA(int stage, cudaStream_t st, const StepConst& c, const SArr<D>& S, const PairBuf& B);
+int launch_pairA(int stage, cudaStream_t st, const StepConst& c, const SArr<D>& S, const PairBuf& B, int64_t pairs_est);
 // The next step's binning started by pass B2 (update! every step): each
 // particle's cell key and arrival slot from its new position, and, in the
 // last block, the cell starts (CellCore::sort with keys_ready goes on from
