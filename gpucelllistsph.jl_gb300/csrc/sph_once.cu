@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(32 * L) k_pairB1(StepConst c, const Scal* __re
 // also the next binning's keys, slots and (last block) cell starts
 template <int D, int L>
 __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict__ sc, int64_t N, SArr<D> S,
-                                                   PairBuf B, NextBin nb) {
+                                                   PairBuf B, NextBin nb, PosCopy pc) {
   if (*S.ovf) return;  // uniform over the grid, before the barriers below
   __shared__ RowSums R;
   const bool w0 = threadIdx.x < 32;
@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict
       S.xho[d][k] = xv;
       S.xo[d][k] = xv;
       xn[d] = xv;
+      if (pc.f[0]) pc.f[d][k] = (float)(xv - pc.off[d]);
     }
     if (nb.key) {
       const int32_t ck = cell_key_v<D>(xn, nb.g);
@@ -456,6 +457,303 @@ __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict
   }
 }
 
+
+// ---------------------------------------------------------------------------
+// The gathers of a split-row step and the sums of a call: L lanes walk a
+// particle's row, GATHER_U entries of each lane in flight at a time (a row's
+// loads depend on its entry's index: at one entry a time these passes waited
+// on that chain).  Their FP64 instructions are the second bound, so divisions
+// and roots take the same forms as pass A's.
+// ---------------------------------------------------------------------------
+constexpr int GATHER_U = 4;
+
+// the sums s[0 .. n) of a row over its L lanes, on every lane (lanes_total4's
+// exchange, then the owners' values back)
+template <int L>
+__device__ __forceinline__ void lanes_sum4(double* s, int lane, unsigned gm) {
+  const bool b0 = lane & 1, b1 = lane & 2;
+  double k0 = b0 ? s[2] : s[0], k1 = b0 ? s[3] : s[1];
+  k0 += __shfl_xor_sync(gm, b0 ? s[0] : s[2], 1, L);
+  k1 += __shfl_xor_sync(gm, b0 ? s[1] : s[3], 1, L);
+  if constexpr (L == 2) {
+    s[0] = __shfl_sync(gm, k0, 0, L);
+    s[1] = __shfl_sync(gm, k1, 0, L);
+    s[2] = __shfl_sync(gm, k0, 1, L);
+    s[3] = __shfl_sync(gm, k1, 1, L);
+  } else {
+    double t = b1 ? k1 : k0;
+    t += __shfl_xor_sync(gm, b1 ? k0 : k1, 2, L);
+#pragma unroll
+    for (int o = 4; o < L; o <<= 1) t += __shfl_xor_sync(gm, t, o, L);
+    s[0] = __shfl_sync(gm, t, 0, L);
+    s[1] = __shfl_sync(gm, t, 2, L);
+    s[2] = __shfl_sync(gm, t, 1, L);
+    s[3] = __shfl_sync(gm, t, 3, L);
+  }
+}
+
+// dpcreg! + update_dpcreg!  (src/gpukernels_sph.jl:1500-1553, :1617-1632).
+// W = 0 from u = r / l₀ >= 1 on, so χ = 0, the factor (u >= dpckernlim) is χ
+// and Pᵇ = 0: such a pair adds an exact zero to either branch's sum.  l₀ lies
+// well under the spacing, so nearly every entry is one of those, and it is
+// told apart in FP32 on pass B2's copy of the positions: with R the largest
+// |x - offset| component of the particle, the copies of a pair with |Δx| <= l
+// differ by at most l + 2^-23 (R + l) per component, so past
+// (l + 2^-21 (R + l))² (1 + 2^-20) in FP32 it is beyond l = l₀ (1 + 1e-6).  The
+// rest take the FP64 test and terms.  (390k particles, 3-D: the FP64 test of
+// every entry cost 1.07 ms a step.)
+template <int D, int L>
+__global__ void __launch_bounds__(STPB) k_dpc_rows(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S,
+                                                   PosCopy pc) {
+  if (*S.ovf) return;
+  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t k = gt / L;
+  const int lane = (int)(gt % L);
+  if (k >= N) return;  // whole groups leave together
+  double sum[4] = {0.0, 0.0, 0.0, 0.0};
+  const int ptk = S.pt[k];
+  const double Pk = S.P1[k];
+  double xk[D], vk[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    xk[d] = S.x[d][k];
+    vk[d] = S.v[d][k];
+  }
+  if (ptk > 0) {
+    const double rk = S.rho[k], dt = sc->dt;
+    float fk[D];
+    double R = 0.0;
+    bool nan = false;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      fk[d] = pc.f[d][k];
+      R = fmax(R, fabs(xk[d] - pc.off[d]));
+      nan |= fk[d] != fk[d];
+    }
+    const double l = 1.000001 / c.dpc_l0inv;
+    const double lim = l + 0x1p-21 * (R + l);
+    const float thr = nan ? INFINITY : __double2float_ru(lim * lim * (1.0 + 0x1p-20));
+    const int64_t e1 = S.rs[k + 1];
+    for (int64_t e = S.rs[k] + lane; e < e1; e += GATHER_U * L) {
+      int32_t m[GATHER_U];
+      float r2f[GATHER_U];
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) m[j] = e + j * L < e1 ? S.nbr[e + j * L] : (int32_t)k;
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        r2f[j] = 0.f;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const float df = fk[d] - pc.f[d][m[j]];
+          r2f[j] = fmaf(df, df, r2f[j]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        if (r2f[j] > thr || m[j] == k) continue;
+        const int32_t i = m[j];
+        if (!(S.pt[i] > 0)) continue;
+        double dx[D], dv[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) dx[d] = xk[d] - S.x[d][i];
+        const double r2 = dotD<D>(dx, dx);
+        if (r2 > c.dpc_r2cut) continue;
+        const double u = sqrt(r2) * c.dpc_l0inv;
+        if (!(u < 1.0)) continue;
+#pragma unroll
+        for (int d = 0; d < D; ++d) dv[d] = vk[d] - S.v[d][i];
+        const double chi = sqrt(wc2_w(u, c.dpc_nW) * c.dpc_whinv);
+        const double vr = dotD<D>(dv, dx);
+        double f;
+        if (vr < 0.0) {
+          f = -(u < c.dpc_kernlim ? 1.0 : chi) * (vr / (r2 + c.dpc_eta2));
+        } else {
+          const double Pb =
+              chi * jl_max(jl_min(c.dpc_lambda * fabs(Pk + S.P1[i]), c.dpc_lambda * c.dpc_pmax), c.dpc_pmin);
+          f = 2.0 * dt * Pb / ((rk + S.rho[i]) * (r2 + c.dpc_eta2));
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d) sum[d] += f * dx[d];
+      }
+    }
+    lanes_sum4<L>(sum, lane, group_mask<L>());
+  }
+  if (lane != 0) return;
+  const double dt = sc->dt;
+  S.Plast[k] = Pk;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    S.buf2[d][k] = sum[d];
+    double nv = vk[d], nx = xk[d];
+    if (ptk > 1) {
+      nv = vk[d] + sum[d];
+      nx = xk[d] + sum[d] * dt;
+    }
+    S.vo[d][k] = nv;
+    S.xo[d][k] = nx;
+  }
+}
+
+// xsphcorr! + update_xsphcorr!  (:1757-1779, :1827-1838), stage-1 W
+template <int D, int L>
+__global__ void __launch_bounds__(STPB) k_xsph_rows(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S) {
+  if (*S.ovf) return;
+  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t k = gt / L;
+  const int lane = (int)(gt % L);
+  if (k >= N) return;
+  double sum[4] = {0.0, 0.0, 0.0, 0.0};
+  const int ptk = S.pt[k];
+  if (ptk > 1) {
+    double vk[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) vk[d] = S.v[d][k];
+    const double rk = S.rho[k];
+    const int64_t e1 = S.rs[k + 1];
+    for (int64_t e = S.rs[k] + lane; e < e1; e += GATHER_U * L) {
+      int32_t m[GATHER_U];
+      int pt[GATHER_U];
+      double w[GATHER_U], rm[GATHER_U], vm[GATHER_U][D];
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        const bool in = e + j * L < e1;
+        m[j] = in ? S.nbr[e + j * L] : (int32_t)k;
+        w[j] = in ? S.We[e + j * L] : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        pt[j] = S.pt[m[j]];
+        rm[j] = S.rho[m[j]];
+#pragma unroll
+        for (int d = 0; d < D; ++d) vm[j][d] = S.v[d][m[j]];
+      }
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        if (!(pt[j] > 1) || m[j] == k) continue;
+        const double xs = c.xsph_c * w[j] * rcp_nr(rk + rm[j]);
+#pragma unroll
+        for (int d = 0; d < D; ++d) sum[d] += (vm[j][d] - vk[d]) * xs;
+      }
+    }
+    lanes_sum4<L>(sum, lane, group_mask<L>());
+  }
+  if (lane != 0) return;
+  const double dt = sc->dt;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    S.buf2[d][k] = sum[d];
+    if (ptk > 1) S.x[d][k] = S.x[d][k] + sum[d] * dt;
+  }
+}
+
+// cspmcorr!  (:1693-1719), stage-1 W; writes ρ to the other buffer
+template <int D, int L>
+__global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr<D> S) {
+  if (*S.ovf) return;
+  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t k = gt / L;
+  const int lane = (int)(gt % L);
+  if (k >= N) return;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  const int ptk = S.pt[k];
+  if (ptk > 0) {
+    const int64_t e1 = S.rs[k + 1];
+    for (int64_t e = S.rs[k] + lane; e < e1; e += GATHER_U * L) {
+      int32_t m[GATHER_U];
+      int pt[GATHER_U];
+      double w[GATHER_U], rm[GATHER_U];
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        const bool in = e + j * L < e1;
+        m[j] = in ? S.nbr[e + j * L] : (int32_t)k;
+        w[j] = in ? S.We[e + j * L] : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        pt[j] = S.pt[m[j]];
+        rm[j] = S.rho[m[j]];
+      }
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) {
+        if (!(pt[j] > 0) || m[j] == k) continue;
+        const double mw = c.m0 * w[j];
+        s[0] += mw;
+        s[1] += mw * rcp_nr(rm[j]);
+      }
+    }
+    lanes_sum4<L>(s, lane, group_mask<L>());
+  }
+  if (lane != 0) return;
+  const double rk = S.rho[k];
+  const double nr = s[0] / s[1];
+  const double rv = isnan(nr) ? rk : nr;
+  S.rhoo[k] = rv;
+  S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
+  S.ir[k] = 1.0 / rv;
+  S.buf2[0][k] = s[0];
+  S.buf2[1][k] = s[1];
+  if (D == 3) S.buf2[2][k] = 0.0;
+}
+
+// post-batch sph∑W! + sph∑∇W!  (:139-156, :332-359).  The kernel's factors
+// come out of the sums: ∑W = nW ∑ (1 + 4u)(1 - u)^4, ∑∇W = dWg ∑ Δx (1 - u)^3.
+template <int D, int L>
+__global__ void __launch_bounds__(STPB) k_sums_rows(StepConst c, int64_t N, const int64_t* __restrict__ rs,
+                                                    const int32_t* __restrict__ nbr, PostSums Q,
+                                                    const int* __restrict__ ovf) {
+  if (*ovf) return;
+  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t k = gt / L;
+  const int lane = (int)(gt % L);
+  if (k >= N) return;
+  const int32_t ik = Q.map ? Q.map[k] : (int32_t)k;
+  double xk[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) xk[d] = Q.x[d][ik];
+  const bool real = Q.pt[ik] > 0;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  const int64_t e1 = rs[k + 1];
+  for (int64_t e = rs[k] + lane; e < e1; e += GATHER_U * L) {
+    int32_t m[GATHER_U];
+    int pt[GATHER_U];
+    double xm[GATHER_U][D];
+#pragma unroll
+    for (int j = 0; j < GATHER_U; ++j) m[j] = e + j * L < e1 ? nbr[e + j * L] : -1;
+    if (Q.map) {
+#pragma unroll
+      for (int j = 0; j < GATHER_U; ++j) m[j] = m[j] < 0 ? -1 : Q.map[m[j]];
+    }
+#pragma unroll
+    for (int j = 0; j < GATHER_U; ++j) {
+      const int32_t i = m[j] < 0 ? ik : m[j];
+      pt[j] = Q.pt[i];
+#pragma unroll
+      for (int d = 0; d < D; ++d) xm[j][d] = Q.x[d][i];
+    }
+#pragma unroll
+    for (int j = 0; j < GATHER_U; ++j) {
+      if (m[j] < 0 || (pt[j] > 0) != real) continue;
+      double dx[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) dx[d] = xk[d] - xm[j][d];
+      const double r2 = dotD<D>(dx, dx);
+      const bool r2pos = dbits(r2) != 0;
+      const double u = r2pos ? sqrt_nr(r2) * c.Hinv : 0.0;
+      if (!(dbits(u) < ONE_BITS)) continue;
+      const double t = 1.0 - u, t2 = t * t;
+      s[0] += fma(4.0, u, 1.0) * (t2 * t2);
+      const double t3 = r2pos ? t2 * t : NAN;  // the reference's d𝒲(0)/0
+#pragma unroll
+      for (int d = 0; d < D; ++d) s[1 + d] += dx[d] * t3;
+    }
+  }
+  lanes_sum4<L>(s, lane, group_mask<L>());
+  if (lane != 0) return;
+  const int32_t o = Q.orig[k];
+  Q.sumW[o] = s[0] * c.nW;
+#pragma unroll
+  for (int d = 0; d < D; ++d) Q.sg[d][o] = s[1 + d] * c.dWg;
+}
 
 template <int D, int STAGE, bool QUEUE>
 static int pairA_grid(int* g) {
@@ -497,14 +795,15 @@ int launch_pairA(int stage, cudaStream_t st, const StepConst& c, const SArr<D>& 
 
 template <int D>
 int launch_pairB(int stage, int L, int64_t N, cudaStream_t st, const StepConst& c, Scal* sc, const SArr<D>& S,
-                 const PairBuf& B, const NextBin* nb) {
+                 const PairBuf& B, const NextBin* nb, const PosCopy* pc) {
   const int g = nblocks(N, 32);  // 32 particles per block, 32 L threads
   const NextBin nbv = nb ? *nb : NextBin{};
+  const PosCopy pcv = pc ? *pc : PosCopy{};
 #define GC_PAIRB(LL)                                                        \
   if (stage == 1)                                                          \
     k_pairB1<D, LL><<<g, 32 * LL, 0, st>>>(c, sc, N, S, B);                \
   else                                                                     \
-    k_pairB2<D, LL><<<g, 32 * LL, 0, st>>>(c, sc, N, S, B, nbv);
+    k_pairB2<D, LL><<<g, 32 * LL, 0, st>>>(c, sc, N, S, B, nbv, pcv);
   switch (L) {
     case 2: GC_PAIRB(2) break;
     case 4: GC_PAIRB(4) break;
@@ -517,11 +816,55 @@ int launch_pairB(int stage, int L, int64_t N, cudaStream_t st, const StepConst& 
   return GCSPH_OK;
 }
 
+#define GC_ROWS(KER, ...)                                          \
+  do {                                                             \
+    const int g = nblocks(N * (int64_t)L, STPB);                   \
+    switch (L) {                                                   \
+      case 2: KER<D, 2><<<g, STPB, 0, st>>>(__VA_ARGS__); break;   \
+      case 4: KER<D, 4><<<g, STPB, 0, st>>>(__VA_ARGS__); break;   \
+      case 8: KER<D, 8><<<g, STPB, 0, st>>>(__VA_ARGS__); break;   \
+      case 16: KER<D, 16><<<g, STPB, 0, st>>>(__VA_ARGS__); break; \
+      default: KER<D, 32><<<g, STPB, 0, st>>>(__VA_ARGS__); break; \
+    }                                                              \
+    GC_LAUNCHED();                                                 \
+    return GCSPH_OK;                                               \
+  } while (0)
+
+template <int D>
+int launch_dpc(int L, int64_t N, cudaStream_t st, const StepConst& c, const Scal* sc, const SArr<D>& S,
+               const PosCopy& pc) {
+  GC_ROWS(k_dpc_rows, c, sc, N, S, pc);
+}
+template <int D>
+int launch_xsph(int L, int64_t N, cudaStream_t st, const StepConst& c, const Scal* sc, const SArr<D>& S) {
+  GC_ROWS(k_xsph_rows, c, sc, N, S);
+}
+template <int D>
+int launch_cspm(int L, int64_t N, cudaStream_t st, const StepConst& c, const SArr<D>& S) {
+  GC_ROWS(k_cspm_rows, c, N, S);
+}
+template <int D>
+int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, const int64_t* rs, const int32_t* nbr,
+                     const PostSums& Q, const int* ovf) {
+  GC_ROWS(k_sums_rows, c, N, rs, nbr, Q, ovf);
+}
+#undef GC_ROWS
+
+#define GC_INST(D)                                                                                                \
+  template int launch_dpc<D>(int, int64_t, cudaStream_t, const StepConst&, const Scal*, const SArr<D>&,          \
+                             const PosCopy&);                                                                     \
+  template int launch_xsph<D>(int, int64_t, cudaStream_t, const StepConst&, const Scal*, const SArr<D>&);         \
+  template int launch_cspm<D>(int, int64_t, cudaStream_t, const StepConst&, const SArr<D>&);                      \
+  template int launch_sums_post<D>(int, int64_t, cudaStream_t, const StepConst&, const int64_t*, const int32_t*,  \
+                                   const PostSums&, const int*);
+GC_INST(2)
+GC_INST(3)
+#undef GC_INST
 template int launch_pairA<2>(int, cudaStream_t, const StepConst&, const SArr<2>&, const PairBuf&, int64_t);
 template int launch_pairA<3>(int, cudaStream_t, const StepConst&, const SArr<3>&, const PairBuf&, int64_t);
 template int launch_pairB<2>(int, int, int64_t, cudaStream_t, const StepConst&, Scal*, const SArr<2>&,
-                             const PairBuf&, const NextBin*);
+                             const PairBuf&, const NextBin*, const PosCopy*);
 template int launch_pairB<3>(int, int, int64_t, cudaStream_t, const StepConst&, Scal*, const SArr<3>&,
-                             const PairBuf&, const NextBin*);
+                             const PairBuf&, const NextBin*, const PosCopy*);
 
 }  // namespace gcsph

@@ -191,14 +191,11 @@ __global__ void __launch_bounds__(256) k_pair_quads(int64_t N, const int64_t* __
 // ---------------------------------------------------------------------------
 // dpcreg! + update_dpcreg!  (:1500-1553, :1617-1632)
 // ---------------------------------------------------------------------------
-template <int D, int L>
+template <int D>
 __global__ void __launch_bounds__(STPB) k_dpc(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S) {
   if (*S.ovf) return;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t k = gt / L;
-  const int lane = (int)(gt % L);
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
-  const unsigned gm = group_mask<L>();
   const double dt = sc->dt;
   double xk[D], vk[D], sum[D];
 #pragma unroll
@@ -207,7 +204,7 @@ __global__ void __launch_bounds__(STPB) k_dpc(StepConst c, const Scal* __restric
   const int ptk = S.pt[k];
   const int64_t e0 = S.rs[k], e1 = S.rs[k + 1];
   if (ptk > 0) {
-    for (int64_t e = e0 + lane; e < e1; e += L) {
+    for (int64_t e = e0; e < e1; ++e) {
       const int32_t m = S.nbr[e];
       if (!(S.pt[m] > 0)) continue;
       double dx[D], dv[D];
@@ -242,9 +239,6 @@ __global__ void __launch_bounds__(STPB) k_dpc(StepConst c, const Scal* __restric
       }
     }
   }
-#pragma unroll
-  for (int d = 0; d < D; ++d) sum[d] = group_sum<L>(sum[d], gm);
-  if (lane != 0) return;
   S.Plast[k] = Pk;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -262,14 +256,11 @@ __global__ void __launch_bounds__(STPB) k_dpc(StepConst c, const Scal* __restric
 // ---------------------------------------------------------------------------
 // xsphcorr! + update_xsphcorr!  (:1757-1779, :1827-1838), stage-1 W
 // ---------------------------------------------------------------------------
-template <int D, int L>
+template <int D>
 __global__ void __launch_bounds__(STPB) k_xsph(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S) {
   if (*S.ovf) return;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t k = gt / L;
-  const int lane = (int)(gt % L);
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
-  const unsigned gm = group_mask<L>();
   const double dt = sc->dt;
   double vk[D], sum[D];
 #pragma unroll
@@ -278,7 +269,7 @@ __global__ void __launch_bounds__(STPB) k_xsph(StepConst c, const Scal* __restri
   const int ptk = S.pt[k];
   if (ptk > 1) {
     const int64_t e0 = S.rs[k], e1 = S.rs[k + 1];
-    for (int64_t e = e0 + lane; e < e1; e += L) {
+    for (int64_t e = e0; e < e1; ++e) {
       const int32_t m = S.nbr[e];
       if (!(S.pt[m] > 1)) continue;
       const double xs = c.xsph_c * S.We[e] / (rk + S.rho[m]);
@@ -286,9 +277,6 @@ __global__ void __launch_bounds__(STPB) k_xsph(StepConst c, const Scal* __restri
       for (int d = 0; d < D; ++d) sum[d] += (S.v[d][m] - vk[d]) * xs;
     }
   }
-#pragma unroll
-  for (int d = 0; d < D; ++d) sum[d] = group_sum<L>(sum[d], gm);
-  if (lane != 0) return;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     S.buf2[d][k] = sum[d];
@@ -299,20 +287,17 @@ __global__ void __launch_bounds__(STPB) k_xsph(StepConst c, const Scal* __restri
 // ---------------------------------------------------------------------------
 // cspmcorr!  (:1693-1719), stage-1 W; writes ρ to the other buffer
 // ---------------------------------------------------------------------------
-template <int D, int L>
+template <int D>
 __global__ void __launch_bounds__(STPB) k_cspm(StepConst c, int64_t N, SArr<D> S) {
   if (*S.ovf) return;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t k = gt / L;
-  const int lane = (int)(gt % L);
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
-  const unsigned gm = group_mask<L>();
   const double rk = S.rho[k];
   const int ptk = S.pt[k];
   double s1 = 0.0, s2 = 0.0;
   if (ptk > 0) {
     const int64_t e0 = S.rs[k], e1 = S.rs[k + 1];
-    for (int64_t e = e0 + lane; e < e1; e += L) {
+    for (int64_t e = e0; e < e1; ++e) {
       const int32_t m = S.nbr[e];
       if (!(S.pt[m] > 0)) continue;
       const double w = S.We[e];
@@ -320,9 +305,6 @@ __global__ void __launch_bounds__(STPB) k_cspm(StepConst c, int64_t N, SArr<D> S
       s2 += w * c.m0 / S.rho[m];
     }
   }
-  s1 = group_sum<L>(s1, gm);
-  s2 = group_sum<L>(s2, gm);
-  if (lane != 0) return;
   double nr = s1 / s2;
   double rv = isnan(nr) ? rk : nr;
   S.rhoo[k] = rv;
@@ -379,7 +361,7 @@ __global__ void k_step_end(StepConst c, Scal* __restrict__ sc) {
 // ---------------------------------------------------------------------------
 // post-batch sph∑W! + sph∑∇W! (:139-156, :332-359) on original-order arrays
 // ---------------------------------------------------------------------------
-template <int D, int L>
+template <int D>
 __global__ void __launch_bounds__(STPB) k_sums_post(StepConst c, int64_t N, const int64_t* __restrict__ rs,
                                                      const int32_t* __restrict__ nbr, const int32_t* __restrict__ orig,
                                                      const int32_t* __restrict__ pt, const double* __restrict__ x0,
@@ -388,11 +370,8 @@ __global__ void __launch_bounds__(STPB) k_sums_post(StepConst c, int64_t N, cons
                                                      double* __restrict__ sg1, double* __restrict__ sg2,
                                                      const int* __restrict__ ovf) {
   if (*ovf) return;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t k = gt / L;
-  const int lane = (int)(gt % L);
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
-  const unsigned gm = group_mask<L>();
   const double* X[3] = {x0, x1, x2};
   const int32_t o = orig[k];
   double xk[D];
@@ -402,7 +381,7 @@ __global__ void __launch_bounds__(STPB) k_sums_post(StepConst c, int64_t N, cons
   double sw = 0.0, sg[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) sg[d] = 0.0;
-  for (int64_t e = rs[k] + lane; e < rs[k + 1]; e += L) {
+  for (int64_t e = rs[k]; e < rs[k + 1]; ++e) {
     const int32_t om = orig[nbr[e]];
     if ((pt[om] > 0) != rk) continue;
     double dx[D];
@@ -415,10 +394,6 @@ __global__ void __launch_bounds__(STPB) k_sums_post(StepConst c, int64_t N, cons
 #pragma unroll
     for (int d = 0; d < D; ++d) sg[d] += dx[d] * dwk_r;
   }
-  sw = group_sum<L>(sw, gm);
-#pragma unroll
-  for (int d = 0; d < D; ++d) sg[d] = group_sum<L>(sg[d], gm);
-  if (lane != 0) return;
   sumW[o] = sw;
   double* SG[3] = {sg0, sg1, sg2};
 #pragma unroll
@@ -705,7 +680,8 @@ static StepConst make_const(const sph_handle* h) {
     c.nW = wc2_norm_w<3>(c.Hinv);
     c.nDW = wc2_norm_dw<3>(c.Hinv);
   }
-  c.dWr = -20.0 * c.nDW * c.Hinv * p.m0;
+  c.dWg = -20.0 * c.nDW * c.Hinv;
+  c.dWr = c.dWg * p.m0;
   c.avK = 2.0 * p.alpha * p.c0 * p.h;
   c.visc4 = 4.0 * p.nu;
   c.twoh = 2.0 * p.h;
@@ -933,20 +909,6 @@ static int rebuild(sph_handle* h, const StepConst& c, int* ovf_dev) {
   return GCSPH_OK;
 }
 
-// L lanes per particle: one launch per pair pass, N*L threads
-#define PAIR_LAUNCH(KER, L, ...)                                                              \
-  do {                                                                                        \
-    const int _g = nblocks(h->N * (int64_t)(L), STPB);                                        \
-    switch (L) {                                                                              \
-      case 1: KER<D, 1><<<_g, STPB, 0, st>>>(__VA_ARGS__); break;                             \
-      case 2: KER<D, 2><<<_g, STPB, 0, st>>>(__VA_ARGS__); break;                             \
-      case 4: KER<D, 4><<<_g, STPB, 0, st>>>(__VA_ARGS__); break;                             \
-      case 8: KER<D, 8><<<_g, STPB, 0, st>>>(__VA_ARGS__); break;                             \
-      case 16: KER<D, 16><<<_g, STPB, 0, st>>>(__VA_ARGS__); break;                           \
-      default: KER<D, 32><<<_g, STPB, 0, st>>>(__VA_ARGS__); break;                           \
-    }                                                                                         \
-  } while (0)
-
 // pass A: one thread per pair, one block per SM (the pair count itself
 // stays on the device); pass B: L lanes per row
 #define PAIRA_LAUNCH(STAGE, ...)                                                              \
@@ -961,13 +923,20 @@ static int rebuild(sph_handle* h, const StepConst& c, int* ovf_dev) {
     if (_rc) return _rc;                                                                      \
   } while (0)
 
+// Lanes per particle in the row sums and gathers: about four neighbours per
+// lane, but no more than four lanes from 6,000 particles on and eight below.
+// More lanes mean more short rows' tails and more of the sums' exchanges; four
+// fill the GPU once there are a few thousand particles (one GB300, a call at
+// 4 / 8 / 16 / 32 lanes: 390k particles in 3-D 26.8 / 27.2 / 28.2 / 31.5 ms,
+// 65k in 2-D 7.0 / 7.4 / 8.0 / 9.8 ms, 6.5k in 2-D 1.39 / 1.40 / 1.41 / 1.60 ms,
+// 1.7k in 2-D 0.87 / 0.81 / 0.81 / 0.86 ms).
 static int choose_lanes(const sph_handle* h) {
   if (h->lanes > 0) return h->lanes;
   const CellCore& core = h->cl->core;
-  double mean = h->N > 0 ? (double)core.nfull_est / (double)h->N : 0.0;
-  // about four neighbours per lane
+  const double mean = h->N > 0 ? (double)core.nfull_est / (double)h->N : 0.0;
+  const int most = h->N >= 6000 ? 4 : 8;
   int L = 1;
-  while (L < 32 && (double)L * 4.0 < mean) L <<= 1;
+  while (L < most && (double)L * 4.0 < mean) L <<= 1;
   return L;
 }
 
@@ -976,6 +945,7 @@ static int finish_call(sph_handle* h, const StepConst& c, Scal* dsc) {
   CellCore& core = h->cl->core;
   cudaStream_t st = core.st;
   int rc;
+  const bool was_in_cell_order = h->in_cell_order;
   if (h->in_cell_order && (rc = scatter_state<D>(h))) return rc;
   if (core.built && core.rows_upper) {
     // no update! ran in this call (n = 0) and the last pair set is the cell
@@ -991,11 +961,28 @@ static int finish_call(sph_handle* h, const StepConst& c, Scal* dsc) {
     double* sg2 = D == 3 ? h->sumgW_o[2].as<double>() : h->sumgW_o[0].as<double>();
     timer_begin(T_POST, st);
     const int L = choose_lanes(h);
-    PAIR_LAUNCH(k_sums_post, L, c, h->N, core.rs_full.as<int64_t>(), core.nbr.as<int32_t>(),
-                                        core.orig.as<int32_t>(), h->pt_u, h->cl->xuser[0], h->cl->xuser[1], x2,
-                                        h->sumW_o.as<double>(), h->sumgW_o[0].as<double>(),
-                                        h->sumgW_o[1].as<double>(), sg2, &dsc->ovf);
-    GC_LAUNCHED();
+    if (L > 1) {
+      // after a step the cell-order state holds the final points in the
+      // list's own order; without one (n = 0) they are read through the map
+      PostSums Q{};
+      const bool own = was_in_cell_order;
+      for (int d = 0; d < D; ++d) {
+        Q.x[d] = own ? h->X[h->ix][d].as<double>() : h->cl->xuser[d];
+        Q.sg[d] = h->sumgW_o[d].as<double>();
+      }
+      Q.pt = own ? h->PT.as<int32_t>() : h->pt_u;
+      Q.map = own ? nullptr : core.orig.as<int32_t>();
+      Q.orig = core.orig.as<int32_t>();
+      Q.sumW = h->sumW_o.as<double>();
+      if ((rc = launch_sums_post<D>(L, h->N, st, c, core.rs_full.as<int64_t>(), core.nbr.as<int32_t>(), Q, &dsc->ovf)))
+        return rc;
+    } else {
+      k_sums_post<D><<<nblocks(h->N, STPB), STPB, 0, st>>>(
+          c, h->N, core.rs_full.as<int64_t>(), core.nbr.as<int32_t>(), core.orig.as<int32_t>(), h->pt_u,
+          h->cl->xuser[0], h->cl->xuser[1], x2, h->sumW_o.as<double>(), h->sumgW_o[0].as<double>(),
+          h->sumgW_o[1].as<double>(), sg2, &dsc->ovf);
+      GC_LAUNCHED();
+    }
     timer_end(T_POST, st);
   }
   return GCSPH_OK;
@@ -1023,6 +1010,8 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
   // (the call's ∑W is recomputed from the positions at its end)
   c.need_w = (p.xsph_eps > 0) || (p.cspmn > 0 && cspmcnt == p.cspmn);
   bool folded = false;  // k_step_end's work done by pass B2's last block
+  PosCopy pc{};
+  int rc;
   // stage 1 (predictor) and stage 2 (corrector); the pair-once form times
   // pass A as the stage and the two row-sum passes together
   if (once) {
@@ -1062,7 +1051,15 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
       nb.g = core.g;
       h->keys_ready = true;
     }
-    PAIRB_LAUNCH(2, L, c2, dsc, make_arr<D>(h), make_pairbuf<D>(h), &nb);
+    // dpcreg!'s prefilter copy of the new positions goes over the pair
+    // build's, which this step's list no longer reads
+    if (p.dpc_l0 > 0) {
+      for (int d = 0; d < D; ++d) {
+        pc.f[d] = core.pf[d].as<float>();
+        pc.off[d] = core.g.offset[d];
+      }
+    }
+    PAIRB_LAUNCH(2, L, c2, dsc, make_arr<D>(h), make_pairbuf<D>(h), &nb, &pc);
     folded = c2.fold_end != 0;
     timer_end(T_ROWSUM, st);
   } else {
@@ -1077,22 +1074,34 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
   h->irhoh ^= 1;
   if (p.dpc_l0 > 0) {
     timer_begin(T_DPC, st);
-    PAIR_LAUNCH(k_dpc, L, c, dsc, h->N, make_arr<D>(h));
-    GC_LAUNCHED();
+    if (once) {
+      if ((rc = launch_dpc<D>(L, h->N, st, c, dsc, make_arr<D>(h), pc))) return rc;
+    } else {
+      k_dpc<D><<<nb, STPB, 0, st>>>(c, dsc, h->N, make_arr<D>(h));
+      GC_LAUNCHED();
+    }
     timer_end(T_DPC, st);
     h->iv ^= 1;
     h->ix ^= 1;
   }
   if (p.xsph_eps > 0) {
     timer_begin(T_XSPH, st);
-    PAIR_LAUNCH(k_xsph, L, c, dsc, h->N, make_arr<D>(h));
-    GC_LAUNCHED();
+    if (once) {
+      if ((rc = launch_xsph<D>(L, h->N, st, c, dsc, make_arr<D>(h)))) return rc;
+    } else {
+      k_xsph<D><<<nb, STPB, 0, st>>>(c, dsc, h->N, make_arr<D>(h));
+      GC_LAUNCHED();
+    }
     timer_end(T_XSPH, st);
   }
   if (p.cspmn > 0 && cspmcnt == p.cspmn) {
     timer_begin(T_CSPM, st);
-    PAIR_LAUNCH(k_cspm, L, c, h->N, make_arr<D>(h));
-    GC_LAUNCHED();
+    if (once) {
+      if ((rc = launch_cspm<D>(L, h->N, st, c, make_arr<D>(h)))) return rc;
+    } else {
+      k_cspm<D><<<nb, STPB, 0, st>>>(c, h->N, make_arr<D>(h));
+      GC_LAUNCHED();
+    }
     timer_end(T_CSPM, st);
     h->irho ^= 1;
     cspmcnt = 0;

@@ -18,6 +18,7 @@ struct StepConst {
   // pair-once products of the constants: m₀ d𝒲/r = dWr (1 - u)^3 (u / r = H⁻¹),
   // ∂v∂t_av!'s 2 α c₀ h and ∂v∂t_visc!'s 4 ν
   double dWr, avK, visc4;
+  double dWg;                   // d𝒲/r = dWg (1 - u)^3 (∑∇W of a call)
   double twoh, pfc, hp1;        // 2h, 1.5*pi, 0.1h  (∂v∂tpF!)
   double pfk, pfs;              // 1.5 pi / 2h and s / m₀ (∂v∂tpF! of the pair-once pass)
   double dpc_l0inv, dpc_nW, dpc_whinv, dpc_pmin, dpc_pmax, dpc_lambda, dpc_kernlim, dpc_eta2;
@@ -399,8 +400,36 @@ struct NextBin {
   int32_t* cellstart;
   Grid g;
 };
+// the FP32 copy (x - offset) of the particles' new positions that pass B2
+// writes for dpcreg!'s prefilter; f[0] == nullptr: none
+struct PosCopy {
+  float* f[3];
+  double off[3];
+};
 template <int D>
 int launch_pairB(int stage, int L, int64_t N, cudaStream_t st, const StepConst& c, Scal* sc, const SArr<D>& S,
-                 const PairBuf& B, const NextBin* nb = nullptr);
+                 const PairBuf& B, const NextBin* nb = nullptr, const PosCopy* pc = nullptr);
+
+// the gathers of a split-row step (L >= 2 lanes per particle)
+template <int D>
+int launch_dpc(int L, int64_t N, cudaStream_t st, const StepConst& c, const Scal* sc, const SArr<D>& S,
+               const PosCopy& pc);
+template <int D>
+int launch_xsph(int L, int64_t N, cudaStream_t st, const StepConst& c, const Scal* sc, const SArr<D>& S);
+template <int D>
+int launch_cspm(int L, int64_t N, cudaStream_t st, const StepConst& c, const SArr<D>& S);
+// ∑W and ∑∇W of a call.  X: the positions and pt the ptypes, by cell-order
+// index (map null) or by map[cell-order index]; results go to orig's places.
+struct PostSums {
+  const double* x[3];
+  const int32_t* pt;
+  const int32_t* map;
+  const int32_t* orig;
+  double* sumW;
+  double* sg[3];
+};
+template <int D>
+int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, const int64_t* rs, const int32_t* nbr,
+                     const PostSums& Q, const int* ovf);
 
 }  // namespace gcsph

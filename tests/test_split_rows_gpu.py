@@ -38,3 +38,37 @@ def test_pair_classes(gpu_pkg, orc, D, layers, lanes):
     for _ in range(2):  # the second call replays the captured graph
         run_both(prob, ref, 4)
     check(orc, prob, ref, case, lanes, [(4, {}), (4, {})], v=v)
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("lanes", [2, 8, 32])
+def test_dpc_prefilter(gpu_pkg, orc, D, lanes):
+    """dpcreg! with pairs on both sides of l₀ (fluid jittered by up to a
+    quarter of the spacing, l₀ = 0.7 dx): the FP32 test must pass on every pair
+    the FP64 one takes."""
+    case = _case(gpu_pkg, D, (1, 0, 0))
+    rng = np.random.default_rng(3)
+    fl = case.ptype > 1
+    case.x[:, fl] += rng.uniform(-0.2, 0.2, (D, int(fl.sum()))) * case.dx
+    case.extra = dict(case.extra, dpc_l0=0.7 * case.dx, dpc_lambda=0.005, dpc_pmax=36000.0)
+    v = well_conditioned_v(case)
+    prob, ref = make_pair(gpu_pkg, orc, case, lanes, v=v)
+    run_both(prob, ref, 6)
+    assert np.abs(ref.get("buf2")).max() > 0
+    check(orc, prob, ref, case, lanes, [(6, {})], v=v)
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("lanes", [2, 4, 32])
+def test_sums_without_a_step(gpu_pkg, orc, D, lanes):
+    """A call of no steps sums W and ∇W over the caller's points through the
+    map, one of a step over the cell-order state."""
+    case = _case(gpu_pkg, D, (1, 0, 0))
+    prob, ref = make_pair(gpu_pkg, orc, case, lanes)
+    for n in (0, 1):
+        run_both(prob, ref, n)
+        for f in ("sumW", "sumgW"):
+            got, want = prob.field(f), ref.get(f)
+            got = np.stack([t.cpu().numpy() for t in got]) if isinstance(got, tuple) else got.cpu().numpy()
+            # eight roundings per term of up to 200 terms against ∑|terms| <= 4x the largest sum
+            assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max(), f
