@@ -116,7 +116,9 @@ __global__ void k_cellkey(const double* __restrict__ x0, const double* __restric
   if (popmax) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) pop = max(pop, __shfl_xor_sync(0xffffffffu, pop, o));
-    if ((threadIdx.x & 31) == 0 && pop > 0) atomicMax(popmax, pop);
+    // (a lane that sees a larger value already there leaves the word alone: an
+    // atomic per warp on one word took 0.1 ms at 4M points)
+    if ((threadIdx.x & 31) == 0 && pop > *(volatile int*)popmax) atomicMax(popmax, pop);
   }
   if (fold_cnt && last_block_of_grid(fold_cnt)) {
     block_exclusive_scan<int32_t>(count, cellstart, g.ncell);
@@ -629,7 +631,7 @@ void CellCore::sort_done() {
   std::swap(orig.bytes, orig_b.bytes);
   sorted = true;
   built = false;
-  up_valid = false;
+  up_valid = up_scanned = false;
 }
 
 int CellCore::read_popmax() {
@@ -1152,8 +1154,9 @@ int CellCore::ensure_pf() {
   for (int d = 0; d < D; ++d)
     if ((rc = pf[d].ensure(sizeof(float) * N, st))) return rc;
   if ((rc = pfthr.ensure(sizeof(float2), st))) return rc;
-  if ((rc = pfcnt.ensure(sizeof(unsigned), st, true))) return rc;
-  return pfmax.ensure(sizeof(unsigned long long), st, true);
+  // zeroed once: the pass that accumulates them leaves both at zero
+  if (!pfcnt.p && (rc = pfcnt.ensure(sizeof(unsigned), st, true))) return rc;
+  return pfmax.p ? GCSPH_OK : pfmax.ensure(sizeof(unsigned long long), st, true);
 }
 
 int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, bool pf_ready, int4* pq,
@@ -1253,6 +1256,7 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
   timer_end(T_PAIRS, st);
   built = true;
   up_valid = false;
+  up_scanned = scan_up || fold;
   rows_upper = up;
   return GCSPH_OK;
 }
@@ -1274,12 +1278,15 @@ int CellCore::read_nfull() {
   return GCSPH_OK;
 }
 
-// offsets of each sorted particle's pairs in the (min,max) list: scanned on
-// demand, the stepping loop never needs them
+// offsets of each sorted particle's pairs in the (min,max) list: scanned with
+// the build where it needed them itself, else on demand
 int CellCore::ensure_up() {
   if (up_valid) return GCSPH_OK;
-  int rc = exclusive_scan_i32_to_i64(cnt_up.as<int32_t>(), rs_up.as<int64_t>(), N, scratch.as<int64_t>(), st);
-  if (rc) return rc;
+  int rc;
+  if (!up_scanned &&
+      (rc = exclusive_scan_i32_to_i64(cnt_up.as<int32_t>(), rs_up.as<int64_t>(), N, scratch.as<int64_t>(), st)))
+    return rc;
+  up_scanned = true;
   GC_CUDA(cudaMemcpyAsync(pin + 1, rs_up.as<int64_t>() + N, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   GC_CUDA(cudaStreamSynchronize(st));
   nup = pin[1];

@@ -96,7 +96,8 @@ __device__ inline void pf_thresholds_from(unsigned long long bits, double dist2,
 
 // The pass that accumulates the bound (max |x - offset|, atomically, per
 // warp) ends with this, every thread of every block: the last block to
-// finish turns the bound into the two thresholds and resets the counter.
+// finish turns the bound into the two thresholds and resets the bound and the
+// counter (both zero at rest: no memset before a build).
 template <int D>
 __device__ inline void pf_thresholds_last_block(unsigned long long* bmax, double dist2, float2* thr, unsigned* cnt) {
   __shared__ int s_last;
@@ -109,7 +110,7 @@ __device__ inline void pf_thresholds_last_block(unsigned long long* bmax, double
   if (s_last && threadIdx.x == 0) {
     __threadfence();
     float lo, hi;
-    pf_thresholds_from<D>(atomicAdd(bmax, 0ull), dist2, &lo, &hi);
+    pf_thresholds_from<D>(atomicExch(bmax, 0ull), dist2, &lo, &hi);
     *thr = make_float2(lo, hi);
     *cnt = 0u;
   }
@@ -156,6 +157,7 @@ struct CellCore {
   int64_t nfull_est = 0;  // last neighbour-entry count read back (lane choice); nfull is -1 while unknown
   int64_t gen = 0;        // bumped whenever a buffer a captured step graph points into is reallocated
   bool sorted = false, built = false, up_valid = false;
+  bool up_scanned = false;  // rs_up holds the last build's offsets (nup may still be unread)
   bool rows_upper = false;  // the last build stored the larger-index part of each row only
   int lanes = 0;  // lanes per particle in the pair search; 0 = by mean candidate count
   int sort_mode = 0;    // in-cell order: 0 by the population, 1 counting sort's rank, 2 radix sort

@@ -158,10 +158,14 @@ __host__ __device__ inline double eos(double rho, int gamma, double rho0, double
   return P0 * (ipow(rho / rho0, gamma) - 1.0);
 }
 
-// positive doubles order like their bit patterns: atomicMax on the bits
+// positive doubles order like their bit patterns: atomicMax on the bits.  The
+// word only grows while it is accumulated, so a value not above what a plain
+// read sees cannot raise it: after the first few warps hardly any atomic is
+// left on the word (one per warp on one word took 0.1 ms at 4M points).
 __device__ inline void atomic_max_pos(unsigned long long* addr, double v) {
   if (!(v > 0.0)) return;
-  atomicMax(addr, (unsigned long long)__double_as_longlong(v));
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  if (b > *(volatile unsigned long long*)addr) atomicMax(addr, b);
 }
 
 // Warp/block max of a non-negative double, one atomic per block
@@ -175,13 +179,14 @@ __device__ inline double warp_max(double v) {
 // ----------------------------------------------------------------------------
 // out[i] = sum_{j<i} in[j] for i in [0, n]; out[n] = total.  scratch must
 // hold scan_scratch_elems(n + 1) int64 values.  Arrays of up to
-// SCAN_SINGLE_MAX items take one single-block launch; longer ones are
-// scanned in tiles of SCAN_TILE items, with the tile totals scanned
-// recursively in the scratch.
+// SCAN_SINGLE_MAX items take one single-block launch (8 us for 6.5k items, 23
+// for 26k, 52 for 65k: one block walks them); longer ones are scanned in tiles
+// of SCAN_TILE items, with the tile totals scanned recursively in the scratch
+// (three launches, 11 us at 65k).
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int64_t SCAN_TILE = (int64_t)SCAN_THREADS * SCAN_ITEMS;
-constexpr int64_t SCAN_SINGLE_MAX = 65536;
+constexpr int64_t SCAN_SINGLE_MAX = 16384;
 constexpr int64_t scan_scratch_elems(int64_t m) {
   return (m + SCAN_TILE - 1) / SCAN_TILE <= 1
              ? 1

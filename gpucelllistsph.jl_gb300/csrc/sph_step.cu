@@ -594,7 +594,7 @@ struct HostSide {
   void* pt[2];
   void* buf2[3][2];
   void* orig[2];
-  bool sorted, built, up_valid, in_cell_order, rows_upper;
+  bool sorted, built, up_valid, up_scanned, in_cell_order, rows_upper;
   int64_t nfull;
 };
 
@@ -1229,6 +1229,7 @@ static HostSide host_side(const sph_handle* h) {
   s.sorted = core.sorted;
   s.built = core.built;
   s.up_valid = core.up_valid;
+  s.up_scanned = core.up_scanned;
   s.rows_upper = core.rows_upper;
   s.in_cell_order = h->in_cell_order;
   s.nfull = core.nfull;
@@ -1255,6 +1256,7 @@ static void set_host_side(sph_handle* h, const HostSide& s) {
   core.sorted = s.sorted;
   core.built = s.built;
   core.up_valid = s.up_valid;
+  core.up_scanned = s.up_scanned;
   core.rows_upper = s.rows_upper;
   h->in_cell_order = s.in_cell_order;
   core.nfull = s.nfull;
@@ -1279,7 +1281,7 @@ static GraphKey graph_key(const sph_handle* h, int32_t n, int timestepping, doub
   k.at = host_side(h);
   // flags and counts the capture does not depend on (it always starts by
   // binning the caller's points) stay out of the key
-  k.at.sorted = k.at.built = k.at.up_valid = k.at.in_cell_order = k.at.rows_upper = false;
+  k.at.sorted = k.at.built = k.at.up_valid = k.at.up_scanned = k.at.in_cell_order = k.at.rows_upper = false;
   k.at.nfull = 0;
   for (int d = 0; d < 3; ++d) {
     k.user[d] = h->cl->xuser[d];
