@@ -80,7 +80,7 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
 #pragma unroll
     for (int d = 0; d < D; ++d) dx[d] = S.x[d][k] - S.x[d][m];
     const double r2 = dotD<D>(dx, dx);
-    if (!(dbits(r2) > dbits(c.fb_r2cut))) fb_pair<D>(c, dx, r2, dbits(r2) != 0 ? sqrt_nr(r2) : 0.0, f);
+    if (!(dbits(r2) > dbits(c.fb_r2cut))) fb_pair<D>(c, dx, r2, dbits(r2) != 0 ? sqrt_nr2(r2) : 0.0, f);
   } else {
     const double* const* XP = STAGE == 1 ? S.x : S.xh;
     const double* const* VP = STAGE == 1 ? S.v : S.vh;

@@ -327,6 +327,20 @@ __device__ inline double sqrt_nr(double x) {
   return fma(s, e * fma(0.375, e, 0.5), s);
 }
 
+// sqrt(x) as above by two Newton steps on the reciprocal root, y <- y + y (1/2 -
+// (x/2) y^2), then x y.  fbmolforce! takes it: lattice walls hold pairs at
+// exactly r₀, where the last bit of r decides whether the pair has a force.
+__device__ inline double sqrt_nr2(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double hx = 0.5 * x;
+  double e = fma(-hx, y * y, 0.5);
+  y = fma(y, e, y);
+  e = fma(-hx, y * y, 0.5);
+  y = fma(y, e, y);
+  return x * y;
+}
+
 // cos(t) for 0 <= t < 3π/2 (∂v∂tpF! inside 2h): reduction by the nearest
 // multiple of π/2 (head and tail in FMAs), then one Taylor series, cosine's or
 // sine's by the quadrant's parity -- the coefficients are selected on the
