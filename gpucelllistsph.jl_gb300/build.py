@@ -22,6 +22,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 UNITS = {
     "common.cu": [],
     "celllist.cu": ["-fmad=false"],
+    "celllist_upper.cu": ["-fmad=false"],
     "sph_step.cu": ["-fmad=false"],
     "sph_once.cu": [],
     "sph_pairs.cu": ["-fmad=false"],

@@ -141,6 +141,25 @@ __global__ void k_scatter_arrival(const int32_t* __restrict__ key, const int32_t
   if (tord) tord[pos] = ord ? ord[i] : (int32_t)i;
 }
 
+// the arrival lists as records (the input order is the original order)
+template <int D>
+__global__ void __launch_bounds__(TPB) k_scatter_records(const double* __restrict__ x0, const double* __restrict__ x1,
+                                                         const double* __restrict__ x2,
+                                                         const int32_t* __restrict__ key,
+                                                         const int32_t* __restrict__ slot,
+                                                         const int32_t* __restrict__ cellstart, int64_t N,
+                                                         PointRec* __restrict__ rec) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const int32_t c = key[i];
+  const double a = x0[i], b = x1[i], z = D == 3 ? x2[i] : 0.0;
+  const long long ik = (long long)(unsigned)(int32_t)i | ((long long)c << 32);  // i, key
+  PointRec* p = rec + cellstart[c] + slot[i];
+  asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(__double_as_longlong(a)),
+               "l"(__double_as_longlong(b)), "l"(__double_as_longlong(z)), "l"(ik)
+               : "memory");
+}
+
 // rank of each cell member by original index: stable, history-free order.
 // Cost is sum over cells of n_c^2 integer compares (the reference's own pair
 // search is quadratic per cell too).
@@ -280,18 +299,6 @@ __global__ void k_gather_pos(const int32_t* __restrict__ idx, int64_t N, const d
 // ---------------------------------------------------------------------------
 // pair search over the 3^D stencil, as 3^(D-1) contiguous x-rows
 // ---------------------------------------------------------------------------
-template <int D>
-__device__ inline double r2_ref(double ax, double ay, double az, double bx, double by, double bz) {
-  double d0 = ax - bx;
-  double d1 = ay - by;
-  double s = d0 * d0 + d1 * d1;
-  if (D == 3) {
-    double d2 = az - bz;
-    s = s + d2 * d2;
-  }
-  return s;
-}
-
 // MODE 0: count (full, up); MODE 1: fill nbr.  L lanes share one particle:
 // the candidates of each x-row are tested L at a time, and the fill keeps the
 // row ascending by compacting each round's hits with a sub-warp ballot.
@@ -482,6 +489,8 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
     if (ncell > 0x7ffffff0LL) return fail(GCSPH_EINVAL, "cell grid too large (%lld cells)", (long long)ncell);
   }
   for (int d = D; d < 3; ++d) { g.offset[d] = 0; g.hinv[d] = 0; g.nc[d] = 1; }
+  g.fx.set(g.nc[0]);
+  g.fy.set(g.nc[1]);
   g.D = D;
   g.ncell = ncell;
   g.dist2 = dist * dist;
@@ -517,6 +526,7 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
     if ((rc = rhist.ensure(sizeof(int32_t) * 256 * ntiles, st))) return rc;
     if ((rc = rhoff.ensure(sizeof(int32_t) * (256 * ntiles + 1), st))) return rc;
     if ((rc = popmax.ensure(sizeof(int), st, true))) return rc;
+    GC_CUDA(cudaEventCreateWithFlags(&ev_pop, cudaEventDisableTiming));
     if (scan_scratch_elems(256 * ntiles + 1) > sc) return fail(GCSPH_EINVAL, "radix scan scratch");
   }
   return GCSPH_OK;
@@ -525,14 +535,17 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
 void CellCore::release() {
   DevBuf* all[] = {&count, &cellstart, &key, &slot, &tmp, &tord, &perm, &skey, &orig, &cnt_full, &cnt_up, &rs_full,
                    &rs_up, &nbr, &scratch, &pf[0], &pf[1], &pf[2], &pfmax, &pfthr, &pfcnt, &orig_b, &stage,
-                   &foldcnt, &foldsum, &rkey[0], &rkey[1], &rval[0], &rval[1], &rhist, &rhoff, &popmax};
+                   &foldcnt, &foldsum, &rkey[0], &rkey[1], &rval[0], &rval[1], &rhist, &rhoff, &popmax,
+                   &upf, &upmask, &uptot, &upbase, &upstat, &uprec};
   for (DevBuf* b : all) b->release();
+  if (ev_pop) cudaEventDestroy(ev_pop);
+  ev_pop = nullptr;
   if (pin) cudaFreeHost(pin);
   pin = nullptr;
 }
 
 int CellCore::sort(const double* const* xin, const int32_t* ord, bool may_sync, bool* rank_deferred,
-                   bool keys_ready) {
+                   bool keys_ready, PointRec* rec) {
   timer_begin(T_SORT, st);
   if (rank_deferred) *rank_deferred = false;
   if (keys_ready && !keys_in_step())
@@ -560,7 +573,30 @@ int CellCore::sort(const double* const* xin, const int32_t* ord, bool may_sync, 
     if (rc) return rc;
     GC_CUDA(cudaMemsetAsync(count.p, 0, sizeof(int32_t) * g.ncell, st));
   }
-  if (pm && may_sync && sort_mode == 0 && (rc = read_popmax())) return rc;
+  // small sets: 64-thread blocks, so these latency-bound passes spread over more SMs
+  const int tb = N <= RADIX_MIN_N ? 64 : TPB;
+  bool lists = false;  // the arrival lists are made
+  auto arrival = [&]() {
+    if (rec && D == 2)
+      k_scatter_records<2><<<nblocks(N, tb), tb, 0, st>>>(xin[0], xin[1], x2, key.as<int32_t>(), slot.as<int32_t>(),
+                                                          cellstart.as<int32_t>(), N, rec);
+    else if (rec)
+      k_scatter_records<3><<<nblocks(N, tb), tb, 0, st>>>(xin[0], xin[1], x2, key.as<int32_t>(), slot.as<int32_t>(),
+                                                          cellstart.as<int32_t>(), N, rec);
+    else
+      k_scatter_arrival<<<nblocks(N, tb), tb, 0, st>>>(key.as<int32_t>(), slot.as<int32_t>(), cellstart.as<int32_t>(),
+                                                      N, tmp.as<int32_t>(), ord, tord.as<int32_t>());
+    GC_LAUNCHED();
+    lists = true;
+    return (int)GCSPH_OK;
+  };
+  if (pm && may_sync && sort_mode == 0) {
+    GC_CUDA(cudaMemcpyAsync(pin + 7, pm, sizeof(int), cudaMemcpyDeviceToHost, st));
+    GC_CUDA(cudaEventRecord(ev_pop, st));
+    if ((rc = arrival())) return rc;
+    GC_CUDA(cudaEventSynchronize(ev_pop));
+    take_popmax();
+  }
   // the in-cell order: the counting sort's rank costs the square of a cell's
   // population per cell, the radix sort a fixed few passes over the set
   const bool radix = N > RADIX_MIN_N && (sort_mode == 2 || (sort_mode == 0 && last_popmax > RADIX_MIN_POP));
@@ -605,11 +641,7 @@ int CellCore::sort(const double* const* xin, const int32_t* ord, bool may_sync, 
                                                    orig_b.as<int32_t>());
     GC_LAUNCHED();
   } else {
-    // small sets: 64-thread blocks, so these latency-bound passes spread over more SMs
-    const int tb = N <= RADIX_MIN_N ? 64 : TPB;
-    k_scatter_arrival<<<nblocks(N, tb), tb, 0, st>>>(key.as<int32_t>(), slot.as<int32_t>(), cellstart.as<int32_t>(),
-                                                      N, tmp.as<int32_t>(), ord, tord.as<int32_t>());
-    GC_LAUNCHED();
+    if (!lists && (rc = arrival())) return rc;
     if (rank_deferred) {
       // the caller ranks (rank_in_cell) and applies the order in its own pass
       *rank_deferred = true;
@@ -638,34 +670,16 @@ int CellCore::read_popmax() {
   if (N <= RADIX_MIN_N || !popmax.p) return GCSPH_OK;
   GC_CUDA(cudaMemcpyAsync(pin + 7, popmax.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   GC_CUDA(cudaStreamSynchronize(st));
+  take_popmax();
+  return GCSPH_OK;
+}
+
+void CellCore::take_popmax() {
   const bool before = last_popmax > RADIX_MIN_POP;
   last_popmax = *(const int*)(pin + 7);
   // a captured step graph holds the ordering it was captured with: a change
   // of the choice retires the captured graphs
   if ((last_popmax > RADIX_MIN_POP) != before) ++gen;
-  return GCSPH_OK;
-}
-
-int CellCore::gather_positions(const double* const* xin, double* const* xs) {
-  const double* a2 = D == 3 ? xin[2] : xin[0];
-  double* b2 = D == 3 ? xs[2] : xs[0];
-  if (D == 2)
-    k_gather_pos<2><<<nblocks(N, TPB), TPB, 0, st>>>(perm.as<int32_t>(), N, xin[0], xin[1], a2, xs[0], xs[1], b2);
-  else
-    k_gather_pos<3><<<nblocks(N, TPB), TPB, 0, st>>>(perm.as<int32_t>(), N, xin[0], xin[1], a2, xs[0], xs[1], b2);
-  GC_LAUNCHED();
-  return GCSPH_OK;
-}
-
-int CellCore::gather_positions_by_orig(const double* const* xorig, double* const* xs) {
-  const double* a2 = D == 3 ? xorig[2] : xorig[0];
-  double* b2 = D == 3 ? xs[2] : xs[0];
-  if (D == 2)
-    k_gather_pos<2><<<nblocks(N, TPB), TPB, 0, st>>>(orig.as<int32_t>(), N, xorig[0], xorig[1], a2, xs[0], xs[1], b2);
-  else
-    k_gather_pos<3><<<nblocks(N, TPB), TPB, 0, st>>>(orig.as<int32_t>(), N, xorig[0], xorig[1], a2, xs[0], xs[1], b2);
-  GC_LAUNCHED();
-  return GCSPH_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -729,15 +743,11 @@ __device__ __forceinline__ void pairs32_row(const double* __restrict__ x0, const
                                                  int32_t* __restrict__ cnt_full, int32_t* __restrict__ cnt_up,
                                                  const int64_t* __restrict__ rs_full, int32_t* __restrict__ nbr,
                                                  int64_t cap, int* __restrict__ ovf, int32_t* __restrict__ stg,
-                                                 int S, const int32_t* fold_buf, bool up) {
+                                                 int S, const int32_t* fold_buf) {
   // MODE 0: count; MODE 2: count and stage the row (ascending) in stg[k*S ..]
   // when it fits; MODE 1: fill the CSR row -- a copy of the staged row when
   // the count pass staged it, else the search again.  MODE 1 reads the row
   // starts from the count pass's fold buffer where it folded (FoldRows).
-  // up: the half stencil, candidates m > k only (the cell list's own
-  // (min, max) list): the rows whose cells all come before k's in key order
-  // are skipped and k's own row starts at k + 1, so a row holds exactly the
-  // larger-index part of the full row, in the same order
   const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t k = gt / L;
   const int lane = (int)(gt % L);
@@ -835,11 +845,10 @@ __device__ __forceinline__ void pairs32_row(const double* __restrict__ x0, const
       for (int r = 0; r < NR; ++r) {
         const int z = cz + (r / 3 - 1), y = cy + (r % 3 - 1);
         int32_t m0 = 0, m1 = 0;
-        if (z >= 0 && z < nz && y >= 0 && y < ny && !(up && r < NR / 2)) {
+        if (z >= 0 && z < nz && y >= 0 && y < ny) {
           const int64_t base = (int64_t)nx * ((int64_t)y + (int64_t)ny * z);
           m0 = cellstart[base + xlo];
           m1 = cellstart[base + xhi + 1];
-          if (up && r == NR / 2) m0 = (int32_t)(k + 1);  // k's own row: k lies in it
         }
         rows[r] = tot;
         rows[NR + 1 + r] = m0 - tot;
@@ -869,11 +878,10 @@ __device__ __forceinline__ void pairs32_row(const double* __restrict__ x0, const
     for (int r = 0; r < 3; ++r) {
       const int dy = r - 1, y = cy + dy;
       rm0[r] = rm1[r] = 0;
-      if (!(up && dy < 0) && y >= 0 && y < ny) {
+      if (y >= 0 && y < ny) {
         const int64_t base = (int64_t)nx * (int64_t)y;
         rm0[r] = cellstart[base + xlo];
         rm1[r] = cellstart[base + xhi + 1];
-        if (up && dy == 0) rm0[r] = (int32_t)(k + 1);  // k's own row: k lies in it
       }
     }
 #pragma unroll
@@ -1052,7 +1060,7 @@ __global__ void __launch_bounds__(TPB) k_pairs32(const double* __restrict__ x0, 
                                                  int64_t cap, int* __restrict__ ovf, int32_t* __restrict__ stg,
                                                  int S, int64_t* fold_rs_full, int64_t* fold_rs_up,
                                                  unsigned* fold_cnt, const int64_t* __restrict__ rs_up,
-                                                 int4* __restrict__ pq, int32_t* fold_buf, bool up) {
+                                                 int4* __restrict__ pq, int32_t* fold_buf) {
   if ((MODE == 1 || MODE == 3) && fold_buf) {
     // small sets: the final row starts, from the count pass's two levels
     const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1064,7 +1072,7 @@ __global__ void __launch_bounds__(TPB) k_pairs32(const double* __restrict__ x0, 
   }
   pairs32_row<D, MODE == 3 ? 1 : (MODE == 4 ? 2 : MODE), L>(x0, x1, x2, f0, f1, f2, thr, skey, cellstart, N, g,
                                                              cnt_full, cnt_up, rs_full, nbr, cap, ovf, stg, S,
-                                                             fold_buf, up);
+                                                             fold_buf);
   if (MODE == 4) rows_fold<L>(cnt_full, cnt_up, N, fold_rs_full, fold_rs_up, fold_buf, fold_cnt);
   if (MODE == 3) {
     __syncwarp();  // a recomputed row's entries, written by the group's lanes, are read back
@@ -1153,6 +1161,11 @@ int CellCore::ensure_pf() {
   int rc;
   for (int d = 0; d < D; ++d)
     if ((rc = pf[d].ensure(sizeof(float) * N, st))) return rc;
+  return ensure_pf_scalars();
+}
+
+int CellCore::ensure_pf_scalars() {
+  int rc;
   if ((rc = pfthr.ensure(sizeof(float2), st))) return rc;
   // zeroed once: the pass that accumulates them leaves both at zero
   if (!pfcnt.p && (rc = pfcnt.ensure(sizeof(unsigned), st, true))) return rc;
@@ -1160,14 +1173,8 @@ int CellCore::ensure_pf() {
 }
 
 int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, bool pf_ready, int4* pq,
-                          bool* pq_done, bool up) {
+                          bool* pq_done) {
   if (pq_done) *pq_done = false;
-  if (up) {
-    // the half stencil: every row is its larger-index part, so both counts
-    // and both row-start scans are the same; no pair list for the step
-    scan_up = true;
-    pq = nullptr;
-  }
   if (!sorted) return fail(GCSPH_ESTATE, "pair build before binning");
   const double* x2 = D == 3 ? xs[2] : xs[0];
   timer_begin(T_PAIRS, st);
@@ -1188,8 +1195,7 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
     GC_LAUNCHED();
   }
   // rows of up to S neighbours are staged by the count pass and copied by the fill
-  // nfull_est counts full rows (a half-stencil build records twice its count)
-  const double mean = N > 0 && nfull_est > 0 ? (up ? 0.5 : 1.0) * (double)nfull_est / (double)N : 0.0;
+  const double mean = N > 0 && nfull_est > 0 ? (double)nfull_est / (double)N : 0.0;
   int S = 16;
   while (S < 256 && (double)S < 1.5 * mean + 8.0) S <<= 1;
   int32_t* sp = nullptr;
@@ -1206,15 +1212,15 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
     PAIRS32_LAUNCH(4, L, xs[0], xs[1], x2, pf[0].as<float>(), pf[1].as<float>(), f2, thr, skey.as<int32_t>(),
                    cellstart.as<int32_t>(), N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(), nullptr, nullptr, 0,
                    nullptr, sp, S, rs_full.as<int64_t>(), rs_up.as<int64_t>(), fc, nullptr, nullptr,
-                   foldsum.as<int32_t>(), up);
+                   foldsum.as<int32_t>());
   else if (sp)
     PAIRS32_LAUNCH(2, L, xs[0], xs[1], x2, pf[0].as<float>(), pf[1].as<float>(), f2, thr, skey.as<int32_t>(),
                    cellstart.as<int32_t>(), N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(), nullptr, nullptr, 0,
-                   nullptr, sp, S, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, up);
+                   nullptr, sp, S, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
   else
     PAIRS32_LAUNCH(0, L, xs[0], xs[1], x2, pf[0].as<float>(), pf[1].as<float>(), f2, thr, skey.as<int32_t>(),
                    cellstart.as<int32_t>(), N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(), nullptr, nullptr, 0,
-                   nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, up);
+                   nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
   GC_LAUNCHED();
   int rc = GCSPH_OK;
   if (!fold)
@@ -1234,7 +1240,7 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
     GC_CUDA(cudaStreamSynchronize(st));
     timer_collect();
     nfull = pin[0];
-    nfull_est = up ? 2 * nfull : nfull;
+    nfull_est = nfull;
     if (nfull > nbr_cap && (rc = grow_nbr(nfull))) return rc;
   }
   timer_begin(T_PAIRS, st);
@@ -1245,19 +1251,19 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
     PAIRS32_LAUNCH(3, L, xs[0], xs[1], x2, pf[0].as<float>(), pf[1].as<float>(), f2, thr, skey.as<int32_t>(),
                    cellstart.as<int32_t>(), N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(),
                    rs_full.as<int64_t>(), nbr.as<int32_t>(), nbr_cap, ovf_dev, sp, S, frs_full, frs_up, nullptr,
-                   rs_up.as<int64_t>(), pq, fbuf, false);
+                   rs_up.as<int64_t>(), pq, fbuf);
     if (pq_done) *pq_done = true;
   } else {
     PAIRS32_LAUNCH(1, L, xs[0], xs[1], x2, pf[0].as<float>(), pf[1].as<float>(), f2, thr, skey.as<int32_t>(),
                    cellstart.as<int32_t>(), N, g, nullptr, nullptr, rs_full.as<int64_t>(), nbr.as<int32_t>(), nbr_cap,
-                   ovf_dev, sp, S, frs_full, frs_up, nullptr, nullptr, nullptr, fbuf, up);
+                   ovf_dev, sp, S, frs_full, frs_up, nullptr, nullptr, nullptr, fbuf);
   }
   GC_LAUNCHED();
   timer_end(T_PAIRS, st);
   built = true;
   up_valid = false;
   up_scanned = scan_up || fold;
-  rows_upper = up;
+  rows_upper = false;
   return GCSPH_OK;
 }
 
@@ -1274,7 +1280,7 @@ int CellCore::read_nfull() {
   GC_CUDA(cudaMemcpyAsync(pin, rs_full.as<int64_t>() + N, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   GC_CUDA(cudaStreamSynchronize(st));
   nfull = pin[0];
-  nfull_est = rows_upper ? 2 * nfull : nfull;
+  nfull_est = nfull;
   return GCSPH_OK;
 }
 
@@ -1302,7 +1308,9 @@ int CellCore::emit(int32_t* pairs, int64_t cap, int fillzero, int64_t* pairsn) {
   if (pairsn) *pairsn = nup;
   if (cap > 0 && !pairs) return fail(GCSPH_EINVAL, "null pair buffer");
   if (cap > 0) {
-    if (((uintptr_t)pairs & 7u) == 0) {
+    if (rows_upper) {
+      if ((rc0 = emit_upper(pairs, cap))) return rc0;
+    } else if (((uintptr_t)pairs & 7u) == 0) {
       // lanes per point: about four pairs each, from the mean upper row
       const double mean = N > 0 ? (double)nup / (double)N : 0.0;
       int L = 1;
@@ -1325,7 +1333,7 @@ int CellCore::emit(int32_t* pairs, int64_t cap, int fillzero, int64_t* pairsn) {
       k_emit_pairs<<<nblocks(N, TPB), TPB, 0, st>>>(rs_full.as<int64_t>(), rs_up.as<int64_t>(), nbr.as<int32_t>(),
                                                      orig.as<int32_t>(), N, cap, pairs);
     }
-    GC_LAUNCHED();
+    if (!rows_upper) GC_LAUNCHED();
     if (fillzero && nup < cap)
       GC_CUDA(cudaMemsetAsync(pairs + 2 * nup, 0, sizeof(int32_t) * 2 * (size_t)(cap - nup), st));
   }
@@ -1352,14 +1360,11 @@ int CellCore::maxpairs(int64_t* out) {
 // ---------------------------------------------------------------------------
 using namespace gcsph;
 
-// update! and partialupdate! return the pairs k < m only: their builds take
-// the half stencil
-static int gcl_full_update(gcl_handle* h) {
-  int rc = h->core.sort(h->xuser, nullptr, true);
-  if (rc) return rc;
+// update! and partialupdate! return the pairs k < m only: their builds search
+// the half stencil (celllist_upper.cu)
+static int gcl_build(gcl_handle* h, bool rebin) {
   double* xs[3] = {h->xs[0].as<double>(), h->xs[1].as<double>(), h->core.D == 3 ? h->xs[2].as<double>() : nullptr};
-  if ((rc = h->core.gather_positions(h->xuser, xs))) return rc;
-  return h->core.build_pairs((const double* const*)xs, nullptr, false, false, nullptr, nullptr, true);
+  return h->core.build_upper(h->xuser, xs, rebin);
 }
 
 extern "C" {
@@ -1376,7 +1381,7 @@ int gcl_create(int32_t D, int64_t N, const double* const* x_dev, const double* c
   int rc = h->core.init(D, N, cellsize, dist, MIN_or_null, MAX_or_null, x_dev, (cudaStream_t)stream);
   if (!rc)
     for (int d = 0; d < D && !rc; ++d) rc = h->xs[d].ensure(sizeof(double) * N, h->core.st);
-  if (!rc) rc = gcl_full_update(h);
+  if (!rc) rc = gcl_build(h, true);
   if (rc) {
     std::string keep = gcsph_last_error();
     h->core.release();
@@ -1409,24 +1414,18 @@ int gcl_grid(const gcl_handle* h, double* cs, double* offset, int64_t* cell) {
 
 int gcl_update(gcl_handle* h, int64_t* pairsn_out) {
   if (!h) return fail(GCSPH_EINVAL, "null handle");
-  int rc = gcl_full_update(h);
+  int rc = gcl_build(h, true);
   if (rc) return rc;
-  if ((rc = h->core.ensure_up())) return rc;
   if (pairsn_out) *pairsn_out = h->core.nup;
-  GC_CUDA(cudaStreamSynchronize(h->core.st));
   return GCSPH_OK;
 }
 
 int gcl_partialupdate(gcl_handle* h, int64_t* pairsn_out) {
   if (!h) return fail(GCSPH_EINVAL, "null handle");
   if (!h->core.sorted) return fail(GCSPH_ESTATE, "partialupdate before any update");
-  double* xs[3] = {h->xs[0].as<double>(), h->xs[1].as<double>(), h->core.D == 3 ? h->xs[2].as<double>() : nullptr};
-  int rc = h->core.gather_positions_by_orig(h->xuser, xs);
+  int rc = gcl_build(h, false);
   if (rc) return rc;
-  if ((rc = h->core.build_pairs((const double* const*)xs, nullptr, false, false, nullptr, nullptr, true))) return rc;
-  if ((rc = h->core.ensure_up())) return rc;
   if (pairsn_out) *pairsn_out = h->core.nup;
-  GC_CUDA(cudaStreamSynchronize(h->core.st));
   return GCSPH_OK;
 }
 

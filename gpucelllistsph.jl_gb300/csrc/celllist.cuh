@@ -18,6 +18,22 @@
 
 namespace gcsph {
 
+// n / d for 0 <= n < 2^31 by one multiplication: m = ceil(2^(31+s) / d) with
+// 2^(s-1) < d <= 2^s (Granlund and Montgomery's division by an invariant)
+struct FastDiv {
+  unsigned m;
+  int s, d;
+  void set(int div) {
+    d = div;
+    s = 0;
+    while ((1LL << s) < div) ++s;
+    m = (unsigned)((((unsigned long long)1 << (31 + s)) + (unsigned)div - 1) / (unsigned)div);
+  }
+  __device__ __forceinline__ int quot(int n) const {
+    return (int)(((unsigned long long)(unsigned)n * m) >> (31 + s));
+  }
+};
+
 struct Grid {
   int D;
   double offset[3];
@@ -25,22 +41,25 @@ struct Grid {
   int nc[3];
   int64_t ncell;
   double dist2;
+  FastDiv fx, fy;  // by nc[0] and nc[1]
 };
 
 // the cell of point i (0-based linear key, x fastest): kernel_cellmap!'s
-// clamped ceil((x - offset) / cellsize), src/gpukernels_cls.jl:28-60
+// ceil of the clamped (x - offset) / cellsize, src/gpukernels_cls.jl:28-60.  The
+// ceil is taken first and the clamp in integers, which gives the same cell
+// (the conversion saturates; NaN converts below 1, where the reference's clamp
+// puts it): compares, the ceil and two conversions in FP64 kept the FP64 pipe
+// 85% busy over 4M points.
 template <int D>
 __device__ inline int32_t cell_key_v(const double* xv, const Grid& g) {
-  int64_t lin = 0, stride = 1;
+  int lin = 0, stride = 1;  // fewer than 2^31 cells
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     const double p = (xv[d] - g.offset[d]) * g.hinv[d];
-    const double c = fmin(fmax(p, 1.0), (double)g.nc[d]);
-    const int ci = (int)ceil(c);
-    lin += (int64_t)(ci - 1) * stride;
+    lin += (min(max(__double2int_ru(p), 1), g.nc[d]) - 1) * stride;
     stride *= g.nc[d];
   }
-  return (int32_t)lin;
+  return lin;
 }
 template <int D>
 __device__ inline int32_t cell_key(const double* x0, const double* x1, const double* x2, int64_t i, const Grid& g) {
@@ -116,6 +135,37 @@ __device__ inline void pf_thresholds_last_block(unsigned long long* bmax, double
   }
 }
 
+// the reference's squared distance, left to right and without contraction
+// (the units that test pairs are compiled with -fmad=false)
+template <int D>
+__device__ inline double r2_ref(double ax, double ay, double az, double bx, double by, double bz) {
+  double d0 = ax - bx;
+  double d1 = ay - by;
+  double s = d0 * d0 + d1 * d1;
+  if (D == 3) {
+    double d2 = az - bz;
+    s = s + d2 * d2;
+  }
+  return s;
+}
+
+// a point of the arrival lists with its position: one full sector, so the
+// list's random writes are whole sectors and the pass that ranks the points
+// reads them in order (indices alone made it gather every coordinate and the
+// key, a sector each: 1.0 GB for 4M points in 3-D against 0.34)
+struct __align__(32) PointRec {
+  double x[3];  // 2-D: x[2] unused
+  int32_t i, key;
+};
+
+// candidate statistics of a mask search (celllist_upper.cu)
+struct UpStat {
+  unsigned long long words;  // mask words of the points of every UP_SAMPLE-th block
+  int most;                  // the most words of a point
+  int pad;
+};
+constexpr int UP_SAMPLE = 16;
+
 // bounding box of D coordinate arrays (celllist.jl:41-43) with one launch
 // of nb blocks per dimension and one wait; a NaN coordinate is refused with
 // GCSPH_EINVAL.  part_dev and part_host hold 2 * D * nb doubles.
@@ -158,7 +208,14 @@ struct CellCore {
   int64_t gen = 0;        // bumped whenever a buffer a captured step graph points into is reallocated
   bool sorted = false, built = false, up_valid = false;
   bool up_scanned = false;  // rs_up holds the last build's offsets (nup may still be unread)
-  bool rows_upper = false;  // the last build stored the larger-index part of each row only
+  bool rows_upper = false;  // the last build is the list's own (pairs k < m alone, as masks)
+  // the mask search: FP32 vectors, words per point, block totals and starts, statistics
+  DevBuf upf, upmask, uptot, upbase, upstat, uprec;
+  double* up_xs[3] = {nullptr, nullptr, nullptr};  // the positions it was made on
+  int up_w = 0;          // words stored per point
+  int up_most = 0;       // the most words a point needed, last time
+  double up_mean = 0.0;  // and their mean
+  cudaEvent_t ev_pop = nullptr;  // the most crowded cell's read-back
   int lanes = 0;  // lanes per particle in the pair search; 0 = by mean candidate count
   int sort_mode = 0;    // in-cell order: 0 by the population, 1 counting sort's rank, 2 radix sort
   int last_popmax = 0;  // largest cell population seen (large sets; read where the host waits anyway)
@@ -174,25 +231,30 @@ struct CellCore {
   // bin xin (input order) into the frozen grid and sort by (cell, ord[i]);
   // ord == nullptr means the input order is the original order.
   // may_sync: the caller waits anyway, so the most crowded cell of this very
-  // binning is read back to pick the ordering (else the last one read)
+  // binning is read back to pick the ordering (else the last one read), while
+  // the arrival lists are made
   // rank_deferred (the counting sort's path only, where it is set true):
   // stop after the arrival lists; the caller ranks each point with
   // rank_in_cell in a pass of its own and then calls sort_done
   // keys_ready: the cell keys, arrival slots and cell starts of xin were
   // written by the step's last pass (small sets whose cell starts that pass
   // scans, see keys_in_step), so the binning starts at the arrival lists
+  // rec (with rank_deferred): the arrival lists are made as records of xin in
+  // rec instead of tmp / tord (PointRec)
   int sort(const double* const* xin, const int32_t* ord, bool may_sync = false, bool* rank_deferred = nullptr,
-           bool keys_ready = false);
+           bool keys_ready = false, PointRec* rec = nullptr);
   // whether the next binning's keys may come from the step's last pass: a
   // grid whose cell starts one block scans, and the counting sort's order
   bool keys_in_step() const { return g.ncell + 1 <= SCAN_FOLD_MAX && N <= RADIX_MIN_N && sort_mode != 2; }
   // the bookkeeping after a binning into perm / skey / orig_b (orig_b becomes orig)
   void sort_done();
   int read_popmax();
-  // gather xs[d][k] = xin[d][perm[k]] (and orig[k] = ord[perm[k]] is done by sort)
-  int gather_positions(const double* const* xin, double* const* xs);
-  // gather xs[d][k] = xorig[d][orig[k]] for partial updates
-  int gather_positions_by_orig(const double* const* xorig, double* const* xs);
+  void take_popmax();  // the value read back into pin[7]
+  // the list's own pair set, k < m, as masks (celllist_upper.cu): rebin bins
+  // xin first; otherwise the cells stay as they are and xin are moved points.
+  // xs takes the positions in cell order.  Waits for the pair count (nup).
+  int build_upper(const double* const* xin, double* const* xs, bool rebin);
+  int emit_upper(int32_t* pairs, int64_t cap);
   // count + scan + fill of the neighbour CSR on sorted positions xs.  With
   // ovf_dev (and buffers already sized once) the fill does not wait for the
   // count: rows past nbr_cap raise *ovf_dev instead (see grow_nbr).  scan_up
@@ -203,11 +265,10 @@ struct CellCore {
   // pair-once passes when the count pass staged the rows and the fill runs without a host
   // round trip (the capacity unchanged: pq must hold nbr_cap / 2 + 1 pairs); *pq_done says
   // whether it did
-  // up: the half stencil (only the m > k part of each row is searched and
-  // stored: rs_full == rs_up), for callers that need the pairs k < m alone
   int build_pairs(const double* const* xs, int* ovf_dev = nullptr, bool scan_up = false, bool pf_ready = false,
-                  int4* pq = nullptr, bool* pq_done = nullptr, bool up = false);
+                  int4* pq = nullptr, bool* pq_done = nullptr);
   int ensure_pf();
+  int ensure_pf_scalars();
   int grow_nbr(int64_t need);
   int read_nfull();
   int ensure_up();

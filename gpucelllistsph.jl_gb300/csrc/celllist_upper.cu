@@ -1,0 +1,532 @@
+// celllist_upper.cu -- the cell list's own pair list (update! / partialupdate!
+// and their emit): the pairs k < m alone, searched as bit masks.
+//
+// Each sorted point k has one sequence of candidates, m = k + 1 .. in its own
+// x-row and then the rows of the half stencil that follow in key order (1 more
+// row in 2-D, 4 more in 3-D).  The search keeps one bit per candidate, 32 to a
+// word, in candidate order; the emit expands the bits straight into the
+// caller's (min, max) list.  Ascending m is the order of the bits, so the list
+// is the one a search that writes neighbours in turn would give.
+//
+// Why masks and one thread per point: with a group of lanes per point, every
+// candidate paid for a ballot, two popcounts and a scattered store besides its
+// five floating-point instructions -- some 84 instructions per 32 candidates
+// and point, and the neighbour rows went through memory three times (staged,
+// copied into a CSR, read back by the emit).  A thread that walks its own
+// candidates needs about ten per candidate, the lanes of a warp are points of
+// the same or neighbouring cells, so that their loads fall on the same few
+// lines, and the masks are an eighth of a neighbour row's bytes or less.
+// Measured (one GB300, search alone): 200k uniform 2-D points (79 pairs a
+// point) 131 -> 45 us; 4M uniform 3-D points (4.3 a point) 685 -> 220 us.
+//
+// Compiled without FMA contraction: r2_ref is the reference's expression.
+#include "celllist.cuh"
+
+namespace gcsph {
+
+static constexpr int UTPB = 256;
+// pairs staged per block of the sparse emit (16 KB)
+static constexpr int EMIT_STAGE = 2048;
+
+// the FP32 prefilter copy, one vector per point
+template <int D> struct PfVec;
+template <> struct PfVec<2> { using T = float2; };
+template <> struct PfVec<3> { using T = float4; };
+template <int D>
+__device__ __forceinline__ typename PfVec<D>::T pf_make(const float* v) {
+  if constexpr (D == 2) return make_float2(v[0], v[1]);
+  else return make_float4(v[0], v[1], v[2], 0.f);
+}
+
+// one point's positions into cell order: FP64 copies, the FP32 prefilter
+// vector and its bound
+template <int D>
+__device__ __forceinline__ double place_point(const double* xv, const Grid& g, int64_t k, double* const* xs,
+                                              typename PfVec<D>::T* pf) {
+  double b = 0.0;
+  float f[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    xs[d][k] = xv[d];
+    const double v = xv[d] - g.offset[d];
+    f[d] = (float)v;
+    b = fmax(b, fabs(v));
+    if (v != v) b = INFINITY;  // NaN coordinate: every candidate of the set goes to FP64
+  }
+  pf[k] = pf_make<D>(f);
+  return b;
+}
+
+struct Pos3 {
+  const double* in[3];
+  double* out[3];
+};
+
+// the block's largest bound, one atomic per block, and the thresholds from
+// the last block
+template <int D>
+__device__ __forceinline__ void bound_block(double b, unsigned long long* bmax, double dist2, float2* thr,
+                                            unsigned* cnt) {
+  __shared__ double s_b[UTPB / 32];
+  b = warp_max(b);
+  if ((threadIdx.x & 31) == 0) s_b[threadIdx.x >> 5] = b;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < UTPB / 32; ++w) b = fmax(b, s_b[w]);
+    atomic_max_pos(bmax, b);
+  }
+  pf_thresholds_last_block<D>(bmax, dist2, thr, cnt);
+}
+
+// the rank of each point of the arrival lists among its cell's by original
+// index, and its place in cell order at once
+template <int D>
+__global__ void __launch_bounds__(UTPB) k_rank_place(const PointRec* __restrict__ rec,
+                                                     const int32_t* __restrict__ cellstart, int64_t N, Grid g,
+                                                     int32_t* __restrict__ perm, int32_t* __restrict__ skey,
+                                                     int32_t* __restrict__ orig, Pos3 P,
+                                                     typename PfVec<D>::T* __restrict__ pf, unsigned long long* bmax,
+                                                     float2* thr, unsigned* cnt) {
+  const int64_t q = (int64_t)blockIdx.x * UTPB + threadIdx.x;
+  double b = 0.0;
+  if (q < N) {
+    const PointRec p = rec[q];
+    const int32_t s = cellstart[p.key], e = cellstart[p.key + 1];
+    int32_t r = 0;
+#pragma unroll 4
+    for (int32_t t = s; t < e; ++t) r += rec[t].i < p.i;
+    const int64_t k = s + r;
+    perm[k] = p.i;
+    skey[k] = p.key;
+    orig[k] = p.i;
+    b = place_point<D>(p.x, g, k, P.out, pf);
+  }
+  bound_block<D>(b, bmax, g.dist2, thr, cnt);
+}
+
+// positions by a map (a radix-sorted binning, or stale cells with moved points)
+template <int D>
+__global__ void __launch_bounds__(UTPB) k_place(const int32_t* __restrict__ map, int64_t N, Grid g, Pos3 P,
+                                                typename PfVec<D>::T* __restrict__ pf, unsigned long long* bmax,
+                                                float2* thr, unsigned* cnt) {
+  const int64_t k = (int64_t)blockIdx.x * UTPB + threadIdx.x;
+  double b = 0.0;
+  if (k < N) {
+    const int32_t i = map[k];
+    double xv[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) xv[d] = P.in[d][i];
+    b = place_point<D>(xv, g, k, P.out, pf);
+  }
+  bound_block<D>(b, bmax, g.dist2, thr, cnt);
+}
+
+// The candidate rows of point k, in key order: its own row from k + 1 on,
+// then the stencil's later rows (empty outside the grid).  Row r holds the
+// candidates c[r - 1] <= t < c[r] of the sequence, candidate t is the point
+// t + dl[r].
+template <int D>
+struct UpRows {
+  static constexpr int R = D == 2 ? 2 : 5;
+  int32_t dl[R], c[R];
+  __device__ __forceinline__ int32_t total() const { return c[R - 1]; }
+  __device__ __forceinline__ int32_t at(int32_t t) const {
+    int32_t d = dl[0];
+#pragma unroll
+    for (int r = 1; r < R; ++r)
+      if (t >= c[r - 1]) d = dl[r];
+    return t + d;
+  }
+};
+
+template <int D>
+__device__ __forceinline__ UpRows<D> up_rows(int64_t k, int32_t key, const int32_t* __restrict__ cellstart,
+                                             const Grid& g) {
+  const int nx = g.nc[0], ny = g.nc[1], nz = D == 3 ? g.nc[2] : 1;
+  const int t = g.fx.quot(key);
+  const int cx = key - t * nx;
+  const int cz = D == 3 ? g.fy.quot(t) : 0;
+  const int cy = t - cz * ny;
+  const int xlo = cx > 0 ? cx - 1 : 0, xhi = cx < nx - 1 ? cx + 1 : nx - 1;
+  constexpr int R = UpRows<D>::R;
+  int32_t m0[R], m1[R];
+  m0[0] = (int32_t)k + 1;
+  m1[0] = cellstart[key - cx + xhi + 1];
+#pragma unroll
+  for (int r = 1; r < R; ++r) {
+    const int dy = r == 1 ? 1 : r - 3, dz = r == 1 ? 0 : 1;
+    const int y = cy + dy, z = cz + dz;
+    m0[r] = m1[r] = 0;
+    if (y >= 0 && y < ny && z < nz) {
+      const int base = nx * (y + ny * z);  // fewer than 2^31 cells
+      m0[r] = cellstart[base + xlo];
+      m1[r] = cellstart[base + xhi + 1];
+    }
+  }
+  UpRows<D> U;
+  int32_t c = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    U.dl[r] = m0[r] - c;
+    c += m1[r] - m0[r];
+    U.c[r] = c;
+  }
+  return U;
+}
+
+// the FP32 squared distance (any rounding of it lies inside the band)
+template <int D>
+__device__ __forceinline__ float r2_pf(const typename PfVec<D>::T& a, const typename PfVec<D>::T& b) {
+  const float d0 = a.x - b.x, d1 = a.y - b.y;
+  float r2 = fmaf(d1, d1, d0 * d0);
+  if constexpr (D == 3) {
+    const float d2 = a.z - b.z;
+    r2 = fmaf(d2, d2, r2);
+  }
+  return r2;
+}
+
+// the reference's FP64 test of a candidate inside the band
+template <int D>
+__device__ __forceinline__ bool hit_exact(int64_t k, int32_t m, double* const* xs, double dist2) {
+  return r2_ref<D>(xs[0][k], xs[1][k], D == 3 ? xs[2][k] : 0.0, xs[0][m], xs[1][m], D == 3 ? xs[2][m] : 0.0) < dist2;
+}
+
+// one thread walks all candidates of point k; put(w, word) gets each word of
+// its mask in turn.  The vectors past the last point that a group of four may
+// read are padding (their bits are cut off).
+template <int D, class F>
+__device__ __forceinline__ void up_walk(int64_t k, const UpRows<D>& U, const typename PfVec<D>::T* __restrict__ pf,
+                                        double* const* xs, float2 tt, double dist2, F put) {
+  const typename PfVec<D>::T a = pf[k];
+  unsigned long long acc = 0;
+  int fill = 0, w = 0;
+#pragma unroll
+  for (int r = 0; r < UpRows<D>::R; ++r) {
+    const int32_t m1 = U.c[r] + U.dl[r];
+    for (int32_t m = (r ? U.c[r ? r - 1 : 0] : 0) + U.dl[r]; m < m1; m += 32) {
+      const int n = min(32, m1 - m);
+      unsigned in = 0, ok = 0;  // surely in; not surely out
+      for (int j = 0; j < n; j += 4) {
+        unsigned i4 = 0, o4 = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float r2 = r2_pf<D>(a, pf[m + j + q]);
+          if (r2 < tt.x) i4 |= 1u << q;
+          if (!(r2 > tt.y)) o4 |= 1u << q;
+        }
+        in |= i4 << j;
+        ok |= o4 << j;
+      }
+      const unsigned cut = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+      in &= cut;
+      unsigned band = ok & cut & ~in;
+      while (band) {
+        const int b = __ffs(band) - 1;
+        band &= band - 1;
+        if (hit_exact<D>(k, m + b, xs, dist2)) in |= 1u << b;
+      }
+      acc |= (unsigned long long)in << fill;
+      fill += n;
+      if (fill >= 32) {
+        put(w++, (unsigned)acc);
+        acc >>= 32;
+        fill -= 32;
+      }
+    }
+  }
+  if (fill > 0) put(w, (unsigned)acc);
+}
+
+// Count pass: the mask words of each point (point-major, the first W of
+// them), its offset among the pairs of its block, the blocks' totals and the
+// candidate statistics; the last block of a grid of up to SCAN_FOLD_MAX blocks
+// scans the totals into the blocks' starts (base[gridDim.x] is the total).
+template <int D>
+__global__ void __launch_bounds__(UTPB) k_up_count(const typename PfVec<D>::T* __restrict__ pf, Pos3 P,
+                                                   const float2* __restrict__ thr, const int32_t* __restrict__ skey,
+                                                   const int32_t* __restrict__ cellstart, int64_t N, Grid g,
+                                                   unsigned* __restrict__ mask, int W, int32_t* __restrict__ loc,
+                                                   int32_t* __restrict__ total, int64_t* __restrict__ base,
+                                                   UpStat* stat, unsigned* fold_cnt) {
+  const int64_t k = (int64_t)blockIdx.x * UTPB + threadIdx.x;
+  int32_t cnt = 0, nw = 0;
+  if (k < N) {
+    const UpRows<D> U = up_rows<D>(k, skey[k], cellstart, g);
+    nw = (U.total() + 31) >> 5;
+    unsigned* mk = mask + k * W;
+    up_walk<D>(k, U, pf, P.out, *thr, g.dist2, [&](int w, unsigned word) {
+      cnt += __popc(word);
+      if (w < W) mk[w] = word;
+    });
+  }
+  // the block's exclusive scan of the counts; sum and maximum of the words
+  __shared__ int32_t s_c[UTPB / 32], s_s[UTPB / 32], s_m[UTPB / 32];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  int32_t inc = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  const int32_t ws = __reduce_add_sync(0xffffffffu, nw), wm = __reduce_max_sync(0xffffffffu, nw);
+  if (lane == 31) {
+    s_c[wp] = inc;
+    s_s[wp] = ws;
+    s_m[wp] = wm;
+  }
+  __syncthreads();
+  int32_t before = 0, all = 0, sum = 0, mx = 0;
+#pragma unroll
+  for (int v = 0; v < UTPB / 32; ++v) {
+    if (v < wp) before += s_c[v];
+    all += s_c[v];
+    sum += s_s[v];
+    mx = max(mx, s_m[v]);
+  }
+  if (k < N) loc[k] = before + inc - cnt;
+  if (threadIdx.x == 0) {
+    total[blockIdx.x] = all;
+    if (blockIdx.x % UP_SAMPLE == 0) atomicAdd(&stat->words, (unsigned long long)sum);
+    if (mx > *(volatile int*)&stat->most) atomicMax(&stat->most, mx);
+  }
+  if (fold_cnt && last_block_of_grid(fold_cnt)) block_exclusive_scan<int64_t>(total, base, gridDim.x);
+}
+
+// (min, max) 1-based original indices of a pair
+__device__ __forceinline__ int2 make_pair1(int32_t ok, int32_t om) {
+  return make_int2(ok < om ? ok : om, ok < om ? om : ok);
+}
+__device__ __forceinline__ void store_pair(int32_t* pairs, int64_t pos, int2 v, bool aligned) {
+  if (aligned) {
+    reinterpret_cast<int2*>(pairs)[pos] = v;
+  } else {
+    pairs[2 * pos] = v.x;
+    pairs[2 * pos + 1] = v.y;
+  }
+}
+
+// Emit, one warp per point: each lane takes one bit of a word, so a word's
+// pairs are one contiguous store.  The words past the stored W are searched
+// again, 32 candidates at a time.
+template <int D>
+__global__ void __launch_bounds__(UTPB) k_up_emit_warp(const typename PfVec<D>::T* __restrict__ pf, Pos3 P,
+                                                       const float2* __restrict__ thr,
+                                                       const int32_t* __restrict__ skey,
+                                                       const int32_t* __restrict__ cellstart,
+                                                       const int32_t* __restrict__ orig, int64_t N, Grid g,
+                                                       const unsigned* __restrict__ mask, int W,
+                                                       const int32_t* __restrict__ loc,
+                                                       const int64_t* __restrict__ base, int64_t cap,
+                                                       int32_t* __restrict__ pairs, bool aligned) {
+  const int64_t k = ((int64_t)blockIdx.x * UTPB + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (k >= N) return;
+  const UpRows<D> U = up_rows<D>(k, skey[k], cellstart, g);
+  const int32_t tot = U.total();
+  const int nw = (tot + 31) >> 5;
+  const int32_t ok = orig[k] + 1;
+  const int64_t pos = base[k / UTPB] + loc[k];
+  int32_t* out = pairs + 2 * pos;
+  const int lim = (int)max((int64_t)0, min(cap - pos, (int64_t)0x7fffffff));  // pairs of this point that fit
+  const unsigned bit = 1u << lane, lt = bit - 1u;
+  int off = 0;
+  const int stored = min(nw, W);
+  for (int w0 = 0; w0 < stored; w0 += 32) {
+    const unsigned mine = w0 + lane < stored ? mask[k * W + w0 + lane] : 0u;
+    const int n = min(32, stored - w0);
+#pragma unroll 4
+    for (int w = 0; w < n; ++w) {
+      const unsigned word = __shfl_sync(0xffffffffu, mine, w);
+      const int at = off + __popc(word & lt);
+      if ((word & bit) && at < lim)
+        store_pair(out, at, make_pair1(ok, orig[U.at((w0 + w) * 32 + lane)] + 1), aligned);
+      off += __popc(word);
+    }
+  }
+  for (int w = stored; w < nw; ++w) {
+    const int32_t t = w * 32 + lane;
+    const int32_t m = t < tot ? U.at(t) : (int32_t)k;
+    bool hit = false;
+    if (t < tot) {
+      const float r2 = r2_pf<D>(pf[k], pf[m]);
+      hit = r2 < thr->x || (!(r2 > thr->y) && hit_exact<D>(k, m, P.out, g.dist2));
+    }
+    const unsigned word = __ballot_sync(0xffffffffu, hit);
+    const int at = off + __popc(word & lt);
+    if (hit && at < lim) store_pair(out, at, make_pair1(ok, orig[m] + 1), aligned);
+    off += __popc(word);
+  }
+}
+
+// Emit, one thread per point, for lists of few pairs a point (a warp per
+// point would leave most lanes without a bit): a block's pairs are contiguous
+// in the list, so they are collected in shared memory and stored as one run.
+template <int D>
+__global__ void __launch_bounds__(UTPB) k_up_emit_thread(const typename PfVec<D>::T* __restrict__ pf, Pos3 P,
+                                                         const float2* __restrict__ thr,
+                                                         const int32_t* __restrict__ skey,
+                                                         const int32_t* __restrict__ cellstart,
+                                                         const int32_t* __restrict__ orig, int64_t N, Grid g,
+                                                         const unsigned* __restrict__ mask, int W,
+                                                         const int32_t* __restrict__ loc,
+                                                         const int32_t* __restrict__ total,
+                                                         const int64_t* __restrict__ base, int64_t cap,
+                                                         int32_t* __restrict__ pairs, bool aligned) {
+  __shared__ int2 s_p[EMIT_STAGE];
+  const int64_t k = (int64_t)blockIdx.x * UTPB + threadIdx.x;
+  const int64_t b0 = base[blockIdx.x];
+  const int32_t all = total[blockIdx.x];
+  const bool staged = all <= EMIT_STAGE;
+  if (k < N) {
+    const UpRows<D> U = up_rows<D>(k, skey[k], cellstart, g);
+    const int nw = (U.total() + 31) >> 5;
+    const int32_t ok = orig[k] + 1;
+    int32_t at = loc[k];
+    auto expand = [&](int w, unsigned word) {
+      while (word) {
+        const int b = __ffs(word) - 1;
+        word &= word - 1;
+        const int2 v = make_pair1(ok, orig[U.at(w * 32 + b)] + 1);
+        if (staged) s_p[at] = v;
+        else if (b0 + at < cap) store_pair(pairs, b0 + at, v, aligned);
+        ++at;
+      }
+    };
+    if (nw <= W) {
+      for (int w = 0; w < nw; ++w) expand(w, mask[k * W + w]);
+    } else {
+      up_walk<D>(k, U, pf, P.out, *thr, g.dist2, expand);
+    }
+  }
+  if (!staged) return;  // uniform over the block
+  __syncthreads();
+  for (int32_t i = threadIdx.x; i < all; i += UTPB)
+    if (b0 + i < cap) store_pair(pairs, b0 + i, s_p[i], aligned);
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+template <int D>
+static Pos3 pos3(const double* const* in, double* const* out) {
+  Pos3 P{};
+  for (int d = 0; d < D; ++d) {
+    P.in[d] = in ? in[d] : nullptr;
+    P.out[d] = out[d];
+  }
+  return P;
+}
+
+template <int D>
+static int build_upper_impl(CellCore& C, const double* const* xin, double* const* xs, bool rebin) {
+  using V = typename PfVec<D>::T;
+  cudaStream_t st = C.st;
+  const int64_t N = C.N;
+  const int nb = nblocks(N, UTPB);
+  int rc;
+  if ((rc = C.ensure_pf_scalars())) return rc;
+  // four vectors of padding, which a walk may read and cut off
+  if (!C.upf.p && (rc = C.upf.ensure(sizeof(V) * (N + 4), st, true))) return rc;
+  if ((rc = C.uptot.ensure(sizeof(int32_t) * ((size_t)nb + 4), st))) return rc;
+  if ((rc = C.upbase.ensure(sizeof(int64_t) * ((size_t)nb + 1), st))) return rc;
+  if ((rc = C.upstat.ensure(sizeof(UpStat), st))) return rc;
+  V* pf = C.upf.as<V>();
+  const Pos3 P = pos3<D>(xin, xs);
+  unsigned long long* bm = C.pfmax.as<unsigned long long>();
+  float2* thr = C.pfthr.as<float2>();
+  unsigned* cnt = C.pfcnt.as<unsigned>();
+  bool deferred = false;
+  if (rebin) {
+    if ((rc = C.uprec.ensure(sizeof(PointRec) * N, st))) return rc;
+    if ((rc = C.sort(xin, nullptr, true, &deferred, false, C.uprec.as<PointRec>()))) return rc;
+  }
+  if (!C.sorted && !deferred) return fail(GCSPH_ESTATE, "pair build before binning");
+  timer_begin(T_SORT, st);
+  if (deferred) {
+    k_rank_place<D><<<nb, UTPB, 0, st>>>(C.uprec.as<PointRec>(), C.cellstart.as<int32_t>(), N, C.g,
+                                         C.perm.as<int32_t>(), C.skey.as<int32_t>(), C.orig_b.as<int32_t>(), P, pf,
+                                         bm, thr, cnt);
+    GC_LAUNCHED();
+    C.sort_done();
+  } else {
+    // stale cells: the points are the caller's, by original index
+    k_place<D><<<nb, UTPB, 0, st>>>(rebin ? C.perm.as<int32_t>() : C.orig.as<int32_t>(), N, C.g, P, pf, bm, thr, cnt);
+    GC_LAUNCHED();
+  }
+  timer_end(T_SORT, st);
+  timer_begin(T_PAIRS, st);
+  // mask words a point: as many as the last search needed, up to three times
+  // its mean (a crowded cell's points search their last words again in the emit)
+  int W = 0;
+  if (C.up_most > 0) {
+    W = C.up_most;
+    if ((double)W > 3.0 * C.up_mean + 4.0) W = (int)(3.0 * C.up_mean + 4.0);
+    if ((rc = C.upmask.ensure(sizeof(unsigned) * (size_t)N * (size_t)W, st))) return rc;
+  }
+  C.up_w = W;
+  GC_CUDA(cudaMemsetAsync(C.upstat.p, 0, sizeof(UpStat), st));
+  const bool fold = nb <= SCAN_FOLD_MAX;
+  k_up_count<D><<<nb, UTPB, 0, st>>>(pf, P, thr, C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), N, C.g,
+                                     C.upmask.as<unsigned>(), W, C.cnt_up.as<int32_t>(), C.uptot.as<int32_t>(),
+                                     C.upbase.as<int64_t>(), C.upstat.as<UpStat>(),
+                                     fold ? C.foldcnt.as<unsigned>() + 1 : nullptr);
+  GC_LAUNCHED();
+  if (!fold && (rc = exclusive_scan_i32_to_i64(C.uptot.as<int32_t>(), C.upbase.as<int64_t>(), nb,
+                                               C.scratch.as<int64_t>(), st)))
+    return rc;
+  timer_end(T_PAIRS, st);
+  GC_CUDA(cudaMemcpyAsync(C.pin, C.upbase.as<int64_t>() + nb, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  GC_CUDA(cudaMemcpyAsync(C.pin + 2, C.upstat.p, sizeof(UpStat), cudaMemcpyDeviceToHost, st));
+  GC_CUDA(cudaStreamSynchronize(st));
+  timer_collect();
+  UpStat s;
+  memcpy(&s, C.pin + 2, sizeof(s));
+  int64_t sampled = (int64_t)((nb + UP_SAMPLE - 1) / UP_SAMPLE) * UTPB;
+  if (sampled > N) sampled = N;
+  C.up_mean = (double)s.words / (double)sampled;
+  C.up_most = s.most;
+  C.nup = C.pin[0];
+  C.nfull = C.nup;
+  C.nfull_est = 2 * C.nup;
+  C.built = true;
+  C.up_valid = true;
+  C.rows_upper = true;
+  return GCSPH_OK;
+}
+
+template <int D>
+static int emit_upper_impl(CellCore& C, double* const* xs, int32_t* pairs, int64_t cap) {
+  using V = typename PfVec<D>::T;
+  cudaStream_t st = C.st;
+  const int64_t N = C.N;
+  const Pos3 P = pos3<D>(nullptr, xs);
+  const bool aligned = ((uintptr_t)pairs & 7u) == 0;
+  // up to two words a point (about 64 candidates, some ten pairs) a thread per
+  // point; above, a warp per point
+  if (C.up_mean <= 2.0)
+    k_up_emit_thread<D><<<nblocks(N, UTPB), UTPB, 0, st>>>(
+        C.upf.as<V>(), P, C.pfthr.as<float2>(), C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), C.orig.as<int32_t>(),
+        N, C.g, C.upmask.as<unsigned>(), C.up_w, C.cnt_up.as<int32_t>(), C.uptot.as<int32_t>(),
+        C.upbase.as<int64_t>(), cap, pairs, aligned);
+  else
+    k_up_emit_warp<D><<<nblocks(N * 32, UTPB), UTPB, 0, st>>>(
+        C.upf.as<V>(), P, C.pfthr.as<float2>(), C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), C.orig.as<int32_t>(),
+        N, C.g, C.upmask.as<unsigned>(), C.up_w, C.cnt_up.as<int32_t>(), C.upbase.as<int64_t>(), cap, pairs, aligned);
+  GC_LAUNCHED();
+  return GCSPH_OK;
+}
+
+int CellCore::build_upper(const double* const* xin, double* const* xs, bool rebin) {
+  up_xs[0] = xs[0];
+  up_xs[1] = xs[1];
+  up_xs[2] = D == 3 ? xs[2] : nullptr;
+  return D == 2 ? build_upper_impl<2>(*this, xin, xs, rebin) : build_upper_impl<3>(*this, xin, xs, rebin);
+}
+
+int CellCore::emit_upper(int32_t* pairs, int64_t cap) {
+  return D == 2 ? emit_upper_impl<2>(*this, up_xs, pairs, cap) : emit_upper_impl<3>(*this, up_xs, pairs, cap);
+}
+
+}  // namespace gcsph
