@@ -536,7 +536,7 @@ void CellCore::release() {
   DevBuf* all[] = {&count, &cellstart, &key, &slot, &tmp, &tord, &perm, &skey, &orig, &cnt_full, &cnt_up, &rs_full,
                    &rs_up, &nbr, &scratch, &pf[0], &pf[1], &pf[2], &pfmax, &pfthr, &pfcnt, &orig_b, &stage,
                    &foldcnt, &foldsum, &rkey[0], &rkey[1], &rval[0], &rval[1], &rhist, &rhoff, &popmax,
-                   &upf, &upmask, &uptot, &upbase, &upstat, &uprec};
+                   &upf, &upkept, &uptot, &upbase, &upstat, &uprec};
   for (DevBuf* b : all) b->release();
   if (ev_pop) cudaEventDestroy(ev_pop);
   ev_pop = nullptr;
@@ -701,7 +701,7 @@ __global__ void k_make_pf(const double* __restrict__ x0, const double* __restric
                           float* __restrict__ f1, float* __restrict__ f2, unsigned long long* __restrict__ bmax,
                           float2* __restrict__ thr, unsigned* __restrict__ cnt) {
   int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double b = 0.0;
+  unsigned b = 0;  // a NaN coordinate bounds as infinity: every candidate of the set goes to FP64
   if (k < N) {
     const double* X[3] = {x0, x1, x2};
     float* F[3] = {f0, f1, f2};
@@ -709,12 +709,10 @@ __global__ void k_make_pf(const double* __restrict__ x0, const double* __restric
     for (int d = 0; d < D; ++d) {
       const double v = X[d][k] - g.offset[d];
       F[d][k] = (float)v;
-      b = fmax(b, fabs(v));
+      b = max(b, abs_hi(v));
     }
-    if (b != b) b = INFINITY;  // NaN coordinate: every candidate of the set goes to FP64
   }
-  b = warp_max(b);
-  if ((threadIdx.x & 31) == 0) atomic_max_pos(bmax, b);
+  atomic_max_hi(bmax, b);
   pf_thresholds_last_block<D>(bmax, g.dist2, thr, cnt);
 }
 

@@ -158,10 +158,10 @@ struct __align__(32) PointRec {
   int32_t i, key;
 };
 
-// candidate statistics of a mask search (celllist_upper.cu)
+// candidate statistics of such a search (celllist_upper.cu)
 struct UpStat {
-  unsigned long long words;  // mask words of the points of every UP_SAMPLE-th block
-  int most;                  // the most words of a point
+  unsigned long long words;  // words of candidates of the points of every UP_SAMPLE-th block
+  int most;                  // the most words or neighbours (what is kept) of a point
   int pad;
 };
 constexpr int UP_SAMPLE = 16;
@@ -208,13 +208,12 @@ struct CellCore {
   int64_t gen = 0;        // bumped whenever a buffer a captured step graph points into is reallocated
   bool sorted = false, built = false, up_valid = false;
   bool up_scanned = false;  // rs_up holds the last build's offsets (nup may still be unread)
-  bool rows_upper = false;  // the last build is the list's own (pairs k < m alone, as masks)
-  // the mask search: FP32 vectors, words per point, block totals and starts, statistics
-  DevBuf upf, upmask, uptot, upbase, upstat, uprec;
+  bool rows_upper = false;  // the last build is the list's own (pairs k < m alone, as masks or rows)
+  // their search: FP32 vectors, what each point keeps, block totals and starts, statistics
+  DevBuf upf, upkept, uptot, upbase, upstat, uprec;
   double* up_xs[3] = {nullptr, nullptr, nullptr};  // the positions it was made on
-  int up_w = 0;          // words stored per point
-  int up_most = 0;       // the most words a point needed, last time
-  double up_mean = 0.0;  // and their mean
+  int up_w = 0;          // entries kept per point
+  bool up_rows = false;  // neighbours rather than words
   cudaEvent_t ev_pop = nullptr;  // the most crowded cell's read-back
   int lanes = 0;  // lanes per particle in the pair search; 0 = by mean candidate count
   int sort_mode = 0;    // in-cell order: 0 by the population, 1 counting sort's rank, 2 radix sort
@@ -250,7 +249,7 @@ struct CellCore {
   void sort_done();
   int read_popmax();
   void take_popmax();  // the value read back into pin[7]
-  // the list's own pair set, k < m, as masks (celllist_upper.cu): rebin bins
+  // the list's own pair set, k < m, as masks or rows (celllist_upper.cu): rebin bins
   // xin first; otherwise the cells stay as they are and xin are moved points.
   // xs takes the positions in cell order.  Waits for the pair count (nup).
   int build_upper(const double* const* xin, double* const* xs, bool rebin);

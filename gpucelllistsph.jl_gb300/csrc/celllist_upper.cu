@@ -1,23 +1,26 @@
 // celllist_upper.cu -- the cell list's own pair list (update! / partialupdate!
-// and their emit): the pairs k < m alone, searched as bit masks.
+// and their emit): the pairs k < m alone, one thread per point.
 //
 // Each sorted point k has one sequence of candidates, m = k + 1 .. in its own
 // x-row and then the rows of the half stencil that follow in key order (1 more
-// row in 2-D, 4 more in 3-D).  The search keeps one bit per candidate, 32 to a
-// word, in candidate order; the emit expands the bits straight into the
-// caller's (min, max) list.  Ascending m is the order of the bits, so the list
-// is the one a search that writes neighbours in turn would give.
+// row in 2-D, 4 more in 3-D).  A thread walks its point's candidates 32 at a
+// time into a word of hit bits.  Sets of few candidates a point (UP_FEW words)
+// keep the words; denser ones keep the neighbours themselves, expanded from
+// each word as it is made.  The emit turns either into the caller's (min, max)
+// list.  Ascending m is the order of both, so the list is the one a search that
+// writes neighbours in turn would give.
 //
-// Why masks and one thread per point: with a group of lanes per point, every
-// candidate paid for a ballot, two popcounts and a scattered store besides its
-// five floating-point instructions -- some 84 instructions per 32 candidates
-// and point, and the neighbour rows went through memory three times (staged,
+// Why one thread per point: with a group of lanes per point, every candidate
+// paid for a ballot, two popcounts and a scattered store besides its five
+// floating-point instructions -- some 84 instructions per 32 candidates and
+// point -- and the neighbour rows went through memory three times (staged,
 // copied into a CSR, read back by the emit).  A thread that walks its own
-// candidates needs about ten per candidate, the lanes of a warp are points of
-// the same or neighbouring cells, so that their loads fall on the same few
-// lines, and the masks are an eighth of a neighbour row's bytes or less.
-// Measured (one GB300, search alone): 200k uniform 2-D points (79 pairs a
-// point) 131 -> 45 us; 4M uniform 3-D points (4.3 a point) 685 -> 220 us.
+// candidates needs about ten per candidate, and the lanes of a warp are points
+// of the same or neighbouring cells, so their loads fall on the same few
+// lines.  Measured (one GB300): search and emit of 200k uniform 2-D points (79
+// pairs a point) 131 + 61 + 67 -> 71 + 43 us; of 333k uniform 3-D points (43 a
+// point) 354 + 89 + 58 -> 108 + 49 us; of 4M uniform 3-D points (4.3 a point) 685 +
+// 125 + 86 -> 202 + 100 us.
 //
 // Compiled without FMA contraction: r2_ref is the reference's expression.
 #include "celllist.cuh"
@@ -25,7 +28,9 @@
 namespace gcsph {
 
 static constexpr int UTPB = 256;
-// pairs staged per block of the sparse emit (16 KB)
+// sets of up to this many words of candidates a point keep the words
+static constexpr double UP_FEW = 2.0;
+// pairs collected per block of their emit (16 KB)
 static constexpr int EMIT_STAGE = 2048;
 
 // the FP32 prefilter copy, one vector per point
@@ -38,20 +43,23 @@ __device__ __forceinline__ typename PfVec<D>::T pf_make(const float* v) {
   else return make_float4(v[0], v[1], v[2], 0.f);
 }
 
-// one point's positions into cell order: FP64 copies, the FP32 prefilter
-// vector and its bound
 template <int D>
-__device__ __forceinline__ double place_point(const double* xv, const Grid& g, int64_t k, double* const* xs,
+constexpr int UP_GROUP = D == 2 ? 8 : 4;  // candidates tested at a time, and the vectors' padding
+
+// one point's positions into cell order: FP64 copies, the FP32 prefilter
+// vector and its bound (abs_hi; a NaN coordinate sends every candidate of the
+// set to FP64)
+template <int D>
+__device__ __forceinline__ unsigned place_point(const double* xv, const Grid& g, int64_t k, double* const* xs,
                                               typename PfVec<D>::T* pf) {
-  double b = 0.0;
+  unsigned b = 0;
   float f[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     xs[d][k] = xv[d];
     const double v = xv[d] - g.offset[d];
     f[d] = (float)v;
-    b = fmax(b, fabs(v));
-    if (v != v) b = INFINITY;  // NaN coordinate: every candidate of the set goes to FP64
+    b = max(b, abs_hi(v));
   }
   pf[k] = pf_make<D>(f);
   return b;
@@ -61,23 +69,6 @@ struct Pos3 {
   const double* in[3];
   double* out[3];
 };
-
-// the block's largest bound, one atomic per block, and the thresholds from
-// the last block
-template <int D>
-__device__ __forceinline__ void bound_block(double b, unsigned long long* bmax, double dist2, float2* thr,
-                                            unsigned* cnt) {
-  __shared__ double s_b[UTPB / 32];
-  b = warp_max(b);
-  if ((threadIdx.x & 31) == 0) s_b[threadIdx.x >> 5] = b;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 1; w < UTPB / 32; ++w) b = fmax(b, s_b[w]);
-    atomic_max_pos(bmax, b);
-  }
-  pf_thresholds_last_block<D>(bmax, dist2, thr, cnt);
-}
 
 // the rank of each point of the arrival lists among its cell's by original
 // index, and its place in cell order at once
@@ -89,7 +80,7 @@ __global__ void __launch_bounds__(UTPB) k_rank_place(const PointRec* __restrict_
                                                      typename PfVec<D>::T* __restrict__ pf, unsigned long long* bmax,
                                                      float2* thr, unsigned* cnt) {
   const int64_t q = (int64_t)blockIdx.x * UTPB + threadIdx.x;
-  double b = 0.0;
+  unsigned b = 0;
   if (q < N) {
     const PointRec p = rec[q];
     const int32_t s = cellstart[p.key], e = cellstart[p.key + 1];
@@ -102,7 +93,8 @@ __global__ void __launch_bounds__(UTPB) k_rank_place(const PointRec* __restrict_
     orig[k] = p.i;
     b = place_point<D>(p.x, g, k, P.out, pf);
   }
-  bound_block<D>(b, bmax, g.dist2, thr, cnt);
+  atomic_max_hi(bmax, b);
+  pf_thresholds_last_block<D>(bmax, g.dist2, thr, cnt);
 }
 
 // positions by a map (a radix-sorted binning, or stale cells with moved points)
@@ -111,7 +103,7 @@ __global__ void __launch_bounds__(UTPB) k_place(const int32_t* __restrict__ map,
                                                 typename PfVec<D>::T* __restrict__ pf, unsigned long long* bmax,
                                                 float2* thr, unsigned* cnt) {
   const int64_t k = (int64_t)blockIdx.x * UTPB + threadIdx.x;
-  double b = 0.0;
+  unsigned b = 0;
   if (k < N) {
     const int32_t i = map[k];
     double xv[D];
@@ -119,7 +111,8 @@ __global__ void __launch_bounds__(UTPB) k_place(const int32_t* __restrict__ map,
     for (int d = 0; d < D; ++d) xv[d] = P.in[d][i];
     b = place_point<D>(xv, g, k, P.out, pf);
   }
-  bound_block<D>(b, bmax, g.dist2, thr, cnt);
+  atomic_max_hi(bmax, b);
+  pf_thresholds_last_block<D>(bmax, g.dist2, thr, cnt);
 }
 
 // The candidate rows of point k, in key order: its own row from k + 1 on,
@@ -193,31 +186,32 @@ __device__ __forceinline__ bool hit_exact(int64_t k, int32_t m, double* const* x
   return r2_ref<D>(xs[0][k], xs[1][k], D == 3 ? xs[2][k] : 0.0, xs[0][m], xs[1][m], D == 3 ? xs[2][m] : 0.0) < dist2;
 }
 
-// one thread walks all candidates of point k; put(w, word) gets each word of
-// its mask in turn.  The vectors past the last point that a group of four may
-// read are padding (their bits are cut off).
+// One thread walks all candidates of point k: chunk(m, n, in) gets the hit bits
+// of the n <= 32 candidates from m on, in order.  UP_GROUP candidates at a time:
+// eight in 2-D, four in 3-D, whose rows are short (8 there: 219 -> 230 us at 4M
+// points; 4 in 2-D: 37 -> 41 us at 200k).  The vectors past the last point that
+// a group may read are padding (their bits are cut off).
 template <int D, class F>
 __device__ __forceinline__ void up_walk(int64_t k, const UpRows<D>& U, const typename PfVec<D>::T* __restrict__ pf,
-                                        double* const* xs, float2 tt, double dist2, F put) {
+                                        double* const* xs, float2 tt, double dist2, F chunk) {
+  constexpr int G = UP_GROUP<D>;
   const typename PfVec<D>::T a = pf[k];
-  unsigned long long acc = 0;
-  int fill = 0, w = 0;
 #pragma unroll
   for (int r = 0; r < UpRows<D>::R; ++r) {
     const int32_t m1 = U.c[r] + U.dl[r];
     for (int32_t m = (r ? U.c[r ? r - 1 : 0] : 0) + U.dl[r]; m < m1; m += 32) {
       const int n = min(32, m1 - m);
       unsigned in = 0, ok = 0;  // surely in; not surely out
-      for (int j = 0; j < n; j += 4) {
-        unsigned i4 = 0, o4 = 0;
+      for (int j = 0; j < n; j += G) {
+        unsigned ig = 0, og = 0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < G; ++q) {
           const float r2 = r2_pf<D>(a, pf[m + j + q]);
-          if (r2 < tt.x) i4 |= 1u << q;
-          if (!(r2 > tt.y)) o4 |= 1u << q;
+          if (r2 < tt.x) ig |= 1u << q;
+          if (!(r2 > tt.y)) og |= 1u << q;
         }
-        in |= i4 << j;
-        ok |= o4 << j;
+        in |= ig << j;
+        ok |= og << j;
       }
       const unsigned cut = n == 32 ? 0xffffffffu : (1u << n) - 1u;
       in &= cut;
@@ -227,41 +221,66 @@ __device__ __forceinline__ void up_walk(int64_t k, const UpRows<D>& U, const typ
         band &= band - 1;
         if (hit_exact<D>(k, m + b, xs, dist2)) in |= 1u << b;
       }
-      acc |= (unsigned long long)in << fill;
-      fill += n;
-      if (fill >= 32) {
-        put(w++, (unsigned)acc);
-        acc >>= 32;
-        fill -= 32;
-      }
+      chunk(m, n, in);
     }
   }
-  if (fill > 0) put(w, (unsigned)acc);
 }
 
-// Count pass: the mask words of each point (point-major, the first W of
-// them), its offset among the pairs of its block, the blocks' totals and the
-// candidate statistics; the last block of a grid of up to SCAN_FOLD_MAX blocks
-// scans the totals into the blocks' starts (base[gridDim.x] is the total).
-template <int D>
-__global__ void __launch_bounds__(UTPB) k_up_count(const typename PfVec<D>::T* __restrict__ pf, Pos3 P,
-                                                   const float2* __restrict__ thr, const int32_t* __restrict__ skey,
-                                                   const int32_t* __restrict__ cellstart, int64_t N, Grid g,
-                                                   unsigned* __restrict__ mask, int W, int32_t* __restrict__ loc,
-                                                   int32_t* __restrict__ total, int64_t* __restrict__ base,
-                                                   UpStat* stat, unsigned* fold_cnt) {
+// Count pass: what each point keeps (ROWS: its neighbours, else its words; W of
+// either, point-major), its offset among the pairs of its block, the blocks'
+// totals and the candidate statistics; the last block of a grid of up to
+// SCAN_FOLD_MAX blocks scans the totals into the blocks' starts
+// (base[gridDim.x] is the total).
+template <int D, bool ROWS>
+__global__ void __launch_bounds__(UTPB, D == 2 ? 4 : 5) k_up_count(
+    const typename PfVec<D>::T* __restrict__ pf, Pos3 P, const float2* __restrict__ thr,
+    const int32_t* __restrict__ skey, const int32_t* __restrict__ cellstart, int64_t N, Grid g,
+    unsigned* __restrict__ kept, int W, int32_t* __restrict__ loc, int32_t* __restrict__ total,
+    int64_t* __restrict__ base, UpStat* stat, unsigned* fold_cnt) {
   const int64_t k = (int64_t)blockIdx.x * UTPB + threadIdx.x;
   int32_t cnt = 0, nw = 0;
   if (k < N) {
     const UpRows<D> U = up_rows<D>(k, skey[k], cellstart, g);
     nw = (U.total() + 31) >> 5;
-    unsigned* mk = mask + k * W;
-    up_walk<D>(k, U, pf, P.out, *thr, g.dist2, [&](int w, unsigned word) {
-      cnt += __popc(word);
-      if (w < W) mk[w] = word;
-    });
+    unsigned* kp = kept + k * W;
+    if constexpr (ROWS) {
+      // four neighbours to a store (W is a multiple of four)
+      int4 v = make_int4(0, 0, 0, 0);
+      up_walk<D>(k, U, pf, P.out, *thr, g.dist2, [&](int32_t m, int, unsigned in) {
+        while (in) {
+          const int b = __ffs(in) - 1;
+          in &= in - 1;
+          v = make_int4(v.y, v.z, v.w, m + b);
+          ++cnt;
+          if ((cnt & 3) == 0 && cnt <= W) *reinterpret_cast<int4*>(kp + cnt - 4) = v;
+        }
+      });
+      const int left = cnt & 3;
+      if (cnt < W) {
+        unsigned* e = kp + (cnt - left);
+        if (left == 3) e[0] = v.y;
+        if (left >= 2) e[left - 2] = v.z;
+        if (left >= 1) e[left - 1] = v.w;
+      }
+    } else {
+      unsigned long long acc = 0;
+      int fill = 0, w = 0;
+      up_walk<D>(k, U, pf, P.out, *thr, g.dist2, [&](int32_t, int n, unsigned in) {
+        cnt += __popc(in);
+        acc |= (unsigned long long)in << fill;
+        fill += n;
+        if (fill >= 32) {
+          if (w < W) kp[w] = (unsigned)acc;
+          ++w;
+          acc >>= 32;
+          fill -= 32;
+        }
+      });
+      if (fill > 0 && w < W) kp[w] = (unsigned)acc;
+    }
   }
-  // the block's exclusive scan of the counts; sum and maximum of the words
+  // the block's exclusive scan of the counts; the sum of the words, and the
+  // most of what a point keeps
   __shared__ int32_t s_c[UTPB / 32], s_s[UTPB / 32], s_m[UTPB / 32];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   int32_t inc = cnt;
@@ -270,7 +289,7 @@ __global__ void __launch_bounds__(UTPB) k_up_count(const typename PfVec<D>::T* _
     const int32_t y = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += y;
   }
-  const int32_t ws = __reduce_add_sync(0xffffffffu, nw), wm = __reduce_max_sync(0xffffffffu, nw);
+  const int32_t ws = __reduce_add_sync(0xffffffffu, nw), wm = __reduce_max_sync(0xffffffffu, ROWS ? cnt : nw);
   if (lane == 31) {
     s_c[wp] = inc;
     s_s[wp] = ws;
@@ -294,9 +313,9 @@ __global__ void __launch_bounds__(UTPB) k_up_count(const typename PfVec<D>::T* _
   if (fold_cnt && last_block_of_grid(fold_cnt)) block_exclusive_scan<int64_t>(total, base, gridDim.x);
 }
 
-// (min, max) 1-based original indices of a pair
+// (min, max) of a pair's 1-based original indices, and its store
 __device__ __forceinline__ int2 make_pair1(int32_t ok, int32_t om) {
-  return make_int2(ok < om ? ok : om, ok < om ? om : ok);
+  return make_int2(min(ok, om), max(ok, om));
 }
 __device__ __forceinline__ void store_pair(int32_t* pairs, int64_t pos, int2 v, bool aligned) {
   if (aligned) {
@@ -307,73 +326,23 @@ __device__ __forceinline__ void store_pair(int32_t* pairs, int64_t pos, int2 v, 
   }
 }
 
-// Emit, one warp per point: each lane takes one bit of a word, so a word's
-// pairs are one contiguous store.  The words past the stored W are searched
-// again, 32 candidates at a time.
-template <int D>
-__global__ void __launch_bounds__(UTPB) k_up_emit_warp(const typename PfVec<D>::T* __restrict__ pf, Pos3 P,
-                                                       const float2* __restrict__ thr,
-                                                       const int32_t* __restrict__ skey,
-                                                       const int32_t* __restrict__ cellstart,
-                                                       const int32_t* __restrict__ orig, int64_t N, Grid g,
-                                                       const unsigned* __restrict__ mask, int W,
-                                                       const int32_t* __restrict__ loc,
-                                                       const int64_t* __restrict__ base, int64_t cap,
-                                                       int32_t* __restrict__ pairs, bool aligned) {
-  const int64_t k = ((int64_t)blockIdx.x * UTPB + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (k >= N) return;
-  const UpRows<D> U = up_rows<D>(k, skey[k], cellstart, g);
-  const int32_t tot = U.total();
-  const int nw = (tot + 31) >> 5;
-  const int32_t ok = orig[k] + 1;
-  const int64_t pos = base[k / UTPB] + loc[k];
-  int32_t* out = pairs + 2 * pos;
-  const int lim = (int)max((int64_t)0, min(cap - pos, (int64_t)0x7fffffff));  // pairs of this point that fit
-  const unsigned bit = 1u << lane, lt = bit - 1u;
-  int off = 0;
-  const int stored = min(nw, W);
-  for (int w0 = 0; w0 < stored; w0 += 32) {
-    const unsigned mine = w0 + lane < stored ? mask[k * W + w0 + lane] : 0u;
-    const int n = min(32, stored - w0);
-#pragma unroll 4
-    for (int w = 0; w < n; ++w) {
-      const unsigned word = __shfl_sync(0xffffffffu, mine, w);
-      const int at = off + __popc(word & lt);
-      if ((word & bit) && at < lim)
-        store_pair(out, at, make_pair1(ok, orig[U.at((w0 + w) * 32 + lane)] + 1), aligned);
-      off += __popc(word);
-    }
-  }
-  for (int w = stored; w < nw; ++w) {
-    const int32_t t = w * 32 + lane;
-    const int32_t m = t < tot ? U.at(t) : (int32_t)k;
-    bool hit = false;
-    if (t < tot) {
-      const float r2 = r2_pf<D>(pf[k], pf[m]);
-      hit = r2 < thr->x || (!(r2 > thr->y) && hit_exact<D>(k, m, P.out, g.dist2));
-    }
-    const unsigned word = __ballot_sync(0xffffffffu, hit);
-    const int at = off + __popc(word & lt);
-    if (hit && at < lim) store_pair(out, at, make_pair1(ok, orig[m] + 1), aligned);
-    off += __popc(word);
-  }
+// pairs of point k: those of its block's list from loc[k] on
+__device__ __forceinline__ int32_t up_pairs(int64_t k, int64_t N, const int32_t* __restrict__ loc,
+                                            const int32_t* __restrict__ total) {
+  const int64_t kn = k + 1;
+  return (kn < N && kn % UTPB != 0 ? loc[kn] : total[k / UTPB]) - loc[k];
 }
 
-// Emit, one thread per point, for lists of few pairs a point (a warp per
-// point would leave most lanes without a bit): a block's pairs are contiguous
-// in the list, so they are collected in shared memory and stored as one run.
+// Emit from words, one thread per point: a block's pairs are one run of the
+// list, so they are collected in shared memory and stored as such.  A point
+// with more words than are kept is searched again.
 template <int D>
-__global__ void __launch_bounds__(UTPB) k_up_emit_thread(const typename PfVec<D>::T* __restrict__ pf, Pos3 P,
-                                                         const float2* __restrict__ thr,
-                                                         const int32_t* __restrict__ skey,
-                                                         const int32_t* __restrict__ cellstart,
-                                                         const int32_t* __restrict__ orig, int64_t N, Grid g,
-                                                         const unsigned* __restrict__ mask, int W,
-                                                         const int32_t* __restrict__ loc,
-                                                         const int32_t* __restrict__ total,
-                                                         const int64_t* __restrict__ base, int64_t cap,
-                                                         int32_t* __restrict__ pairs, bool aligned) {
+__global__ void __launch_bounds__(UTPB, 6) k_up_emit_words(
+    const typename PfVec<D>::T* __restrict__ pf, Pos3 P, const float2* __restrict__ thr,
+    const int32_t* __restrict__ skey, const int32_t* __restrict__ cellstart, const int32_t* __restrict__ orig,
+    int64_t N, Grid g, const unsigned* __restrict__ kept, int W, const int32_t* __restrict__ loc,
+    const int32_t* __restrict__ total, const int64_t* __restrict__ base, int64_t cap, int32_t* __restrict__ pairs,
+    bool aligned) {
   __shared__ int2 s_p[EMIT_STAGE];
   const int64_t k = (int64_t)blockIdx.x * UTPB + threadIdx.x;
   const int64_t b0 = base[blockIdx.x];
@@ -384,26 +353,88 @@ __global__ void __launch_bounds__(UTPB) k_up_emit_thread(const typename PfVec<D>
     const int nw = (U.total() + 31) >> 5;
     const int32_t ok = orig[k] + 1;
     int32_t at = loc[k];
-    auto expand = [&](int w, unsigned word) {
-      while (word) {
-        const int b = __ffs(word) - 1;
-        word &= word - 1;
-        const int2 v = make_pair1(ok, orig[U.at(w * 32 + b)] + 1);
-        if (staged) s_p[at] = v;
-        else if (b0 + at < cap) store_pair(pairs, b0 + at, v, aligned);
-        ++at;
-      }
+    auto pair = [&](int32_t m) {
+      const int2 v = make_pair1(ok, orig[m] + 1);
+      if (staged) s_p[at] = v;
+      else if (b0 + at < cap) store_pair(pairs, b0 + at, v, aligned);
+      ++at;
     };
     if (nw <= W) {
-      for (int w = 0; w < nw; ++w) expand(w, mask[k * W + w]);
+      for (int w = 0; w < nw; ++w) {
+        unsigned word = kept[k * W + w];
+        while (word) {
+          pair(U.at(w * 32 + __ffs(word) - 1));
+          word &= word - 1;
+        }
+      }
     } else {
-      up_walk<D>(k, U, pf, P.out, *thr, g.dist2, expand);
+      up_walk<D>(k, U, pf, P.out, *thr, g.dist2, [&](int32_t m, int, unsigned in) {
+        while (in) {
+          pair(m + __ffs(in) - 1);
+          in &= in - 1;
+        }
+      });
     }
   }
   if (!staged) return;  // uniform over the block
   __syncthreads();
   for (int32_t i = threadIdx.x; i < all; i += UTPB)
     if (b0 + i < cap) store_pair(pairs, b0 + i, s_p[i], aligned);
+}
+
+// Emit from neighbour rows, L lanes per point, four entries of each in flight
+// (at one the pass waits for its loads).  A row that outgrew its W entries is
+// searched again by the group, L candidates at a time.
+template <int D, int L>
+__global__ void __launch_bounds__(UTPB) k_up_emit_rows(
+    const typename PfVec<D>::T* __restrict__ pf, Pos3 P, const float2* __restrict__ thr,
+    const int32_t* __restrict__ skey, const int32_t* __restrict__ cellstart, const int32_t* __restrict__ orig,
+    int64_t N, Grid g, const unsigned* __restrict__ kept, int W, const int32_t* __restrict__ loc,
+    const int32_t* __restrict__ total, const int64_t* __restrict__ base, int64_t cap, int32_t* __restrict__ pairs,
+    bool aligned) {
+  const int64_t gt = (int64_t)blockIdx.x * UTPB + threadIdx.x;
+  const int64_t k = gt / L;
+  const int lane = (int)(gt % L);
+  if (k >= N) return;  // whole groups leave together
+  const int32_t n = up_pairs(k, N, loc, total);
+  const int32_t ok = orig[k] + 1;
+  const int64_t pos = base[k / UTPB] + loc[k];
+  int32_t* out = pairs + 2 * pos;
+  const int32_t lim = (int32_t)max((int64_t)0, min(cap - pos, (int64_t)n));  // of this point's pairs, those that fit
+  if (n <= W) {
+    const int32_t* row = reinterpret_cast<const int32_t*>(kept) + k * W;
+    for (int32_t t = lane; t < lim; t += 4 * L) {
+      int32_t om[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) om[j] = t + j * L < lim ? row[t + j * L] : (int32_t)k;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) om[j] = orig[om[j]] + 1;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (t + j * L < lim) store_pair(out, t + j * L, make_pair1(ok, om[j]), aligned);
+    }
+    return;
+  }
+  const unsigned gbase = threadIdx.x & 31u & ~(unsigned)(L - 1);
+  const unsigned gm = L == 32 ? 0xffffffffu : ((1u << L) - 1u) << gbase;
+  const UpRows<D> U = up_rows<D>(k, skey[k], cellstart, g);
+  const int32_t tot = U.total();
+  const typename PfVec<D>::T a = pf[k];
+  int32_t off = 0;
+  for (int32_t tb = 0; tb < tot; tb += L) {
+    const int32_t t = tb + lane;
+    int32_t m = 0;
+    bool hit = false;
+    if (t < tot) {
+      m = U.at(t);
+      const float r2 = r2_pf<D>(a, pf[m]);
+      hit = r2 < thr->x || (!(r2 > thr->y) && hit_exact<D>(k, m, P.out, g.dist2));
+    }
+    const unsigned bal = (__ballot_sync(gm, hit) >> gbase) & (L == 32 ? 0xffffffffu : (1u << L) - 1u);
+    const int32_t at = off + __popc(bal & ((1u << lane) - 1u));
+    if (hit && at < lim) store_pair(out, at, make_pair1(ok, orig[m] + 1), aligned);
+    off += __popc(bal);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -427,8 +458,8 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
   const int nb = nblocks(N, UTPB);
   int rc;
   if ((rc = C.ensure_pf_scalars())) return rc;
-  // four vectors of padding, which a walk may read and cut off
-  if (!C.upf.p && (rc = C.upf.ensure(sizeof(V) * (N + 4), st, true))) return rc;
+  // a group of padding, which a walk may read and cut off
+  if (!C.upf.p && (rc = C.upf.ensure(sizeof(V) * (N + UP_GROUP<D>), st, true))) return rc;
   if ((rc = C.uptot.ensure(sizeof(int32_t) * ((size_t)nb + 4), st))) return rc;
   if ((rc = C.upbase.ensure(sizeof(int64_t) * ((size_t)nb + 1), st))) return rc;
   if ((rc = C.upstat.ensure(sizeof(UpStat), st))) return rc;
@@ -457,36 +488,55 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
   }
   timer_end(T_SORT, st);
   timer_begin(T_PAIRS, st);
-  // mask words a point: as many as the last search needed, up to three times
-  // its mean (a crowded cell's points search their last words again in the emit)
-  int W = 0;
-  if (C.up_most > 0) {
-    W = C.up_most;
-    if ((double)W > 3.0 * C.up_mean + 4.0) W = (int)(3.0 * C.up_mean + 4.0);
-    if ((rc = C.upmask.ensure(sizeof(unsigned) * (size_t)N * (size_t)W, st))) return rc;
-  }
-  C.up_w = W;
-  GC_CUDA(cudaMemsetAsync(C.upstat.p, 0, sizeof(UpStat), st));
+  // What a point keeps: as much as the last search's fullest point needed and
+  // a quarter more, up to about three times the mean (a crowded cell's points
+  // are searched again in the emit).  A search that finds its points in need
+  // of more, or of the other form, is run again.  The first one guesses from
+  // the grid-wide mean of candidates, of which about a third are pairs in 2-D
+  // and a sixth in 3-D.
   const bool fold = nb <= SCAN_FOLD_MAX;
-  k_up_count<D><<<nb, UTPB, 0, st>>>(pf, P, thr, C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), N, C.g,
-                                     C.upmask.as<unsigned>(), W, C.cnt_up.as<int32_t>(), C.uptot.as<int32_t>(),
-                                     C.upbase.as<int64_t>(), C.upstat.as<UpStat>(),
-                                     fold ? C.foldcnt.as<unsigned>() + 1 : nullptr);
-  GC_LAUNCHED();
-  if (!fold && (rc = exclusive_scan_i32_to_i64(C.uptot.as<int32_t>(), C.upbase.as<int64_t>(), nb,
-                                               C.scratch.as<int64_t>(), st)))
-    return rc;
+  if (C.up_w == 0) {
+    const double cand = 0.5 * C.candidates_per_point(), top = 4096.0;
+    C.up_rows = cand > 32.0 * UP_FEW;
+    const double need = C.up_rows ? cand * (D == 2 ? 0.7 : 0.35) : cand / 16.0;
+    C.up_w = ((int)(need < top ? need : top) + 8) / 4 * 4;
+  }
+  for (;;) {
+    if (C.up_w > 0 && (rc = C.upkept.ensure(sizeof(unsigned) * (size_t)N * (size_t)C.up_w, st))) return rc;
+    GC_CUDA(cudaMemsetAsync(C.upstat.p, 0, sizeof(UpStat), st));
+    const auto count = C.up_rows ? k_up_count<D, true> : k_up_count<D, false>;
+    count<<<nb, UTPB, 0, st>>>(pf, P, thr, C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), N, C.g,
+                               C.upkept.as<unsigned>(), C.up_w, C.cnt_up.as<int32_t>(), C.uptot.as<int32_t>(),
+                               C.upbase.as<int64_t>(), C.upstat.as<UpStat>(),
+                               fold ? C.foldcnt.as<unsigned>() + 1 : nullptr);
+    GC_LAUNCHED();
+    if (!fold && (rc = exclusive_scan_i32_to_i64(C.uptot.as<int32_t>(), C.upbase.as<int64_t>(), nb,
+                                                 C.scratch.as<int64_t>(), st)))
+      return rc;
+    GC_CUDA(cudaMemcpyAsync(C.pin, C.upbase.as<int64_t>() + nb, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    GC_CUDA(cudaMemcpyAsync(C.pin + 2, C.upstat.p, sizeof(UpStat), cudaMemcpyDeviceToHost, st));
+    GC_CUDA(cudaStreamSynchronize(st));
+    UpStat s;
+    memcpy(&s, C.pin + 2, sizeof(s));
+    int64_t sampled = (int64_t)((nb + UP_SAMPLE - 1) / UP_SAMPLE) * UTPB;
+    if (sampled > N) sampled = N;
+    const double words = (double)s.words / (double)sampled;
+    const double mean = C.up_rows ? (double)C.pin[0] / (double)N : words;
+    // (a set near the line between the forms stays with the one it has)
+    if (C.up_rows ? words < 0.8 * UP_FEW : words > UP_FEW) {
+      C.up_rows = !C.up_rows;
+      // the other form's need: at a first guess its mean
+      const double other = C.up_rows ? (double)C.pin[0] / (double)N : words;
+      C.up_w = ((int)(1.5 * other) + 8 + 3) / 4 * 4;
+      continue;
+    }
+    const double bound = 3.0 * mean + 16.0;
+    const int most = (double)s.most < bound ? s.most : (int)bound;
+    if (most <= C.up_w) break;
+    C.up_w = (most + most / 4 + 3) / 4 * 4;
+  }
   timer_end(T_PAIRS, st);
-  GC_CUDA(cudaMemcpyAsync(C.pin, C.upbase.as<int64_t>() + nb, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  GC_CUDA(cudaMemcpyAsync(C.pin + 2, C.upstat.p, sizeof(UpStat), cudaMemcpyDeviceToHost, st));
-  GC_CUDA(cudaStreamSynchronize(st));
   timer_collect();
-  UpStat s;
-  memcpy(&s, C.pin + 2, sizeof(s));
-  int64_t sampled = (int64_t)((nb + UP_SAMPLE - 1) / UP_SAMPLE) * UTPB;
-  if (sampled > N) sampled = N;
-  C.up_mean = (double)s.words / (double)sampled;
-  C.up_most = s.most;
   C.nup = C.pin[0];
   C.nfull = C.nup;
   C.nfull_est = 2 * C.nup;
@@ -503,17 +553,22 @@ static int emit_upper_impl(CellCore& C, double* const* xs, int32_t* pairs, int64
   const int64_t N = C.N;
   const Pos3 P = pos3<D>(nullptr, xs);
   const bool aligned = ((uintptr_t)pairs & 7u) == 0;
-  // up to two words a point (about 64 candidates, some ten pairs) a thread per
-  // point; above, a warp per point
-  if (C.up_mean <= 2.0)
-    k_up_emit_thread<D><<<nblocks(N, UTPB), UTPB, 0, st>>>(
-        C.upf.as<V>(), P, C.pfthr.as<float2>(), C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), C.orig.as<int32_t>(),
-        N, C.g, C.upmask.as<unsigned>(), C.up_w, C.cnt_up.as<int32_t>(), C.uptot.as<int32_t>(),
-        C.upbase.as<int64_t>(), cap, pairs, aligned);
-  else
-    k_up_emit_warp<D><<<nblocks(N * 32, UTPB), UTPB, 0, st>>>(
-        C.upf.as<V>(), P, C.pfthr.as<float2>(), C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), C.orig.as<int32_t>(),
-        N, C.g, C.upmask.as<unsigned>(), C.up_w, C.cnt_up.as<int32_t>(), C.upbase.as<int64_t>(), cap, pairs, aligned);
+#define UP_EMIT(KER, T)                                                                                            \
+  KER<<<nblocks(T, UTPB), UTPB, 0, st>>>(C.upf.as<V>(), P, C.pfthr.as<float2>(), C.skey.as<int32_t>(),             \
+                                         C.cellstart.as<int32_t>(), C.orig.as<int32_t>(), N, C.g,                  \
+                                         C.upkept.as<unsigned>(), C.up_w, C.cnt_up.as<int32_t>(),                  \
+                                         C.uptot.as<int32_t>(), C.upbase.as<int64_t>(), cap, pairs, aligned)
+  if (!C.up_rows) {
+    UP_EMIT((k_up_emit_words<D>), N);
+  } else {
+    // lanes per point: about four or five of its pairs each
+    const double mean = (double)C.nup / (double)N;
+    if (mean <= 24.0) UP_EMIT((k_up_emit_rows<D, 4>), N * 4);
+    else if (mean <= 48.0) UP_EMIT((k_up_emit_rows<D, 8>), N * 8);
+    else if (mean <= 96.0) UP_EMIT((k_up_emit_rows<D, 16>), N * 16);
+    else UP_EMIT((k_up_emit_rows<D, 32>), N * 32);
+  }
+#undef UP_EMIT
   GC_LAUNCHED();
   return GCSPH_OK;
 }

@@ -168,6 +168,21 @@ __device__ inline void atomic_max_pos(unsigned long long* addr, double v) {
   if (b > *(volatile unsigned long long*)addr) atomicMax(addr, b);
 }
 
+// Upper bounds of |v| on the integer pipe: the high word of |v|, rounded up,
+// orders like |v|; NaN and infinity give infinity's.  (FP64 compares and their
+// reduction kept the FP64 pipe busier than the memory in the passes that take
+// this bound.)
+constexpr unsigned HI_INF = 0x7ff00000u;
+__device__ __forceinline__ unsigned abs_hi(double v) {
+  return min(((unsigned)(__double_as_longlong(v) >> 32) & 0x7fffffffu) + 1u, HI_INF);
+}
+// the largest of a warp's bounds (all lanes, 0: none) into *addr
+__device__ __forceinline__ void atomic_max_hi(unsigned long long* addr, unsigned hi) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned long long b = (unsigned long long)m << 32;
+  if ((threadIdx.x & 31) == 0 && b > *(volatile unsigned long long*)addr) atomicMax(addr, b);
+}
+
 // Warp/block max of a non-negative double, one atomic per block
 __device__ inline double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));

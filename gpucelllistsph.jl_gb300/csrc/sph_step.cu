@@ -491,17 +491,14 @@ __device__ __forceinline__ PermVals<D> perm_load(const SArr<D>& S, int64_t i) {
 // the max |x - offset| of the FP32 prefilter copy
 template <int D>
 __device__ __forceinline__ void perm_store(const StepConst& c, const SArr<D>& S, const PermOut<D>& O,
-                                           const PermVals<D>& p, int64_t k, double& b) {
-  double bk = 0.0;
+                                           const PermVals<D>& p, int64_t k, unsigned& b) {
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     O.x[d][k] = p.x[d];
     const double rel = p.x[d] - O.off[d];
     O.pf[d][k] = (float)rel;
-    bk = fmax(bk, fabs(rel));
+    b = max(b, abs_hi(rel));
   }
-  if (bk != bk) bk = INFINITY;  // NaN coordinate: every candidate of the set goes to FP64
-  b = fmax(b, bk);
   O.pt[k] = p.pt;
   O.rho[k] = p.rho;
   O.rhoh[k] = p.rhoh;
@@ -519,7 +516,7 @@ __device__ __forceinline__ void perm_store(const StepConst& c, const SArr<D>& S,
 // new[k] = old[i] for the whole cell-order state of one particle
 template <int D>
 __device__ __forceinline__ void permute_one(const StepConst& c, const SArr<D>& S, const PermOut<D>& O, int64_t i,
-                                            int64_t k, double& b) {
+                                            int64_t k, unsigned& b) {
   perm_store<D>(c, S, O, perm_load<D>(S, i), k, b);
 }
 
@@ -527,10 +524,9 @@ __device__ __forceinline__ void permute_one(const StepConst& c, const SArr<D>& S
 template <int D>
 __global__ void k_permute_state(StepConst c, int64_t N, const int32_t* __restrict__ perm, SArr<D> S, PermOut<D> O) {
   int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double b = 0.0;
+  unsigned b = 0;
   if (k < N) permute_one<D>(c, S, O, perm[k], k, b);
-  b = warp_max(b);
-  if ((threadIdx.x & 31) == 0) atomic_max_pos(O.pfmax, b);
+  atomic_max_hi(O.pfmax, b);
   pf_thresholds_last_block<D>(O.pfmax, O.dist2, O.thr, O.cnt);
 }
 
@@ -545,7 +541,7 @@ __global__ void k_rank_permute(StepConst c, int64_t N, const int32_t* __restrict
                                int32_t* __restrict__ skey, int32_t* __restrict__ orig, SArr<D> S, PermOut<D> O,
                                const int32_t* __restrict__ tord) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double b = 0.0;
+  unsigned b = 0;
   if (q < N) {
     // the particle's state is loaded as soon as its index is known, so that
     // these loads overlap the rank's (the rank's stores could alias them)
@@ -554,8 +550,7 @@ __global__ void k_rank_permute(StepConst c, int64_t N, const int32_t* __restrict
     const int64_t k = rank_in_cell(tmp, key, cellstart, ord, q, perm, skey, orig, nullptr, tord);
     perm_store<D>(c, S, O, pv, k, b);
   }
-  b = warp_max(b);
-  if ((threadIdx.x & 31) == 0) atomic_max_pos(O.pfmax, b);
+  atomic_max_hi(O.pfmax, b);
   pf_thresholds_last_block<D>(O.pfmax, O.dist2, O.thr, O.cnt);
 }
 

@@ -1,7 +1,7 @@
-"""The cell list's mask search and its two emits, pairs and order: rows of
+"""The cell list's own search and its two emits, pairs and order: rows of
 exactly 32 candidates and their neighbours, few and many pairs a point, a
-crowded cell whose masks pass the stored words (searched again in the emit), a
-first build (no masks stored yet) against later ones, moved points on stale
+crowded cell whose points outgrow what is kept (searched again in the emit), a
+first build against later ones, moved points on stale
 cells, lists cut by their capacity.  The list is exactly the oracle's pair set
 ordered by (rank of the first, rank of the second), ranks by (cell, index)."""
 import ctypes as C
@@ -50,11 +50,11 @@ def _points(kind, D, N, seed):
     ("uniform", 2, 1, 0.1), ("uniform", 2, 257, 0.03), ("uniform", 2, 5000, 0.1), ("uniform", 2, 70001, 0.01),
     ("uniform", 3, 255, 0.3), ("uniform", 3, 9001, 0.04), ("uniform", 3, 9001, 0.2),
     ("cluster", 2, 3000, 0.02), ("cluster", 3, 3000, 0.05)])
-def test_masks_give_the_ordered_list(gpu_pkg, orc, kind, D, N, dist):
+def test_ordered_list(gpu_pkg, orc, kind, D, N, dist):
     x = _points(kind, D, N, 7 + D)
     c = gpu_pkg.GPUCellList(tuple(x), (dist,) * D, dist)
     want = _expected(orc, x, dist)
-    assert np.array_equal(c.neighborlistview().cpu().numpy(), want)  # first build: no masks stored
+    assert np.array_equal(c.neighborlistview().cpu().numpy(), want)  # first build
     c.update()
     assert np.array_equal(c.neighborlistview().cpu().numpy(), want)
     # a list cut by its capacity, 8-byte aligned and not
@@ -77,8 +77,8 @@ def test_masks_give_the_ordered_list(gpu_pkg, orc, kind, D, N, dist):
 
 
 def test_crowding_between_updates(gpu_pkg, orc):
-    """Masks stored for a sparse set, then all points move into a few cells:
-    the words stored are too few, then the next update stores enough."""
+    """Words kept for a sparse set, then all points move into a few cells:
+    the next search keeps rows, and enough of them."""
     D, N, dist = 2, 2000, 0.02
     x = _points("uniform", D, N, 3)
     c = gpu_pkg.GPUCellList(tuple(x), (dist,) * D, dist, MIN=(0, 0), MAX=(1, 1))
