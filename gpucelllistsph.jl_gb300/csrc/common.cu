@@ -181,7 +181,9 @@ void DevBuf::release() {
 
 template <class TIn, class TOut>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile(const TIn* __restrict__ in, TOut* __restrict__ out,
-                                                            int64_t n_in, int64_t m, int64_t* __restrict__ bsum) {
+                                                            int64_t n_in, int64_t m, int64_t* __restrict__ bsum,
+                                                            const int* __restrict__ run) {
+  if (run && !*run) return;
   __shared__ long long wtot[SCAN_THREADS / 32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)tid * SCAN_ITEMS;
@@ -223,7 +225,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile(const TIn* __restric
 }
 
 template <class TOut>
-__global__ void k_scan_add(TOut* __restrict__ out, int64_t m, const int64_t* __restrict__ boff) {
+__global__ void k_scan_add(TOut* __restrict__ out, int64_t m, const int64_t* __restrict__ boff,
+                           const int* __restrict__ run) {
+  if (run && !*run) return;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m) out[i] = (TOut)((long long)out[i] + boff[i / SCAN_TILE]);
 }
@@ -236,7 +240,8 @@ __global__ void k_scan_add(TOut* __restrict__ out, int64_t m, const int64_t* __r
 template <class TIn, class TOut>
 __global__ void __launch_bounds__(1024) k_scan_single(const TIn* __restrict__ in0, TOut* __restrict__ out0,
                                                       const TIn* __restrict__ in1, TOut* __restrict__ out1,
-                                                      int64_t n_in, int64_t m) {
+                                                      int64_t n_in, int64_t m, const int* __restrict__ run) {
+  if (run && !*run) return;
   constexpr int TILE = 1024 * SCAN_ITEMS;
   // 32-bit inputs go through shared memory (32 KB); 64-bit ones (block totals) are read directly
   constexpr bool SMEM = sizeof(TIn) == 4;
@@ -300,22 +305,23 @@ __global__ void __launch_bounds__(1024) k_scan_single(const TIn* __restrict__ in
 }
 
 template <class TIn, class TOut>
-static int scan_impl(const TIn* in, TOut* out, int64_t n_in, int64_t m, int64_t* scratch, cudaStream_t s) {
+static int scan_impl(const TIn* in, TOut* out, int64_t n_in, int64_t m, int64_t* scratch, cudaStream_t s,
+                     const int* run = nullptr) {
   if (m <= SCAN_SINGLE_MAX) {
-    k_scan_single<TIn, TOut><<<1, 1024, 0, s>>>(in, out, nullptr, nullptr, n_in, m);
+    k_scan_single<TIn, TOut><<<1, 1024, 0, s>>>(in, out, nullptr, nullptr, n_in, m, run);
     GC_LAUNCHED();
     return GCSPH_OK;
   }
   int64_t nb = (m + SCAN_TILE - 1) / SCAN_TILE;
   if (nb < 1) nb = 1;
   if (nb > 0x7fffffffLL) return fail(GCSPH_EINVAL, "scan too large");
-  k_scan_tile<TIn, TOut><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n_in, m, scratch);
+  k_scan_tile<TIn, TOut><<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n_in, m, scratch, run);
   GC_LAUNCHED();
   if (nb == 1) return GCSPH_OK;
   int64_t* bscan = scratch + nb;
-  int rc = scan_impl<int64_t, int64_t>(scratch, bscan, nb, nb, bscan + nb + 1, s);
+  int rc = scan_impl<int64_t, int64_t>(scratch, bscan, nb, nb, bscan + nb + 1, s, run);
   if (rc) return rc;
-  k_scan_add<TOut><<<nblocks(m, 256), 256, 0, s>>>(out, m, bscan);
+  k_scan_add<TOut><<<nblocks(m, 256), 256, 0, s>>>(out, m, bscan, run);
   GC_LAUNCHED();
   return GCSPH_OK;
 }
@@ -323,13 +329,14 @@ static int scan_impl(const TIn* in, TOut* out, int64_t n_in, int64_t m, int64_t*
 int exclusive_scan_i32_to_i64(const int32_t* in, int64_t* out, int64_t n, int64_t* scratch, cudaStream_t s) {
   return scan_impl<int32_t, int64_t>(in, out, n, n + 1, scratch, s);
 }
-int exclusive_scan_i32_to_i32(const int32_t* in, int32_t* out, int64_t n, int64_t* scratch, cudaStream_t s) {
-  return scan_impl<int32_t, int32_t>(in, out, n, n + 1, scratch, s);
+int exclusive_scan_i32_to_i32(const int32_t* in, int32_t* out, int64_t n, int64_t* scratch, cudaStream_t s,
+                              const int* run) {
+  return scan_impl<int32_t, int32_t>(in, out, n, n + 1, scratch, s, run);
 }
 int exclusive_scan2_i32_to_i64(const int32_t* in0, int64_t* out0, const int32_t* in1, int64_t* out1, int64_t n,
                                int64_t* scratch, cudaStream_t s) {
   if (n + 1 <= SCAN_SINGLE_MAX) {
-    k_scan_single<int32_t, int64_t><<<2, 1024, 0, s>>>(in0, out0, in1, out1, n, n + 1);
+    k_scan_single<int32_t, int64_t><<<2, 1024, 0, s>>>(in0, out0, in1, out1, n, n + 1, nullptr);
     GC_LAUNCHED();
     return GCSPH_OK;
   }

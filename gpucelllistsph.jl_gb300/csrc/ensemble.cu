@@ -111,6 +111,7 @@ struct EnsArr {
   float4* r4;
   const int32_t* istep;      // steps done per instance (cspmcorr! schedule)
   const int* rb;             // per instance: this step rebuilds the instance's cells and list
+  const int* any;            // [0] some instance does, [1] some instance's cspmcorr! is due
   float* ob[3];              // offsets at the instance's last list build (same cell corner as off)
   // dpcreg!'s row bound (null: every row is scanned): the smallest r² of each
   // row at the step's start (stage 1) and, per instance, the largest |Δx|² of
@@ -273,54 +274,68 @@ __device__ __forceinline__ void cell_of(int key, const EnsInst& I, int& c0, int&
 // An instance that keeps its list keeps its particles' cells (the key they
 // were sorted by, skey): the sort then leaves its particles where they are,
 // so the list's instance-local indices stay valid.
+//
+// any[0] (k_ens_tick): some instance rebuilds at this step.  Where none does,
+// the order stays as it is and the binning's passes return at once, on small
+// grids -- they took a tenth of a 2-D step (69 of 545 us at 743k particles).
+constexpr int BIN_TPB = 256;
+inline int bin_grid(int64_t n) { return (int)std::min<int64_t>(nblocks(n, BIN_TPB), 152 * 8); }
+
 template <int D>
 __global__ void k_ens_key(int64_t N, const int32_t* __restrict__ inst, const double* __restrict__ x0,
                           const double* __restrict__ x1, const double* __restrict__ x2,
                           const EnsInst* __restrict__ T, const int* __restrict__ rb,
                           const int32_t* __restrict__ skey, int32_t* __restrict__ key, int32_t* __restrict__ slot,
-                          int32_t* __restrict__ count) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const int si = inst[i];
-  int k;
-  if (!rb[si]) {
-    k = skey[i];
-  } else {
-    const EnsInst& I = T[si];
-    const double xs[3] = {x0[i], x1[i], D == 3 ? x2[i] : 0.0};
-    int c[3] = {0, 0, 0};
+                          int32_t* __restrict__ count, const int* __restrict__ any) {
+  if (!any[0]) return;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
+    const int si = inst[i];
+    int k;
+    if (!rb[si]) {
+      k = skey[i];
+    } else {
+      const EnsInst& I = T[si];
+      const double xs[3] = {x0[i], x1[i], D == 3 ? x2[i] : 0.0};
+      int c[3] = {0, 0, 0};
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      double f = floor((xs[d] - I.origin[d]) * I.csinv);
-      f = f >= 0.0 ? f : 0.0;  // also NaN -> 0: points outside the frozen grid clamp to its edge cells
-      c[d] = f < (double)(I.nc[d] - 1) ? (int)f : I.nc[d] - 1;
+      for (int d = 0; d < D; ++d) {
+        double f = floor((xs[d] - I.origin[d]) * I.csinv);
+        f = f >= 0.0 ? f : 0.0;  // also NaN -> 0: points outside the frozen grid clamp to its edge cells
+        c[d] = f < (double)(I.nc[d] - 1) ? (int)f : I.nc[d] - 1;
+      }
+      k = I.key_off + c[0] + I.nc[0] * (c[1] + I.nc[1] * c[2]);
     }
-    k = I.key_off + c[0] + I.nc[0] * (c[1] + I.nc[1] * c[2]);
+    key[i] = k;
+    slot[i] = atomicAdd(&count[k], 1);
   }
-  key[i] = k;
-  slot[i] = atomicAdd(&count[k], 1);
 }
 
+// the arrival lists; the counts, scanned by now, are zeroed for the next binning
 __global__ void k_ens_scatter(int64_t N, const int32_t* __restrict__ key, const int32_t* __restrict__ slot,
-                              const int32_t* __restrict__ cellstart, int32_t* __restrict__ tmp) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  tmp[cellstart[key[i]] + slot[i]] = (int32_t)i;
+                              const int32_t* __restrict__ cellstart, int32_t* __restrict__ tmp, int64_t K,
+                              int32_t* __restrict__ count, const int* __restrict__ any) {
+  if (!any[0]) return;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = t0; i < N; i += stride) tmp[cellstart[key[i]] + slot[i]] = (int32_t)i;
+  for (int64_t c = t0; c < K; c += stride) count[c] = 0;
 }
 
 // rank inside the cell by instance-local id (ids are unique inside an instance)
 __global__ void k_ens_rank(int64_t N, const int32_t* __restrict__ tmp, const int32_t* __restrict__ key,
                            const int32_t* __restrict__ cellstart, const int32_t* __restrict__ id,
-                           int32_t* __restrict__ perm) {
-  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= N) return;
-  const int32_t i = tmp[q];
-  const int32_t c = key[i];
-  const int32_t s = cellstart[c], e = cellstart[c + 1];
-  const int32_t oi = id[i];
-  int32_t r = 0;
-  for (int32_t t = s; t < e; ++t) r += id[tmp[t]] < oi;
-  perm[s + r] = i;
+                           int32_t* __restrict__ perm, const int* __restrict__ any) {
+  if (!any[0]) return;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += stride) {
+    const int32_t i = tmp[q];
+    const int32_t c = key[i];
+    const int32_t s = cellstart[c], e = cellstart[c + 1];
+    const int32_t oi = id[i];
+    int32_t r = 0;
+    for (int32_t t = s; t < e; ++t) r += id[tmp[t]] < oi;
+    perm[s + r] = i;
+  }
 }
 
 struct EnsState {
@@ -334,44 +349,72 @@ struct EnsState {
   int32_t* id;
 };
 
-// new[k] = old[perm[k]]; FP32 offsets from the new cell's corner
+// out[k] = in[perm[k]] for the whole state, and the sorted keys
 template <int D>
-__global__ void k_ens_permute(int64_t N, const int32_t* __restrict__ perm, const int32_t* __restrict__ key,
-                              const int32_t* __restrict__ inst, const EnsInst* __restrict__ T, EnsState in,
-                              EnsState out, int32_t* __restrict__ skey, float* __restrict__ o0,
-                              float* __restrict__ o1, float* __restrict__ o2, float4* __restrict__ r1,
-                              const int* __restrict__ rb, float* __restrict__ b0, float* __restrict__ b1,
-                              float* __restrict__ b2) {
+__global__ void k_ens_move(int64_t N, const int32_t* __restrict__ perm, const int32_t* __restrict__ key, EnsState in,
+                           EnsState out, int32_t* __restrict__ skey, const int* __restrict__ any) {
+  if (!any[0]) return;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < N; k += stride) {
+    const int32_t i = perm[k];
+    skey[k] = key[i];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      out.x[d][k] = in.x[d][i];
+      out.v[d][k] = in.v[d][i];
+      out.dxb[d][k] = in.dxb[d][i];
+      out.dvb[d][k] = in.dvb[d][i];
+    }
+    out.dr[k] = in.dr[i];
+    out.drb[k] = in.drb[i];
+    out.pt[k] = in.pt[i];
+    out.id[k] = in.id[i];
+  }
+}
+
+// The step's start: FP32 offsets from each particle's cell corner and the
+// stage-1 records; after a binning also the moved state back from `moved`
+// (so the state stays in one set of buffers, whether or not a step re-sorts)
+// and a rebuilding instance's build offsets.
+template <int D>
+__global__ void k_ens_start(int64_t N, const int32_t* __restrict__ skey, const int32_t* __restrict__ inst,
+                            const EnsInst* __restrict__ T, EnsState st, EnsState moved, float* __restrict__ o0,
+                            float* __restrict__ o1, float* __restrict__ o2, float4* __restrict__ r1,
+                            const int* __restrict__ rb, float* __restrict__ b0, float* __restrict__ b1,
+                            float* __restrict__ b2, const int* __restrict__ any) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
-  const int32_t i = perm[k];
-  const int32_t kk = key[i];
-  skey[k] = kk;
-  const bool reb = rb[inst[k]] != 0;
-  const EnsInst& I = T[inst[k]];
+  const int si = inst[k];
+  const EnsInst& I = T[si];
+  const bool re = any[0] != 0;
+  const bool reb = re && rb[si] != 0;
   int c0, c1, c2;
-  cell_of(kk, I, c0, c1, c2);
+  cell_of(skey[k], I, c0, c1, c2);
   float ov[D], vv[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    const double xv = in.x[d][i];
-    out.x[d][k] = xv;
-    vv[d] = in.v[d][i];
-    out.v[d][k] = vv[d];
-    out.dxb[d][k] = in.dxb[d][i];
-    out.dvb[d][k] = in.dvb[d][i];
+    const double xv = re ? moved.x[d][k] : st.x[d][k];
+    vv[d] = re ? moved.v[d][k] : st.v[d][k];
+    if (re) {
+      st.x[d][k] = xv;
+      st.v[d][k] = vv[d];
+      st.dxb[d][k] = moved.dxb[d][k];
+      st.dvb[d][k] = moved.dvb[d][k];
+    }
     const int cd = d == 0 ? c0 : (d == 1 ? c1 : c2);
     float* o = d == 0 ? o0 : (d == 1 ? o1 : o2);
     ov[d] = (float)(xv - (I.origin[d] + (double)cd * I.cs));
     o[k] = ov[d];
     if (reb) (d == 0 ? b0 : (d == 1 ? b1 : b2))[k] = ov[d];
   }
-  const float dr = in.dr[i];
-  const int pt = in.pt[i];
-  out.dr[k] = dr;
-  out.drb[k] = in.drb[i];
-  out.pt[k] = pt;
-  out.id[k] = in.id[i];
+  const float dr = re ? moved.dr[k] : st.dr[k];
+  const int pt = re ? moved.pt[k] : st.pt[k];
+  if (re) {
+    st.dr[k] = dr;
+    st.drb[k] = moved.drb[k];
+    st.pt[k] = pt;
+    st.id[k] = moved.id[k];
+  }
   put_r1<D>(r1, k, ov, vv, dr, pt, D == 2 ? eos32(dr, pt, I) : 0.f);
 }
 
@@ -437,7 +480,7 @@ __device__ __forceinline__ void nl_close(const EnsArr& A, int64_t i, int lane, i
 // L lanes share a particle: candidates go in chunks of L
 template <int D, int L>
 __global__ void __launch_bounds__(ENS_MAX_TPB) k_ens_nlist(EnsArr A, const EnsInst* __restrict__ T) {
-  if (*A.ovf) return;
+  if (!A.any[0] || *A.ovf) return;
   const unsigned lanew = threadIdx.x & 31u;
   const unsigned gbase = lanew & ~(unsigned)(L - 1);
   const unsigned gm = L == 32 ? 0xffffffffu : (((1u << L) - 1u) << gbase);
@@ -638,7 +681,7 @@ template <int D, int L, int DEPTH>
 __global__ void __launch_bounds__(TILE_TPB) k_ens_nlist_tile(EnsArr A, const EnsInst* __restrict__ T,
                                                              const int* __restrict__ tile_off, int ninst, int cpb,
                                                              int cap) {
-  if (*A.ovf) return;
+  if (!A.any[0] || *A.ovf) return;
   extern __shared__ float4 tile_smem[];
   float* const sbuf = reinterpret_cast<float*>(tile_smem);
   __shared__ TileSm G[DEPTH];
@@ -714,6 +757,114 @@ __device__ __forceinline__ float lane_total(const KSum& k, unsigned gm) {
   return s - c;
 }
 
+// A particle's walk over its list.  FLUID: both sums; else (a real wall
+// particle, ptype 1) ∂ρ/∂t alone -- its acceleration moves nothing and is no
+// output of the engine.
+template <int D, int STAGE, bool RM, bool FLUID>
+__device__ __forceinline__ void stage_row(const EnsArr& A, const EnsInst& I, int64_t i, int lane, const float* oi,
+                                          const float* ohi, const float* vi, float dri, float rhoi, float irhoi,
+                                          float Pi, KSum& drho, KSum2& accxy, KSum& accz, float& rm2) {
+  constexpr int L = stage_lanes<D>();
+  const int nn = A.nlc[i];
+  // the next entry is loaded one iteration ahead: the list streams from
+  // DRAM, and its latency then overlaps the current neighbour's arithmetic
+  int nxt = lane < nn ? A.nl[(int64_t)lane * A.ncap + i] : 0;
+  for (int e = lane; e < nn; e += L) {
+    const int ent = nxt;
+    if (e + L < nn) nxt = A.nl[(int64_t)(e + L) * A.ncap + i];
+    const Rec<D, STAGE> rec = load_rec<D, STAGE>(A.r1, A.r2, I.p_off + ent_index(ent));
+    float sh[D];
+    ent_shift<D>(ent, sh);
+    // the neighbour's record: offsets (at x, and at xΔt½ in stage 2), velocity, δρ, ptype
+    float oj[D], hj[D], vj[D], drj, Prec = 0.f;
+    int ptj;
+    decode_rec<D, STAGE>(rec, oj, hj, vj, drj, ptj, Prec);
+    const float4 kA = I.kA;  // H², 1/H, dwc, cell edge
+    float d[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) d[q] = fmaf(-sh[q], kA.w, oi[q] - oj[q]);
+    const float r2 = dot32<D>(d, d);
+    if (STAGE == 1 && RM) rm2 = fminf(rm2, r2);
+    if (!(r2 < kA.x)) continue;  // in the list's skin: not a pair of this step
+    if (!FLUID && !(ptj > 0)) continue;
+    // sph∇W!: W'(r)/r of WendlandC2 = -20 nDW Hinv (1-q)^3.  Reciprocals and
+    // roots here are the approximate intrinsics (within 2 ulp each), far
+    // inside the FP32 path's error against FP64.
+    const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
+    const float u = r * kA.y;
+    const float t = u < 1.f ? 1.f - u : 0.f;
+    const float dwr = kA.z * (t * t * t);
+    float gw[D], dd[D], dv[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+      gw[q] = d[q] * dwr;
+      dd[q] = STAGE == 1 ? d[q] : fmaf(-sh[q], kA.w, ohi[q] - hj[q]);
+      dv[q] = vi[q] - vj[q];
+    }
+    const float4 kB = I.kB;  // ρ₀, η², m₀, DDTgz
+    if (!FLUID) {
+      drho.add(kB.z * dot32<D>(dv, gw));
+      continue;
+    }
+    // gsc: the factor of ∇W of ∂v∂t! and ∂v∂t_av! together; f: the
+    // viscous, surface-tension and boundary terms
+    float gsc = 0.f, f[D];
+#pragma unroll
+    for (int q = 0; q < D; ++q) f[q] = 0.f;
+    if (ptj > 0) {
+      const float r2d = STAGE == 1 ? r2 : dot32<D>(dd, dd);
+      const float rhoj = kB.x + drj;
+      const float irhoj = __fdividef(1.f, rhoj);
+      const float inv = __fdividef(1.f, r2d + kB.y);
+      // ∂v∂t!
+      float Pj = Prec;
+      if (!rec_has_p<D, STAGE>()) Pj = eos32(drj, ptj, I);
+      gsc = -kB.z * (Pi + Pj) * (irhoi * irhoj);
+      const float4 kC = I.kC;  // kddt, kav, kvisc
+      const float ddgw = dot32<D>(dd, gw);
+      // ∂ρ∂tDDT!
+      float term = kB.z * dot32<D>(dv, gw);
+      const float dp = kB.x * root_m1g(kB.w * dd[1], I.kE, I.gamma);
+      term += kC.x * ((drj - dri) - dp) * inv * (-ddgw) * irhoj;
+      drho.add(term);
+      const float cond = dot32<D>(dv, dd);
+      if (cond < 0.f || I.use_visc) {
+        const float ii = __fdividef(1.f, rhoi + rhoj) * inv;
+        // ∂v∂t_av!: -Π m₀ = 2 α c₀ h m₀ (Δv·Δx) / ((r² + η²)(ρi + ρj))
+        if (cond < 0.f) gsc += kC.y * cond * ii;
+        if (I.use_visc) {
+          // ∂v∂t_visc!
+          const float nt = kC.z * ddgw * ii;
+#pragma unroll
+          for (int q = 0; q < D; ++q) f[q] = nt * dv[q];
+        }
+      }
+      if (I.use_pF) {
+        // ∂v∂tpF! (in stage 1 the separation is r itself)
+        const float4 kD = I.kD;  // pfcr, hp1, 2h, kpf
+        const float rd = STAGE == 1 ? r : (r2d > 0.f ? r2d * rsqrtf(r2d) : 0.f);
+        if (rd < kD.z) {
+          const float scos = kD.w * __cosf(kD.x * rd) * __fdividef(1.f, rd + kD.y);  // argument in [0, 1.5π)
+#pragma unroll
+          for (int q = 0; q < D; ++q) f[q] = fmaf(scos, dd[q], f[q]);
+        }
+      }
+    } else {
+      const float4 kF = I.kFB[STAGE - 1];  // fb_d, fb_r0, fb_eta2
+      if (r < kF.y) {
+        // fbmolforce! at x
+        const float qq = kF.y * __fdividef(1.f, r + kF.z);
+        const float q2 = qq * qq, q4 = q2 * q2, q8 = q4 * q4;
+        const float Fc = kF.x * (q8 * q4 - q4) * __fdividef(1.f, r2 + kF.z);
+#pragma unroll
+        for (int q = 0; q < D; ++q) f[q] += d[q] * Fc;
+      }
+    }
+    accxy.add(make_float2(fmaf(gsc, gw[0], f[0]), fmaf(gsc, gw[1], f[1])));
+    if (D == 3) accz.add(fmaf(gsc, gw[D - 1], f[D - 1]));
+  }
+}
+
 // two blocks of 512 per SM: at most 64 registers.  RM (stage 1): keep each
 // row's smallest r² for dpcreg!'s row bound (a separate instantiation, so the
 // ensembles without dpcreg! run the loop without it)
@@ -740,110 +891,17 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const En
     const float rhoi = I.rho0 + dri;
     const float irhoi = __fdividef(1.f, rhoi);
     const float Pi = eos32(dri, pti, I);
-    const int fbs = STAGE - 1;
     KSum drho;
     KSum2 accxy;  // the x and y components of the acceleration, packed
     KSum accz;
     float rm2 = INFINITY;  // stage 1: the row's smallest r² (dpcreg!'s row bound)
-    const int nn = A.nlc[i];
-    // the next entry is loaded one iteration ahead: the list streams from
-    // DRAM, and its latency then overlaps the current neighbour's arithmetic
-    int nxt = lane < nn ? A.nl[(int64_t)lane * A.ncap + i] : 0;
-    for (int e = lane; e < nn; e += L) {
-      const int ent = nxt;
-      if (e + L < nn) nxt = A.nl[(int64_t)(e + L) * A.ncap + i];
-      const Rec<D, STAGE> rec = load_rec<D, STAGE>(A.r1, A.r2, I.p_off + ent_index(ent));
-      float sh[D];
-      ent_shift<D>(ent, sh);
-      // the neighbour's record: offsets (at x, and at xΔt½ in stage 2), velocity, δρ, ptype
-      float oj[D], hj[D], vj[D], drj, Prec = 0.f;
-      int ptj;
-      decode_rec<D, STAGE>(rec, oj, hj, vj, drj, ptj, Prec);
-      const float4 kA = I.kA;  // H², 1/H, dwc, cell edge
-      float d[D];
-#pragma unroll
-      for (int q = 0; q < D; ++q) d[q] = fmaf(-sh[q], kA.w, oi[q] - oj[q]);
-      const float r2 = dot32<D>(d, d);
-      if (STAGE == 1 && RM) rm2 = fminf(rm2, r2);
-      if (!(r2 < kA.x)) continue;  // in the list's skin: not a pair of this step
-      // sph∇W!: W'(r)/r of WendlandC2 = -20 nDW Hinv (1-q)^3.  Reciprocals and
-      // roots here are the approximate intrinsics (within 2 ulp each), far
-      // inside the FP32 path's error against FP64.
-      const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
-      const float u = r * kA.y;
-      const float t = u < 1.f ? 1.f - u : 0.f;
-      const float dwr = kA.z * (t * t * t);
-      float gw[D], dd[D], dv[D];
-#pragma unroll
-      for (int q = 0; q < D; ++q) {
-        gw[q] = d[q] * dwr;
-        dd[q] = STAGE == 1 ? d[q] : fmaf(-sh[q], kA.w, ohi[q] - hj[q]);
-        dv[q] = vi[q] - vj[q];
-      }
-      const float4 kB = I.kB;  // ρ₀, η², m₀, DDTgz
-      const float r2d = STAGE == 1 ? r2 : dot32<D>(dd, dd);
-      const float rhoj = kB.x + drj;
-      const float irhoj = __fdividef(1.f, rhoj);
-      const bool both = pti > 0 && ptj > 0;
-      const float inv = __fdividef(1.f, r2d + kB.y);
-      // gsc: the factor of ∇W of ∂v∂t! and ∂v∂t_av! together; f: the
-      // viscous, surface-tension and boundary terms
-      float gsc = 0.f, f[D];
-#pragma unroll
-      for (int q = 0; q < D; ++q) f[q] = 0.f;
-      if (pti * ptj > 0) {
-        // ∂v∂t!
-        float Pj = Prec;
-        if (!rec_has_p<D, STAGE>()) Pj = eos32(drj, ptj, I);
-        gsc = -kB.z * (Pi + Pj) * (irhoi * irhoj);
-      }
-      if (both) {
-        const float4 kC = I.kC;  // kddt, kav, kvisc
-        const float ddgw = dot32<D>(dd, gw);
-        // ∂ρ∂tDDT!
-        float term = kB.z * dot32<D>(dv, gw);
-        if (pti > 1) {
-          const float dp = kB.x * root_m1g(kB.w * dd[1], I.kE, I.gamma);
-          term += kC.x * ((drj - dri) - dp) * inv * (-ddgw) * irhoj;
-        }
-        drho.add(term);
-        const float cond = dot32<D>(dv, dd);
-        if (cond < 0.f || I.use_visc) {
-          const float ii = __fdividef(1.f, rhoi + rhoj) * inv;
-          // ∂v∂t_av!: -Π m₀ = 2 α c₀ h m₀ (Δv·Δx) / ((r² + η²)(ρi + ρj))
-          if (cond < 0.f) gsc += kC.y * cond * ii;
-          if (I.use_visc) {
-            // ∂v∂t_visc!
-            const float nt = kC.z * ddgw * ii;
-#pragma unroll
-            for (int q = 0; q < D; ++q) f[q] = nt * dv[q];
-          }
-        }
-        if (I.use_pF) {
-          // ∂v∂tpF! (in stage 1 the separation is r itself)
-          const float4 kD = I.kD;  // pfcr, hp1, 2h, kpf
-          const float rd = STAGE == 1 ? r : (r2d > 0.f ? r2d * rsqrtf(r2d) : 0.f);
-          if (rd < kD.z) {
-            const float scos = kD.w * __cosf(kD.x * rd) * __fdividef(1.f, rd + kD.y);  // argument in [0, 1.5π)
-#pragma unroll
-            for (int q = 0; q < D; ++q) f[q] = fmaf(scos, dd[q], f[q]);
-          }
-        }
-      }
-      if ((pti > 0) != (ptj > 0)) {
-        const float4 kF = I.kFB[fbs];  // fb_d, fb_r0, fb_eta2
-        if (r < kF.y) {
-          // fbmolforce! at x
-          const float qq = kF.y * __fdividef(1.f, r + kF.z);
-          const float q2 = qq * qq, q4 = q2 * q2, q8 = q4 * q4;
-          const float Fc = kF.x * (q8 * q4 - q4) * __fdividef(1.f, r2 + kF.z);
-#pragma unroll
-          for (int q = 0; q < D; ++q) f[q] += d[q] * Fc;
-        }
-      }
-      accxy.add(make_float2(fmaf(gsc, gw[0], f[0]), fmaf(gsc, gw[1], f[1])));
-      if (D == 3) accz.add(fmaf(gsc, gw[D - 1], f[D - 1]));
-    }
+    // What a row's sums feed decides what its entries run: a fluid particle
+    // both, a real wall particle ∂ρ/∂t, any other wall particle neither (390k
+    // particles in 3-D, two thirds of them walls, stage 1 357 -> 276 us)
+    if (pti > 1)
+      stage_row<D, STAGE, RM, true>(A, I, i, lane, oi, ohi, vi, dri, rhoi, irhoi, Pi, drho, accxy, accz, rm2);
+    else if (pti > 0)
+      stage_row<D, STAGE, RM, false>(A, I, i, lane, oi, ohi, vi, dri, rhoi, irhoi, Pi, drho, accxy, accz, rm2);
     KSum acc[D];
     acc[0] = accxy.part(0);
     acc[1] = accxy.part(1);
@@ -1088,7 +1146,7 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 3) k_ens_xsph(EnsArr A, const Ens
 template <int D>
 __global__ void __launch_bounds__(ENS_MAX_TPB) k_ens_cspm(EnsArr A, const EnsInst* __restrict__ T,
                                                           const int32_t* __restrict__ istep) {
-  if (*A.ovf) return;
+  if (!A.any[1] || *A.ovf) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.N; i += stride) {
     const int s = A.inst[i];
@@ -1135,12 +1193,13 @@ __global__ void __launch_bounds__(ENS_MAX_TPB) k_ens_cspm(EnsArr A, const EnsIns
 
 __global__ void k_ens_cspm_apply(int64_t N, const int32_t* __restrict__ inst, const EnsInst* __restrict__ T,
                                  const int32_t* __restrict__ istep, const float* __restrict__ drh,
-                                 float* __restrict__ dr, const int* __restrict__ ovf) {
-  if (*ovf) return;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const int s = inst[i];
-  if (cspm_due(T[s], istep, s)) dr[i] = drh[i];
+                                 float* __restrict__ dr, const int* __restrict__ ovf, const int* __restrict__ any) {
+  if (!any[1] || *ovf) return;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
+    const int s = inst[i];
+    if (cspm_due(T[s], istep, s)) dr[i] = drh[i];
+  }
 }
 
 // the largest squared displacement since the last list build, per instance
@@ -1187,20 +1246,33 @@ __global__ void k_ens_disp(EnsArr A, const EnsInst* __restrict__ T, unsigned* __
 }
 
 // one more step done, per instance, and for the call; whether the instance
-// rebuilds its list at the next step (always without a skin)
-__global__ void k_ens_tick(int ninst, int32_t* __restrict__ istep, const int* __restrict__ ovf,
-                           int* __restrict__ done, const EnsInst* __restrict__ T, int* __restrict__ rb,
-                           int* __restrict__ nreb, unsigned* __restrict__ dmax, unsigned* __restrict__ sdmax) {
+// rebuilds its list at the next step (always without a skin), and whether any
+// does or has a cspmcorr! due.  One block.
+constexpr int TICK_TPB = 512;
+__global__ void __launch_bounds__(TICK_TPB) k_ens_tick(int ninst, int32_t* __restrict__ istep,
+                                                       const int* __restrict__ ovf, int* __restrict__ done,
+                                                       const EnsInst* __restrict__ T, int* __restrict__ rb,
+                                                       int* __restrict__ nreb, unsigned* __restrict__ dmax,
+                                                       unsigned* __restrict__ sdmax, int* __restrict__ any) {
   if (*ovf) return;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < ninst) {
+  int reb = 0, due = 0;
+  for (int s = threadIdx.x; s < ninst; s += TICK_TPB) {
     istep[s] += 1;
     if (rb[s]) nreb[s] += 1;
-    rb[s] = T[s].reuse ? (__uint_as_float(dmax[s]) > T[s].dthr2 ? 1 : 0) : 1;
+    const int r = T[s].reuse ? (__uint_as_float(dmax[s]) > T[s].dthr2 ? 1 : 0) : 1;
+    rb[s] = r;
+    reb |= r;
+    due |= cspm_due(T[s], istep, s) ? 1 : 0;
     dmax[s] = 0u;
     sdmax[s] = 0u;
   }
-  if (s == 0) *done += 1;
+  reb = __syncthreads_or(reb);
+  due = __syncthreads_or(due);
+  if (threadIdx.x == 0) {
+    *done += 1;
+    any[0] = reb != 0;
+    any[1] = due != 0;
+  }
 }
 
 // gather one instance's field into its original particle order
@@ -1326,6 +1398,7 @@ struct gcsph_ens {
   DevBuf R3, R4;         // packed neighbour records of the correction passes
   DevBuf OB[3];          // offsets at each instance's last list build
   DevBuf RB, NREB, DMAX; // per instance: rebuild at the next step, list builds, largest displacement²
+  DevBuf ANY;            // some instance rebuilds / has a cspmcorr! due at the next step
   DevBuf SDMAX;          // per instance: largest |Δx|² of the step (dpcreg!'s row bound)
   DevBuf RMIN;           // per particle: smallest r² of the row at the step's start (dpcreg!'s row bound)
   bool dpc_bound = true; // dpcreg! skips the rows the bound clears (the results are the same)
@@ -1422,6 +1495,7 @@ EnsArr ens_arr(gcsph_ens* e) {
   A.r2 = e->R2.as<float4>();
   A.pt = e->PT[e->cur].as<int32_t>();
   A.rb = e->RB.as<int>();
+  A.any = e->ANY.as<int>();
   A.r3 = e->any_dpc ? e->R3.as<float4>() : nullptr;
   A.r4 = (e->any_dpc || e->any_xsph || e->any_cspm) ? e->R4.as<float4>() : nullptr;
   A.istep = e->ISTEP.as<int32_t>();
@@ -1594,6 +1668,11 @@ int ens_relayout(gcsph_ens* e) {
   }
   int rc;
   if ((rc = ens_reserve_cells(e, k))) return rc;
+  // the counts are zero at rest; both flags stand until a step's end says
+  // otherwise (memset to bytes of 1: any nonzero value)
+  if (k > 0) GC_CUDA(cudaMemsetAsync(e->COUNT.p, 0, sizeof(int32_t) * k, e->st));
+  if ((rc = e->ANY.ensure(sizeof(int) * 2, e->st))) return rc;
+  GC_CUDA(cudaMemsetAsync(e->ANY.p, 0x01, sizeof(int) * 2, e->st));
   std::vector<EnsInst> tab(e->inst.size());
   for (size_t s = 0; s < e->inst.size(); ++s) tab[s] = e->inst[s].dev;
   if ((rc = e->TAB.ensure(sizeof(EnsInst) * std::max<size_t>(tab.size(), 1), e->st))) return rc;
@@ -1732,33 +1811,33 @@ template <int D>
 int ens_enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
   const int64_t N = e->N;
   const EnsInst* T = e->TAB.as<EnsInst>();
-  GC_CUDA(cudaMemsetAsync(e->COUNT.p, 0, sizeof(int32_t) * e->K, st));
+  const int* any = e->ANY.as<int>();
   const double* x2 = D == 3 ? e->X[e->cur][2].as<double>() : e->X[e->cur][0].as<double>();
-  k_ens_key<D><<<nblocks(N, 256), 256, 0, st>>>(N, e->INST.as<int32_t>(), e->X[e->cur][0].as<double>(),
-                                                 e->X[e->cur][1].as<double>(), x2, T, e->RB.as<int>(),
-                                                 e->SKEY.as<int32_t>(), e->KEY.as<int32_t>(),
-                                                 e->SLOT.as<int32_t>(), e->COUNT.as<int32_t>());
+  const int bg = bin_grid(N);
+  k_ens_key<D><<<bg, BIN_TPB, 0, st>>>(N, e->INST.as<int32_t>(), e->X[e->cur][0].as<double>(),
+                                       e->X[e->cur][1].as<double>(), x2, T, e->RB.as<int>(), e->SKEY.as<int32_t>(),
+                                       e->KEY.as<int32_t>(), e->SLOT.as<int32_t>(), e->COUNT.as<int32_t>(), any);
   GC_LAUNCHED();
   int rc = exclusive_scan_i32_to_i32(e->COUNT.as<int32_t>(), e->CELLSTART.as<int32_t>(), e->K,
-                                     e->SCRATCH.as<int64_t>(), st);
+                                     e->SCRATCH.as<int64_t>(), st, any);
   if (rc) return rc;
-  k_ens_scatter<<<nblocks(N, 256), 256, 0, st>>>(N, e->KEY.as<int32_t>(), e->SLOT.as<int32_t>(),
-                                                 e->CELLSTART.as<int32_t>(), e->TMP.as<int32_t>());
+  k_ens_scatter<<<bg, BIN_TPB, 0, st>>>(N, e->KEY.as<int32_t>(), e->SLOT.as<int32_t>(), e->CELLSTART.as<int32_t>(),
+                                        e->TMP.as<int32_t>(), e->K, e->COUNT.as<int32_t>(), any);
   GC_LAUNCHED();
-  k_ens_rank<<<nblocks(N, 256), 256, 0, st>>>(N, e->TMP.as<int32_t>(), e->KEY.as<int32_t>(),
-                                              e->CELLSTART.as<int32_t>(), e->ID[e->cur].as<int32_t>(),
-                                              e->PERM.as<int32_t>());
+  k_ens_rank<<<bg, BIN_TPB, 0, st>>>(N, e->TMP.as<int32_t>(), e->KEY.as<int32_t>(), e->CELLSTART.as<int32_t>(),
+                                     e->ID[e->cur].as<int32_t>(), e->PERM.as<int32_t>(), any);
+  GC_LAUNCHED();
+  k_ens_move<D><<<bg, BIN_TPB, 0, st>>>(N, e->PERM.as<int32_t>(), e->KEY.as<int32_t>(), ens_state(e, e->cur),
+                                        ens_state(e, e->cur ^ 1), e->SKEY.as<int32_t>(), any);
   GC_LAUNCHED();
   float* o2 = D == 3 ? e->OFF[2].as<float>() : e->OFF[0].as<float>();
-  k_ens_permute<D><<<nblocks(N, 256), 256, 0, st>>>(N, e->PERM.as<int32_t>(), e->KEY.as<int32_t>(),
-                                                     e->INST.as<int32_t>(), T, ens_state(e, e->cur),
-                                                     ens_state(e, e->cur ^ 1), e->SKEY.as<int32_t>(),
-                                                     e->OFF[0].as<float>(), e->OFF[1].as<float>(), o2,
-                                                     e->R1.as<float4>(), e->RB.as<int>(), e->OB[0].as<float>(),
-                                                     e->OB[1].as<float>(),
-                                                     D == 3 ? e->OB[2].as<float>() : e->OB[0].as<float>());
+  k_ens_start<D><<<nblocks(N, 256), 256, 0, st>>>(N, e->SKEY.as<int32_t>(), e->INST.as<int32_t>(), T,
+                                                   ens_state(e, e->cur), ens_state(e, e->cur ^ 1),
+                                                   e->OFF[0].as<float>(), e->OFF[1].as<float>(), o2,
+                                                   e->R1.as<float4>(), e->RB.as<int>(), e->OB[0].as<float>(),
+                                                   e->OB[1].as<float>(),
+                                                   D == 3 ? e->OB[2].as<float>() : e->OB[0].as<float>(), any);
   GC_LAUNCHED();
-  e->cur ^= 1;
   const int t = tpb_index(tpb);
   const int64_t want = (N + tpb - 1) / tpb;
   const int grid = wave_grid(want, (int64_t)e->sms * e->occ[t]);
@@ -1829,17 +1908,16 @@ int ens_enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
     timer_begin(T_CSPM, st);
     k_ens_cspm<D><<<grid, tpb, 0, st>>>(A, T, e->ISTEP.as<int32_t>());
     GC_LAUNCHED();
-    k_ens_cspm_apply<<<nblocks(N, 256), 256, 0, st>>>(N, e->INST.as<int32_t>(), T, e->ISTEP.as<int32_t>(),
-                                                      e->DRH.as<float>(), e->DR[e->cur].as<float>(), A.ovf);
+    k_ens_cspm_apply<<<bg, BIN_TPB, 0, st>>>(N, e->INST.as<int32_t>(), T, e->ISTEP.as<int32_t>(), e->DRH.as<float>(),
+                                             e->DR[e->cur].as<float>(), A.ovf, any);
     GC_LAUNCHED();
     timer_end(T_CSPM, st);
   }
   k_ens_disp<D, false><<<nblocks(N, 256), 256, 0, st>>>(A, T, e->DMAX.as<unsigned>());
   GC_LAUNCHED();
-  k_ens_tick<<<nblocks(std::max(ninst, 1), 128), 128, 0, st>>>(ninst, e->ISTEP.as<int32_t>(), A.ovf,
-                                                                  A.ovf + 2, T, e->RB.as<int>(),
-                                                                  e->NREB.as<int>(), e->DMAX.as<unsigned>(),
-                                                                  e->SDMAX.as<unsigned>());
+  k_ens_tick<<<1, TICK_TPB, 0, st>>>(ninst, e->ISTEP.as<int32_t>(), A.ovf, A.ovf + 2, T, e->RB.as<int>(),
+                                     e->NREB.as<int>(), e->DMAX.as<unsigned>(), e->SDMAX.as<unsigned>(),
+                                     e->ANY.as<int>());
   GC_LAUNCHED();
   return GCSPH_OK;
 }
@@ -1858,6 +1936,7 @@ int enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
 //      staging depth 1, then the best at depth 2 (10 steps).
 // A phase runs when the call has the steps for it; the rest wait for a later
 // call.  A particle count that moves past 2x of the tuned one starts over.
+// Phases 2 and 3 are for ensembles without a skin, whose every step builds.
 int ens_autotune(gcsph_ens* e, int32_t budget, int32_t* steps_used) {
   *steps_used = 0;
   if (e->tpb_fixed) return GCSPH_OK;
@@ -1895,6 +1974,17 @@ int ens_autotune(gcsph_ens* e, int32_t budget, int32_t* steps_used) {
     e->tpb = pick;
     e->tuned_n = e->N;
     e->tune_phase = 1;
+  }
+  if (e->tune_phase == 1 && !e->nl_fixed && e->skin > 0) {
+    // with a skin most steps build no list, so there is nothing to time: a
+    // thread group per particle, eight lanes in 3-D, in 2-D one, or as many (up
+    // to eight) as fill the GPU (the fastest where every step built: 11.5M
+    // 2-D particles 3.43 ms with one lane, 390k in 3-D 0.91 with eight)
+    e->nl_cpb = 0;
+    e->nl_depth = 1;
+    e->nl_lanes = e->D == 3 ? 8 : 1;
+    while (e->nl_lanes < 8 && e->N * e->nl_lanes < (int64_t)e->sms * 2048) e->nl_lanes *= 2;
+    e->tune_phase = 3;
   }
   if (e->tune_phase == 1 && e->nl_fixed) e->tune_phase = 3;
   if (rc == GCSPH_OK && e->tune_phase == 1 && budget - *steps_used >= 8) {
@@ -1958,7 +2048,6 @@ int ens_run_graph(gcsph_ens* e, int32_t n) {
       if (!c.exec || c.used < g->used) g = &c;
     graph_free(*g);
     if (!e->cap) GC_CUDA(cudaStreamCreateWithFlags(&e->cap, cudaStreamNonBlocking));
-    const int cur0 = e->cur;
     const unsigned long long l0 = gcsph_launch_count();
     GC_CUDA(cudaStreamBeginCapture(e->cap, cudaStreamCaptureModeThreadLocal));
     timer_capture_to(&g->timers);
@@ -1969,8 +2058,6 @@ int ens_run_graph(gcsph_ens* e, int32_t n) {
     cudaError_t ce = cudaStreamEndCapture(e->cap, &graph);
     const unsigned long long l1 = gcsph_launch_count();
     count_launch(-(int)(l1 - l0));
-    const int cur1 = e->cur;
-    e->cur = cur0;
     if (rc == GCSPH_OK && ce != cudaSuccess) rc = cuda_fail(ce, "cudaStreamEndCapture", __FILE__, __LINE__);
     if (rc == GCSPH_OK) {
       ce = cudaGraphInstantiate(&g->exec, graph, 0);
@@ -1992,10 +2079,9 @@ int ens_run_graph(gcsph_ens* e, int32_t n) {
     g->N = e->N;
     g->K = e->K;
     g->gen = e->gen;
-    g->cur = cur0;
+    g->cur = e->cur;
     g->tpb = e->tpb;
     g->launches = (long long)(l1 - l0);
-    (void)cur1;
     e->n_captures += 1;
   }
   g->used = ++e->clock;
@@ -2003,7 +2089,6 @@ int ens_run_graph(gcsph_ens* e, int32_t n) {
   GC_CUDA(cudaStreamSynchronize(e->st));
   count_launch((int)g->launches);
   timer_account(g->timers);
-  if (n & 1) e->cur ^= 1;
   e->n_replays += 1;
   return GCSPH_OK;
 }
@@ -2070,7 +2155,7 @@ void ens_destroy(gcsph_ens* e) {
     e->PT[b].release();
     e->ID[b].release();
   }
-  DevBuf* one[] = {&e->INST, &e->KEY, &e->SLOT, &e->TMP, &e->PERM, &e->SKEY, &e->DRH, &e->COUNT, &e->CELLSTART,
+  DevBuf* one[] = {&e->ANY, &e->INST, &e->KEY, &e->SLOT, &e->TMP, &e->PERM, &e->SKEY, &e->DRH, &e->COUNT, &e->CELLSTART,
                    &e->SCRATCH, &e->TAB, &e->MOVES, &e->OUT, &e->ISTEP, &e->NL, &e->NLC, &e->FLAGS,
                    &e->R1, &e->R2};
   for (DevBuf* b : one) b->release();
@@ -2320,6 +2405,7 @@ int ens_step(gcsph_ens* e, int32_t n) {
   if (e->lists_lost) {
     // no list survived: every instance builds one at its next step
     GC_CUDA(cudaMemsetAsync(e->RB.p, 0x01, sizeof(int32_t) * e->inst.size(), e->st));
+    GC_CUDA(cudaMemsetAsync(e->ANY.p, 0x01, sizeof(int) * 2, e->st));
     e->lists_lost = false;
   }
   int32_t left = n;

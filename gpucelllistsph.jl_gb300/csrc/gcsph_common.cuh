@@ -298,8 +298,9 @@ __device__ void block_exclusive_scan(const int32_t* in, TOut* out, int64_t n) {
 
 int exclusive_scan_i32_to_i64(const int32_t* in, int64_t* out, int64_t n, int64_t* scratch,
                               cudaStream_t s);
+// run (may be null): a device word; where it is zero the scan does nothing
 int exclusive_scan_i32_to_i32(const int32_t* in, int32_t* out, int64_t n, int64_t* scratch,
-                              cudaStream_t s);
+                              cudaStream_t s, const int* run = nullptr);
 // two scans of n items each (one launch when they are small)
 int exclusive_scan2_i32_to_i64(const int32_t* in0, int64_t* out0, const int32_t* in1, int64_t* out1, int64_t n,
                                int64_t* scratch, cudaStream_t s);
