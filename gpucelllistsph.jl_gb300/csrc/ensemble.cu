@@ -757,6 +757,21 @@ __device__ __forceinline__ float lane_total(const KSum& k, unsigned gm) {
   return s - c;
 }
 
+// a particle's instance: from the table, or (an ensemble of one) from the
+// launch's parameters
+template <bool ONE>
+struct EnsOne {
+  EnsInst one;
+  __device__ __forceinline__ const EnsInst& pick(const EnsInst*, const int32_t*, int64_t) const { return one; }
+};
+template <>
+struct EnsOne<false> {
+  int none;
+  __device__ __forceinline__ const EnsInst& pick(const EnsInst* T, const int32_t* inst, int64_t i) const {
+    return T[inst[i]];
+  }
+};
+
 // A particle's walk over its list.  FLUID: both sums; else (a real wall
 // particle, ptype 1) ∂ρ/∂t alone -- its acceleration moves nothing and is no
 // output of the engine.
@@ -868,8 +883,12 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const EnsInst& I, int
 // two blocks of 512 per SM: at most 64 registers.  RM (stage 1): keep each
 // row's smallest r² for dpcreg!'s row bound (a separate instantiation, so the
 // ensembles without dpcreg! run the loop without it)
-template <int D, int STAGE, bool RM = false>
-__global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const EnsInst* __restrict__ T) {
+// ONE: an ensemble of one instance takes its constants from the launch's
+// parameters (constant-bank operands) instead of loading them from the table,
+// 16 bytes at a time, for every entry.
+template <int D, int STAGE, bool RM, bool ONE>
+__global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const EnsInst* __restrict__ T,
+                                                              const __grid_constant__ EnsOne<ONE> one) {
   if (*A.ovf) return;
   constexpr int L = stage_lanes<D>();
   const unsigned lanew = threadIdx.x & 31u;
@@ -878,7 +897,7 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const En
   const int lane = (int)(lanew - gbase);
   const int64_t groups = ((int64_t)gridDim.x * blockDim.x) / L;
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L; i < A.N; i += groups) {
-    const EnsInst& I = T[A.inst[i]];
+    const EnsInst& I = one.pick(T, A.inst, i);
     float oi[D], ohi[D], vi[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -1086,8 +1105,9 @@ __global__ void k_ens_dpc_apply(EnsArr A, const EnsInst* __restrict__ T) {
 // moves x only.  Reads neighbours' v, writes its own x: one pass.  Little
 // arithmetic per neighbour and a record gather each: latency-bound, so three
 // blocks of 512 per SM (at most 42 registers) rather than the stage passes' two
+constexpr int XSPH_U = 2;
 template <int D>
-__global__ void __launch_bounds__(ENS_MAX_TPB, 3) k_ens_xsph(EnsArr A, const EnsInst* __restrict__ T) {
+__global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_xsph(EnsArr A, const EnsInst* __restrict__ T) {
   if (*A.ovf) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.N; i += stride) {
@@ -1102,29 +1122,42 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 3) k_ens_xsph(EnsArr A, const Ens
     const float rhoi = I.rho0 + A.dr[i];
     KSum sum[D];
     const int nn = A.nlc[i];
-    int nxt = nn > 0 ? A.nl[i] : 0;  // entries one iteration ahead (as in the stage passes)
-    for (int e = 0; e < nn; ++e) {
-      const int ent = nxt;
-      if (e + 1 < nn) nxt = A.nl[(int64_t)(e + 1) * A.ncap + i];
-      const int j = I.p_off + ent_index(ent);
-      float oj[D], hj[D], vj[D], drj, pu;
-      int ptj;
-      decode_rec<D, 1>(load_rec<D, 1>(A.r4, nullptr, j), oj, hj, vj, drj, ptj, pu);
-      if (!(ptj > 1)) continue;
-      float sh[D];
-      ent_shift<D>(ent, sh);
-      float d[D];
+    // XSPH_U entries' records in flight at a time (their sums keep the list's
+    // order), and the next entries loaded ahead of them
+    const int* np = A.nl + i;
+    int nxt[XSPH_U];
 #pragma unroll
-      for (int q = 0; q < D; ++q) d[q] = fmaf(-sh[q], I.csf, oi[q] - oj[q]);
-      const float r2 = dot32<D>(d, d);
-      if (!(r2 < I.H2)) continue;  // in the list's skin
-      const float u = sqrt_fast(r2) * I.Hinv;
-      const float t = u < 1.f ? 1.f - u : 0.f;
-      const float t2 = t * t;
-      const float w = (1.f + 4.f * u) * (t2 * t2) * I.nW;
-      const float xs = I.xsph_c * w * __fdividef(1.f, rhoi + (I.rho0 + drj));
+    for (int j = 0; j < XSPH_U; ++j) nxt[j] = j < nn ? np[(int64_t)j * A.ncap] : 0;
+    for (int e = 0; e < nn; e += XSPH_U) {
+      Rec<D, 1> rec[XSPH_U];
+      float sh[XSPH_U][D];
 #pragma unroll
-      for (int q = 0; q < D; ++q) sum[q].add((vj[q] - vi[q]) * xs);
+      for (int j = 0; j < XSPH_U; ++j) {
+        rec[j] = load_rec<D, 1>(A.r4, nullptr, I.p_off + ent_index(nxt[j]));
+        ent_shift<D>(nxt[j], sh[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < XSPH_U; ++j)
+        nxt[j] = e + XSPH_U + j < nn ? np[(int64_t)(e + XSPH_U + j) * A.ncap] : 0;
+#pragma unroll
+      for (int j = 0; j < XSPH_U; ++j) {
+        float oj[D], hj[D], vj[D], drj, pu;
+        int ptj;
+        decode_rec<D, 1>(rec[j], oj, hj, vj, drj, ptj, pu);
+        if (e + j >= nn || !(ptj > 1)) continue;
+        float d[D];
+#pragma unroll
+        for (int q = 0; q < D; ++q) d[q] = fmaf(-sh[j][q], I.csf, oi[q] - oj[q]);
+        const float r2 = dot32<D>(d, d);
+        if (!(r2 < I.H2)) continue;  // in the list's skin
+        const float u = sqrt_fast(r2) * I.Hinv;
+        const float t = u < 1.f ? 1.f - u : 0.f;
+        const float t2 = t * t;
+        const float w = (1.f + 4.f * u) * (t2 * t2) * I.nW;
+        const float xs = I.xsph_c * w * __fdividef(1.f, rhoi + (I.rho0 + drj));
+#pragma unroll
+        for (int q = 0; q < D; ++q) sum[q].add((vj[q] - vi[q]) * xs);
+      }
     }
 #pragma unroll
     for (int q = 0; q < D; ++q) {
@@ -1760,9 +1793,9 @@ int ens_occupancy(gcsph_ens* e) {
   for (int t = 0; t < 3; ++t) {
     int b = 0;
     if (e->D == 2)
-      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_ens_stage<2, 2>, kTpbs[t], 0));
+      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (k_ens_stage<2, 2, false, false>), kTpbs[t], 0));
     else
-      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_ens_stage<3, 2>, kTpbs[t], 0));
+      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (k_ens_stage<3, 2, false, false>), kTpbs[t], 0));
     e->occ[t] = std::max(b, 1);
     int b2 = 0;
     if (e->D == 2)
@@ -1875,14 +1908,25 @@ int ens_enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
   // 3-D dam break's stage passes 8% faster at 0.4 M and 2 M particles)
   const int sgrid = (int)std::max<int64_t>(1, swant);
   timer_begin(T_STAGE1, st);
-  if (A.rmin2)
-    k_ens_stage<D, 1, true><<<sgrid, tpb, 0, st>>>(A, T);
+  const bool one = e->inst.size() == 1;
+  EnsOne<true> o1{};
+  if (one) o1.one = e->inst[0].dev;
+  const EnsOne<false> o0{};
+  if (A.rmin2 && one)
+    k_ens_stage<D, 1, true, true><<<sgrid, tpb, 0, st>>>(A, T, o1);
+  else if (A.rmin2)
+    k_ens_stage<D, 1, true, false><<<sgrid, tpb, 0, st>>>(A, T, o0);
+  else if (one)
+    k_ens_stage<D, 1, false, true><<<sgrid, tpb, 0, st>>>(A, T, o1);
   else
-    k_ens_stage<D, 1, false><<<sgrid, tpb, 0, st>>>(A, T);
+    k_ens_stage<D, 1, false, false><<<sgrid, tpb, 0, st>>>(A, T, o0);
   GC_LAUNCHED();
   timer_end(T_STAGE1, st);
   timer_begin(T_STAGE2, st);
-  k_ens_stage<D, 2><<<sgrid, tpb, 0, st>>>(A, T);
+  if (one)
+    k_ens_stage<D, 2, false, true><<<sgrid, tpb, 0, st>>>(A, T, o1);
+  else
+    k_ens_stage<D, 2, false, false><<<sgrid, tpb, 0, st>>>(A, T, o0);
   GC_LAUNCHED();
   timer_end(T_STAGE2, st);
   const int32_t ninst = (int32_t)e->inst.size();
