@@ -6,8 +6,19 @@
 // pair, FP64 atomics into both particles.  These are the drop-in for users who
 // call the kernels one by one; stepsolve! itself runs the fused gather path in
 // sph_step.cu.
+//
+// What is written per pair or per particle (W, ∇W, P, the updates) keeps the
+// reference's expressions and IEEE divisions and roots, bit for bit.  The
+// terms that go into sums are bound by the FP64 pipe (80 to 87% busy, the
+// atomics well behind), so they take the pair-once forms of the fused step:
+// reciprocals, roots and the cosine by rcp_pair, sqrt_pair and cos_fast,
+// powfancy7th by its series, dot products and products of constants fused.
+// Measured with the queue below (one GB300, 10.5M pairs of a 3-D tank, 179k
+// particles): ∂v∂tpF! 1577 -> 388 us, ∂ρ∂tDDT! 1403 -> 478, sph∑W! 499 -> 310,
+// ∂v∂t_visc! 475 -> 281, fbmolforce! 449 -> 223, ∂v∂t_av! 425 -> 263, ∂v∂t! 231 -> 180,
+// xsphcorr! 179 -> 151.
 #include <math.h>
-#include "gcsph_common.cuh"
+#include "sph_step.cuh"
 
 namespace gcsph {
 
@@ -39,6 +50,7 @@ static int vec_out(int D, double* const* src, W3* out, const char* name) {
   return GCSPH_OK;
 }
 
+// the reference's dot product (no contraction) ...
 template <int D>
 __device__ inline double dotp(const double* a, const double* b) {
   double s = a[0] * b[0];
@@ -47,11 +59,113 @@ __device__ inline double dotp(const double* a, const double* b) {
   return s;
 }
 
+// ... and the fused one of the summed terms
+template <int D>
+__device__ inline double dotf(const double* a, const double* b) {
+  double s = a[0] * b[0];
+#pragma unroll
+  for (int d = 1; d < D; ++d) s = fma(a[d], b[d], s);
+  return s;
+}
+
+// whether x's exponent lies in a range where the corrected approximations
+// hold (2^-900 .. 2^900); zeros, denormals, infinities and NaN take the IEEE
+// operations
+__device__ inline bool mid_range(double x) {
+  return ((unsigned)(dbits(x) >> 32) & 0x7fffffffu) - 0x07b00000u < 0x70800000u;
+}
+__device__ inline double rcp_pair(double x) { return mid_range(x) ? rcp_nr(x) : 1.0 / x; }
+__device__ inline double sqrt_pair(double x) { return mid_range(x) ? sqrt_nr(x) : sqrt(x); }
+
 __device__ inline bool pair_at(const int32_t* pairs, int64_t p, int64_t* i, int64_t* j) {
   int32_t a = pairs[2 * p], b = pairs[2 * p + 1];
   *i = (int64_t)a - 1;
   *j = (int64_t)b - 1;
   return a != 0;
+}
+
+// A summed term over the pair list.  F: take(pt of i, pt of j) says whether a
+// pair has the term, run(p, i, j) adds it.  QUEUE: a warp's FP64 instruction
+// costs the same for one active lane as for 32, and in a tank most lanes hold
+// pairs without the term (walls); each warp collects the pairs of its chunks
+// that have it and runs 32 at a time.  A list of about one chunk a warp has
+// nothing to collect and is run as it comes, and so are the terms that gained
+// nothing.  (10.5M pairs of a 3-D tank, 179k particles of them 50k fluid,
+// without and with the queue: ∂v∂tpF! 504 and 388 us, sph∑W! 384 and 310,
+// ∂v∂t_visc! 345 and 281, fbmolforce! 374 and 223, ∂v∂t_av! 265 and 263, ∂v∂t! 198
+// and 180; ∂ρ∂tDDT! 478 and 485, xsphcorr! 151 and 164.)
+constexpr int PW = PTPB / 32;
+template <class F, bool QUEUE>
+__global__ void __launch_bounds__(PTPB) k_pair_term(int64_t P, const int32_t* __restrict__ pairs, const F f) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if constexpr (!QUEUE) {
+    const int64_t p = (int64_t)blockIdx.x * PTPB + threadIdx.x;
+    if (p >= P) return;
+    const int32_t a = pairs[2 * p], b = pairs[2 * p + 1];
+    if (a > 0 && f.take(f.pt[a - 1], f.pt[b - 1])) f.run(p, (int64_t)a - 1, (int64_t)b - 1);
+    return;
+  }
+  __shared__ int64_t s_q[PW][64];  // at most 31 waiting and 32 new ones
+  int64_t* q = s_q[w];
+  int cnt = 0;
+  const int64_t nchunk = (P + 31) / 32, step = (int64_t)gridDim.x * PW;
+  int64_t ch = (int64_t)blockIdx.x * PW + w;
+  bool more;
+  do {
+    more = ch < nchunk;
+    const int64_t p = ch * 32 + lane;
+    bool on = false;
+    if (p < P) {
+      const int32_t a = pairs[2 * p], b = pairs[2 * p + 1];
+      on = a > 0 && f.take(f.pt[a - 1], f.pt[b - 1]);
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, on);
+    if (on) q[cnt + __popc(bal & ((1u << lane) - 1u))] = p;
+    cnt += __popc(bal);
+    __syncwarp();
+    // a full warp's worth, or after the last chunk what is left (under 32)
+    const int base = cnt >= 32 ? cnt - 32 : (more ? cnt : 0);
+    if (base + lane < cnt) {
+      const int64_t u = q[base + lane];
+      f.run(u, (int64_t)pairs[2 * u] - 1, (int64_t)pairs[2 * u + 1] - 1);
+    }
+    cnt = base;
+    __syncwarp();
+    ch += step;
+  } while (more);
+}
+
+template <class F>
+static int launch_pair_term(int64_t P, const int32_t* pairs, const F& f, cudaStream_t st) {
+  // the queue form's blocks stay resident: as many as fit
+  static int64_t grid = 0;
+  if (grid == 0) {
+    int dev = 0, sms = 0, per = 0;
+    GC_CUDA(cudaGetDevice(&dev));
+    GC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_term<F, true>, PTPB, 0));
+    grid = (int64_t)sms * (per > 0 ? per : 1);
+  }
+  if (!F::QUEUE || P <= 2 * grid * PTPB)
+    k_pair_term<F, false><<<nblocks(P, PTPB), PTPB, 0, st>>>(P, pairs, f);
+  else
+    k_pair_term<F, true><<<(unsigned)grid, PTPB, 0, st>>>(P, pairs, f);
+  GC_LAUNCHED();
+  return GCSPH_OK;
+}
+
+template <int D>
+__device__ inline void pair_dx(const V3& x, int64_t i, int64_t j, double* dx) {
+#pragma unroll
+  for (int d = 0; d < D; ++d) dx[d] = x.p[d][i] - x.p[d][j];
+}
+template <int D>
+__device__ inline void scatter_pm(const W3& a, int64_t i, int64_t j, const double* f) {
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    atomicAdd(&a.p[d][i], f[d]);
+    atomicAdd(&a.p[d][j], -f[d]);
+  }
 }
 
 // kernel_sphW! (:84-100) and kernel_sph∇W! (:196-213)
@@ -76,71 +190,75 @@ __global__ void k_fn_w(int64_t P, const int32_t* __restrict__ pairs, V3 x, doubl
   }
 }
 
-// kernel_sph∑W! (:139-156), kernel_sph∑∇W! (:332-359)
+// kernel_sph∑W! (:139-156), kernel_sph∑∇W! (:332-359).  nn: the norm of 𝒲, or
+// of d𝒲 times -20 H⁻¹ (d𝒲/r = nn (1 - u)^3, u / r = H⁻¹)
 template <int D, int GRAD>
-__global__ void k_fn_sumw(int64_t P, const int32_t* __restrict__ pairs, V3 x, double Hinv, double nn,
-                          const int32_t* __restrict__ pt, double* __restrict__ sumW, W3 sg) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t i, j;
-  if (!pair_at(pairs, p, &i, &j)) return;
-  if ((pt[i] > 0) != (pt[j] > 0)) return;
-  double dx[D];
+struct TermSumW {
+  static constexpr bool QUEUE = true;
+  V3 x;
+  double Hinv, nn;
+  const int32_t* pt;
+  double* sumW;
+  W3 sg;
+  __device__ bool take(int pi, int pj) const { return (pi > 0) == (pj > 0); }
+  __device__ void run(int64_t, int64_t i, int64_t j) const {
+    double dx[D];
+    pair_dx<D>(x, i, j, dx);
+    const double r2 = dotf<D>(dx, dx);
+    const double u = sqrt_pair(r2) * Hinv;
+    // (a NaN distance adds 0 to ∑W and NaN to ∑∇W, an infinite one NaN to ∑∇W)
+    if (GRAD ? u >= 1.0 && r2 < INFINITY : !(u < 1.0)) return;
+    const double t = u < 1.0 ? 1.0 - u : 0.0, t2 = t * t;
+    if (GRAD) {
+      const double dwk_r = r2 > 0.0 ? nn * (t2 * t) : NAN;  // the reference's d𝒲(0)/0
+      double g[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) dx[d] = x.p[d][i] - x.p[d][j];
-  double r = sqrt(dotp<D>(dx, dx));
-  double u = r * Hinv;
-  if (GRAD) {
-    double dwk_r = wc2_dw(u, nn) / r;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      double g = dx[d] * dwk_r;
-      atomicAdd(&sg.p[d][i], g);
-      atomicAdd(&sg.p[d][j], -g);
+      for (int d = 0; d < D; ++d) g[d] = dx[d] * dwk_r;
+      scatter_pm<D>(sg, i, j, g);
+    } else {
+      const double w = fma(4.0, u, 1.0) * (t2 * t2) * nn;
+      atomicAdd(&sumW[i], w);
+      atomicAdd(&sumW[j], w);
     }
-  } else {
-    double w = wc2_w(u, nn);
-    atomicAdd(&sumW[i], w);
-    atomicAdd(&sumW[j], w);
   }
-}
+};
 
 // kernel_∂ρ∂tDDT! (:571-631)
 template <int D>
-__global__ void k_fn_ddt(int64_t P, const int32_t* __restrict__ pairs, V3 gW, const double* __restrict__ rho, V3 v,
-                         V3 x, double eta2, double m0, double rho0, double ginv, int gamma, double DDTkh, double DDTgz,
-                         const int32_t* __restrict__ pt, double* __restrict__ out) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int32_t a = pairs[2 * p], b = pairs[2 * p + 1];
-  if (!(a > 0)) return;
-  int64_t i = a - 1, j = b - 1;
-  if (!(pt[i] > 0 && pt[j] > 0)) return;
-  double dx[D], dv[D], gw[D];
+struct TermDDT {
+  static constexpr bool QUEUE = false;
+  V3 gW, v, x;
+  const double* rho;
+  double eta2, m0, rho0, ginv, DDTkhm0, DDTgz;
+  int gamma;
+  const int32_t* pt;
+  double* out;
+  __device__ bool take(int pi, int pj) const { return pi > 0 && pj > 0; }
+  __device__ void run(int64_t p, int64_t i, int64_t j) const {
+    double dx[D], dv[D], gw[D];
+    pair_dx<D>(x, i, j, dx);
+    pair_dx<D>(v, i, j, dv);
 #pragma unroll
-  for (int d = 0; d < D; ++d) {
-    dx[d] = x.p[d][i] - x.p[d][j];
-    dv[d] = v.p[d][i] - v.p[d][j];
-    gw[d] = gW.p[d][p];
+    for (int d = 0; d < D; ++d) gw[d] = gW.p[d][p];
+    const double ri = rho[i], rj = rho[j];
+    const int pi = pt[i], pj = pt[j];
+    double si = m0 * dotf<D>(dv, gw), sj = si;
+    if (pi > 1 || pj > 1) {
+      const double com = DDTkhm0 * -dotf<D>(dx, gw) * rcp_pair(dotf<D>(dx, dx) + eta2);
+      const double ez = DDTgz * dx[1], drr = rj - ri;
+      if (pi > 1) {
+        const double dp = fma(rho0, 1.0 + pf7m1_fast(ez, ginv, gamma), -rho0);
+        si = fma((drr - dp) * com, rcp_pair(rj), si);
+      }
+      if (pj > 1) {
+        const double dn = fma(rho0, 1.0 + pf7m1_fast(-ez, ginv, gamma), -rho0);
+        sj = fma((-drr - dn) * com, rcp_pair(ri), sj);
+      }
+    }
+    atomicAdd(&out[i], si);
+    atomicAdd(&out[j], sj);
   }
-  double r2 = dotp<D>(dx, dx);
-  double ri = rho[i], rj = rho[j];
-  double dot3 = -dotp<D>(dx, gw);
-  double m0dot = m0 * dotp<D>(dv, gw);
-  double si = m0dot, sj = m0dot;
-  if (pt[i] > 1) {
-    double drhopvp = rho0 * powfancy7th(1.0 + DDTgz * dx[1], ginv, gamma) - rho0;
-    double vd = DDTkh * ((rj - ri) - drhopvp) / (r2 + eta2);
-    si += vd * dot3 * m0 / rj;
-  }
-  atomicAdd(&out[i], si);
-  if (pt[j] > 1) {
-    double drhopvn = rho0 * powfancy7th(1.0 - DDTgz * dx[1], ginv, gamma) - rho0;
-    double vd = DDTkh * ((ri - rj) - drhopvn) / (r2 + eta2);
-    sj += vd * dot3 * m0 / ri;
-  }
-  atomicAdd(&out[j], sj);
-}
+};
 
 __global__ void k_fn_pressure(int64_t N, const double* __restrict__ rho, int gamma, double rho0, double P0,
                               const int32_t* __restrict__ pt, double* __restrict__ P) {
@@ -148,85 +266,72 @@ __global__ void k_fn_pressure(int64_t N, const double* __restrict__ rho, int gam
   if (i < N) P[i] = eos(rho[i], gamma, rho0, P0, pt[i]);
 }
 
-template <int D>
-__device__ inline void scatter_pm(W3 a, int64_t i, int64_t j, const double* f) {
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    atomicAdd(&a.p[d][i], f[d]);
-    atomicAdd(&a.p[d][j], -f[d]);
-  }
-}
-
 // kernel_∂v∂t! (:750-776)
 template <int D>
-__global__ void k_fn_dvdt(int64_t P, const int32_t* __restrict__ pairs, V3 gW, const double* __restrict__ Pr,
-                          double m0, const double* __restrict__ rho, const int32_t* __restrict__ pt, W3 a) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t i, j;
-  if (!pair_at(pairs, p, &i, &j)) return;
-  if (!(pt[i] * pt[j] > 0)) return;
-  double Pfac = (Pr[i] + Pr[j]) / (rho[i] * rho[j]);
-  double s = -m0 * Pfac;
-  double f[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) f[d] = s * gW.p[d][p];
-  scatter_pm<D>(a, i, j, f);
-}
-
-// kernel_∂v∂t_av! (:863-901)
-template <int D>
-__global__ void k_fn_av(int64_t P, const int32_t* __restrict__ pairs, V3 gW, V3 x, double h, double eta2,
-                        const double* __restrict__ rho, double alpha, V3 v, double c0, double m0,
-                        const int32_t* __restrict__ pt, W3 a) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t i, j;
-  if (!pair_at(pairs, p, &i, &j)) return;
-  if (!(pt[i] > 0 && pt[j] > 0)) return;
-  double dx[D], dv[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    dx[d] = x.p[d][i] - x.p[d][j];
-    dv[d] = v.p[d][i] - v.p[d][j];
-  }
-  double r2 = dotp<D>(dx, dx);
-  double rhom = (rho[i] + rho[j]) * 0.5;
-  double cond = dotp<D>(dv, dx);
-  if (cond < 0.0) {
-    double dmu = h * cond / (r2 + eta2);
-    double dPi = (-alpha * c0 * dmu) / rhom;
-    double s = -dPi * m0;
+struct TermPress {
+  static constexpr bool QUEUE = true;
+  V3 gW;
+  const double* Pr;
+  const double* rho;
+  double m0;
+  const int32_t* pt;
+  W3 a;
+  __device__ bool take(int pi, int pj) const { return pi * pj > 0; }
+  __device__ void run(int64_t p, int64_t i, int64_t j) const {
+    const double s = -m0 * (Pr[i] + Pr[j]) * rcp_pair(rho[i] * rho[j]);
     double f[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) f[d] = s * gW.p[d][p];
     scatter_pm<D>(a, i, j, f);
   }
-}
+};
 
-// kernel_∂v∂t_visc! (:962-991)
+// kernel_∂v∂t_av! (:863-901): -Π m₀ = avk (Δv·Δx) / ((r² + η²)(ρi + ρj)), avk = 2 α c₀ h m₀
 template <int D>
-__global__ void k_fn_visc(int64_t P, const int32_t* __restrict__ pairs, V3 gW, V3 v, const double* __restrict__ rho,
-                          V3 x, double eta2, double m0, double nu, const int32_t* __restrict__ pt, W3 a) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t i, j;
-  if (!pair_at(pairs, p, &i, &j)) return;
-  if (!(pt[i] > 0 && pt[j] > 0)) return;
-  double dx[D], dv[D], gw[D];
+struct TermAv {
+  static constexpr bool QUEUE = true;
+  V3 gW, x, v;
+  const double* rho;
+  double eta2, avk;
+  const int32_t* pt;
+  W3 a;
+  __device__ bool take(int pi, int pj) const { return pi > 0 && pj > 0; }
+  __device__ void run(int64_t p, int64_t i, int64_t j) const {
+    double dx[D], dv[D];
+    pair_dx<D>(x, i, j, dx);
+    pair_dx<D>(v, i, j, dv);
+    const double cond = dotf<D>(dv, dx);
+    if (!(cond < 0.0)) return;
+    const double s = avk * cond * rcp_pair((dotf<D>(dx, dx) + eta2) * (rho[i] + rho[j]));
+    double f[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) {
-    dx[d] = x.p[d][i] - x.p[d][j];
-    dv[d] = v.p[d][i] - v.p[d][j];
-    gw[d] = gW.p[d][p];
+    for (int d = 0; d < D; ++d) f[d] = s * gW.p[d][p];
+    scatter_pm<D>(a, i, j, f);
   }
-  double r2 = dotp<D>(dx, dx);
-  double nuterm = 4.0 * nu * m0 * dotp<D>(dx, gw) / ((rho[i] + rho[j]) * (r2 + eta2));
-  double f[D];
+};
+
+// kernel_∂v∂t_visc! (:962-991), nu4 = 4 ν m₀
+template <int D>
+struct TermVisc {
+  static constexpr bool QUEUE = true;
+  V3 gW, v, x;
+  const double* rho;
+  double eta2, nu4;
+  const int32_t* pt;
+  W3 a;
+  __device__ bool take(int pi, int pj) const { return pi > 0 && pj > 0; }
+  __device__ void run(int64_t p, int64_t i, int64_t j) const {
+    double dx[D], dv[D], gw[D], f[D];
+    pair_dx<D>(x, i, j, dx);
+    pair_dx<D>(v, i, j, dv);
 #pragma unroll
-  for (int d = 0; d < D; ++d) f[d] = nuterm * dv[d];
-  scatter_pm<D>(a, i, j, f);
-}
+    for (int d = 0; d < D; ++d) gw[d] = gW.p[d][p];
+    const double nt = nu4 * dotf<D>(dx, gw) * rcp_pair((rho[i] + rho[j]) * (dotf<D>(dx, dx) + eta2));
+#pragma unroll
+    for (int d = 0; d < D; ++d) f[d] = nt * dv[d];
+    scatter_pm<D>(a, i, j, f);
+  }
+};
 
 template <int D>
 __global__ void k_fn_grav(int64_t N, double g, W3 a) {
@@ -236,52 +341,55 @@ __global__ void k_fn_grav(int64_t N, double g, W3 a) {
   for (int d = 0; d < D; ++d) a.p[d][i] = a.p[d][i] - (d == 1 ? g : 0.0);
 }
 
-// kernel_fbmolforce! (:1885-1913)
+// kernel_fbmolforce! (:1885-1913).  Lattice walls hold pairs at exactly r₀: the
+// distance and its compare are the reference's to the bit (past r2cut =
+// r₀² (1 + 1e-6) it fails for certain)
 template <int D>
-__global__ void k_fn_fbmol(int64_t P, const int32_t* __restrict__ pairs, V3 x, double dd, double r0, double eta2,
-                           const int32_t* __restrict__ pt, W3 a) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t i, j;
-  if (!pair_at(pairs, p, &i, &j)) return;
-  if ((pt[i] > 0) == (pt[j] > 0)) return;
-  double dx[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) dx[d] = x.p[d][i] - x.p[d][j];
-  double r2 = dotp<D>(dx, dx);
-  double r = sqrt(r2);
-  if (r < r0) {
-    double q = r0 / (r + eta2);
-    double q2 = q * q, q4 = q2 * q2, q8 = q4 * q4, q12 = q8 * q4;
-    double Fc = dd * (q12 - q4) / (r2 + eta2);
+struct TermWall {
+  static constexpr bool QUEUE = true;
+  V3 x;
+  double dd, r0, eta2, r2cut;
+  const int32_t* pt;
+  W3 a;
+  __device__ bool take(int pi, int pj) const { return (pi > 0) != (pj > 0); }
+  __device__ void run(int64_t, int64_t i, int64_t j) const {
+    double dx[D];
+    pair_dx<D>(x, i, j, dx);
+    const double r2 = dotp<D>(dx, dx);
+    if (r2 > r2cut) return;
+    const double r = sqrt(r2);
+    if (!(r < r0)) return;
+    const double q = r0 * rcp_pair(r + eta2);
+    const double q2 = q * q, q4 = q2 * q2, q8 = q4 * q4, q12 = q8 * q4;
+    const double Fc = dd * (q12 - q4) * rcp_pair(r2 + eta2);
     double f[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) f[d] = dx[d] * Fc;
     scatter_pm<D>(a, i, j, f);
   }
-}
+};
 
-// kernel_∂v∂tpF! (:1382-1409)
+// kernel_∂v∂tpF! (:1382-1409): sm = s/m₀, pfk = 1.5π/2h, hp1 = 0.1h
 template <int D>
-__global__ void k_fn_pF(int64_t P, const int32_t* __restrict__ pairs, V3 x, double s, double h, double m0,
-                        const int32_t* __restrict__ pt, W3 a) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t i, j;
-  if (!pair_at(pairs, p, &i, &j)) return;
-  if (!(pt[i] > 0 && pt[j] > 0)) return;
-  double dx[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) dx[d] = x.p[d][i] - x.p[d][j];
-  double r = sqrt(dotp<D>(dx, dx));
-  if (r < 2.0 * h) {
-    double scos = s * gc_cos((1.5 * GCSPH_PI64) * r / (2.0 * h)) / (r + 0.1 * h);
+struct TermTension {
+  static constexpr bool QUEUE = true;
+  V3 x;
+  double sm, twoh, pfk, hp1;
+  const int32_t* pt;
+  W3 a;
+  __device__ bool take(int pi, int pj) const { return pi > 0 && pj > 0; }
+  __device__ void run(int64_t, int64_t i, int64_t j) const {
+    double dx[D];
+    pair_dx<D>(x, i, j, dx);
+    const double r = sqrt_pair(dotf<D>(dx, dx));
+    if (!(r < twoh)) return;
+    const double scos = sm * cos_fast(pfk * r) * rcp_pair(r + hp1);
     double f[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) f[d] = scos * dx[d] / m0;
+    for (int d = 0; d < D; ++d) f[d] = scos * dx[d];
     scatter_pm<D>(a, i, j, f);
   }
-}
+};
 
 __global__ void k_fn_update_rho(int64_t N, double* __restrict__ rho, const double* __restrict__ drho, double dt,
                                 double rho0, const int32_t* __restrict__ pt) {
@@ -387,21 +495,25 @@ __global__ void k_fn_update_dpc(int64_t N, W3 v, W3 x, V3 buf, double dt, const 
   }
 }
 
-// kernel_xsphcorr! (:1757-1779)
+// kernel_xsphcorr! (:1757-1779), xc = 2 m₀ ε
 template <int D>
-__global__ void k_fn_xsph(int64_t P, W3 buf, const int32_t* __restrict__ pairs, const double* __restrict__ W,
-                          const double* __restrict__ rho, V3 v, double m0, double eps, const int32_t* __restrict__ pt) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  int64_t i, j;
-  if (!pair_at(pairs, p, &i, &j)) return;
-  if (!(pt[i] > 1 && pt[j] > 1)) return;
-  double xs = 2.0 * m0 * eps * W[p] / (rho[i] + rho[j]);
-  double f[D];
+struct TermXsph {
+  static constexpr bool QUEUE = false;
+  V3 v;
+  const double* W;
+  const double* rho;
+  double xc;
+  const int32_t* pt;
+  W3 buf;
+  __device__ bool take(int pi, int pj) const { return pi > 1 && pj > 1; }
+  __device__ void run(int64_t p, int64_t i, int64_t j) const {
+    const double xs = xc * W[p] * rcp_pair(rho[i] + rho[j]);
+    double f[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) f[d] = (v.p[d][j] - v.p[d][i]) * xs;
-  scatter_pm<D>(buf, i, j, f);
-}
+    for (int d = 0; d < D; ++d) f[d] = (v.p[d][j] - v.p[d][i]) * xs;
+    scatter_pm<D>(buf, i, j, f);
+  }
+};
 
 template <int D>
 __global__ void k_fn_update_xsph(int64_t N, W3 x, V3 buf, double dt, const int32_t* __restrict__ pt) {
@@ -467,6 +579,14 @@ using namespace gcsph;
     GC_LAUNCHED();                                \
     GC_CUDA(cudaStreamSynchronize((st)));         \
     return GCSPH_OK;                              \
+  } while (0)
+// a summed term over the pairs, then the wait that ends the call
+#define TERM(D, ST, F2, F3)                                                                        \
+  do {                                                                                             \
+    const int _rc = (D) == 2 ? launch_pair_term(P, pairs, F2, (ST)) : launch_pair_term(P, pairs, F3, (ST)); \
+    if (_rc) return _rc;                                                                           \
+    GC_CUDA(cudaStreamSynchronize((ST)));                                                          \
+    return GCSPH_OK;                                                                               \
   } while (0)
 #define DISPATCH(D, KER, GRID, ST, ...)                                  \
   do {                                                                   \
@@ -545,10 +665,8 @@ int gcsph_sphsumW(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const d
   cudaStream_t st = (cudaStream_t)stream;
   double nn = D == 2 ? wc2_norm_w<2>(Hinv) : wc2_norm_w<3>(Hinv);
   W3 none{};
-  if (D == 2) k_fn_sumw<2, 0><<<nblocks(P, PTPB), PTPB, 0, st>>>(P, pairs, x, Hinv, nn, pt, sumW, none);
-  else k_fn_sumw<3, 0><<<nblocks(P, PTPB), PTPB, 0, st>>>(P, pairs, x, Hinv, nn, pt, sumW, none);
   (void)N;
-  FINISH(st);
+  TERM(D, st, (TermSumW<2, 0>{x, Hinv, nn, pt, sumW, none}), (TermSumW<3, 0>{x, Hinv, nn, pt, sumW, none}));
 }
 
 int gcsph_sphsumgradW(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const double* const* x_dev, double Hinv,
@@ -563,11 +681,9 @@ int gcsph_sphsumgradW(int32_t D, int64_t N, int64_t P, const int32_t* pairs, con
   if (!pt) return fail(GCSPH_EINVAL, "null ptype");
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  double nn = D == 2 ? wc2_norm_dw<2>(Hinv) : wc2_norm_dw<3>(Hinv);
-  if (D == 2) k_fn_sumw<2, 1><<<nblocks(P, PTPB), PTPB, 0, st>>>(P, pairs, x, Hinv, nn, pt, nullptr, g);
-  else k_fn_sumw<3, 1><<<nblocks(P, PTPB), PTPB, 0, st>>>(P, pairs, x, Hinv, nn, pt, nullptr, g);
+  double nn = -20.0 * (D == 2 ? wc2_norm_dw<2>(Hinv) : wc2_norm_dw<3>(Hinv)) * Hinv;
   (void)N;
-  FINISH(st);
+  TERM(D, st, (TermSumW<2, 1>{x, Hinv, nn, pt, nullptr, g}), (TermSumW<3, 1>{x, Hinv, nn, pt, nullptr, g}));
 }
 
 int gcsph_drhodt_ddt(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const double* const* gW_dev,
@@ -590,11 +706,9 @@ int gcsph_drhodt_ddt(int32_t D, int64_t N, int64_t P, const int32_t* pairs, cons
   double DDTkh = 2.0 * h * delta * c0;
   double Cb = (c0 * c0 * rho0) * ginv;
   double DDTgz = rho0 * g / Cb;
-  if (P > 0) {
-    DISPATCH(D, k_fn_ddt, nblocks(P, PTPB), st, P, pairs, gw, rho, v, x, eta2, m0, rho0, ginv, gamma, DDTkh, DDTgz,
-             pt, out);
-    GC_LAUNCHED();
-  }
+  if (P > 0)
+    TERM(D, st, (TermDDT<2>{gw, v, x, rho, eta2, m0, rho0, ginv, DDTkh * m0, DDTgz, gamma, pt, out}),
+         (TermDDT<3>{gw, v, x, rho, eta2, m0, rho0, ginv, DDTkh * m0, DDTgz, gamma, pt, out}));
   GC_CUDA(cudaStreamSynchronize(st));
   return GCSPH_OK;
 }
@@ -622,9 +736,8 @@ int gcsph_dvdt(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const doub
   if (!Pr || !rho || !pt) return fail(GCSPH_EINVAL, "null argument");
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  DISPATCH(D, k_fn_dvdt, nblocks(P, PTPB), st, P, pairs, gw, Pr, m0, rho, pt, a);
   (void)N;
-  FINISH(st);
+  TERM(D, st, (TermPress<2>{gw, Pr, rho, m0, pt, a}), (TermPress<3>{gw, Pr, rho, m0, pt, a}));
 }
 
 int gcsph_dvdt_av(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const double* const* gW_dev,
@@ -643,9 +756,9 @@ int gcsph_dvdt_av(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const d
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
   double eta2 = (0.1 * h) * (0.1 * h);
-  DISPATCH(D, k_fn_av, nblocks(P, PTPB), st, P, pairs, gw, x, h, eta2, rho, alpha, v, c0, m0, pt, a);
+  const double avk = 2.0 * alpha * c0 * h * m0;
   (void)N;
-  FINISH(st);
+  TERM(D, st, (TermAv<2>{gw, x, v, rho, eta2, avk, pt, a}), (TermAv<3>{gw, x, v, rho, eta2, avk, pt, a}));
 }
 
 int gcsph_dvdt_visc(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const double* const* gW_dev,
@@ -664,9 +777,9 @@ int gcsph_dvdt_visc(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
   double eta2 = (0.1 * h) * (0.1 * h);
-  DISPATCH(D, k_fn_visc, nblocks(P, PTPB), st, P, pairs, gw, v, rho, x, eta2, m0, nu, pt, a);
+  const double nu4 = 4.0 * nu * m0;
   (void)N;
-  FINISH(st);
+  TERM(D, st, (TermVisc<2>{gw, v, x, rho, eta2, nu4, pt, a}), (TermVisc<3>{gw, v, x, rho, eta2, nu4, pt, a}));
 }
 
 int gcsph_addgrav(int32_t D, int64_t N, double g, double* const* a_dev, void* stream) {
@@ -693,9 +806,9 @@ int gcsph_fbmolforce(int32_t D, int64_t N, int64_t P, const int32_t* pairs, cons
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
   double eta2 = 0.01 * (r0 * r0);
-  DISPATCH(D, k_fn_fbmol, nblocks(P, PTPB), st, P, pairs, x, d, r0, eta2, pt, a);
+  const double cut = r0 * r0 * (1.0 + 1e-6);
   (void)N;
-  FINISH(st);
+  TERM(D, st, (TermWall<2>{x, d, r0, eta2, cut, pt, a}), (TermWall<3>{x, d, r0, eta2, cut, pt, a}));
 }
 
 int gcsph_dvdt_pF(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const double* const* x_dev, double s,
@@ -710,9 +823,9 @@ int gcsph_dvdt_pF(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const d
   if (!pt) return fail(GCSPH_EINVAL, "null ptype");
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  DISPATCH(D, k_fn_pF, nblocks(P, PTPB), st, P, pairs, x, s, h, m0, pt, a);
+  const double sm = s / m0, twoh = 2.0 * h, pfk = 1.5 * GCSPH_PI64 / twoh, hp1 = 0.1 * h;
   (void)N;
-  FINISH(st);
+  TERM(D, st, (TermTension<2>{x, sm, twoh, pfk, hp1, pt, a}), (TermTension<3>{x, sm, twoh, pfk, hp1, pt, a}));
 }
 
 int gcsph_update_rho(int64_t N, double* rho, const double* drho, double dt, double rho0, const int32_t* pt,
@@ -830,10 +943,8 @@ int gcsph_xsphcorr(int32_t D, int64_t N, int64_t P, double* const* buf_dev, cons
   if (!W || !rho || !pt) return fail(GCSPH_EINVAL, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
   for (int d = 0; d < D; ++d) GC_CUDA(cudaMemsetAsync(buf.p[d], 0, sizeof(double) * (size_t)N, st));
-  if (P > 0) {
-    DISPATCH(D, k_fn_xsph, nblocks(P, PTPB), st, P, buf, pairs, W, rho, v, m0, eps, pt);
-    GC_LAUNCHED();
-  }
+  const double xc = 2.0 * m0 * eps;
+  if (P > 0) TERM(D, st, (TermXsph<2>{v, W, rho, xc, pt, buf}), (TermXsph<3>{v, W, rho, xc, pt, buf}));
   GC_CUDA(cudaStreamSynchronize(st));
   return GCSPH_OK;
 }
