@@ -1158,7 +1158,7 @@ int CellCore::pair_lanes() const {
 int CellCore::ensure_pf() {
   int rc;
   for (int d = 0; d < D; ++d)
-    if ((rc = pf[d].ensure(sizeof(float) * N, st))) return rc;
+    if ((rc = pf[d].ensure(sizeof(float) * (N + 8), st))) return rc;  // a group of padding (k_full_count)
   return ensure_pf_scalars();
 }
 
@@ -1211,7 +1211,9 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
                    cellstart.as<int32_t>(), N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(), nullptr, nullptr, 0,
                    nullptr, sp, S, rs_full.as<int64_t>(), rs_up.as<int64_t>(), fc, nullptr, nullptr,
                    foldsum.as<int32_t>());
-  else if (sp)
+  else if (sp && N >= ROWS_THREAD_MIN_N) {
+    if ((rc0 = count_rows(xs, sp, S))) return rc0;
+  } else if (sp)
     PAIRS32_LAUNCH(2, L, xs[0], xs[1], x2, pf[0].as<float>(), pf[1].as<float>(), f2, thr, skey.as<int32_t>(),
                    cellstart.as<int32_t>(), N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(), nullptr, nullptr, 0,
                    nullptr, sp, S, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
@@ -1286,7 +1288,7 @@ int CellCore::read_nfull() {
 // the build where it needed them itself, else on demand
 int CellCore::ensure_up() {
   if (up_valid) return GCSPH_OK;
-  int rc;
+  int rc = GCSPH_OK;
   if (!up_scanned &&
       (rc = exclusive_scan_i32_to_i64(cnt_up.as<int32_t>(), rs_up.as<int64_t>(), N, scratch.as<int64_t>(), st)))
     return rc;

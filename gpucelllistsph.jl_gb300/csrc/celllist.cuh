@@ -180,6 +180,11 @@ constexpr int64_t RADIX_MIN_N = 65536;
 // ... and then only where a cell holds more than this many points (below it
 // the rank's cost is a few loads per point and takes fewer launches)
 constexpr int RADIX_MIN_POP = 128;
+// sets of at least this many points give each point of the step's pair search a
+// thread (celllist_upper.cu); below, the lanes of pair_lanes (one GB300, the
+// search and its fill together with lanes and with a thread: 3-D 26k points 107
+// and 125 us, 46k 160 and 146, 390k 1277 and 764; 2-D 40k 61 and 49)
+constexpr int64_t ROWS_THREAD_MIN_N = 32768;
 // blocks of the count pass whose row-start scan it folds (rows_fold)
 constexpr int ROWS_FOLD_MAX_BLOCKS = 2048;
 
@@ -254,6 +259,8 @@ struct CellCore {
   // xs takes the positions in cell order.  Waits for the pair count (nup).
   int build_upper(const double* const* xin, double* const* xs, bool rebin);
   int emit_upper(int32_t* pairs, int64_t cap);
+  // the step's counts and staged rows of a large set (celllist_upper.cu)
+  int count_rows(const double* const* xs, int32_t* stg, int S);
   // count + scan + fill of the neighbour CSR on sorted positions xs.  With
   // ovf_dev (and buffers already sized once) the fill does not wait for the
   // count: rows past nbr_cap raise *ovf_dev instead (see grow_nbr).  scan_up

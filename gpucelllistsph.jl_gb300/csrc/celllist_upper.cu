@@ -438,6 +438,100 @@ __global__ void __launch_bounds__(UTPB) k_up_emit_rows(
 }
 
 // ---------------------------------------------------------------------------
+// The step's rows (both directions), one thread per point: k_pairs32's MODE 2
+// -- the two counts, and the row staged ascending at stg[k * S ..] -- for sets
+// large enough to fill the GPU with a thread each.  The prefilter's copies are
+// the step's (one array per dimension, a group of padding past the last point).
+// ---------------------------------------------------------------------------
+template <int D>
+__global__ void __launch_bounds__(UTPB, 4) k_full_count(
+    const float* __restrict__ f0, const float* __restrict__ f1, const float* __restrict__ f2, Pos3 P,
+    const float2* __restrict__ thr, const int32_t* __restrict__ skey, const int32_t* __restrict__ cellstart, int64_t N,
+    Grid g, int32_t* __restrict__ cnt_full, int32_t* __restrict__ cnt_up, int32_t* __restrict__ stg, int S) {
+  const int64_t k64 = (int64_t)blockIdx.x * UTPB + threadIdx.x;
+  if (k64 >= N) return;
+  const int32_t k = (int32_t)k64;
+  constexpr int NR = D == 2 ? 3 : 9, G = 8;
+  const int nx = g.nc[0], ny = g.nc[1], nz = D == 3 ? g.nc[2] : 1;
+  const int32_t key = skey[k];
+  const int t = g.fx.quot(key);
+  const int cx = key - t * nx;
+  const int cz = D == 3 ? g.fy.quot(t) : 0;
+  const int cy = t - cz * ny;
+  const int xlo = cx > 0 ? cx - 1 : 0, xhi = cx < nx - 1 ? cx + 1 : nx - 1;
+  auto range = [&](int r, int32_t& a, int32_t& b) {
+    const int y = cy + r % 3 - 1, z = cz + (D == 3 ? r / 3 - 1 : 0);
+    a = b = 0;
+    if (y >= 0 && y < ny && z >= 0 && z < nz) {
+      const int base = nx * (y + ny * z);
+      a = cellstart[base + xlo];
+      b = cellstart[base + xhi + 1];
+    }
+  };
+  const float2 tt = *thr;
+  const float ax = f0[k], ay = f1[k], az = D == 3 ? f2[k] : 0.f;
+  int32_t* row = stg + k64 * S;
+  int32_t cnt = 0, up = 0;
+  int4 v = make_int4(0, 0, 0, 0);
+  int32_t m0, m1;
+  range(0, m0, m1);
+#pragma unroll 1
+  for (int r = 0; r < NR; ++r) {
+    int32_t a = m0;
+    const int32_t b = m1;
+    if (r + 1 < NR) range(r + 1, m0, m1);  // the next row's range, a row ahead
+    for (; a < b; a += 32) {
+      const int n = min(32, b - a);
+      unsigned in = 0, ok = 0;  // surely in; not surely out
+      for (int j = 0; j < n; j += G) {
+        unsigned ig = 0, og = 0;
+#pragma unroll
+        for (int q = 0; q < G; ++q) {
+          const int32_t m = a + j + q;
+          const float d0 = ax - f0[m], d1 = ay - f1[m];
+          float r2 = fmaf(d1, d1, d0 * d0);
+          if (D == 3) {
+            const float d2 = az - f2[m];
+            r2 = fmaf(d2, d2, r2);
+          }
+          if (r2 < tt.x) ig |= 1u << q;
+          if (!(r2 > tt.y)) og |= 1u << q;
+        }
+        in |= ig << j;
+        ok |= og << j;
+      }
+      unsigned cut = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+      if (k >= a && k < a + n) cut &= ~(1u << (k - a));
+      in &= cut;
+      unsigned band = ok & cut & ~in;
+      while (band) {
+        const int e = __ffs(band) - 1;
+        band &= band - 1;
+        if (hit_exact<D>(k, a + e, P.out, g.dist2)) in |= 1u << e;
+      }
+      // the bits above k: all of a chunk past k, none of one before it
+      up += __popc(a > k ? in : (a + 31 <= k ? 0u : in & (0xfffffffeu << (k - a))));
+      while (in) {
+        const int e = __ffs(in) - 1;
+        in &= in - 1;
+        v = make_int4(v.y, v.z, v.w, a + e);
+        ++cnt;
+        if ((cnt & 3) == 0 && cnt <= S) *reinterpret_cast<int4*>(row + cnt - 4) = v;
+      }
+    }
+  }
+  const int left = cnt & 3;
+  if (cnt < S) {  // S is a multiple of four
+    int32_t* e = row + (cnt - left);
+    if (left == 3) e[0] = v.y;
+    if (left >= 2) e[left - 2] = v.z;
+    if (left >= 1) e[left - 1] = v.w;
+  }
+  cnt_full[k] = cnt;
+  cnt_up[k] = up;
+}
+
+// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 template <int D>
@@ -571,6 +665,22 @@ static int emit_upper_impl(CellCore& C, double* const* xs, int32_t* pairs, int64
 #undef UP_EMIT
   GC_LAUNCHED();
   return GCSPH_OK;
+}
+
+int CellCore::count_rows(const double* const* xs, int32_t* stg, int S) {
+  Pos3 P{};
+  for (int d = 0; d < D; ++d) P.out[d] = const_cast<double*>(xs[d]);
+  const int nb = nblocks(N, UTPB);
+  const float* f0 = pf[0].as<float>();
+  const float* f1 = pf[1].as<float>();
+  if (D == 2)
+    k_full_count<2><<<nb, UTPB, 0, st>>>(f0, f1, f0, P, pfthr.as<float2>(), skey.as<int32_t>(), cellstart.as<int32_t>(),
+                                         N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(), stg, S);
+  else
+    k_full_count<3><<<nb, UTPB, 0, st>>>(f0, f1, pf[2].as<float>(), P, pfthr.as<float2>(), skey.as<int32_t>(),
+                                         cellstart.as<int32_t>(), N, g, cnt_full.as<int32_t>(), cnt_up.as<int32_t>(),
+                                         stg, S);
+  return GCSPH_OK;  // the caller counts and checks the launch
 }
 
 int CellCore::build_upper(const double* const* xin, double* const* xs, bool rebin) {

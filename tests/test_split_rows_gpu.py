@@ -72,3 +72,23 @@ def test_sums_without_a_step(gpu_pkg, orc, D, lanes):
             got = np.stack([t.cpu().numpy() for t in got]) if isinstance(got, tuple) else got.cpu().numpy()
             # eight roundings per term of up to 200 terms against ∑|terms| <= 4x the largest sum
             assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max(), f
+
+
+@pytest.mark.parametrize("D", [2, 3])
+def test_rows_by_a_thread_per_point(gpu_pkg, orc, D):
+    """Sets past 32,768 particles search their rows with a thread per point:
+    on serial rows, whose sums follow the rows' order, two calls are the
+    oracle's to the bit."""
+    if D == 2:
+        case = gpu_pkg.workloads.dam_break_2d(dx=0.0078)
+    else:
+        case = gpu_pkg.workloads.dam_break_3d(dx=0.042, fluid=(1.0, 1.2, 0.7), tank=(2.4, 1.6, 1.2), full_physics=False)
+    assert 32768 <= case.N <= 65536
+    rng = np.random.default_rng(2)
+    fl = case.ptype > 1
+    case.x = case.x.copy()
+    case.x[:, fl] += rng.uniform(-0.2, 0.2, (D, int(fl.sum()))) * case.dx
+    prob, ref = make_pair(gpu_pkg, orc, case, 1)
+    for _ in range(2):
+        run_both(prob, ref, 1)
+    check(orc, prob, ref, case, 1, [(1, {}), (1, {})])
