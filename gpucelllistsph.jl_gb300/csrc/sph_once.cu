@@ -697,10 +697,12 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
 
 // post-batch sph∑W! + sph∑∇W!  (:139-156, :332-359).  The kernel's factors
 // come out of the sums: ∑W = nW ∑ (1 + 4u)(1 - u)^4, ∑∇W = dWg ∑ Δx (1 - u)^3.
-template <int D, int L>
+// With SCATTER the lanes of a particle also write its state back to the
+// original order, an array in turn each.
+template <int D, int L, bool SCATTER>
 __global__ void __launch_bounds__(STPB) k_sums_rows(StepConst c, int64_t N, const int64_t* __restrict__ rs,
                                                     const int32_t* __restrict__ nbr, PostSums Q,
-                                                    const int* __restrict__ ovf) {
+                                                    const int* __restrict__ ovf, StateIO<D> O, SArr<D> S) {
   if (*ovf) return;
   const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t k = gt / L;
@@ -748,8 +750,30 @@ __global__ void __launch_bounds__(STPB) k_sums_rows(StepConst c, int64_t N, cons
     }
   }
   lanes_sum4<L>(s, lane, group_mask<L>());
-  if (lane != 0) return;
   const int32_t o = Q.orig[k];
+  if constexpr (SCATTER) {
+    if (lane == 0) {
+      O.rho[o] = S.rho[k];
+      O.rhoh[o] = S.rhoh[k];
+      O.drho[o] = S.drho[k];
+      O.P[o] = S.Plast[k];
+    }
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      if (lane == (1 + 2 * d) % L) {
+        O.x[d][o] = xk[d];
+        O.v[d][o] = S.v[d][k];
+        O.vh[d][o] = S.vh[d][k];
+      }
+      if (lane == (2 + 2 * d) % L) {
+        O.xh[d][o] = S.xh[d][k];
+        O.cdx[d][o] = S.cdx[d][k];
+        O.a[d][o] = S.a[d][k];
+        O.buf2[d][o] = S.buf2[d][k];
+      }
+    }
+  }
+  if (lane != 0) return;
   Q.sumW[o] = s[0] * c.nW;
 #pragma unroll
   for (int d = 0; d < D; ++d) Q.sg[d][o] = s[1 + d] * c.dWg;
@@ -845,8 +869,22 @@ int launch_cspm(int L, int64_t N, cudaStream_t st, const StepConst& c, const SAr
 }
 template <int D>
 int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, const int64_t* rs, const int32_t* nbr,
-                     const PostSums& Q, const int* ovf) {
-  GC_ROWS(k_sums_rows, c, N, rs, nbr, Q, ovf);
+                     const PostSums& Q, const int* ovf, bool scatter, const StateIO<D>& O, const SArr<D>& S) {
+#define GC_SUMS(LL)                                                                                            \
+  if (scatter)                                                                                                 \
+    k_sums_rows<D, LL, true><<<nblocks(N * (int64_t)LL, STPB), STPB, 0, st>>>(c, N, rs, nbr, Q, ovf, O, S);     \
+  else                                                                                                         \
+    k_sums_rows<D, LL, false><<<nblocks(N * (int64_t)LL, STPB), STPB, 0, st>>>(c, N, rs, nbr, Q, ovf, O, S);
+  switch (L) {
+    case 2: GC_SUMS(2) break;
+    case 4: GC_SUMS(4) break;
+    case 8: GC_SUMS(8) break;
+    case 16: GC_SUMS(16) break;
+    default: GC_SUMS(32) break;
+  }
+#undef GC_SUMS
+  GC_LAUNCHED();
+  return GCSPH_OK;
 }
 #undef GC_ROWS
 
@@ -856,7 +894,7 @@ int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, cons
   template int launch_xsph<D>(int, int64_t, cudaStream_t, const StepConst&, const Scal*, const SArr<D>&);         \
   template int launch_cspm<D>(int, int64_t, cudaStream_t, const StepConst&, const SArr<D>&);                      \
   template int launch_sums_post<D>(int, int64_t, cudaStream_t, const StepConst&, const int64_t*, const int32_t*,  \
-                                   const PostSums&, const int*);
+                                   const PostSums&, const int*, bool, const StateIO<D>&, const SArr<D>&);
 GC_INST(2)
 GC_INST(3)
 #undef GC_INST

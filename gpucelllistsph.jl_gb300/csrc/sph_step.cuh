@@ -414,6 +414,23 @@ struct NextBin {
   int32_t* cellstart;
   Grid g;
 };
+// the caller's and the library's original-order arrays
+template <int D>
+struct StateIO {
+  double* x[3];
+  double* v[3];
+  double* rho;
+  const int32_t* pt;
+  double* rhoh;
+  double* vh[3];
+  double* xh[3];
+  double* cdx[3];
+  double* a[3];
+  double* drho;
+  double* buf2[3];
+  double* P;
+};
+
 // the FP32 copy (x - offset) of the particles' new positions that pass B2
 // writes for dpcreg!'s prefilter; f[0] == nullptr: none
 struct PosCopy {
@@ -434,6 +451,8 @@ template <int D>
 int launch_cspm(int L, int64_t N, cudaStream_t st, const StepConst& c, const SArr<D>& S);
 // ∑W and ∑∇W of a call.  X: the positions and pt the ptypes, by cell-order
 // index (map null) or by map[cell-order index]; results go to orig's places.
+// scatter: the cell-order state S goes to the original-order arrays O as well
+// (k_scatter_state's work, without its launch).
 struct PostSums {
   const double* x[3];
   const int32_t* pt;
@@ -444,6 +463,6 @@ struct PostSums {
 };
 template <int D>
 int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, const int64_t* rs, const int32_t* nbr,
-                     const PostSums& Q, const int* ovf);
+                     const PostSums& Q, const int* ovf, bool scatter, const StateIO<D>& O, const SArr<D>& S);
 
 }  // namespace gcsph
