@@ -86,11 +86,19 @@ class GPUCellList:
 
     # ------------------------------------------------------------------ internals
     def _refresh_cellpnum(self):
-        ncell = 1
-        for g in self.grid:
-            ncell *= g
-        self.cellpnum = torch.empty(ncell, dtype=torch.int32, device="cuda")
+        self.cellpnum = self._new_cellpnum()
         _lib.check(_lib.load().gcl_cellpnum(self._h, _lib.dptr(self.cellpnum)))
+
+    def _new_cellpnum(self):
+        return torch.empty(math.prod(self.grid), dtype=torch.int32, device="cuda")
+
+    def _refresh(self, fillzero):
+        """cellpnum and the pair list, with one wait."""
+        n = C.c_int64()
+        cap = int(self.pairs.shape[0])
+        self.cellpnum = self._new_cellpnum()
+        _lib.check(_lib.load().gcl_refresh(self._h, _lib.dptr(self.cellpnum), _lib.dptr(self.pairs) if cap else None,
+                                           cap, int(bool(fillzero)), C.byref(n)))
 
     def _emit(self, fillzero=True, allow_overflow=False) -> int:
         n = C.c_int64()
@@ -101,7 +109,7 @@ class GPUCellList:
         return int(n.value)
 
     def _apply_update_policy(self, prev_pairsn: int, total: int, fillzero: bool):
-        """Capacity policy of update!, src/celllist.jl:117-133."""
+        """Capacity policy of update!, src/celllist.jl:117-133; then the user-visible fields."""
         cap = int(self.pairs.shape[0])
         realloc = False
         if prev_pairsn > cap or prev_pairsn < cap * 0.6:
@@ -112,7 +120,7 @@ class GPUCellList:
             realloc = True
         if realloc:
             self.pairs = torch.zeros((cap, 2), dtype=torch.int32, device="cuda")
-        self._emit(fillzero=fillzero or realloc)
+        self._refresh(fillzero or realloc)
         self.pairsn = total
 
     # ------------------------------------------------------------------ API
@@ -120,7 +128,6 @@ class GPUCellList:
         """update!(c, fillzero) -- src/celllist.jl:95-134."""
         n = C.c_int64()
         _lib.check(_lib.load().gcl_update(self._h, C.byref(n)))
-        self._refresh_cellpnum()
         self._apply_update_policy(self.pairsn, int(n.value), fillzero)
 
     def partialupdate(self, fillzero: bool = True):

@@ -1293,11 +1293,20 @@ int CellCore::ensure_up() {
       (rc = exclusive_scan_i32_to_i64(cnt_up.as<int32_t>(), rs_up.as<int64_t>(), N, scratch.as<int64_t>(), st)))
     return rc;
   up_scanned = true;
-  GC_CUDA(cudaMemcpyAsync(pin + 1, rs_up.as<int64_t>() + N, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  if ((rc = enqueue_nup())) return rc;
   GC_CUDA(cudaStreamSynchronize(st));
+  take_nup();
+  return GCSPH_OK;
+}
+
+int CellCore::enqueue_nup() {
+  GC_CUDA(cudaMemcpyAsync(pin + 1, rs_up.as<int64_t>() + N, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  return GCSPH_OK;
+}
+
+void CellCore::take_nup() {
   nup = pin[1];
   up_valid = true;
-  return GCSPH_OK;
 }
 
 int CellCore::emit(int32_t* pairs, int64_t cap, int fillzero, int64_t* pairsn) {
@@ -1434,13 +1443,29 @@ int gcl_emit_pairs(gcl_handle* h, int32_t* pairs_dev, int64_t cap, int fillzero,
   return h->core.emit(pairs_dev, cap, fillzero, pairsn_out);
 }
 
-int gcl_cellpnum(gcl_handle* h, int32_t* cellpnum_dev) {
-  if (!h || !cellpnum_dev) return fail(GCSPH_EINVAL, "null argument");
+static int enqueue_cellpnum(gcl_handle* h, int32_t* cellpnum_dev) {
   const int64_t nc = h->core.g.ncell;
   k_cell_pop<<<nblocks(nc, TPB), TPB, 0, h->core.st>>>(h->core.cellstart.as<int32_t>(), nc, cellpnum_dev);
   GC_LAUNCHED();
+  return GCSPH_OK;
+}
+
+int gcl_cellpnum(gcl_handle* h, int32_t* cellpnum_dev) {
+  if (!h || !cellpnum_dev) return fail(GCSPH_EINVAL, "null argument");
+  int rc = enqueue_cellpnum(h, cellpnum_dev);
+  if (rc) return rc;
   GC_CUDA(cudaStreamSynchronize(h->core.st));
   return GCSPH_OK;
+}
+
+int gcl_refresh(gcl_handle* h, int32_t* cellpnum_dev, int32_t* pairs_dev, int64_t cap, int fillzero,
+                int64_t* pairsn_out) {
+  if (!h || !cellpnum_dev) return fail(GCSPH_EINVAL, "null argument");
+  int rc = enqueue_cellpnum(h, cellpnum_dev);
+  if (rc) return rc;
+  rc = h->core.emit(pairs_dev, cap, fillzero, pairsn_out);  // waits, except where it refuses the call
+  if (rc != GCSPH_OK && rc != GCSPH_ECAPACITY) cudaStreamSynchronize(h->core.st);
+  return rc;
 }
 
 int gcl_maxpairs(gcl_handle* h, int64_t* out) {

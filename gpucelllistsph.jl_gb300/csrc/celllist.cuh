@@ -278,6 +278,10 @@ struct CellCore {
   int grow_nbr(int64_t need);
   int read_nfull();
   int ensure_up();
+  // the pair count of scanned offsets (up_scanned), read with whatever the
+  // caller waits for next
+  int enqueue_nup();
+  void take_nup();
   // (min,max) 1-based original indices of every pair, first cap written
   int emit(int32_t* pairs, int64_t cap, int fillzero, int64_t* pairsn);
   // мaxpairs over the current counts (src/gpukernels_cls.jl:109-286)

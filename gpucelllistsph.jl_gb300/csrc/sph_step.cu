@@ -1235,7 +1235,10 @@ static int step_eager(sph_handle* h, StepConst c, int32_t n, int64_t* updaten_ou
   }
   if ((rc = finish_call<D>(h, c, dsc))) return rc;
   GC_CUDA(cudaMemcpyAsync(h->pin, dsc, sizeof(Scal), cudaMemcpyDeviceToHost, st));
+  const bool nup = core.built && core.up_scanned && !core.up_valid;
+  if (nup && (rc = core.enqueue_nup())) return rc;
   GC_CUDA(cudaStreamSynchronize(st));
+  if (nup) core.take_nup();
   timer_collect();
   h->prm.dt = h->pin->dt;
   h->prm.etime = h->pin->etime;
@@ -1423,10 +1426,12 @@ static int step_graph(sph_handle* h, const StepConst& c, int32_t n, int timestep
     h->n_captures += 1;
   }
   g->used = ++h->graph_clock;
+  int rc_up;
   init_scal(h, n);
   GC_CUDA(cudaMemcpyAsync(dsc, h->pin, sizeof(Scal), cudaMemcpyHostToDevice, st));
   GC_CUDA(cudaGraphLaunch(g->exec, st));
   GC_CUDA(cudaMemcpyAsync(h->pin, dsc, sizeof(Scal), cudaMemcpyDeviceToHost, st));
+  if (g->after.up_scanned && (rc_up = core.enqueue_nup())) return rc_up;
   GC_CUDA(cudaStreamSynchronize(st));
   count_launch((int)g->launches);
   timer_account(g->timers);
@@ -1440,6 +1445,7 @@ static int step_graph(sph_handle* h, const StepConst& c, int32_t n, int timestep
     return GCSPH_OK;  // not done: the eager loop runs the call
   }
   set_host_side(h, g->after);
+  if (core.up_scanned) core.take_nup();
   h->n_replays += 1;
   h->prm.dt = h->pin->dt;
   h->prm.etime = h->pin->etime;

@@ -153,7 +153,8 @@ class SPHProblem:
         Returns (updaten, maxcΔxout).  The default timelims are
         (sqrt(eps()), CFL*H/3c₀) as in _stepsolve! (:207)."""
         if timelims is None:
-            timelims = (math.sqrt(_EPS), self.CFL * self.H / (3 * self.c0))
+            p = self._params()
+            timelims = (math.sqrt(_EPS), p.CFL * p.H / (3 * p.c0))
         un = C.c_int64()
         mc = C.c_double()
         prev = self.system.pairsn
@@ -161,7 +162,6 @@ class SPHProblem:
                                         float(timelims[1]), C.byref(un), C.byref(mc)))
         if un.value > 0:
             # update! ran inside: refresh the cell list's user-visible fields
-            self.system._refresh_cellpnum()
             tot = C.c_int64()
             _lib.load().gcl_emit_pairs(self.system._h, None, 0, 0, C.byref(tot))
             self.system._apply_update_policy(prev, int(tot.value), True)

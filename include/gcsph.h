@@ -87,6 +87,11 @@ int gcl_emit_pairs(gcl_handle* h, int32_t* pairs_dev, int64_t cap, int fillzero,
 /* c.cellpnum (Int32[CELL...], column-major) -- src/gpukernels_cls.jl:29-60 */
 int gcl_cellpnum(gcl_handle* h, int32_t* cellpnum_dev);
 
+/* gcl_cellpnum and gcl_emit_pairs with one wait: what a host refreshes after
+ * update! and stepsolve! */
+int gcl_refresh(gcl_handle* h, int32_t* cellpnum_dev, int32_t* pairs_dev, int64_t cap, int fillzero,
+                int64_t* pairsn_out);
+
 /* мaxpairs(c.cellpnum) -- src/gpukernels_cls.jl:109-286 */
 int gcl_maxpairs(gcl_handle* h, int64_t* out);
 
