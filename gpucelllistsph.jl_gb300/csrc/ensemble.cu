@@ -33,16 +33,21 @@ namespace {
 
 constexpr int ENS_MAX_TPB = 512;
 
+// what the stage passes read of an instance for every list entry, in 16-byte
+// groups, so that a branch loads the group it needs with one vector load
+struct __align__(16) StageK {
+  float4 A;  // H², 1/H, dwc, cell edge
+  float4 B;  // ρ₀, η², m₀, DDTgz
+  float4 C;  // kddt, kav, kvisc, (unused)
+  float4 D;  // pfcr, hp1, 2h, kpf
+  float4 E;  // pc[0..3]
+  float4 F;  // fb_d, fb_r0, fb_eta2 of the stage, first particle (int)
+  float4 G;  // 1/ρ₀, P₀, γ (int), bit 0: viscosity, bit 1: surface tension (int)
+};
+
 // per-instance constants (device table, indexed by packing position)
 struct EnsInst {
-  // the stage passes' per-entry constants in 16-byte groups, so that a
-  // branch loads the group it needs with one vector load
-  float4 kA;      // H², 1/H, dwc, cell edge
-  float4 kB;      // ρ₀, η², m₀, DDTgz
-  float4 kC;      // kddt, kav, kvisc, (unused)
-  float4 kD;      // pfcr, hp1, 2h, kpf
-  float4 kE;      // pc[0..3]
-  float4 kFB[2];  // fb_d, fb_r0, fb_eta2, (unused) of stage 1 and stage 2
+  StageK k[2];    // of stage 1 and stage 2
   double origin[3];
   double csinv;  // 1 / cell edge
   double cs;
@@ -252,6 +257,19 @@ __device__ __forceinline__ float eos32(float dr, int pt, const EnsInst& I) {
   return I.P0 * p;
 }
 
+
+// the same from the stage passes' constants
+__device__ __forceinline__ float eos32(float dr, int pt, const StageK& Q) {
+  if (pt <= 1 && dr < 0.f) return 0.f;
+  const float4 g = Q.G;
+  const float e = dr * g.x;
+  float p;
+  if (__float_as_int(g.z) == 7)
+    p = e * (7.f + e * (21.f + e * (35.f + e * (35.f + e * (21.f + e * (7.f + e))))));
+  else
+    p = expm1f((float)__float_as_int(g.z) * log1pf(e));
+  return g.y * p;
+}
 
 // (1+ε)^(1/γ) - 1 (powfancy7th(1+ε) - 1, src/gpukernels_sph.jl:499-515), from
 // the series coefficients pc
@@ -757,44 +775,49 @@ __device__ __forceinline__ float lane_total(const KSum& k, unsigned gm) {
   return s - c;
 }
 
-// a particle's instance: from the table, or (an ensemble of one) from the
-// launch's parameters
-template <bool ONE>
-struct EnsOne {
-  EnsInst one;
-  __device__ __forceinline__ const EnsInst& pick(const EnsInst*, const int32_t*, int64_t) const { return one; }
+// A particle's stage constants: from the launch's parameters, which hold up to
+// N instances', or (N = 0) from the table in global memory.  From the table
+// they were four to five vector loads an entry, a fifth of the requests of an
+// L1 that was 60 to 70% busy; parameters come through the constant cache, and
+// a single instance's as operands.  (20 2-D instances, 743k particles: 453 us a
+// step from the table, 412 from parameters.)
+constexpr int STAGE_TAB = 64;  // 7 KB of parameters, 15 MB in a graph of 1,000 steps
+template <int N, int STAGE>
+struct StageTab {
+  StageK t[N];
+  __device__ __forceinline__ const StageK& pick(const EnsInst*, int s) const { return t[N == 1 ? 0 : s]; }
 };
-template <>
-struct EnsOne<false> {
+template <int STAGE>
+struct StageTab<0, STAGE> {
   int none;
-  __device__ __forceinline__ const EnsInst& pick(const EnsInst* T, const int32_t* inst, int64_t i) const {
-    return T[inst[i]];
-  }
+  __device__ __forceinline__ const StageK& pick(const EnsInst* T, int s) const { return T[s].k[STAGE - 1]; }
 };
 
 // A particle's walk over its list.  FLUID: both sums; else (a real wall
 // particle, ptype 1) ∂ρ/∂t alone -- its acceleration moves nothing and is no
 // output of the engine.
 template <int D, int STAGE, bool RM, bool FLUID>
-__device__ __forceinline__ void stage_row(const EnsArr& A, const EnsInst& I, int64_t i, int lane, const float* oi,
+__device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int64_t i, int lane, const float* oi,
                                           const float* ohi, const float* vi, float dri, float rhoi, float irhoi,
                                           float Pi, KSum& drho, KSum2& accxy, KSum& accz, float& rm2) {
   constexpr int L = stage_lanes<D>();
   const int nn = A.nlc[i];
+  const int p_off = __float_as_int(Q.F.w), gamma = __float_as_int(Q.G.z), opt = __float_as_int(Q.G.w);
+  const bool use_visc = opt & 1, use_pF = opt & 2;
   // the next entry is loaded one iteration ahead: the list streams from
   // DRAM, and its latency then overlaps the current neighbour's arithmetic
   int nxt = lane < nn ? A.nl[(int64_t)lane * A.ncap + i] : 0;
   for (int e = lane; e < nn; e += L) {
     const int ent = nxt;
     if (e + L < nn) nxt = A.nl[(int64_t)(e + L) * A.ncap + i];
-    const Rec<D, STAGE> rec = load_rec<D, STAGE>(A.r1, A.r2, I.p_off + ent_index(ent));
+    const Rec<D, STAGE> rec = load_rec<D, STAGE>(A.r1, A.r2, p_off + ent_index(ent));
     float sh[D];
     ent_shift<D>(ent, sh);
     // the neighbour's record: offsets (at x, and at xΔt½ in stage 2), velocity, δρ, ptype
     float oj[D], hj[D], vj[D], drj, Prec = 0.f;
     int ptj;
     decode_rec<D, STAGE>(rec, oj, hj, vj, drj, ptj, Prec);
-    const float4 kA = I.kA;  // H², 1/H, dwc, cell edge
+    const float4 kA = Q.A;  // H², 1/H, dwc, cell edge
     float d[D];
 #pragma unroll
     for (int q = 0; q < D; ++q) d[q] = fmaf(-sh[q], kA.w, oi[q] - oj[q]);
@@ -816,7 +839,7 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const EnsInst& I, int
       dd[q] = STAGE == 1 ? d[q] : fmaf(-sh[q], kA.w, ohi[q] - hj[q]);
       dv[q] = vi[q] - vj[q];
     }
-    const float4 kB = I.kB;  // ρ₀, η², m₀, DDTgz
+    const float4 kB = Q.B;  // ρ₀, η², m₀, DDTgz
     if (!FLUID) {
       drho.add(kB.z * dot32<D>(dv, gw));
       continue;
@@ -833,30 +856,30 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const EnsInst& I, int
       const float inv = __fdividef(1.f, r2d + kB.y);
       // ∂v∂t!
       float Pj = Prec;
-      if (!rec_has_p<D, STAGE>()) Pj = eos32(drj, ptj, I);
+      if (!rec_has_p<D, STAGE>()) Pj = eos32(drj, ptj, Q);
       gsc = -kB.z * (Pi + Pj) * (irhoi * irhoj);
-      const float4 kC = I.kC;  // kddt, kav, kvisc
+      const float4 kC = Q.C;  // kddt, kav, kvisc
       const float ddgw = dot32<D>(dd, gw);
       // ∂ρ∂tDDT!
       float term = kB.z * dot32<D>(dv, gw);
-      const float dp = kB.x * root_m1g(kB.w * dd[1], I.kE, I.gamma);
+      const float dp = kB.x * root_m1g(kB.w * dd[1], Q.E, gamma);
       term += kC.x * ((drj - dri) - dp) * inv * (-ddgw) * irhoj;
       drho.add(term);
       const float cond = dot32<D>(dv, dd);
-      if (cond < 0.f || I.use_visc) {
+      if (cond < 0.f || use_visc) {
         const float ii = __fdividef(1.f, rhoi + rhoj) * inv;
         // ∂v∂t_av!: -Π m₀ = 2 α c₀ h m₀ (Δv·Δx) / ((r² + η²)(ρi + ρj))
         if (cond < 0.f) gsc += kC.y * cond * ii;
-        if (I.use_visc) {
+        if (use_visc) {
           // ∂v∂t_visc!
           const float nt = kC.z * ddgw * ii;
 #pragma unroll
           for (int q = 0; q < D; ++q) f[q] = nt * dv[q];
         }
       }
-      if (I.use_pF) {
+      if (use_pF) {
         // ∂v∂tpF! (in stage 1 the separation is r itself)
-        const float4 kD = I.kD;  // pfcr, hp1, 2h, kpf
+        const float4 kD = Q.D;  // pfcr, hp1, 2h, kpf
         const float rd = STAGE == 1 ? r : (r2d > 0.f ? r2d * rsqrtf(r2d) : 0.f);
         if (rd < kD.z) {
           const float scos = kD.w * __cosf(kD.x * rd) * __fdividef(1.f, rd + kD.y);  // argument in [0, 1.5π)
@@ -865,7 +888,7 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const EnsInst& I, int
         }
       }
     } else {
-      const float4 kF = I.kFB[STAGE - 1];  // fb_d, fb_r0, fb_eta2
+      const float4 kF = Q.F;  // fb_d, fb_r0, fb_eta2
       if (r < kF.y) {
         // fbmolforce! at x
         const float qq = kF.y * __fdividef(1.f, r + kF.z);
@@ -883,12 +906,9 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const EnsInst& I, int
 // two blocks of 512 per SM: at most 64 registers.  RM (stage 1): keep each
 // row's smallest r² for dpcreg!'s row bound (a separate instantiation, so the
 // ensembles without dpcreg! run the loop without it)
-// ONE: an ensemble of one instance takes its constants from the launch's
-// parameters (constant-bank operands) instead of loading them from the table,
-// 16 bytes at a time, for every entry.
-template <int D, int STAGE, bool RM, bool ONE>
+template <int D, int STAGE, bool RM, int N>
 __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const EnsInst* __restrict__ T,
-                                                              const __grid_constant__ EnsOne<ONE> one) {
+                                                              const __grid_constant__ StageTab<N, STAGE> tab) {
   if (*A.ovf) return;
   constexpr int L = stage_lanes<D>();
   const unsigned lanew = threadIdx.x & 31u;
@@ -897,7 +917,9 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const En
   const int lane = (int)(lanew - gbase);
   const int64_t groups = ((int64_t)gridDim.x * blockDim.x) / L;
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L; i < A.N; i += groups) {
-    const EnsInst& I = one.pick(T, A.inst, i);
+    const int si = A.inst[i];
+    const EnsInst& I = T[si];
+    const StageK& Q = tab.pick(T, si);
     float oi[D], ohi[D], vi[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -918,9 +940,9 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const En
     // both, a real wall particle ∂ρ/∂t, any other wall particle neither (390k
     // particles in 3-D, two thirds of them walls, stage 1 357 -> 276 us)
     if (pti > 1)
-      stage_row<D, STAGE, RM, true>(A, I, i, lane, oi, ohi, vi, dri, rhoi, irhoi, Pi, drho, accxy, accz, rm2);
+      stage_row<D, STAGE, RM, true>(A, Q, i, lane, oi, ohi, vi, dri, rhoi, irhoi, Pi, drho, accxy, accz, rm2);
     else if (pti > 0)
-      stage_row<D, STAGE, RM, false>(A, I, i, lane, oi, ohi, vi, dri, rhoi, irhoi, Pi, drho, accxy, accz, rm2);
+      stage_row<D, STAGE, RM, false>(A, Q, i, lane, oi, ohi, vi, dri, rhoi, irhoi, Pi, drho, accxy, accz, rm2);
     KSum acc[D];
     acc[0] = accxy.part(0);
     acc[1] = accxy.part(1);
@@ -1685,6 +1707,7 @@ int ens_relayout(gcsph_ens* e) {
   for (EnsHostInst& h : e->inst) {
     h.p_off = p;
     h.dev.p_off = (int)p;
+    for (StageK& q : h.dev.k) memcpy(&q.F.w, &h.dev.p_off, sizeof(float));
     h.key_off = k;
     h.dev.key_off = (int)k;
     p += h.n;
@@ -1793,9 +1816,9 @@ int ens_occupancy(gcsph_ens* e) {
   for (int t = 0; t < 3; ++t) {
     int b = 0;
     if (e->D == 2)
-      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (k_ens_stage<2, 2, false, false>), kTpbs[t], 0));
+      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (k_ens_stage<2, 2, false, 0>), kTpbs[t], 0));
     else
-      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (k_ens_stage<3, 2, false, false>), kTpbs[t], 0));
+      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, (k_ens_stage<3, 2, false, 0>), kTpbs[t], 0));
     e->occ[t] = std::max(b, 1);
     int b2 = 0;
     if (e->D == 2)
@@ -1838,6 +1861,32 @@ int tpb_index(int tpb) {
 // waves; persistent 0.15 ms against 0.18 at 0.4 M, 1.7 waves)
 int wave_grid(int64_t want, int64_t slots) {
   return (int)std::max<int64_t>(1, want >= 4 * slots ? want : std::min<int64_t>(want, slots));
+}
+
+template <int D, int STAGE, int N>
+void launch_stage_n(const gcsph_ens* e, const EnsArr& A, const EnsInst* T, int grid, int tpb, cudaStream_t st) {
+  StageTab<N, STAGE> tab{};
+  if constexpr (N > 0)
+    for (size_t q = 0; q < e->inst.size(); ++q) tab.t[q] = e->inst[q].dev.k[STAGE - 1];
+  if constexpr (STAGE == 1) {
+    if (A.rmin2) {
+      k_ens_stage<D, 1, true, N><<<grid, tpb, 0, st>>>(A, T, tab);
+      return;
+    }
+  }
+  k_ens_stage<D, STAGE, false, N><<<grid, tpb, 0, st>>>(A, T, tab);
+}
+
+// a stage pass, its constants from the launch's parameters where they fit
+template <int D, int STAGE>
+void launch_stage(const gcsph_ens* e, const EnsArr& A, const EnsInst* T, int grid, int tpb, cudaStream_t st) {
+  const size_t ni = e->inst.size();
+  if (ni == 1)
+    launch_stage_n<D, STAGE, 1>(e, A, T, grid, tpb, st);
+  else if (ni <= (size_t)STAGE_TAB)
+    launch_stage_n<D, STAGE, STAGE_TAB>(e, A, T, grid, tpb, st);
+  else
+    launch_stage_n<D, STAGE, 0>(e, A, T, grid, tpb, st);
 }
 
 template <int D>
@@ -1908,25 +1957,11 @@ int ens_enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
   // 3-D dam break's stage passes 8% faster at 0.4 M and 2 M particles)
   const int sgrid = (int)std::max<int64_t>(1, swant);
   timer_begin(T_STAGE1, st);
-  const bool one = e->inst.size() == 1;
-  EnsOne<true> o1{};
-  if (one) o1.one = e->inst[0].dev;
-  const EnsOne<false> o0{};
-  if (A.rmin2 && one)
-    k_ens_stage<D, 1, true, true><<<sgrid, tpb, 0, st>>>(A, T, o1);
-  else if (A.rmin2)
-    k_ens_stage<D, 1, true, false><<<sgrid, tpb, 0, st>>>(A, T, o0);
-  else if (one)
-    k_ens_stage<D, 1, false, true><<<sgrid, tpb, 0, st>>>(A, T, o1);
-  else
-    k_ens_stage<D, 1, false, false><<<sgrid, tpb, 0, st>>>(A, T, o0);
+  launch_stage<D, 1>(e, A, T, sgrid, tpb, st);
   GC_LAUNCHED();
   timer_end(T_STAGE1, st);
   timer_begin(T_STAGE2, st);
-  if (one)
-    k_ens_stage<D, 2, false, true><<<sgrid, tpb, 0, st>>>(A, T, o1);
-  else
-    k_ens_stage<D, 2, false, false><<<sgrid, tpb, 0, st>>>(A, T, o0);
+  launch_stage<D, 2>(e, A, T, sgrid, tpb, st);
   GC_LAUNCHED();
   timer_end(T_STAGE2, st);
   const int32_t ninst = (int32_t)e->inst.size();
@@ -2328,12 +2363,21 @@ int ens_add(gcsph_ens* e, int64_t n, const double* x, const double* v, const dou
   I.kav = (float)(2.0 * p->alpha * p->c0 * p->h * p->m0);
   I.kvisc = (float)(4.0 * p->nu * p->m0);
   I.kpf = (float)(p->s / p->m0);
-  I.kA = make_float4(I.H2, I.Hinv, I.dwc, I.csf);
-  I.kB = make_float4(I.rho0, I.eta2, I.m0, I.DDTgz);
-  I.kC = make_float4(I.kddt, I.kav, I.kvisc, 0.f);
-  I.kD = make_float4(I.pfcr, I.hp1, I.twoh, I.kpf);
-  I.kE = make_float4(I.pc[0], I.pc[1], I.pc[2], I.pc[3]);
-  for (int st = 0; st < 2; ++st) I.kFB[st] = make_float4(I.fb_d[st], I.fb_r0[st], I.fb_eta2[st], 0.f);
+  auto as_float = [](int v) {
+    float f;
+    memcpy(&f, &v, sizeof(f));
+    return f;
+  };
+  for (int st = 0; st < 2; ++st) {
+    StageK& K = I.k[st];
+    K.A = make_float4(I.H2, I.Hinv, I.dwc, I.csf);
+    K.B = make_float4(I.rho0, I.eta2, I.m0, I.DDTgz);
+    K.C = make_float4(I.kddt, I.kav, I.kvisc, 0.f);
+    K.D = make_float4(I.pfcr, I.hp1, I.twoh, I.kpf);
+    K.E = make_float4(I.pc[0], I.pc[1], I.pc[2], I.pc[3]);
+    K.F = make_float4(I.fb_d[st], I.fb_r0[st], I.fb_eta2[st], 0.f);  // .w: ens_relayout
+    K.G = make_float4(I.rho0inv, I.P0, as_float(I.gamma), as_float((I.use_visc ? 1 : 0) | (I.use_pF ? 2 : 0)));
+  }
   // host staging in the engine's types
   std::vector<float> vf((size_t)D * n, 0.f), drf((size_t)n);
   std::vector<int32_t> ids((size_t)n);
