@@ -20,6 +20,7 @@ K = 10            # highest power kept in the exact series
 EPS_MAX = F(1, 128)
 EPS_SHORT = F(1, 1024)  # a shorter head of the same series serves |eps| <= EPS_SHORT
 TOL = 2.0 ** -64  # dropped tail, relative to 1
+TOL_SHORT = 2.0 ** -55  # the head's: a quarter of the rounding of the reference's 1 + eps
 
 
 def smul(a, b):
@@ -112,9 +113,9 @@ def horner(c, e):
 
 def short_terms(c):
     """Terms of series c that matter for |eps| <= EPS_SHORT (the dropped
-    tail stays below TOL relative to 1)."""
+    tail stays below TOL_SHORT relative to 1)."""
     n = len(c) - 1
-    while n > 1 and abs(c[n]) * float(EPS_SHORT) ** n < TOL:
+    while n > 1 and abs(c[n]) * float(EPS_SHORT) ** n < TOL_SHORT:
         n -= 1
     return n + 1
 

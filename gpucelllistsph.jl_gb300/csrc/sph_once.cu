@@ -32,7 +32,7 @@ __device__ inline void fb_pair(const StepConst& c, const double* dx, double r2, 
 //  * ∂ρ∂tDDT! (:542-631): both sides share DDTkh m₀ (-Δx·∇W)/(r² + η²);
 //  * ∂v∂t! (:740-776) and ∂v∂t_av! (:852-901) as one factor of m₀∇W,
 //    -(Pk + Pm)/(ρk ρm) + 2 α c₀ h (Δv·Δx)/((r² + η²)(ρk + ρm));
-//  * ∂v∂tpF! (:1373-1409) with the products s/m₀ and 1.5π/2h.
+//  * ∂v∂tpF! (:1373-1409) as one factor of Δx, its cosine from r² (pf_cos).
 // The FP64 pipe bounds the pass, so a pair runs only the terms its ptypes
 // allow (PairClass), and a warp runs 32 pairs of one class: a warp's FP64
 // instruction takes the pipe 16 cycles whatever lanes are active.
@@ -96,15 +96,14 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
     const double r2 = dotD<D>(dx, dx);
     const double cond = dotD<D>(dv, dx);
     const bool r2pos = dbits(r2) != 0;  // r2 is +0 or positive
-    double r = 0.0, dxgw, dvgw;
+    double r = 0.0, dr = 0.0, dxgw, dvgw;
     if (STAGE == 1) {
       if (r2pos) r = sqrt_nr(r2);
-      const double uu = r * c.Hinv;
+      const double t = fma(-r, c.Hinv, 1.0);  // 1 - u
       double w = 0.0, dwr = 0.0;
-      if (dbits(uu) < ONE_BITS) {
-        const double t = 1.0 - uu;
+      if ((unsigned long long)dbits(t) - 1ull < (unsigned long long)ONE_BITS) {  // 0 < 1 - u <= 1, and not NaN
         const double t2 = t * t;
-        if (c.need_w) w = ((1.0 + 4.0 * uu) * (t2 * t2)) * c.nW;
+        if (c.need_w) w = (fma(-4.0, t, 5.0) * (t2 * t2)) * c.nW;
         dwr = (t2 * t) * c.dWr;
       }
       if (!r2pos) dwr = NAN;  // the reference's d𝒲(0)/0
@@ -121,10 +120,10 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
         gw[d] = dx[d] * dwr;
         S.gWe[d][u] = gw[d];
       }
+      dr = dwr;
       dxgw = r2 * dwr;
       dvgw = cond * dwr;
     } else {
-      if (c.use_pF && r2pos) r = sqrt_nr(r2);
 #pragma unroll
       for (int d = 0; d < D; ++d) gw[d] = S.gWe[d][u];
       dxgw = dotD<D>(dx, gw);
@@ -134,36 +133,48 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
     double sg = press ? -((PP[k] + PP[m]) * (irk * irm)) : 0.0;
     double visc = 0.0;
     if (both) {
-      const double inv = rcp_nr(r2 + c.eta2);
+      const double s = rk + rm;
+      const double ii = rcp_nr(s * (r2 + c.eta2));
+      const double g = dxgw * ii;
       dk = dvgw;
       dm = dk;
       if (ptk > 1 || ptm > 1) {
-        const double com = c.DDTkh * (-dxgw) * inv;
+        const double com = -(c.DDTkh * g) * s;
         const double ez = c.DDTgz * dx[1];
         const double drr = rm - rk;
         if (ptk > 1) {
-          const double dp = c.rho0 * (1.0 + pf7m1_fast(ez, c.ginv, c.gamma)) - c.rho0;
+          const double dp = c.rho0 * (1.0 + pf7m1_fast((1.0 + ez) - 1.0, c.ginv, c.gamma)) - c.rho0;
           dk += (drr - dp) * com * irm;
         }
         if (ptm > 1) {
-          const double dn = c.rho0 * (1.0 + pf7m1_fast(-ez, c.ginv, c.gamma)) - c.rho0;
+          const double dn = c.rho0 * (1.0 + pf7m1_fast((1.0 - ez) - 1.0, c.ginv, c.gamma)) - c.rho0;
           dm += (-drr - dn) * com * irk;
         }
       }
-      const bool av = neg_int(cond);
-      if (av || c.use_visc) {
-        const double ii = rcp_nr(rk + rm) * inv;
-        if (av) sg += c.avK * cond * ii;
-        if (c.use_visc) visc = c.visc4 * dxgw * ii;
-      }
+      if (neg_int(cond)) sg += c.avK * (cond * ii);
+      if (c.use_visc) visc = c.visc4 * g;
     }
-#pragma unroll
-    for (int d = 0; d < D; ++d) f[d] = c.use_visc ? fma(visc, dv[d], sg * gw[d]) : sg * gw[d];
-    if (c.use_pF && both && dbits(r) < dbits(c.twoh)) {
-      const double scos = c.pfs * cos_fast(c.pfk * r) * rcp_nr(r + c.hp1);
-#pragma unroll
-      for (int d = 0; d < D; ++d) f[d] = fma(scos, dx[d], f[d]);
+    const bool pF = c.use_pF && both && (STAGE == 1 ? dbits(r) < dbits(c.twoh) : true);
+    double scos = 0.0;
+    if (pF) {
+      if (STAGE == 2 && r2pos) r = sqrt_nr(r2);
+      if (STAGE == 1 || dbits(r) < dbits(c.twoh)) scos = c.pfs * pf_cos(r2, c.pfk2) * rcp_nr(r + c.hp1);
     }
+    if (STAGE == 1 && c.use_pF) {
+      // everything along Δx in one factor
+      const double a = fma(sg, dr, scos);
+#pragma unroll
+      for (int d = 0; d < D; ++d) f[d] = a * dx[d];
+    } else {
+#pragma unroll
+      for (int d = 0; d < D; ++d) f[d] = sg * gw[d];
+      if (pF)
+#pragma unroll
+        for (int d = 0; d < D; ++d) f[d] = fma(scos, dx[d], f[d]);
+    }
+    if (c.use_visc)
+#pragma unroll
+      for (int d = 0; d < D; ++d) f[d] = fma(visc, dv[d], f[d]);
   }
   put_slot(B.ce + e, dk, f[0], f[1], f[2]);
   put_slot(B.ce + me, dm, -f[0], -f[1], -f[2]);

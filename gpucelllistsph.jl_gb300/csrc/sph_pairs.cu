@@ -11,7 +11,7 @@
 // reference's expressions and IEEE divisions and roots, bit for bit.  The
 // terms that go into sums are bound by the FP64 pipe (80 to 87% busy, the
 // atomics well behind), so they take the pair-once forms of the fused step:
-// reciprocals, roots and the cosine by rcp_pair, sqrt_pair and cos_fast,
+// reciprocals, roots and the cosine by rcp_pair, sqrt_pair and pf_cos,
 // powfancy7th by its series, dot products and products of constants fused.
 // Measured with the queue below (one GB300, 10.5M pairs of a 3-D tank, 179k
 // particles): ∂v∂tpF! 1577 -> 388 us, ∂ρ∂tDDT! 1403 -> 478, sph∑W! 499 -> 310,
@@ -247,12 +247,12 @@ struct TermDDT {
       const double com = DDTkhm0 * -dotf<D>(dx, gw) * rcp_pair(dotf<D>(dx, dx) + eta2);
       const double ez = DDTgz * dx[1], drr = rj - ri;
       if (pi > 1) {
-        const double dp = fma(rho0, 1.0 + pf7m1_fast(ez, ginv, gamma), -rho0);
-        si = fma((drr - dp) * com, rcp_pair(rj), si);
+        const double d = fma(-rho0, pf7m1_fast(ez, ginv, gamma), drr);
+        si = fma(d * com, rcp_pair(rj), si);
       }
       if (pj > 1) {
-        const double dn = fma(rho0, 1.0 + pf7m1_fast(-ez, ginv, gamma), -rho0);
-        sj = fma((-drr - dn) * com, rcp_pair(ri), sj);
+        const double d = fma(-rho0, pf7m1_fast(-ez, ginv, gamma), -drr);
+        sj = fma(d * com, rcp_pair(ri), sj);
       }
     }
     atomicAdd(&out[i], si);
@@ -369,21 +369,22 @@ struct TermWall {
   }
 };
 
-// kernel_∂v∂tpF! (:1382-1409): sm = s/m₀, pfk = 1.5π/2h, hp1 = 0.1h
+// kernel_∂v∂tpF! (:1382-1409): sm = s/m₀, pfk2 = 2/(2h)², hp1 = 0.1h
 template <int D>
 struct TermTension {
   static constexpr bool QUEUE = true;
   V3 x;
-  double sm, twoh, pfk, hp1;
+  double sm, twoh, pfk2, hp1;
   const int32_t* pt;
   W3 a;
   __device__ bool take(int pi, int pj) const { return pi > 0 && pj > 0; }
   __device__ void run(int64_t, int64_t i, int64_t j) const {
     double dx[D];
     pair_dx<D>(x, i, j, dx);
-    const double r = sqrt_pair(dotf<D>(dx, dx));
+    const double r2 = dotf<D>(dx, dx);
+    const double r = sqrt_pair(r2);
     if (!(r < twoh)) return;
-    const double scos = sm * cos_fast(pfk * r) * rcp_pair(r + hp1);
+    const double scos = sm * pf_cos(r2, pfk2) * rcp_pair(r + hp1);
     double f[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) f[d] = scos * dx[d];
@@ -823,9 +824,9 @@ int gcsph_dvdt_pF(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const d
   if (!pt) return fail(GCSPH_EINVAL, "null ptype");
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const double sm = s / m0, twoh = 2.0 * h, pfk = 1.5 * GCSPH_PI64 / twoh, hp1 = 0.1 * h;
+  const double sm = s / m0, twoh = 2.0 * h, pfk2 = 2.0 / (twoh * twoh), hp1 = 0.1 * h;
   (void)N;
-  TERM(D, st, (TermTension<2>{x, sm, twoh, pfk, hp1, pt, a}), (TermTension<3>{x, sm, twoh, pfk, hp1, pt, a}));
+  TERM(D, st, (TermTension<2>{x, sm, twoh, pfk2, hp1, pt, a}), (TermTension<3>{x, sm, twoh, pfk2, hp1, pt, a}));
 }
 
 int gcsph_update_rho(int64_t N, double* rho, const double* drho, double dt, double rho0, const int32_t* pt,

@@ -711,7 +711,7 @@ static StepConst make_const(const sph_handle* h) {
   c.visc4 = 4.0 * p.nu;
   c.twoh = 2.0 * p.h;
   c.pfc = 1.5 * GCSPH_PI64;
-  c.pfk = 1.5 * GCSPH_PI64 / (2.0 * p.h);
+  c.pfk2 = 2.0 / ((2.0 * p.h) * (2.0 * p.h));
   c.pfs = p.s / p.m0;
   c.hp1 = 0.1 * p.h;
   c.use_visc = p.nu > 0;

@@ -20,7 +20,7 @@ struct StepConst {
   double dWr, avK, visc4;
   double dWg;                   // d𝒲/r = dWg (1 - u)^3 (∑∇W of a call)
   double twoh, pfc, hp1;        // 2h, 1.5*pi, 0.1h  (∂v∂tpF!)
-  double pfk, pfs;              // 1.5 pi / 2h and s / m₀ (∂v∂tpF! of the pair-once pass)
+  double pfk2, pfs;             // 2 / (2h)² and s / m₀ (∂v∂tpF! of the pair-once pass)
   double dpc_l0inv, dpc_nW, dpc_whinv, dpc_pmin, dpc_pmax, dpc_lambda, dpc_kernlim, dpc_eta2;
   double dpc_r2cut;  // l0² (1 + 1e-6): past it u = √r² / l0 >= 1 whatever the rounding
   double xsph_c;                // 2*m0*eps
@@ -341,42 +341,35 @@ __device__ inline double sqrt_nr2(double x) {
   return x * y;
 }
 
-// cos(t) for 0 <= t < 3π/2 (∂v∂tpF! inside 2h): reduction by the nearest
-// multiple of π/2 (head and tail in FMAs), then one Taylor series, cosine's or
-// sine's by the quadrant's parity -- the coefficients are selected on the
-// integer pipe, so the FP64 pipe runs one series rather than gc_cos's two.
-__device__ inline double cos_fast(double t) {
-  const double C[8] = {-0.5, 0.041666666666666664, -0.001388888888888889, 2.48015873015873e-05,
-                       -2.755731922398589e-07, 2.08767569878681e-09, -1.1470745597729725e-11, 4.779477332387385e-14};
-  const double S[8] = {-0.16666666666666666, 0.008333333333333333, -0.0001984126984126984, 2.7557319223985893e-06,
-                       -2.505210838544172e-08, 1.6059043836821613e-10, -7.647163731819816e-13, 2.8114572543455206e-15};
-  const double MAGIC = 6755399441055744.0;  // 1.5 * 2^52: the sum's low mantissa bits are the rounded integer
-  const double km = fma(t, 0.6366197723675814, MAGIC);
-  const int q = (int)dbits(km);
-  const double kd = km - MAGIC;
-  double r = fma(-kd, 1.5707963267948966, t);
-  r = fma(-kd, 6.123233995736766e-17, r);
-  const double z = r * r;
-  const bool odd = q & 1;
-  double p = odd ? S[7] : C[7];
+// cos(1.5π r/2h) of ∂v∂tpF! inside 2h, from r²: with s = 2 (r/2h)² - 1 it is
+// cos(1.5π sqrt((1 + s)/2)), an entire function of s, and s covers [-1, 1];
+// its Chebyshev series falls by about 100 a term there, and the series to the
+// 12th degree (the next coefficient is 1.9e-17), in powers of s, is the
+// polynomial.  k = 2/(2h)².  13 FP64 instructions and no reduction, where a
+// reduction by π/2 and a Taylor series took 16; the worst error over pairs at
+// random separations is 5.8e-16 (1.5e-15 by way of r).
+__device__ inline double pf_cos(double r2, double k) {
+  const double C[13] = {-0.9818965112591632,  0.31558602480454173,   1.2838905431807321,    -0.7879472662466167,
+                        0.19547895338475096,  -0.027475032586512103, 0.00251908751511393,   -0.00016342789686839775,
+                        7.918215700351492e-06, -2.9785382234404e-07, 8.958338323810472e-09, -2.2072216601308446e-10,
+                        4.5275475585621706e-12};
+  const double s = fma(r2, k, -1.0);
+  double p = C[12];
 #pragma unroll
-  for (int i = 6; i >= 0; --i) p = fma(p, z, odd ? S[i] : C[i]);
-  const double zr = z * r;
-  const double v = fma(odd ? zr : z, p, odd ? r : 1.0);
-  // cos t = cos r, -sin r, -cos r, sin r in the quadrants 0 .. 3
-  return __longlong_as_double(dbits(v) ^ ((long long)((q + 1) & 2) << 62));
+  for (int i = 11; i >= 0; --i) p = fma(p, s, C[i]);
+  return p;
 }
 
-// powfancy7th(x) - 1 for x = 1 + eps, src/gpukernels_sph.jl:499-515.  Where
-// |eps| <= PF7_EPS_MAX the exact Taylor series of that iteration's output
+// powfancy7th(1 + e) - 1, src/gpukernels_sph.jl:499-515.  Where |e| <=
+// PF7_EPS_MAX the exact Taylor series of that iteration's output
 // (gen_pf7_series.py, bias included) replaces its two divisions, and where
-// |eps| <= PF7_EPS_SHORT its first PF7_SHORT_N terms do; elsewhere the
-// iteration itself runs.  eps is taken as (1 + eps) - 1, the argument the
-// reference's rounded x carries.  Callers form ρ0 (1 + r) - ρ0 as the
-// reference forms ρ0 t - ρ0: 1 + r rounds to the t the iteration returns.
-__device__ inline double pf7m1_fast(double eps_in, double ginv, int gamma) {
-  const double x = 1.0 + eps_in;
-  const double e = x - 1.0;  // exact for x in [0.5, 2]
+// |e| <= PF7_EPS_SHORT its first PF7_SHORT_N terms do; elsewhere the iteration
+// itself runs.  e is taken as it is; the step's passes hand in (1 + eps) - 1,
+// the argument that the reference's rounded x carries, and form ρ0 (1 + r) - ρ0
+// as the reference forms ρ0 t - ρ0: near rest the whole term is of the size of
+// these roundings (without them a resting tank's largest ∂ρ/∂t, 1.9e-8, is
+// 1.1e-12 of it off the oracle's).
+__device__ inline double pf7m1_fast(double e, double ginv, int gamma) {
   const long long ae = dbits(e) & 0x7FFFFFFFFFFFFFFFLL;
   static_assert(PF7_UP_N == PF7_LO_N, "series lengths");
   if (gamma == 7 && ae <= dbits(PF7_EPS_MAX)) {
@@ -395,7 +388,7 @@ __device__ inline double pf7m1_fast(double eps_in, double ginv, int gamma) {
     }
     return r;
   }
-  return powfancy7th_1div(x, ginv, gamma) - 1.0;
+  return powfancy7th_1div(1.0 + e, ginv, gamma) - 1.0;
 }
 
 // pair-once passes (sph_once.cu): pass A over the device-side pair count,
