@@ -68,6 +68,32 @@ __device__ __forceinline__ int4 pair_load(const SArr<D>& S, const PairBuf& B, in
   return q;
 }
 
+// -x on the integer pipe
+__device__ __forceinline__ double flip(double x) { return __longlong_as_double(dbits(x) ^ (1ll << 63)); }
+
+// A pair past the reach of every term (H, and 2h with ∂v∂tpF!), as a list with
+// a skin holds them: its slots, W and ∇W are zero.  Stage 2 takes stage 1's ∇W
+// and ∂v∂tpF! at xΔt½.  Such a pair then costs 2 D + 2 FP64 instructions instead
+// of 70 to 90, which every pair pays, so make_const sets far_r2 only for lists
+// that reach 3% past (break-even: 5% of the pairs).  No far pair is NaN or
+// infinite: those run through the terms.
+template <int D, int STAGE>
+__device__ __forceinline__ bool pair_far(const StepConst& c, const SArr<D>& S, int u, const int4 q) {
+  if (STAGE == 2) {
+    long long any = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) any |= dbits(S.gWe[d][u]);
+    if ((any << 1) != 0) return false;
+    if (!c.use_pF) return true;
+  }
+  const double* const* XP = STAGE == 1 ? S.x : S.xh;
+  double dx[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) dx[d] = XP[d][q.x] - XP[d][q.y];
+  const double r2 = dotD<D>(dx, dx);
+  return dbits(r2) > dbits(c.far_r2) && dbits(r2) < dbits((double)INFINITY);
+}
+
 template <int D, int STAGE>
 __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, const PairBuf& B, int u,
                                           const int4 q, const int ptk, const int ptm) {
@@ -103,13 +129,13 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
       double w = 0.0, dwr = 0.0;
       if ((unsigned long long)dbits(t) - 1ull < (unsigned long long)ONE_BITS) {  // 0 < 1 - u <= 1, and not NaN
         const double t2 = t * t;
-        if (c.need_w) w = (fma(-4.0, t, 5.0) * (t2 * t2)) * c.nW;
+        if (c.need_w) w = fma(-4.0, t, 5.0) * (t2 * t2);
         dwr = (t2 * t) * c.dWr;
       }
       if (!r2pos) dwr = NAN;  // the reference's d𝒲(0)/0
       if (c.need_w) {
-        // both rows' slots: xsphcorr! and cspmcorr! walk every row (and read
-        // the pairs of two real sides only)
+        // (without 𝒲's norm) in both rows' slots: xsphcorr! and cspmcorr! walk
+        // every row (and read the pairs of two real sides only)
         S.We[e] = w;
         S.We[me] = w;
       }
@@ -143,11 +169,11 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
         const double ez = c.DDTgz * dx[1];
         const double drr = rm - rk;
         if (ptk > 1) {
-          const double dp = c.rho0 * (1.0 + pf7m1_fast((1.0 + ez) - 1.0, c.ginv, c.gamma)) - c.rho0;
+          const double dp = c.rho0 * pf7_fast(ez, c.ginv, c.gamma) - c.rho0;
           dk += (drr - dp) * com * irm;
         }
         if (ptm > 1) {
-          const double dn = c.rho0 * (1.0 + pf7m1_fast((1.0 - ez) - 1.0, c.ginv, c.gamma)) - c.rho0;
+          const double dn = c.rho0 * pf7_fast(-ez, c.ginv, c.gamma) - c.rho0;
           dm += (-drr - dn) * com * irk;
         }
       }
@@ -158,7 +184,7 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
     double scos = 0.0;
     if (pF) {
       if (STAGE == 2 && r2pos) r = sqrt_nr(r2);
-      if (STAGE == 1 || dbits(r) < dbits(c.twoh)) scos = c.pfs * pf_cos(r2, c.pfk2) * rcp_nr(r + c.hp1);
+      if (STAGE == 1 || dbits(r) < dbits(c.twoh)) scos = pf_cos(r2, c.pfk2, c.pfc_s) * rcp_nr(r + c.hp1);
     }
     if (STAGE == 1 && c.use_pF) {
       // everything along Δx in one factor
@@ -177,7 +203,7 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
       for (int d = 0; d < D; ++d) f[d] = fma(visc, dv[d], f[d]);
   }
   put_slot(B.ce + e, dk, f[0], f[1], f[2]);
-  put_slot(B.ce + me, dm, -f[0], -f[1], -f[2]);
+  put_slot(B.ce + me, dm, flip(f[0]), flip(f[1]), flip(f[2]));
 }
 
 // Pass A over all pairs in chunks of 32 consecutive pairs, one chunk per warp
@@ -210,8 +236,21 @@ __global__ void __launch_bounds__(PA_TPB, 1) k_pairA(StepConst c, SArr<D> S, Pai
     q = pair_load<D, STAGE>(S, B, u);
     ptk = S.pt[q.x];
     ptm = S.pt[q.y];
-    const int cl = pair_class(ptk, ptm);
-    if (STAGE == 1 && cl == PC_NONE) {
+    int cl = pair_class(ptk, ptm);
+    bool far = false;
+    if (QUEUE && c.far_r2 > 0.0 && (cl == PC_FLUID || cl == PC_WALL)) far = pair_far<D, STAGE>(c, S, (int)u, q);
+    if (far) {
+      cl = PC_NONE;
+      if (STAGE == 1) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) S.gWe[d][u] = 0.0;
+        if (c.need_w) {
+          S.We[q.z] = 0.0;
+          S.We[q.w] = 0.0;
+        }
+      }
+    }
+    if ((STAGE == 1 && cl == PC_NONE) || far) {
       put_slot(B.ce + q.z, 0.0, 0.0, 0.0, 0.0);
       put_slot(B.ce + q.w, 0.0, 0.0, 0.0, 0.0);
     }
@@ -641,7 +680,7 @@ __global__ void __launch_bounds__(STPB) k_xsph_rows(StepConst c, const Scal* __r
 #pragma unroll
       for (int j = 0; j < GATHER_U; ++j) {
         if (!(pt[j] > 1) || m[j] == k) continue;
-        const double xs = c.xsph_c * w[j] * rcp_nr(rk + rm[j]);
+        const double xs = w[j] * rcp_nr(rk + rm[j]);
 #pragma unroll
         for (int d = 0; d < D; ++d) sum[d] += (vm[j][d] - vk[d]) * xs;
       }
@@ -652,8 +691,9 @@ __global__ void __launch_bounds__(STPB) k_xsph_rows(StepConst c, const Scal* __r
   const double dt = sc->dt;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    S.buf2[d][k] = sum[d];
-    if (ptk > 1) S.x[d][k] = S.x[d][k] + sum[d] * dt;
+    const double u = sum[d] * (c.xsph_c * c.nW);
+    S.buf2[d][k] = u;
+    if (ptk > 1) S.x[d][k] = S.x[d][k] + u * dt;
   }
 }
 
@@ -687,9 +727,8 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
 #pragma unroll
       for (int j = 0; j < GATHER_U; ++j) {
         if (!(pt[j] > 0) || m[j] == k) continue;
-        const double mw = c.m0 * w[j];
-        s[0] += mw;
-        s[1] += mw * rcp_nr(rm[j]);
+        s[0] += w[j];
+        s[1] += w[j] * rcp_nr(rm[j]);
       }
     }
     lanes_sum4<L>(s, lane, group_mask<L>());
@@ -701,8 +740,9 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
   S.rhoo[k] = rv;
   S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
   S.ir[k] = 1.0 / rv;
-  S.buf2[0][k] = s[0];
-  S.buf2[1][k] = s[1];
+  const double mw = c.m0 * c.nW;
+  S.buf2[0][k] = s[0] * mw;
+  S.buf2[1][k] = s[1] * mw;
   if (D == 3) S.buf2[2][k] = 0.0;
 }
 

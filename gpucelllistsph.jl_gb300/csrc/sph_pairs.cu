@@ -369,14 +369,15 @@ struct TermWall {
   }
 };
 
-// kernel_∂v∂tpF! (:1382-1409): sm = s/m₀, pfk2 = 2/(2h)², hp1 = 0.1h
+// kernel_∂v∂tpF! (:1382-1409): pfk2 = 2/(2h)², hp1 = 0.1h, C: pf_cos_coef of s/m₀
 template <int D>
 struct TermTension {
   static constexpr bool QUEUE = true;
   V3 x;
-  double sm, twoh, pfk2, hp1;
+  double twoh, pfk2, hp1;
   const int32_t* pt;
   W3 a;
+  double C[PF_COS_N];
   __device__ bool take(int pi, int pj) const { return pi > 0 && pj > 0; }
   __device__ void run(int64_t, int64_t i, int64_t j) const {
     double dx[D];
@@ -384,7 +385,7 @@ struct TermTension {
     const double r2 = dotf<D>(dx, dx);
     const double r = sqrt_pair(r2);
     if (!(r < twoh)) return;
-    const double scos = sm * pf_cos(r2, pfk2) * rcp_pair(r + hp1);
+    const double scos = pf_cos(r2, pfk2, C) * rcp_pair(r + hp1);
     double f[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) f[d] = scos * dx[d];
@@ -824,9 +825,13 @@ int gcsph_dvdt_pF(int32_t D, int64_t N, int64_t P, const int32_t* pairs, const d
   if (!pt) return fail(GCSPH_EINVAL, "null ptype");
   if (P == 0) return GCSPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const double sm = s / m0, twoh = 2.0 * h, pfk2 = 2.0 / (twoh * twoh), hp1 = 0.1 * h;
+  const double twoh = 2.0 * h, pfk2 = 2.0 / (twoh * twoh), hp1 = 0.1 * h;
   (void)N;
-  TERM(D, st, (TermTension<2>{x, sm, twoh, pfk2, hp1, pt, a}), (TermTension<3>{x, sm, twoh, pfk2, hp1, pt, a}));
+  TermTension<2> f2{x, twoh, pfk2, hp1, pt, a, {}};
+  TermTension<3> f3{x, twoh, pfk2, hp1, pt, a, {}};
+  pf_cos_coef(s / m0, f2.C);
+  pf_cos_coef(s / m0, f3.C);
+  TERM(D, st, f2, f3);
 }
 
 int gcsph_update_rho(int64_t N, double* rho, const double* drho, double dt, double rho0, const int32_t* pt,

@@ -712,10 +712,14 @@ static StepConst make_const(const sph_handle* h) {
   c.twoh = 2.0 * p.h;
   c.pfc = 1.5 * GCSPH_PI64;
   c.pfk2 = 2.0 / ((2.0 * p.h) * (2.0 * p.h));
-  c.pfs = p.s / p.m0;
+  pf_cos_coef(p.s / p.m0, c.pfc_s);
   c.hp1 = 0.1 * p.h;
   c.use_visc = p.nu > 0;
   c.use_pF = p.s > 0;
+  {
+    const double reach = c.use_pF ? fmax(p.H, c.twoh) : p.H;
+    if (h->cl->core.dist > 1.03 * reach) c.far_r2 = reach * reach * (1.0 + 1e-6);  // see pair_far
+  }
   if (p.dpc_l0 > 0) {
     c.dpc_l0inv = 1.0 / p.dpc_l0;
     c.dpc_r2cut = p.dpc_l0 * p.dpc_l0 * (1.0 + 1e-6);

@@ -11,6 +11,16 @@ namespace gcsph {
 
 static constexpr int STPB = 128;
 
+constexpr int PF_COS_N = 13;
+// pf_cos's coefficients times f
+inline void pf_cos_coef(double f, double* C) {
+  const double T[PF_COS_N] = {
+      -0.9818965112591632,   0.31558602480454173, 1.2838905431807321,     -0.7879472662466167,   0.19547895338475096,
+      -0.027475032586512103, 0.00251908751511393, -0.00016342789686839775, 7.918215700351492e-06, -2.9785382234404e-07,
+      8.958338323810472e-09, -2.2072216601308446e-10, 4.5275475585621706e-12};
+  for (int i = 0; i < PF_COS_N; ++i) C[i] = f * T[i];
+}
+
 struct StepConst {
   double h, eta2, m0, rho0, ginv, DDTkh, DDTgz, P0, alpha, c0, nu, g, s, Hinv, nW, nDW;
   double fb_d, fb_r0, fb_eta2;  // fbmolforce constants of the stage being run
@@ -20,7 +30,9 @@ struct StepConst {
   double dWr, avK, visc4;
   double dWg;                   // d𝒲/r = dWg (1 - u)^3 (∑∇W of a call)
   double twoh, pfc, hp1;        // 2h, 1.5*pi, 0.1h  (∂v∂tpF!)
-  double pfk2, pfs;             // 2 / (2h)² and s / m₀ (∂v∂tpF! of the pair-once pass)
+  double pfk2;                  // 2 / (2h)² and s/m₀ times the cosine's coefficients (∂v∂tpF! of the pair-once pass)
+  double pfc_s[PF_COS_N];
+  double far_r2;                // (reach of the pair terms)² (1 + 1e-6) on lists that hold pairs well past it, else 0
   double dpc_l0inv, dpc_nW, dpc_whinv, dpc_pmin, dpc_pmax, dpc_lambda, dpc_kernlim, dpc_eta2;
   double dpc_r2cut;  // l0² (1 + 1e-6): past it u = √r² / l0 >= 1 whatever the rounding
   double xsph_c;                // 2*m0*eps
@@ -345,18 +357,16 @@ __device__ inline double sqrt_nr2(double x) {
 // cos(1.5π sqrt((1 + s)/2)), an entire function of s, and s covers [-1, 1];
 // its Chebyshev series falls by about 100 a term there, and the series to the
 // 12th degree (the next coefficient is 1.9e-17), in powers of s, is the
-// polynomial.  k = 2/(2h)².  13 FP64 instructions and no reduction, where a
-// reduction by π/2 and a Taylor series took 16; the worst error over pairs at
-// random separations is 5.8e-16 (1.5e-15 by way of r).
-__device__ inline double pf_cos(double r2, double k) {
-  const double C[13] = {-0.9818965112591632,  0.31558602480454173,   1.2838905431807321,    -0.7879472662466167,
-                        0.19547895338475096,  -0.027475032586512103, 0.00251908751511393,   -0.00016342789686839775,
-                        7.918215700351492e-06, -2.9785382234404e-07, 8.958338323810472e-09, -2.2072216601308446e-10,
-                        4.5275475585621706e-12};
+// polynomial.  k = 2/(2h)²; C holds the coefficients times the force's factor,
+// in the launch's parameters, where they are operands of the FMAs.  13 FP64
+// instructions and no reduction, where a reduction by π/2 and a Taylor series
+// took 16; the worst error over pairs at random separations is 5.8e-16 (1.5e-15
+// by way of r).
+__device__ inline double pf_cos(double r2, double k, const double* C) {
   const double s = fma(r2, k, -1.0);
-  double p = C[12];
+  double p = C[PF_COS_N - 1];
 #pragma unroll
-  for (int i = 11; i >= 0; --i) p = fma(p, s, C[i]);
+  for (int i = PF_COS_N - 2; i >= 0; --i) p = fma(p, s, C[i]);
   return p;
 }
 
@@ -364,14 +374,14 @@ __device__ inline double pf_cos(double r2, double k) {
 // PF7_EPS_MAX the exact Taylor series of that iteration's output
 // (gen_pf7_series.py, bias included) replaces its two divisions, and where
 // |e| <= PF7_EPS_SHORT its first PF7_SHORT_N terms do; elsewhere the iteration
-// itself runs.  e is taken as it is; the step's passes hand in (1 + eps) - 1,
-// the argument that the reference's rounded x carries, and form ρ0 (1 + r) - ρ0
-// as the reference forms ρ0 t - ρ0: near rest the whole term is of the size of
-// these roundings (without them a resting tank's largest ∂ρ/∂t, 1.9e-8, is
-// 1.1e-12 of it off the oracle's).
-__device__ inline double pf7m1_fast(double e, double ginv, int gamma) {
+// itself runs.  ROOT: powfancy7th(1 + e) itself, its 1 in the series' constant
+// term (which 1 + a₀ holds to 8e-18).
+template <bool ROOT>
+__device__ inline double pf7_series(double e, double ginv, int gamma) {
   const long long ae = dbits(e) & 0x7FFFFFFFFFFFFFFFLL;
   static_assert(PF7_UP_N == PF7_LO_N, "series lengths");
+  constexpr double A0U[PF7_UP_N] = PF7_UP_C, A0L[PF7_LO_N] = PF7_LO_C;
+  static_assert(A0U[0] == A0L[0], "constant terms");
   if (gamma == 7 && ae <= dbits(PF7_EPS_MAX)) {
     const double cu[PF7_UP_N] = PF7_UP_C;
     const double cl[PF7_LO_N] = PF7_LO_C;
@@ -380,15 +390,25 @@ __device__ inline double pf7m1_fast(double e, double ginv, int gamma) {
     if (ae <= dbits(PF7_EPS_SHORT)) {
       r = up ? cu[PF7_SHORT_N - 1] : cl[PF7_SHORT_N - 1];
 #pragma unroll
-      for (int i = PF7_SHORT_N - 2; i >= 0; --i) r = fma(r, e, up ? cu[i] : cl[i]);
+      for (int i = PF7_SHORT_N - 2; i >= 1; --i) r = fma(r, e, up ? cu[i] : cl[i]);
     } else {
       r = up ? cu[PF7_UP_N - 1] : cl[PF7_UP_N - 1];
 #pragma unroll
-      for (int i = PF7_UP_N - 2; i >= 0; --i) r = fma(r, e, up ? cu[i] : cl[i]);
+      for (int i = PF7_UP_N - 2; i >= 1; --i) r = fma(r, e, up ? cu[i] : cl[i]);
     }
-    return r;
+    return fma(r, e, ROOT ? 1.0 + cu[0] : cu[0]);
   }
-  return powfancy7th_1div(1.0 + e, ginv, gamma) - 1.0;
+  const double t = powfancy7th_1div(1.0 + e, ginv, gamma);
+  return ROOT ? t : t - 1.0;
+}
+// powfancy7th(1 + e) - 1, e taken as it is
+__device__ inline double pf7m1_fast(double e, double ginv, int gamma) { return pf7_series<false>(e, ginv, gamma); }
+// powfancy7th(1 + eps): with e = (1 + eps) - 1, the argument that the
+// reference's rounded x carries, and rounded as its t.  The step's passes take
+// this: near rest ρ0 t - ρ0 is of the size of these roundings (without them a
+// resting tank's largest ∂ρ/∂t, 1.9e-8, is 1.1e-12 of it off the oracle's).
+__device__ inline double pf7_fast(double eps, double ginv, int gamma) {
+  return pf7_series<true>((1.0 + eps) - 1.0, ginv, gamma);
 }
 
 // pair-once passes (sph_once.cu): pass A over the device-side pair count,

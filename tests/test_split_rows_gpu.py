@@ -92,3 +92,32 @@ def test_rows_by_a_thread_per_point(gpu_pkg, orc, D):
     for _ in range(2):
         run_both(prob, ref, 1)
     check(orc, prob, ref, case, 1, [(1, {}), (1, {})])
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("factor", [1.02, 1.1, 1.4])
+@pytest.mark.parametrize("s", [0.0, 0.05])
+def test_pairs_past_the_reach(gpu_pkg, orc, D, factor, s):
+    """Lists with a skin hold pairs past H, which pass A tells apart from 3% on
+    (more pairs than its blocks have threads): over steps that keep the list
+    and steps that bring pairs into reach."""
+    if D == 2:
+        case = gpu_pkg.workloads.dam_break_2d(dx=0.0156, layer_ptype=(1, 0, -1), dist_factor=factor)
+    else:
+        case = gpu_pkg.workloads.dam_break_3d(dx=0.05, fluid=(0.5, 0.6, 0.4), tank=(1.0, 0.8, 0.6),
+                                              layer_ptype=(1, 0, -1), full_physics=False)
+        case.dist = factor * case.H
+        case.cellsize = (case.dist,) * 3
+    case.s = s
+    case.extra = dict(nu=0.2, xsph_eps=0.5, cspmn=3)
+    # walls too: lattice walls of both signs hold pairs at exactly r₀, where the
+    # root's last bit decides fbmolforce!
+    rng = np.random.default_rng(17)
+    case.x = case.x + rng.uniform(-0.2, 0.2, case.x.shape) * case.dx
+    case.rho = case.rho + rng.uniform(0.0, 2.0, case.rho.size)
+    v = well_conditioned_v(case)
+    prob, ref = make_pair(gpu_pkg, orc, case, 4, v=v)
+    assert prob.system.pairsn > 152 * 768
+    for _ in range(2):
+        run_both(prob, ref, 3)
+    check(orc, prob, ref, case, 4, [(3, {}), (3, {})], v=v)
