@@ -36,11 +36,11 @@ constexpr int ENS_MAX_TPB = 512;
 // what the stage passes read of an instance for every list entry, in 16-byte
 // groups, so that a branch loads the group it needs with one vector load
 struct __align__(16) StageK {
-  float4 A;  // H², 1/H, dwc, cell edge
-  float4 B;  // ρ₀, η², m₀, DDTgz
-  float4 C;  // kddt, kav, kvisc, (unused)
+  float4 A;  // H², 1/H, m₀ dwc, cell edge
+  float4 B;  // ρ₀, η², -, DDTgz
+  float4 C;  // DDTkh, 2 α c₀ h, 4 ν, largest |z| of the series E
   float4 D;  // pfcr, hp1, 2h, kpf
-  float4 E;  // pc[0..3]
+  float4 E;  // series of ∂ρ∂tDDT!'s density difference in z (ddt_dp)
   float4 F;  // fb_d, fb_r0, fb_eta2 of the stage, first particle (int)
   float4 G;  // 1/ρ₀, P₀, γ (int), bit 0: viscosity, bit 1: surface tension (int)
 };
@@ -60,16 +60,11 @@ struct EnsInst {
   int use_dpc, use_xsph;
   float csf, H2, h, Hinv, nW, nDW, m0, rho0, c0, P0, alpha, DDTkh, DDTgz, eta2, g, nu, s, twoh, pfc, hp1;
   float fb_d[2], fb_r0[2], fb_eta2[2];  // fbmolforce constants of stage 1 and stage 2
-  float pc[4];                           // (1+ε)^(1/γ) - 1 series coefficients
   float dpc_l0inv, dpc_nW, dpc_whinv, dpc_kernlim, dpc_eta2, dpc_pmin, dpc_pmax, dpc_lambda;
   float xsph_c;                          // 2 m0 ε
   float rho0inv, m0inv;                  // 1/ρ₀, 1/m₀
-  float dwc;                             // -20 nDW / H: W'(r)/r = dwc (1 - r/H)^3
   float pfcr;                            // 1.5π / 2h: the cosine's argument per unit r in ∂v∂tpF!
   // products of the above that the stage passes use as one factor
-  float kddt;                            // DDTkh m₀ (∂ρ∂tDDT!)
-  float kav;                             // 2 α c₀ h m₀: ∂v∂t_av!'s -Π m₀ over (Δv·Δx) / ((r² + η²)(ρi + ρj))
-  float kvisc;                           // 4 ν m₀ (∂v∂t_visc!)
   float kpf;                             // s / m₀ (∂v∂tpF!)
   int p_off;                             // first particle of the instance (list entries are instance-local)
   int reuse;                             // the list is kept while the particles stay within the skin
@@ -234,8 +229,20 @@ struct KSum2 {
   }
 };
 
-// √x for x >= 0 by the approximate reciprocal root (within a few ulp); 0 at 0
-__device__ __forceinline__ float sqrt_fast(float x) { return x > 0.f ? x * rsqrtf(x) : 0.f; }
+// 1/x and √x by the hardware's approximations (within 2 ulp), one instruction
+// for the reciprocal: the .ftz forms leave out the scaling of subnormal
+// arguments that __fdividef and rsqrtf carry (three to four instructions
+// each, on the passes' busiest pipe).  Subnormal x: 1/x is infinite, √x is 0.
+__device__ __forceinline__ float rcp32(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sqrt_fast(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return x >= 1.17549435e-38f ? x * y : 0.f;
+}
 
 template <int D>
 __device__ __forceinline__ float dot32(const float* a, const float* b) {
@@ -271,11 +278,12 @@ __device__ __forceinline__ float eos32(float dr, int pt, const StageK& Q) {
   return g.y * p;
 }
 
-// (1+ε)^(1/γ) - 1 (powfancy7th(1+ε) - 1, src/gpukernels_sph.jl:499-515), from
-// the series coefficients pc
-__device__ __forceinline__ float root_m1g(float eps, const float4& pc, int gamma) {
-  if (fabsf(eps) < 0.01f) return eps * (pc.x + eps * (pc.y + eps * (pc.z + eps * pc.w)));
-  return powf(1.f + eps, 1.f / (float)gamma) - 1.f;
+// ρ₀ ((1+ε)^(1/γ) - 1) at ε = gz z (ρ₀ (powfancy7th(1+ε) - 1),
+// src/gpukernels_sph.jl:499-515): for |z| < lim, where |ε| < 0.01, by a series
+// in z with all constants in its coefficients
+__device__ __forceinline__ float ddt_dp(float z, const float4& pc, float lim, float rho0, float gz, int gamma) {
+  if (fabsf(z) < lim) return z * fmaf(z, fmaf(z, fmaf(z, pc.w, pc.z), pc.y), pc.x);
+  return rho0 * (powf(1.f + gz * z, 1.f / (float)gamma) - 1.f);
 }
 
 __device__ __forceinline__ void cell_of(int key, const EnsInst& I, int& c0, int& c1, int& c2) {
@@ -804,6 +812,7 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int6
   const int nn = A.nlc[i];
   const int p_off = __float_as_int(Q.F.w), gamma = __float_as_int(Q.G.z), opt = __float_as_int(Q.G.w);
   const bool use_visc = opt & 1, use_pF = opt & 2;
+  const float nirhoi = -irhoi;
   // the next entry is loaded one iteration ahead: the list streams from
   // DRAM, and its latency then overlaps the current neighbour's arithmetic
   int nxt = lane < nn ? A.nl[(int64_t)lane * A.ncap + i] : 0;
@@ -817,7 +826,7 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int6
     float oj[D], hj[D], vj[D], drj, Prec = 0.f;
     int ptj;
     decode_rec<D, STAGE>(rec, oj, hj, vj, drj, ptj, Prec);
-    const float4 kA = Q.A;  // H², 1/H, dwc, cell edge
+    const float4 kA = Q.A;  // H², 1/H, m₀ dwc, cell edge
     float d[D];
 #pragma unroll
     for (int q = 0; q < D; ++q) d[q] = fmaf(-sh[q], kA.w, oi[q] - oj[q]);
@@ -825,12 +834,11 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int6
     if (STAGE == 1 && RM) rm2 = fminf(rm2, r2);
     if (!(r2 < kA.x)) continue;  // in the list's skin: not a pair of this step
     if (!FLUID && !(ptj > 0)) continue;
-    // sph∇W!: W'(r)/r of WendlandC2 = -20 nDW Hinv (1-q)^3.  Reciprocals and
+    // m₀ sph∇W!: W'(r)/r of WendlandC2 = -20 nDW Hinv (1-q)^3.  Reciprocals and
     // roots here are the approximate intrinsics (within 2 ulp each), far
     // inside the FP32 path's error against FP64.
-    const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
-    const float u = r * kA.y;
-    const float t = u < 1.f ? 1.f - u : 0.f;
+    const float r = sqrt_fast(r2);
+    const float t = fmaxf(fmaf(-r, kA.y, 1.f), 0.f);
     const float dwr = kA.z * (t * t * t);
     float gw[D], dd[D], dv[D];
 #pragma unroll
@@ -839,9 +847,9 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int6
       dd[q] = STAGE == 1 ? d[q] : fmaf(-sh[q], kA.w, ohi[q] - hj[q]);
       dv[q] = vi[q] - vj[q];
     }
-    const float4 kB = Q.B;  // ρ₀, η², m₀, DDTgz
+    const float4 kB = Q.B;  // ρ₀, η², -, DDTgz
     if (!FLUID) {
-      drho.add(kB.z * dot32<D>(dv, gw));
+      drho.add(dot32<D>(dv, gw));
       continue;
     }
     // gsc: the factor of ∇W of ∂v∂t! and ∂v∂t_av! together; f: the
@@ -852,37 +860,34 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int6
     if (ptj > 0) {
       const float r2d = STAGE == 1 ? r2 : dot32<D>(dd, dd);
       const float rhoj = kB.x + drj;
-      const float irhoj = __fdividef(1.f, rhoj);
-      const float inv = __fdividef(1.f, r2d + kB.y);
+      const float irhoj = rcp32(rhoj);
+      // one reciprocal for 1/(r² + η²) and 1/((r² + η²)(ρi + ρj))
+      const float s = rhoi + rhoj;
+      const float ii = rcp32(s * (r2d + kB.y));
       // ∂v∂t!
       float Pj = Prec;
       if (!rec_has_p<D, STAGE>()) Pj = eos32(drj, ptj, Q);
-      gsc = -kB.z * (Pi + Pj) * (irhoi * irhoj);
-      const float4 kC = Q.C;  // kddt, kav, kvisc
-      const float ddgw = dot32<D>(dd, gw);
+      gsc = (Pi + Pj) * (nirhoi * irhoj);
+      const float4 kC = Q.C;  // kddt, kav, kvisc over m₀; the series' range
+      const float ddgw = dot32<D>(dd, gw) * ii;
       // ∂ρ∂tDDT!
-      float term = kB.z * dot32<D>(dv, gw);
-      const float dp = kB.x * root_m1g(kB.w * dd[1], Q.E, gamma);
-      term += kC.x * ((drj - dri) - dp) * inv * (-ddgw) * irhoj;
-      drho.add(term);
+      const float dp = ddt_dp(dd[1], Q.E, kC.w, kB.x, kB.w, gamma);
+      drho.add(fmaf(-kC.x * ((drj - dri) - dp), ddgw * (s * irhoj), dot32<D>(dv, gw)));
+      // ∂v∂t_av!: -Π m₀ = 2 α c₀ h m₀ (Δv·Δx) / ((r² + η²)(ρi + ρj)) where Δv·Δx < 0
       const float cond = dot32<D>(dv, dd);
-      if (cond < 0.f || use_visc) {
-        const float ii = __fdividef(1.f, rhoi + rhoj) * inv;
-        // ∂v∂t_av!: -Π m₀ = 2 α c₀ h m₀ (Δv·Δx) / ((r² + η²)(ρi + ρj))
-        if (cond < 0.f) gsc += kC.y * cond * ii;
-        if (use_visc) {
-          // ∂v∂t_visc!
-          const float nt = kC.z * ddgw * ii;
+      if (cond < 0.f) gsc = fmaf(kC.y * cond, ii, gsc);
+      if (use_visc) {
+        // ∂v∂t_visc!
+        const float nt = kC.z * ddgw;
 #pragma unroll
-          for (int q = 0; q < D; ++q) f[q] = nt * dv[q];
-        }
+        for (int q = 0; q < D; ++q) f[q] = nt * dv[q];
       }
       if (use_pF) {
         // ∂v∂tpF! (in stage 1 the separation is r itself)
         const float4 kD = Q.D;  // pfcr, hp1, 2h, kpf
-        const float rd = STAGE == 1 ? r : (r2d > 0.f ? r2d * rsqrtf(r2d) : 0.f);
+        const float rd = STAGE == 1 ? r : sqrt_fast(r2d);
         if (rd < kD.z) {
-          const float scos = kD.w * __cosf(kD.x * rd) * __fdividef(1.f, rd + kD.y);  // argument in [0, 1.5π)
+          const float scos = kD.w * __cosf(kD.x * rd) * rcp32(rd + kD.y);  // argument in [0, 1.5π)
 #pragma unroll
           for (int q = 0; q < D; ++q) f[q] = fmaf(scos, dd[q], f[q]);
         }
@@ -891,9 +896,9 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int6
       const float4 kF = Q.F;  // fb_d, fb_r0, fb_eta2
       if (r < kF.y) {
         // fbmolforce! at x
-        const float qq = kF.y * __fdividef(1.f, r + kF.z);
+        const float qq = kF.y * rcp32(r + kF.z);
         const float q2 = qq * qq, q4 = q2 * q2, q8 = q4 * q4;
-        const float Fc = kF.x * (q8 * q4 - q4) * __fdividef(1.f, r2 + kF.z);
+        const float Fc = kF.x * (q8 * q4 - q4) * rcp32(r2 + kF.z);
 #pragma unroll
         for (int q = 0; q < D; ++q) f[q] += d[q] * Fc;
       }
@@ -930,7 +935,7 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const En
     const int pti = A.pt[i];
     const float dri = STAGE == 1 ? A.dr[i] : A.drh[i];
     const float rhoi = I.rho0 + dri;
-    const float irhoi = __fdividef(1.f, rhoi);
+    const float irhoi = rcp32(rhoi);
     const float Pi = eos32(dri, pti, I);
     KSum drho;
     KSum2 accxy;  // the x and y components of the acceleration, packed
@@ -1088,8 +1093,8 @@ __global__ void __launch_bounds__(ENS_MAX_TPB) k_ens_dpc(EnsArr A, const EnsInst
                                            I.dpc_lambda * I.dpc_pmax), I.dpc_pmin);
         const float vr = dot32<D>(dv, dx);
         float c;
-        if (vr < 0.f) c = kk * (-vr * __fdividef(1.f, r2 + I.dpc_eta2));
-        else c = 2.f * dt * Pb * __fdividef(1.f, (rhoi + rhoj) * (r2 + I.dpc_eta2));
+        if (vr < 0.f) c = kk * (-vr * rcp32(r2 + I.dpc_eta2));
+        else c = 2.f * dt * Pb * rcp32((rhoi + rhoj) * (r2 + I.dpc_eta2));
 #pragma unroll
         for (int q = 0; q < D; ++q) sum[q].add(c * dx[q]);
       }
@@ -1176,7 +1181,7 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_xsph(EnsArr A, const Ens
         const float t = u < 1.f ? 1.f - u : 0.f;
         const float t2 = t * t;
         const float w = (1.f + 4.f * u) * (t2 * t2) * I.nW;
-        const float xs = I.xsph_c * w * __fdividef(1.f, rhoi + (I.rho0 + drj));
+        const float xs = I.xsph_c * w * rcp32(rhoi + (I.rho0 + drj));
 #pragma unroll
         for (int q = 0; q < D; ++q) sum[q].add((vj[q] - vi[q]) * xs);
       }
@@ -1237,7 +1242,7 @@ __global__ void __launch_bounds__(ENS_MAX_TPB) k_ens_cspm(EnsArr A, const EnsIns
       const float t = u < 1.f ? 1.f - u : 0.f;
       const float t2 = t * t;
       const float w = (1.f + 4.f * u) * (t2 * t2) * I.nW;
-      const float mw = I.m0 * w * __fdividef(1.f, I.rho0 + drj);
+      const float mw = I.m0 * w * rcp32(I.rho0 + drj);
       s2.add(mw);
       s3.add(mw * drj);
     }
@@ -2351,17 +2356,11 @@ int ens_add(gcsph_ens* e, int64_t n, const double* x, const double* v, const dou
   I.xsph_c = (float)(2.0 * p->m0 * p->xsph_eps);
   const double a = 1.0 / (double)p->gamma;
   const double c1 = a, c2 = c1 * (a - 1.0) / 2.0, c3 = c2 * (a - 2.0) / 3.0, c4 = c3 * (a - 3.0) / 4.0;
-  I.pc[0] = (float)c1;
-  I.pc[1] = (float)c2;
-  I.pc[2] = (float)c3;
-  I.pc[3] = (float)c4;
   I.rho0inv = (float)(1.0 / p->rho0);
   I.m0inv = (float)(1.0 / p->m0);
-  I.dwc = (float)(-20.0 * (D == 2 ? wc2_norm_dw<2>(1.0 / p->H) : wc2_norm_dw<3>(1.0 / p->H)) / p->H);
+  // W'(r)/r = dwc (1 - r/H)^3
+  const double dwc = -20.0 * (D == 2 ? wc2_norm_dw<2>(1.0 / p->H) : wc2_norm_dw<3>(1.0 / p->H)) / p->H;
   I.pfcr = (float)(1.5 * GCSPH_PI64 / (2.0 * p->h));
-  I.kddt = (float)(2.0 * p->h * p->delta * p->c0 * p->m0);
-  I.kav = (float)(2.0 * p->alpha * p->c0 * p->h * p->m0);
-  I.kvisc = (float)(4.0 * p->nu * p->m0);
   I.kpf = (float)(p->s / p->m0);
   auto as_float = [](int v) {
     float f;
@@ -2370,11 +2369,15 @@ int ens_add(gcsph_ens* e, int64_t n, const double* x, const double* v, const dou
   };
   for (int st = 0; st < 2; ++st) {
     StageK& K = I.k[st];
-    K.A = make_float4(I.H2, I.Hinv, I.dwc, I.csf);
-    K.B = make_float4(I.rho0, I.eta2, I.m0, I.DDTgz);
-    K.C = make_float4(I.kddt, I.kav, I.kvisc, 0.f);
+    // m₀ goes into ∇W, ρ₀ and DDTgz into the series of ∂ρ∂tDDT!
+    const double gz = p->rho0 * p->g / ((p->c0 * p->c0 * p->rho0) / (double)p->gamma);
+    K.A = make_float4(I.H2, I.Hinv, (float)(dwc * p->m0), I.csf);
+    K.B = make_float4(I.rho0, I.eta2, 0.f, I.DDTgz);
+    K.C = make_float4((float)(2.0 * p->h * p->delta * p->c0), (float)(2.0 * p->alpha * p->c0 * p->h),
+                      (float)(4.0 * p->nu), gz != 0.0 ? (float)(0.01 / std::fabs(gz)) : INFINITY);
     K.D = make_float4(I.pfcr, I.hp1, I.twoh, I.kpf);
-    K.E = make_float4(I.pc[0], I.pc[1], I.pc[2], I.pc[3]);
+    K.E = make_float4((float)(p->rho0 * c1 * gz), (float)(p->rho0 * c2 * gz * gz),
+                      (float)(p->rho0 * c3 * gz * gz * gz), (float)(p->rho0 * c4 * gz * gz * gz * gz));
     K.F = make_float4(I.fb_d[st], I.fb_r0[st], I.fb_eta2[st], 0.f);  // .w: ens_relayout
     K.G = make_float4(I.rho0inv, I.P0, as_float(I.gamma), as_float((I.use_visc ? 1 : 0) | (I.use_pF ? 2 : 0)));
   }
