@@ -908,11 +908,17 @@ __device__ __forceinline__ void stage_row(const EnsArr& A, const StageK& Q, int6
   }
 }
 
-// two blocks of 512 per SM: at most 64 registers.  RM (stage 1): keep each
-// row's smallest r² for dpcreg!'s row bound (a separate instantiation, so the
-// ensembles without dpcreg! run the loop without it)
+// 48 registers, which leaves room for 40 warps an SM: the passes wait for the
+// neighbours' records (L1, 85% hits) with 60% of the issue slots busy, and the
+// warps hide more of that than the few spilled values cost.  A step of 20 2-D
+// instances (743k particles) / of a 3-D instance with full physics (390k): 56 to 64
+// registers 379 / 635 us, 56 375 / 596, 48 360 / 592, 40 382 / 642; 64 with
+// the next record loaded one entry ahead 435 / 650.
+// RM (stage 1): keep each row's smallest r² for dpcreg!'s row bound (a separate
+// instantiation, so the ensembles without dpcreg! run the loop without it)
+constexpr int STAGE_REGS = 48;
 template <int D, int STAGE, bool RM, int N>
-__global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_stage(EnsArr A, const EnsInst* __restrict__ T,
+__global__ void __maxnreg__(STAGE_REGS) k_ens_stage(EnsArr A, const EnsInst* __restrict__ T,
                                                               const __grid_constant__ StageTab<N, STAGE> tab) {
   if (*A.ovf) return;
   constexpr int L = stage_lanes<D>();
@@ -1130,8 +1136,9 @@ __global__ void k_ens_dpc_apply(EnsArr A, const EnsInst* __restrict__ T) {
 // xsphcorr! + update_xsphcorr! (src/gpukernels_sph.jl:1745-1838): stage-1 W
 // (pairs and distances at x), v and ρ after the corrector and dpcreg!;
 // moves x only.  Reads neighbours' v, writes its own x: one pass.  Little
-// arithmetic per neighbour and a record gather each: latency-bound, so three
-// blocks of 512 per SM (at most 42 registers) rather than the stage passes' two
+// arithmetic per neighbour and a record gather each: latency-bound, so two
+// records are loaded at a time (390k particles in 3-D: a step takes 654 us with
+// two, 678 with one, 686 with four; two with 40 registers a thread 709)
 constexpr int XSPH_U = 2;
 template <int D>
 __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_xsph(EnsArr A, const EnsInst* __restrict__ T) {
