@@ -207,8 +207,8 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
 }
 
 // Pass A over all pairs in chunks of 32 consecutive pairs, one chunk per warp
-// at a time, with one block per SM: PA_TPB threads of about 80 registers
-// leave no room for a second block, and the grid is the SM count.  Block b
+// at a time, with one block per SM: its threads' registers leave no room for
+// a second block, and the grid is the SM count.  Block b
 // takes chunks b, b + G, b + 2G, ... (G blocks) and its warp w every NW-th
 // of those, so every SM gets the same number of chunks (to one) -- a grid of
 // many small blocks leaves some SMs one block more than others -- and
@@ -221,11 +221,20 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
 // Where a warp has one chunk there is nothing to sort into and the queue only
 // adds latency (2-D dam break, 102k pairs: 18.7 us without it, 19.1 with it):
 // such lists are run as they come.
-constexpr int PA_TPB = 768;
+//
+// Threads: 768 of 80 registers in the direct form.  The queue form does better
+// with 640 of 96 (2-D full physics with a skin, 65k particles, a call of ten
+// steps: 512 threads 6114 us, 576 6084, 640 6057, 704 6113, 768 6191, 896 6335,
+// 1024 6506; 3-D full 24.07, 24.22, 24.02, 24.15, 24.21, 25.45, 25.64 ms): the
+// FP64 pipe is about 85% busy from 16 warps on, and fewer registers spill.
+template <bool QUEUE>
+__host__ __device__ constexpr int pa_tpb() {
+  return QUEUE ? 640 : 768;
+}
 template <int D, int STAGE, bool QUEUE>
-__global__ void __launch_bounds__(PA_TPB, 1) k_pairA(StepConst c, SArr<D> S, PairBuf B) {
+__global__ void __launch_bounds__(pa_tpb<QUEUE>(), 1) k_pairA(StepConst c, SArr<D> S, PairBuf B) {
   if (*S.ovf) return;
-  constexpr int NW = PA_TPB / 32, NC = 3;
+  constexpr int NW = pa_tpb<QUEUE>() / 32, NC = 3;
   const int np = (int)*B.npair;    // the pair list holds fewer than 2^31
   const int G = gridDim.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -832,14 +841,14 @@ __global__ void __launch_bounds__(STPB) k_sums_rows(StepConst c, int64_t N, cons
 
 template <int D, int STAGE, bool QUEUE>
 static int pairA_grid(int* g) {
-  // one block per SM (the kernel's registers and PA_TPB leave room for one);
+  // one block per SM (the kernel's registers leave room for one);
   // the occupancy query covers a build where two would fit
   static int grid = 0;
   if (grid == 0) {
     int dev = 0, sms = 0, per = 0;
     GC_CUDA(cudaGetDevice(&dev));
     GC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pairA<D, STAGE, QUEUE>, PA_TPB, 0));
+    GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pairA<D, STAGE, QUEUE>, pa_tpb<QUEUE>(), 0));
     grid = sms * (per > 0 ? per : 1);
   }
   *g = grid;
@@ -850,11 +859,11 @@ template <int D, int STAGE>
 static int run_pairA(cudaStream_t st, const StepConst& c, const SArr<D>& S, const PairBuf& B, int64_t pairs_est) {
   int g = 0, rc;
   if ((rc = pairA_grid<D, STAGE, false>(&g))) return rc;
-  if (pairs_est <= (int64_t)g * PA_TPB) {  // about one chunk a warp
-    k_pairA<D, STAGE, false><<<g, PA_TPB, 0, st>>>(c, S, B);
+  if (pairs_est <= (int64_t)g * pa_tpb<false>()) {  // about one chunk a warp
+    k_pairA<D, STAGE, false><<<g, pa_tpb<false>(), 0, st>>>(c, S, B);
   } else {
     if ((rc = pairA_grid<D, STAGE, true>(&g))) return rc;
-    k_pairA<D, STAGE, true><<<g, PA_TPB, 0, st>>>(c, S, B);
+    k_pairA<D, STAGE, true><<<g, pa_tpb<true>(), 0, st>>>(c, S, B);
   }
   GC_LAUNCHED();
   return GCSPH_OK;
