@@ -755,14 +755,51 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
   if (D == 3) S.buf2[2][k] = 0.0;
 }
 
+// The terms of a call's ∑W and ∑∇W by pair, into both rows' slots: (1 + 4u)
+// (1 - u)^4 and Δx (1 - u)^3 for pairs of one side, zero for others.  FP64-bound,
+// so once a pair; the row sums then read slots (rows that evaluated their
+// entries, each pair twice: 3-D full physics, 23.5M pairs, a call 23.96 ms
+// against 23.46; 3-D plain, 5.5M pairs, 7242 us against 7098; 2-D, 102k pairs,
+// a call of one step 224 against 213).
+constexpr int PS_TPB = 256;
+template <int D>
+__global__ void __launch_bounds__(PS_TPB) k_pair_sums(StepConst c, SArr<D> S, PairBuf B) {
+  if (*S.ovf) return;
+  const int64_t np = *B.npair, stride = (int64_t)gridDim.x * PS_TPB;
+  for (int64_t u = (int64_t)blockIdx.x * PS_TPB + threadIdx.x; u < np; u += stride) {
+    // (the mirrors of a list that an update! at the last step's end rebuilt are open)
+    const int4 q = pair_load<D, 1>(S, B, (int)u);
+    double w = 0.0, g[3] = {0.0, 0.0, 0.0};
+    if ((S.pt[q.x] > 0) == (S.pt[q.y] > 0)) {
+      double dx[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) dx[d] = S.x[d][q.x] - S.x[d][q.y];
+      const double r2 = dotD<D>(dx, dx);
+      const bool r2pos = dbits(r2) != 0;
+      const double t = r2pos ? fma(-sqrt_nr(r2), c.Hinv, 1.0) : 1.0;
+      if ((unsigned long long)dbits(t) - 1ull < (unsigned long long)ONE_BITS) {
+        const double t2 = t * t;
+        w = fma(-4.0, t, 5.0) * (t2 * t2);
+        const double t3 = r2pos ? t2 * t : NAN;  // the reference's d𝒲(0)/0
+#pragma unroll
+        for (int d = 0; d < D; ++d) g[d] = dx[d] * t3;
+      }
+    }
+    put_slot(B.ce + q.z, w, g[0], g[1], g[2]);
+    put_slot(B.ce + q.w, w, flip(g[0]), flip(g[1]), flip(g[2]));
+  }
+}
+
 // post-batch sph∑W! + sph∑∇W!  (:139-156, :332-359).  The kernel's factors
 // come out of the sums: ∑W = nW ∑ (1 + 4u)(1 - u)^4, ∑∇W = dWg ∑ Δx (1 - u)^3.
-// With SCATTER the lanes of a particle also write its state back to the
-// original order, an array in turn each.
+// With SCATTER (after a step) the terms are k_pair_sums's slots, and the lanes
+// of a particle also write its state back to the original order, an array in
+// turn each; without (no step in the call) the rows evaluate their entries.
 template <int D, int L, bool SCATTER>
 __global__ void __launch_bounds__(STPB) k_sums_rows(StepConst c, int64_t N, const int64_t* __restrict__ rs,
                                                     const int32_t* __restrict__ nbr, PostSums Q,
-                                                    const int* __restrict__ ovf, StateIO<D> O, SArr<D> S) {
+                                                    const int* __restrict__ ovf, StateIO<D> O, SArr<D> S,
+                                                    const PairOut* ce) {
   if (*ovf) return;
   const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t k = gt / L;
@@ -775,38 +812,53 @@ __global__ void __launch_bounds__(STPB) k_sums_rows(StepConst c, int64_t N, cons
   const bool real = Q.pt[ik] > 0;
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   const int64_t e1 = rs[k + 1];
-  for (int64_t e = rs[k] + lane; e < e1; e += GATHER_U * L) {
-    int32_t m[GATHER_U];
-    int pt[GATHER_U];
-    double xm[GATHER_U][D];
+  if constexpr (SCATTER) {
+    for (int64_t e = rs[k] + lane; e < e1; e += 4 * L) {
+      double v[4][4];
 #pragma unroll
-    for (int j = 0; j < GATHER_U; ++j) m[j] = e + j * L < e1 ? nbr[e + j * L] : -1;
-    if (Q.map) {
+      for (int j = 0; j < 4; ++j)
+        if (e + j * L < e1) get_slot(ce + e + j * L, v[j]);
 #pragma unroll
-      for (int j = 0; j < GATHER_U; ++j) m[j] = m[j] < 0 ? -1 : Q.map[m[j]];
+      for (int j = 0; j < 4; ++j)
+        if (e + j * L < e1)
+#pragma unroll
+          for (int d = 0; d < 1 + D; ++d) s[d] += v[j][d];
     }
+  }
+  if constexpr (!SCATTER) {
+    for (int64_t e = rs[k] + lane; e < e1; e += GATHER_U * L) {
+      int32_t m[GATHER_U];
+      int pt[GATHER_U];
+      double xm[GATHER_U][D];
 #pragma unroll
-    for (int j = 0; j < GATHER_U; ++j) {
-      const int32_t i = m[j] < 0 ? ik : m[j];
-      pt[j] = Q.pt[i];
+      for (int j = 0; j < GATHER_U; ++j) m[j] = e + j * L < e1 ? nbr[e + j * L] : -1;
+      if (Q.map) {
 #pragma unroll
-      for (int d = 0; d < D; ++d) xm[j][d] = Q.x[d][i];
-    }
+        for (int j = 0; j < GATHER_U; ++j) m[j] = m[j] < 0 ? -1 : Q.map[m[j]];
+      }
 #pragma unroll
-    for (int j = 0; j < GATHER_U; ++j) {
-      if (m[j] < 0 || (pt[j] > 0) != real) continue;
-      double dx[D];
+      for (int j = 0; j < GATHER_U; ++j) {
+        const int32_t i = m[j] < 0 ? ik : m[j];
+        pt[j] = Q.pt[i];
 #pragma unroll
-      for (int d = 0; d < D; ++d) dx[d] = xk[d] - xm[j][d];
-      const double r2 = dotD<D>(dx, dx);
-      const bool r2pos = dbits(r2) != 0;
-      const double u = r2pos ? sqrt_nr(r2) * c.Hinv : 0.0;
-      if (!(dbits(u) < ONE_BITS)) continue;
-      const double t = 1.0 - u, t2 = t * t;
-      s[0] += fma(4.0, u, 1.0) * (t2 * t2);
-      const double t3 = r2pos ? t2 * t : NAN;  // the reference's d𝒲(0)/0
+        for (int d = 0; d < D; ++d) xm[j][d] = Q.x[d][i];
+      }
 #pragma unroll
-      for (int d = 0; d < D; ++d) s[1 + d] += dx[d] * t3;
+      for (int j = 0; j < GATHER_U; ++j) {
+        if (m[j] < 0 || (pt[j] > 0) != real) continue;
+        double dx[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) dx[d] = xk[d] - xm[j][d];
+        const double r2 = dotD<D>(dx, dx);
+        const bool r2pos = dbits(r2) != 0;
+        const double u = r2pos ? sqrt_nr(r2) * c.Hinv : 0.0;
+        if (!(dbits(u) < ONE_BITS)) continue;
+        const double t = 1.0 - u, t2 = t * t;
+        s[0] += fma(4.0, u, 1.0) * (t2 * t2);
+        const double t3 = r2pos ? t2 * t : NAN;  // the reference's d𝒲(0)/0
+#pragma unroll
+        for (int d = 0; d < D; ++d) s[1 + d] += dx[d] * t3;
+      }
     }
   }
   lanes_sum4<L>(s, lane, group_mask<L>());
@@ -929,12 +981,19 @@ int launch_cspm(int L, int64_t N, cudaStream_t st, const StepConst& c, const SAr
 }
 template <int D>
 int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, const int64_t* rs, const int32_t* nbr,
-                     const PostSums& Q, const int* ovf, bool scatter, const StateIO<D>& O, const SArr<D>& S) {
+                     const PostSums& Q, const int* ovf, bool scatter, const StateIO<D>& O, const SArr<D>& S,
+                     const PairBuf& B, int64_t pairs_est) {
+  const PairOut* ce = B.ce;
+  if (scatter) {
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(nblocks(pairs_est, PS_TPB), 152 * 16));
+    k_pair_sums<D><<<g, PS_TPB, 0, st>>>(c, S, B);
+    GC_LAUNCHED();
+  }
 #define GC_SUMS(LL)                                                                                            \
   if (scatter)                                                                                                 \
-    k_sums_rows<D, LL, true><<<nblocks(N * (int64_t)LL, STPB), STPB, 0, st>>>(c, N, rs, nbr, Q, ovf, O, S);     \
+    k_sums_rows<D, LL, true><<<nblocks(N * (int64_t)LL, STPB), STPB, 0, st>>>(c, N, rs, nbr, Q, ovf, O, S, ce); \
   else                                                                                                         \
-    k_sums_rows<D, LL, false><<<nblocks(N * (int64_t)LL, STPB), STPB, 0, st>>>(c, N, rs, nbr, Q, ovf, O, S);
+    k_sums_rows<D, LL, false><<<nblocks(N * (int64_t)LL, STPB), STPB, 0, st>>>(c, N, rs, nbr, Q, ovf, O, S, ce);
   switch (L) {
     case 2: GC_SUMS(2) break;
     case 4: GC_SUMS(4) break;
@@ -954,7 +1013,7 @@ int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, cons
   template int launch_xsph<D>(int, int64_t, cudaStream_t, const StepConst&, const Scal*, const SArr<D>&);         \
   template int launch_cspm<D>(int, int64_t, cudaStream_t, const StepConst&, const SArr<D>&);                      \
   template int launch_sums_post<D>(int, int64_t, cudaStream_t, const StepConst&, const int64_t*, const int32_t*,  \
-                                   const PostSums&, const int*, bool, const StateIO<D>&, const SArr<D>&);
+                                   const PostSums&, const int*, bool, const StateIO<D>&, const SArr<D>&, const PairBuf&, int64_t);
 GC_INST(2)
 GC_INST(3)
 #undef GC_INST

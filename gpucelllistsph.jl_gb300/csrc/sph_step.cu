@@ -1027,7 +1027,7 @@ static int finish_call(sph_handle* h, const StepConst& c, Scal* dsc) {
       Q.orig = core.orig.as<int32_t>();
       Q.sumW = h->sumW_o.as<double>();
       if ((rc = launch_sums_post<D>(L, h->N, st, c, core.rs_full.as<int64_t>(), core.nbr.as<int32_t>(), Q, &dsc->ovf,
-                                    fold, make_io<D>(h), make_arr<D>(h))))
+                                    fold, make_io<D>(h), make_arr<D>(h), make_pairbuf<D>(h), core.nfull_est / 2)))
         return rc;
     } else {
       k_sums_post<D><<<nblocks(h->N, STPB), STPB, 0, st>>>(

@@ -476,6 +476,7 @@ struct PostSums {
 };
 template <int D>
 int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, const int64_t* rs, const int32_t* nbr,
-                     const PostSums& Q, const int* ovf, bool scatter, const StateIO<D>& O, const SArr<D>& S);
+                     const PostSums& Q, const int* ovf, bool scatter, const StateIO<D>& O, const SArr<D>& S,
+                     const PairBuf& B, int64_t pairs_est);
 
 }  // namespace gcsph
