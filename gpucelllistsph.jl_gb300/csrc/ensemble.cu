@@ -347,23 +347,6 @@ __global__ void k_ens_scatter(int64_t N, const int32_t* __restrict__ key, const 
   for (int64_t c = t0; c < K; c += stride) count[c] = 0;
 }
 
-// rank inside the cell by instance-local id (ids are unique inside an instance)
-__global__ void k_ens_rank(int64_t N, const int32_t* __restrict__ tmp, const int32_t* __restrict__ key,
-                           const int32_t* __restrict__ cellstart, const int32_t* __restrict__ id,
-                           int32_t* __restrict__ perm, const int* __restrict__ any) {
-  if (!any[0]) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += stride) {
-    const int32_t i = tmp[q];
-    const int32_t c = key[i];
-    const int32_t s = cellstart[c], e = cellstart[c + 1];
-    const int32_t oi = id[i];
-    int32_t r = 0;
-    for (int32_t t = s; t < e; ++t) r += id[tmp[t]] < oi;
-    perm[s + r] = i;
-  }
-}
-
 struct EnsState {
   double* x[3];
   float* v[3];
@@ -375,15 +358,23 @@ struct EnsState {
   int32_t* id;
 };
 
-// out[k] = in[perm[k]] for the whole state, and the sorted keys
+// the rank of each point of the arrival lists inside its cell by
+// instance-local id (ids are unique inside an instance), and its state and key
+// to its place at once
 template <int D>
-__global__ void k_ens_move(int64_t N, const int32_t* __restrict__ perm, const int32_t* __restrict__ key, EnsState in,
-                           EnsState out, int32_t* __restrict__ skey, const int* __restrict__ any) {
+__global__ void k_ens_move(int64_t N, const int32_t* __restrict__ tmp, const int32_t* __restrict__ key,
+                           const int32_t* __restrict__ cellstart, EnsState in, EnsState out,
+                           int32_t* __restrict__ skey, const int* __restrict__ any) {
   if (!any[0]) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < N; k += stride) {
-    const int32_t i = perm[k];
-    skey[k] = key[i];
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += stride) {
+    const int32_t i = tmp[q];
+    const int32_t c = key[i];
+    const int32_t s = cellstart[c], e = cellstart[c + 1];
+    const int32_t oi = in.id[i];
+    int32_t k = s;
+    for (int32_t t = s; t < e; ++t) k += in.id[tmp[t]] < oi;
+    skey[k] = c;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       out.x[d][k] = in.x[d][i];
@@ -394,7 +385,7 @@ __global__ void k_ens_move(int64_t N, const int32_t* __restrict__ perm, const in
     out.dr[k] = in.dr[i];
     out.drb[k] = in.drb[i];
     out.pt[k] = in.pt[i];
-    out.id[k] = in.id[i];
+    out.id[k] = oi;
   }
 }
 
@@ -1208,7 +1199,7 @@ __global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_xsph(EnsArr A, const Ens
 // over real neighbours at the step's starting positions, with the updated ρ_j;
 // formed as δρ = Σ m0 W δρ_j/ρ_j / Σ m0 W/ρ_j (no cancellation against ρ₀).
 // The result goes to δρ½ (free after the corrector) and is applied by
-// k_ens_cspm_apply, so every particle reads the pre-correction densities.
+// k_ens_disp, so every particle reads the pre-correction densities.
 
 template <int D>
 __global__ void __launch_bounds__(ENS_MAX_TPB) k_ens_cspm(EnsArr A, const EnsInst* __restrict__ T,
@@ -1258,20 +1249,10 @@ __global__ void __launch_bounds__(ENS_MAX_TPB) k_ens_cspm(EnsArr A, const EnsIns
   }
 }
 
-__global__ void k_ens_cspm_apply(int64_t N, const int32_t* __restrict__ inst, const EnsInst* __restrict__ T,
-                                 const int32_t* __restrict__ istep, const float* __restrict__ drh,
-                                 float* __restrict__ dr, const int* __restrict__ ovf, const int* __restrict__ any) {
-  if (!any[1] || *ovf) return;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
-    const int s = inst[i];
-    if (cspm_due(T[s], istep, s)) dr[i] = drh[i];
-  }
-}
-
 // the largest squared displacement since the last list build, per instance
 // (particles are sorted by instance: a warp's lanes of one instance reduce
 // together, one atomic per instance per warp)
+// and, at the step's end, the density that k_ens_cspm left in δρ½.
 // STEP: the largest move of the step (x_{n+1} - x_n, after the corrector) of
 // the instances with dpcreg!, for its row bound; NaN gives +inf (no row skips)
 template <int D, bool STEP>
@@ -1281,6 +1262,7 @@ __global__ void k_ens_disp(EnsArr A, const EnsInst* __restrict__ T, unsigned* __
   const bool in = i < A.N;
   const int s = in ? A.inst[i] : -1;
   unsigned bits = 0u;
+  if (!STEP && in && A.any[1] && cspm_due(T[s], A.istep, s)) A.dr[i] = A.drh[i];
   if (in && (STEP ? T[s].use_dpc : T[s].reuse)) {
     float d2 = 0.f;
 #pragma unroll
@@ -1457,7 +1439,7 @@ struct gcsph_ens {
   // state, double-buffered for the re-sort
   DevBuf X[2][3], V[2][3], DXB[2][3], DVB[2][3], DR[2], DRB[2], PT[2], ID[2];
   DevBuf OFFN[3];
-  DevBuf INST, KEY, SLOT, TMP, PERM, SKEY, OFF[3], OFFH[3], VH[3], DRH, COUNT, CELLSTART, SCRATCH, TAB, MOVES, OUT;
+  DevBuf INST, KEY, SLOT, TMP, SKEY, OFF[3], OFFH[3], VH[3], DRH, COUNT, CELLSTART, SCRATCH, TAB, MOVES, OUT;
   DevBuf ISTEP;          // steps done per instance (cspmcorr! schedule), packing order
   DevBuf NL, NLC;        // neighbour list of the step and its row lengths
   DevBuf FLAGS;          // [0] list overflow, [1] longest row, [2] steps done in the call
@@ -1612,7 +1594,7 @@ int ens_reserve(gcsph_ens* e, int64_t n) {
     if ((rc = keep(e->PT[b], sizeof(int32_t)))) return rc;
     if ((rc = keep(e->ID[b], sizeof(int32_t)))) return rc;
   }
-  DevBuf* i32[] = {&e->INST, &e->KEY, &e->SLOT, &e->TMP, &e->PERM};
+  DevBuf* i32[] = {&e->INST, &e->KEY, &e->SLOT, &e->TMP};
   for (DevBuf* b : i32)
     if ((rc = b->ensure(sizeof(int32_t) * want, e->st))) return rc;
   // kept across the growth: the cells and build offsets of instances that keep their lists
@@ -1918,11 +1900,8 @@ int ens_enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
   k_ens_scatter<<<bg, BIN_TPB, 0, st>>>(N, e->KEY.as<int32_t>(), e->SLOT.as<int32_t>(), e->CELLSTART.as<int32_t>(),
                                         e->TMP.as<int32_t>(), e->K, e->COUNT.as<int32_t>(), any);
   GC_LAUNCHED();
-  k_ens_rank<<<bg, BIN_TPB, 0, st>>>(N, e->TMP.as<int32_t>(), e->KEY.as<int32_t>(), e->CELLSTART.as<int32_t>(),
-                                     e->ID[e->cur].as<int32_t>(), e->PERM.as<int32_t>(), any);
-  GC_LAUNCHED();
-  k_ens_move<D><<<bg, BIN_TPB, 0, st>>>(N, e->PERM.as<int32_t>(), e->KEY.as<int32_t>(), ens_state(e, e->cur),
-                                        ens_state(e, e->cur ^ 1), e->SKEY.as<int32_t>(), any);
+  k_ens_move<D><<<bg, BIN_TPB, 0, st>>>(N, e->TMP.as<int32_t>(), e->KEY.as<int32_t>(), e->CELLSTART.as<int32_t>(),
+                                        ens_state(e, e->cur), ens_state(e, e->cur ^ 1), e->SKEY.as<int32_t>(), any);
   GC_LAUNCHED();
   float* o2 = D == 3 ? e->OFF[2].as<float>() : e->OFF[0].as<float>();
   k_ens_start<D><<<nblocks(N, 256), 256, 0, st>>>(N, e->SKEY.as<int32_t>(), e->INST.as<int32_t>(), T,
@@ -1998,9 +1977,6 @@ int ens_enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
   if (e->any_cspm) {
     timer_begin(T_CSPM, st);
     k_ens_cspm<D><<<grid, tpb, 0, st>>>(A, T, e->ISTEP.as<int32_t>());
-    GC_LAUNCHED();
-    k_ens_cspm_apply<<<bg, BIN_TPB, 0, st>>>(N, e->INST.as<int32_t>(), T, e->ISTEP.as<int32_t>(), e->DRH.as<float>(),
-                                             e->DR[e->cur].as<float>(), A.ovf, any);
     GC_LAUNCHED();
     timer_end(T_CSPM, st);
   }
@@ -2246,7 +2222,7 @@ void ens_destroy(gcsph_ens* e) {
     e->PT[b].release();
     e->ID[b].release();
   }
-  DevBuf* one[] = {&e->ANY, &e->INST, &e->KEY, &e->SLOT, &e->TMP, &e->PERM, &e->SKEY, &e->DRH, &e->COUNT, &e->CELLSTART,
+  DevBuf* one[] = {&e->ANY, &e->INST, &e->KEY, &e->SLOT, &e->TMP, &e->SKEY, &e->DRH, &e->COUNT, &e->CELLSTART,
                    &e->SCRATCH, &e->TAB, &e->MOVES, &e->OUT, &e->ISTEP, &e->NL, &e->NLC, &e->FLAGS,
                    &e->R1, &e->R2};
   for (DevBuf* b : one) b->release();
