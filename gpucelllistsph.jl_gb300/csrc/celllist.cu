@@ -1107,30 +1107,6 @@ int CellCore::pair_lanes() const {
   return L;
 }
 
-#define PAIRS_LAUNCH(MODE, L, ...)                                                               \
-  do {                                                                                           \
-    const int _g = nblocks(N * (int64_t)(L), TPB);                                               \
-    if (D == 2) {                                                                                \
-      switch (L) {                                                                               \
-        case 1: k_pairs<2, MODE, 1><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 2: k_pairs<2, MODE, 2><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 4: k_pairs<2, MODE, 4><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 8: k_pairs<2, MODE, 8><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 16: k_pairs<2, MODE, 16><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                   \
-        default: k_pairs<2, MODE, 32><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                   \
-      }                                                                                          \
-    } else {                                                                                     \
-      switch (L) {                                                                               \
-        case 1: k_pairs<3, MODE, 1><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 2: k_pairs<3, MODE, 2><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 4: k_pairs<3, MODE, 4><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 8: k_pairs<3, MODE, 8><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                     \
-        case 16: k_pairs<3, MODE, 16><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                   \
-        default: k_pairs<3, MODE, 32><<<_g, TPB, 0, st>>>(__VA_ARGS__); break;                   \
-      }                                                                                          \
-    }                                                                                            \
-  } while (0)
-
 #define PAIRS32_LAUNCH(MODE, L, ...)                                                             \
   do {                                                                                           \
     const int _g = nblocks(N * (int64_t)(L), TPB);                                               \

@@ -2238,7 +2238,7 @@ void ens_destroy(gcsph_ens* e) {
 int ens_bytes_per_particle(int32_t D, int64_t* bytes) {
   if (!bytes || (D != 2 && D != 3)) return fail(GCSPH_EINVAL, "bad argument");
   // 2 x (x f64, v f32, x and v base differences f32) per dim + 2 x (δρ,
-  // δρ base, ptype, id) + inst, key, slot, tmp, perm, skey + (off, offh, vh,
+  // δρ base, ptype, id) + inst, key, slot, tmp, skey and 4 spare + (off, offh, vh,
   // offn) per dim + δρ½, plus about one cell per particle
   // + the step's neighbour list (64 entries in 2-D, 256 in 3-D, 4 B each) and its length
   *bytes = 2 * D * (8 + 4 + 8) + 2 * 16 + 6 * 4 + D * 16 + 4 + 8 + (D == 2 ? 64 : 256) * 4 + 4 +
