@@ -459,7 +459,8 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
   if (D != 2 && D != 3) return fail(GCSPH_EINVAL, "wrong dimention: D=%d (2 or 3)", D);
   if (N < 1 || N > 0x7ffffffeLL) return fail(GCSPH_EINVAL, "N=%lld out of range", (long long)N);
   if (!(dist > 0)) return fail(GCSPH_EINVAL, "dist must be > 0");
-  GC_CUDA(cudaMallocHost((void**)&pin, 8 * sizeof(int64_t)));
+  // scalars read back, then the bounding box's partial extents
+  GC_CUDA(cudaMallocHost((void**)&pin, 8 * sizeof(int64_t) + sizeof(double) * 2 * D * minmax_blocks()));
   const double seps = 1.4901161193847656e-08;  // sqrt(eps(Float64)) = 2^-26
   double mn[3], mx[3];
   if (!MIN || !MAX) {
@@ -467,10 +468,7 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
     DevBuf part;
     int rc = part.ensure(sizeof(double) * 2 * D * nb, st);
     if (rc) return rc;
-    double* hp = nullptr;
-    GC_CUDA(cudaMallocHost((void**)&hp, sizeof(double) * 2 * D * nb));
-    rc = bounding_box(D, xin, N, nb, part.as<double>(), hp, st, mn, mx);
-    cudaFreeHost(hp);
+    rc = bounding_box(D, xin, N, nb, part.as<double>(), (double*)(pin + 8), st, mn, mx);
     part.release();
     if (rc) return rc;
   }
@@ -494,41 +492,76 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
   g.D = D;
   g.ncell = ncell;
   g.dist2 = dist * dist;
-  int rc;
-  if ((rc = count.ensure(sizeof(int32_t) * ncell, st, true))) return rc;  // zero at rest
-  if ((rc = cellstart.ensure(sizeof(int32_t) * (ncell + 1), st))) return rc;
-  if ((rc = key.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = slot.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = tmp.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = tord.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = perm.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = skey.ensure(sizeof(int32_t) * N, st))) return rc;
-  // the spare original-index map every binning writes into (then swapped in)
-  if ((rc = orig_b.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = orig.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = cnt_full.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = cnt_up.ensure(sizeof(int32_t) * N, st))) return rc;
-  if ((rc = rs_full.ensure(sizeof(int64_t) * (N + 1), st))) return rc;
-  if ((rc = rs_up.ensure(sizeof(int64_t) * (N + 1), st))) return rc;
+  // What the point count and the grid size is cut from one allocation: a
+  // cudaMalloc takes 11 to 35 us, and these were two thirds of what the
+  // construction of a small list took
   int64_t sc = scan_scratch_elems((ncell > N ? ncell : N) + 1);
-  if ((rc = scratch.ensure(sizeof(int64_t) * (sc + 16), st))) return rc;
-  // zeroed once: each pass that folds a scan resets its counter itself
-  if ((rc = foldcnt.ensure(sizeof(unsigned) * 2, st, true))) return rc;
-  if (N + 1 <= SCAN_FOLD_MAX &&
-      (rc = foldsum.ensure(sizeof(int32_t) * (2 * N + 4 * ROWS_FOLD_MAX_BLOCKS + 2), st)))
-    return rc;
-  if (N > RADIX_MIN_N) {
-    const int64_t ntiles = (N + RADIX_TILE - 1) / RADIX_TILE;
-    for (int b = 0; b < 2; ++b) {
-      if ((rc = rkey[b].ensure(sizeof(int32_t) * N, st))) return rc;
-      if ((rc = rval[b].ensure(sizeof(int32_t) * N, st))) return rc;
-    }
-    if ((rc = rhist.ensure(sizeof(int32_t) * 256 * ntiles, st))) return rc;
-    if ((rc = rhoff.ensure(sizeof(int32_t) * (256 * ntiles + 1), st))) return rc;
-    if ((rc = popmax.ensure(sizeof(int), st, true))) return rc;
-    GC_CUDA(cudaEventCreateWithFlags(&ev_pop, cudaEventDisableTiming));
-    if (scan_scratch_elems(256 * ntiles + 1) > sc) return fail(GCSPH_EINVAL, "radix scan scratch");
+  const bool radix = N > RADIX_MIN_N, small = N + 1 <= SCAN_FOLD_MAX;
+  const int64_t ntiles = (N + RADIX_TILE - 1) / RADIX_TILE;
+  if (radix && scan_scratch_elems(256 * ntiles + 1) > sc) return fail(GCSPH_EINVAL, "radix scan scratch");
+  size_t upf_b, uptot_b, upbase_b, upstat_b, uprec_b;
+  upper_sizes(&upf_b, &uptot_b, &upbase_b, &upstat_b, &uprec_b);
+  const size_t n4 = sizeof(int32_t) * (size_t)N, n8 = sizeof(int64_t) * (size_t)(N + 1);
+  const struct Cut {
+    DevBuf* b;
+    size_t bytes;
+  } cuts[] = {
+      // zero from here to the first of the others: the cell counts (zero at
+      // rest), the counters of the passes whose last block does more (each
+      // resets its own), the bound that a build accumulates
+      {&count, sizeof(int32_t) * (size_t)ncell},
+      {&foldcnt, sizeof(unsigned) * 2},
+      {&popmax, radix ? sizeof(int) : 0},
+      {&pfcnt, sizeof(unsigned)},
+      {&pfmax, sizeof(unsigned long long)},
+      {&cellstart, sizeof(int32_t) * (size_t)(ncell + 1)},
+      {&key, n4},
+      {&slot, n4},
+      {&tmp, n4},
+      {&tord, n4},
+      {&perm, n4},
+      {&skey, n4},
+      {&orig_b, n4},  // the spare original-index map every binning writes into (then swapped in)
+      {&orig, n4},
+      {&cnt_full, n4},
+      {&cnt_up, n4},
+      {&rs_full, n8},
+      {&rs_up, n8},
+      {&scratch, sizeof(int64_t) * (size_t)(sc + 16)},
+      {&foldsum, small ? sizeof(int32_t) * (size_t)(2 * N + 4 * ROWS_FOLD_MAX_BLOCKS + 2) : 0},
+      {&rkey[0], radix ? n4 : 0},
+      {&rkey[1], radix ? n4 : 0},
+      {&rval[0], radix ? n4 : 0},
+      {&rval[1], radix ? n4 : 0},
+      {&rhist, radix ? sizeof(int32_t) * 256 * (size_t)ntiles : 0},
+      {&rhoff, radix ? sizeof(int32_t) * (256 * (size_t)ntiles + 1) : 0},
+      {&pfthr, sizeof(float2)},
+      {&upf, upf_b},
+      {&uptot, uptot_b},
+      {&upbase, upbase_b},
+      {&upstat, upstat_b},
+      {&uprec, uprec_b},
+  };
+  size_t total = 0, zero = 0;
+  for (const Cut& c : cuts) {
+    if (c.b == &cellstart) zero = total;
+    total += (c.bytes + 255) / 256 * 256;
   }
+  int rc;
+  if ((rc = arena.ensure(total, st))) return rc;
+  size_t at = 0;
+  for (const Cut& c : cuts) {
+    if (c.bytes == 0) continue;
+    c.b->p = arena.as<char>() + at;
+    c.b->bytes = c.bytes;
+    c.b->part = true;
+    at += (c.bytes + 255) / 256 * 256;
+  }
+  GC_CUDA(cudaMemsetAsync(arena.p, 0, zero, st));
+  // the vectors past the last point, which a search may read
+  const size_t vec = sizeof(float) * (D == 2 ? 2 : 4);
+  GC_CUDA(cudaMemsetAsync(upf.as<char>() + vec * (size_t)N, 0, upf_b - vec * (size_t)N, st));
+  if (radix) GC_CUDA(cudaEventCreateWithFlags(&ev_pop, cudaEventDisableTiming));
   return GCSPH_OK;
 }
 
@@ -536,7 +569,7 @@ void CellCore::release() {
   DevBuf* all[] = {&count, &cellstart, &key, &slot, &tmp, &tord, &perm, &skey, &orig, &cnt_full, &cnt_up, &rs_full,
                    &rs_up, &nbr, &scratch, &pf[0], &pf[1], &pf[2], &pfmax, &pfthr, &pfcnt, &orig_b, &stage,
                    &foldcnt, &foldsum, &rkey[0], &rkey[1], &rval[0], &rval[1], &rhist, &rhoff, &popmax,
-                   &upf, &upkept, &uptot, &upbase, &upstat, &uprec};
+                   &upf, &upkept, &uptot, &upbase, &upstat, &uprec, &arena};
   for (DevBuf* b : all) b->release();
   if (ev_pop) cudaEventDestroy(ev_pop);
   ev_pop = nullptr;

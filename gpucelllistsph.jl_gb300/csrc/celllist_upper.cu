@@ -544,6 +544,18 @@ static Pos3 pos3(const double* const* in, double* const* out) {
   return P;
 }
 
+// bytes of the search's buffers (cut from the cell list's allocation)
+void CellCore::upper_sizes(size_t* upf_b, size_t* uptot_b, size_t* upbase_b, size_t* upstat_b,
+                           size_t* uprec_b) const {
+  const size_t nb = (size_t)nblocks(N, UTPB), n = (size_t)N;
+  // (a group of padding, which a walk may read and cut off)
+  *upf_b = D == 2 ? sizeof(PfVec<2>::T) * (n + UP_GROUP<2>) : sizeof(PfVec<3>::T) * (n + UP_GROUP<3>);
+  *uptot_b = sizeof(int32_t) * (nb + 4);
+  *upbase_b = sizeof(int64_t) * (nb + 1);
+  *upstat_b = sizeof(UpStat);
+  *uprec_b = sizeof(PointRec) * n;
+}
+
 template <int D>
 static int build_upper_impl(CellCore& C, const double* const* xin, double* const* xs, bool rebin) {
   using V = typename PfVec<D>::T;
@@ -552,11 +564,6 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
   const int nb = nblocks(N, UTPB);
   int rc;
   if ((rc = C.ensure_pf_scalars())) return rc;
-  // a group of padding, which a walk may read and cut off
-  if (!C.upf.p && (rc = C.upf.ensure(sizeof(V) * (N + UP_GROUP<D>), st, true))) return rc;
-  if ((rc = C.uptot.ensure(sizeof(int32_t) * ((size_t)nb + 4), st))) return rc;
-  if ((rc = C.upbase.ensure(sizeof(int64_t) * ((size_t)nb + 1), st))) return rc;
-  if ((rc = C.upstat.ensure(sizeof(UpStat), st))) return rc;
   V* pf = C.upf.as<V>();
   const Pos3 P = pos3<D>(xin, xs);
   unsigned long long* bm = C.pfmax.as<unsigned long long>();
@@ -564,7 +571,6 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
   unsigned* cnt = C.pfcnt.as<unsigned>();
   bool deferred = false;
   if (rebin) {
-    if ((rc = C.uprec.ensure(sizeof(PointRec) * N, st))) return rc;
     if ((rc = C.sort(xin, nullptr, true, &deferred, false, C.uprec.as<PointRec>()))) return rc;
   }
   if (!C.sorted && !deferred) return fail(GCSPH_ESTATE, "pair build before binning");

@@ -150,9 +150,7 @@ int DevBuf::ensure(size_t need, cudaStream_t s, bool zero) {
     if (p) {
       cudaError_t e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__);
-      cudaFree(p);
-      p = nullptr;
-      bytes = 0;
+      release();
     }
     cudaError_t e = cudaMalloc(&p, need);
     if (e != cudaSuccess) {
@@ -169,9 +167,10 @@ int DevBuf::ensure(size_t need, cudaStream_t s, bool zero) {
 }
 
 void DevBuf::release() {
-  if (p) cudaFree(p);
+  if (p && !part) cudaFree(p);
   p = nullptr;
   bytes = 0;
+  part = false;
 }
 
 // ---------------------------------------------------------------------------

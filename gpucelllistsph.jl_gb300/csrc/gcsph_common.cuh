@@ -330,6 +330,7 @@ void timer_release(std::vector<TimerRec>& recs);
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool part = false;  // of another buffer's allocation: not freed by itself
   int ensure(size_t need, cudaStream_t s, bool zero = false);
   void release();
   template <class T> T* as() const { return (T*)p; }
