@@ -107,11 +107,10 @@ def gather_stage_bytes(case, npairs):
 
 def design_stage_bytes(case, npairs):
     """The bytes pass A of this design moves per launch (beyond the
-    algorithmic ones: its pair quads, 16 B a pair, and both sides' entry
-    slots, 2·(8 W + 8D ∇W + 8 ρ̇ + 8D a), which pass B sums from L2):
-    N·(16D + 28) + P·(16 + 2·(16 + 16D))."""
+    algorithmic ones: its pair quads, 16 B a pair, both sides' 32-byte slots,
+    which pass B sums from L2, and ∇W, 8D): N·(16D + 28) + P·(16 + 64 + 8D)."""
     D, N = case.D, case.N
-    return N * (16 * D + 28) + npairs * (16 + 2 * (16 + 16 * D))
+    return N * (16 * D + 28) + npairs * (16 + 64 + 8 * D)
 
 
 def ens_stage_bytes(D, particles, pairs):
@@ -155,14 +154,14 @@ def algorithmic_flops_stage1(case, x, v):
 
 
 # DRAM bytes (read + write) of one stage-1 pass A launch on this workload and
-# its FP64 pipe's busy fraction (of active cycles), from one ncu --set full
+# its FP64 pipe's busy fraction (of active cycles), from one ncu
 # capture of that launch (one block per SM, 103,881 pairs)
-PAIRA_STAGE1_DRAM_BYTES = 2_215_168 + 124_672
-PAIRA_STAGE1_FP64_PIPE = 0.764
+PAIRA_STAGE1_DRAM_BYTES = 2_053_888
+PAIRA_STAGE1_FP64_PIPE = 0.730
 # the FP32 ensemble's stage passes are bound by instruction issue: their busy
-# fraction of the issue slots (of active SMs) in one ncu --set full capture of
+# fraction of the issue slots (of active SMs) in one ncu capture of
 # the 64-instance 2-D ensemble (one launch of each stage)
-ENS_STAGE_ISSUE_FRAC = {"stage1": 0.628, "stage2": 0.673}
+ENS_STAGE_ISSUE_FRAC = {"stage1": 0.710, "stage2": 0.800}
 
 
 class Clocks:
@@ -407,7 +406,7 @@ def run_batched(g, args, plain_c1, hbm_peak):
                         "achieved_gbs": alg / avg_s / 1e9, "frac_of_hbm": alg / avg_s / 1e9 / hbm_peak,
                         "issue_slots_busy_ncu": ENS_STAGE_ISSUE_FRAC[st]}
     roof["note"] = ("bytes = N(12D+16) + 2P*4 with P the pairs within H at the instances' initial states "
-                    "(update!); the passes are bound by instruction issue (63-67% of issue slots in ncu, with "
+                    "(update!); the passes are bound by instruction issue (71-80% of issue slots in ncu, with "
                     "long-scoreboard waits on the neighbour records), their working set per step is re-read "
                     "from L2")
     sizes = sorted(wl, key=lambda t: t[0].N)
@@ -794,8 +793,8 @@ def run_gb300(args):
             "avg_launch_us": avg_s * 1e6, "alg_bytes_per_launch": alg,
             "alg_bytes_rule": "gather-form pair-sum stage: N(24D+28) + 2P*4 (P = pairs k<m)",
             "traffic_design": design_stage_bytes(case, npairs) if stage else None,
-            "traffic_design_rule": "this design's pass A: N(16D+28) + P(16 + 2(16+16D)) (pair quads read, "
-                                   "both entry slots written; pass B sums them from L2)",
+            "traffic_design_rule": "this design's pass A: N(16D+28) + P(16 + 64 + 8D) (pair quads read, "
+                                   "both slots and the kernel gradient written; pass B sums the slots from L2)",
             "fp64_pipe_frac_ncu": PAIRA_STAGE1_FP64_PIPE if top == "stage1" else None,
             "note": "pass A is FP64-pipe bound (GB300 issues 2 FP64 instr/cycle/SM); its working set stays in "
                     "L2, so the HBM fraction against the measured copy bandwidth is small by construction; the "
