@@ -451,7 +451,7 @@ int CellCore::read_scalar(const int64_t* dev, int64_t* host) {
 }
 
 int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, const double* MIN, const double* MAX,
-                   const double* const* xin, cudaStream_t s) {
+                   const double* const* xin, DevBuf* pos, cudaStream_t s) {
   D = D_;
   N = N_;
   dist = dist_;
@@ -463,14 +463,19 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
   GC_CUDA(cudaMallocHost((void**)&pin, 8 * sizeof(int64_t) + sizeof(double) * 2 * D * minmax_blocks()));
   const double seps = 1.4901161193847656e-08;  // sqrt(eps(Float64)) = 2^-26
   double mn[3], mx[3];
+  // the cell-ordered positions and the bounding box's partial extents, one allocation
+  const int nb = minmax_blocks();
+  const size_t xb = (sizeof(double) * (size_t)N + 255) / 256 * 256;
+  int rc = arena_x.ensure(D * xb + sizeof(double) * 2 * D * nb, st);
+  if (rc) return rc;
+  for (int d = 0; d < D; ++d) {
+    pos[d].p = arena_x.as<char>() + d * xb;
+    pos[d].bytes = sizeof(double) * (size_t)N;
+    pos[d].part = true;
+  }
   if (!MIN || !MAX) {
-    const int nb = minmax_blocks();
-    DevBuf part;
-    int rc = part.ensure(sizeof(double) * 2 * D * nb, st);
-    if (rc) return rc;
-    rc = bounding_box(D, xin, N, nb, part.as<double>(), (double*)(pin + 8), st, mn, mx);
-    part.release();
-    if (rc) return rc;
+    double* part = reinterpret_cast<double*>(arena_x.as<char>() + D * xb);
+    if ((rc = bounding_box(D, xin, N, nb, part, (double*)(pin + 8), st, mn, mx))) return rc;
   }
   int64_t ncell = 1;
   for (int d = 0; d < D; ++d) {
@@ -547,7 +552,6 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
     if (c.b == &cellstart) zero = total;
     total += (c.bytes + 255) / 256 * 256;
   }
-  int rc;
   if ((rc = arena.ensure(total, st))) return rc;
   size_t at = 0;
   for (const Cut& c : cuts) {
@@ -569,7 +573,7 @@ void CellCore::release() {
   DevBuf* all[] = {&count, &cellstart, &key, &slot, &tmp, &tord, &perm, &skey, &orig, &cnt_full, &cnt_up, &rs_full,
                    &rs_up, &nbr, &scratch, &pf[0], &pf[1], &pf[2], &pfmax, &pfthr, &pfcnt, &orig_b, &stage,
                    &foldcnt, &foldsum, &rkey[0], &rkey[1], &rval[0], &rval[1], &rhist, &rhoff, &popmax,
-                   &upf, &upkept, &uptot, &upbase, &upstat, &uprec, &arena};
+                   &upf, &upkept, &uptot, &upbase, &upstat, &uprec, &arena, &arena_x};
   for (DevBuf* b : all) b->release();
   if (ev_pop) cudaEventDestroy(ev_pop);
   ev_pop = nullptr;
@@ -1396,9 +1400,7 @@ int gcl_create(int32_t D, int64_t N, const double* const* x_dev, const double* c
     if (!x_dev[d]) return fail(GCSPH_EINVAL, "null coordinate array %d", d + 1);
   gcl_handle* h = new gcl_handle();
   for (int d = 0; d < D; ++d) h->xuser[d] = x_dev[d];
-  int rc = h->core.init(D, N, cellsize, dist, MIN_or_null, MAX_or_null, x_dev, (cudaStream_t)stream);
-  if (!rc)
-    for (int d = 0; d < D && !rc; ++d) rc = h->xs[d].ensure(sizeof(double) * N, h->core.st);
+  int rc = h->core.init(D, N, cellsize, dist, MIN_or_null, MAX_or_null, x_dev, h->xs, (cudaStream_t)stream);
   if (!rc) rc = gcl_build(h, true);
   if (rc) {
     std::string keep = gcsph_last_error();

@@ -216,7 +216,8 @@ struct CellCore {
   bool rows_upper = false;  // the last build is the list's own (pairs k < m alone, as masks or rows)
   // their search: FP32 vectors, what each point keeps, block totals and starts, statistics
   DevBuf upf, upkept, uptot, upbase, upstat, uprec;
-  DevBuf arena;         // holds the buffers whose size the point count and the grid fix (init)
+  // the buffers whose size the point count and the grid fix, and the cell list's positions (init)
+  DevBuf arena, arena_x;
   double* up_xs[3] = {nullptr, nullptr, nullptr};  // the positions it was made on
   int up_w = 0;          // entries kept per point
   bool up_rows = false;  // neighbours rather than words
@@ -232,7 +233,7 @@ struct CellCore {
 
   void upper_sizes(size_t* upf_b, size_t* uptot_b, size_t* upbase_b, size_t* upstat_b, size_t* uprec_b) const;
   int init(int D_, int64_t N_, const double* cellsize, double dist_, const double* MIN, const double* MAX,
-           const double* const* xin, cudaStream_t s);
+           const double* const* xin, DevBuf* pos, cudaStream_t s);
   void release();
   // bin xin (input order) into the frozen grid and sort by (cell, ord[i]);
   // ord == nullptr means the input order is the original order.
