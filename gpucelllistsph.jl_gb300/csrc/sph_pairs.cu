@@ -14,7 +14,7 @@
 // reciprocals, roots and the cosine by rcp_pair, sqrt_pair and pf_cos,
 // powfancy7th by its series, dot products and products of constants fused.
 // Measured with the queue below (one GB300, 10.5M pairs of a 3-D tank, 179k
-// particles): ∂v∂tpF! 1577 -> 388 us, ∂ρ∂tDDT! 1403 -> 478, sph∑W! 499 -> 310,
+// particles): ∂v∂tpF! 1577 -> 366 us, ∂ρ∂tDDT! 1403 -> 403, sph∑W! 499 -> 310,
 // ∂v∂t_visc! 475 -> 281, fbmolforce! 449 -> 223, ∂v∂t_av! 425 -> 263, ∂v∂t! 231 -> 180,
 // xsphcorr! 179 -> 151.
 #include <math.h>
