@@ -144,15 +144,20 @@ template <int D, int S>
 struct Rec {
   float4 a, b, c;
 };
+// A 32-byte record in one load: half the L1 lookups of two 16-byte ones (the
+// stage passes within 0.5%, xsphcorr! see there).  The records start on 32 bytes.
+__device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
 template <int D, int S>
 __device__ __forceinline__ Rec<D, S> load_rec(const float4* __restrict__ r1, const float4* __restrict__ r2, int j) {
   Rec<D, S> x;
   if (S == 1) {
-    x.a = __ldg(r1 + 2 * (int64_t)j);
-    x.b = __ldg(r1 + 2 * (int64_t)j + 1);
+    load32(r1 + 2 * (int64_t)j, x.a, x.b);
   } else if (D == 2) {
-    x.a = __ldg(r2 + 2 * (int64_t)j);
-    x.b = __ldg(r2 + 2 * (int64_t)j + 1);
+    load32(r2 + 2 * (int64_t)j, x.a, x.b);
   } else {
     x.a = __ldg(r2 + 3 * (int64_t)j);
     x.b = __ldg(r2 + 3 * (int64_t)j + 1);
@@ -1128,11 +1133,13 @@ __global__ void k_ens_dpc_apply(EnsArr A, const EnsInst* __restrict__ T) {
 // (pairs and distances at x), v and ρ after the corrector and dpcreg!;
 // moves x only.  Reads neighbours' v, writes its own x: one pass.  Little
 // arithmetic per neighbour and a record gather each: latency-bound, so two
-// records are loaded at a time (390k particles in 3-D: a step takes 654 us with
-// two, 678 with one, 686 with four; two with 40 registers a thread 709)
-constexpr int XSPH_U = 2;
+// records are loaded at a time (390k particles in 3-D: a step took 654 us with
+// two, 678 with one, 686 with four), each as one 32-byte access, at 56
+// registers, which leaves nine blocks of 128 an SM (a step 575 us; 59 registers
+// 610, 48 581, 40 620; two 16-byte accesses 587)
+constexpr int XSPH_U = 2, XSPH_REGS = 56;
 template <int D>
-__global__ void __launch_bounds__(ENS_MAX_TPB, 2) k_ens_xsph(EnsArr A, const EnsInst* __restrict__ T) {
+__global__ void __maxnreg__(XSPH_REGS) k_ens_xsph(EnsArr A, const EnsInst* __restrict__ T) {
   if (*A.ovf) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < A.N; i += stride) {
