@@ -33,6 +33,9 @@ int fail(int code, const char* fmt, ...) {
 
 int cuda_fail(cudaError_t e, const char* what, const char* file, int line) {
   set_error("CUDA error %d (%s) in %s at %s:%d", (int)e, cudaGetErrorString(e), what, file, line);
+  // the caller has it from here: left standing, a refused allocation would be
+  // reported again by the next launch, ours or another library's
+  cudaGetLastError();
   return e == cudaErrorMemoryAllocation ? GCSPH_ENOMEM : GCSPH_ECUDA;
 }
 
