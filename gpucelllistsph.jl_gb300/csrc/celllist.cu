@@ -699,8 +699,7 @@ void CellCore::sort_done() {
   std::swap(orig.p, orig_b.p);
   std::swap(orig.bytes, orig_b.bytes);
   sorted = true;
-  built = false;
-  up_valid = up_scanned = false;
+  list_gone();
 }
 
 int CellCore::read_popmax() {
@@ -1187,6 +1186,7 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
                           bool* pq_done) {
   if (pq_done) *pq_done = false;
   if (!sorted) return fail(GCSPH_ESTATE, "pair build before binning");
+  list_gone();
   const double* x2 = D == 3 ? xs[2] : xs[0];
   timer_begin(T_PAIRS, st);
   const int L = pair_lanes();
@@ -1282,6 +1282,7 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
 
 int CellCore::grow_nbr(int64_t need) {
   const int64_t want = need + need / 4 + 1024;
+  nbr_cap = 0;  // nothing fits a buffer that could not be grown
   int rc = nbr.ensure(sizeof(int32_t) * want, st);
   if (rc) return rc;
   nbr_cap = want;

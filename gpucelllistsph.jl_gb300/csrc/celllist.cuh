@@ -255,6 +255,10 @@ struct CellCore {
   bool keys_in_step() const { return g.ncell + 1 <= SCAN_FOLD_MAX && N <= RADIX_MIN_N && sort_mode != 2; }
   // the bookkeeping after a binning into perm / skey / orig_b (orig_b becomes orig)
   void sort_done();
+  // Every build starts with this and sets the flags again at its end: it
+  // overwrites what the list before it is read from (offsets, kept words or
+  // rows, neighbours), so after a build that failed there is no list.
+  void list_gone() { built = up_valid = up_scanned = rows_upper = false; }
   int read_popmax();
   void take_popmax();  // the value read back into pin[7]
   // the list's own pair set, k < m, as masks or rows (celllist_upper.cu): rebin bins

@@ -602,7 +602,10 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
     C.up_w = ((int)(need < top ? need : top) + 8) / 4 * 4;
   }
   for (;;) {
-    if (C.up_w > 0 && (rc = C.upkept.ensure(sizeof(unsigned) * (size_t)N * (size_t)C.up_w, st))) return rc;
+    if ((rc = C.upkept.ensure(sizeof(unsigned) * (size_t)N * (size_t)C.up_w, st))) {
+      C.up_w = 0;  // the next build guesses anew
+      return rc;
+    }
     GC_CUDA(cudaMemsetAsync(C.upstat.p, 0, sizeof(UpStat), st));
     const auto count = C.up_rows ? k_up_count<D, true> : k_up_count<D, false>;
     count<<<nb, UTPB, 0, st>>>(pf, P, thr, C.skey.as<int32_t>(), C.cellstart.as<int32_t>(), N, C.g,
@@ -690,6 +693,7 @@ int CellCore::count_rows(const double* const* xs, int32_t* stg, int S) {
 }
 
 int CellCore::build_upper(const double* const* xin, double* const* xs, bool rebin) {
+  list_gone();
   up_xs[0] = xs[0];
   up_xs[1] = xs[1];
   up_xs[2] = D == 3 ? xs[2] : nullptr;

@@ -810,6 +810,7 @@ static int grow_entry_arrays(sph_handle* h) {
   if (core.nbr_cap <= h->we_cap) return GCSPH_OK;
   const int64_t want = core.nbr_cap;
   int rc;
+  h->we_cap = 0;  // until every one of them has grown
   if ((rc = h->We.ensure(sizeof(double) * want, core.st))) return rc;
   if ((rc = h->CE.ensure(sizeof(PairOut) * want, core.st))) return rc;
   if (want / 2 + 1 > (int64_t)INT32_MAX) return fail(GCSPH_ECAPACITY, "neighbour entries past 2^31");

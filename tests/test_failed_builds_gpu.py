@@ -40,3 +40,20 @@ def test_a_refused_allocation_is_reported_once(gpu_pkg):
     back()
     d, _, _ = _spread(gpu_pkg)
     assert torch.equal(d.neighborlistview(), before)
+
+
+def test_a_failed_partialupdate_leaves_no_list(gpu_pkg):
+    """The list from before is overwritten by then: none is handed out, and
+    the next update! makes one again."""
+    c, closer, back = _spread(gpu_pkg)
+    before = c.neighborlistview().clone()
+    closer()
+    with pytest.raises(gpu_pkg.GcsphError) as e:
+        c.partialupdate()
+    assert e.value.code == gpu_pkg._lib.GCSPH_ENOMEM
+    L, n = gpu_pkg.load_library(), C.c_int64(-1)
+    # (asks for the count alone: nothing is launched)
+    assert L.gcl_emit_pairs(c._h, None, 0, 0, C.byref(n)) == gpu_pkg._lib.GCSPH_ESTATE
+    back()
+    c.update()
+    assert torch.equal(c.neighborlistview(), before)
