@@ -811,9 +811,9 @@ static int grow_entry_arrays(sph_handle* h) {
   const int64_t want = core.nbr_cap;
   int rc;
   h->we_cap = 0;  // until every one of them has grown
+  if (want / 2 + 1 > (int64_t)INT32_MAX) return fail(GCSPH_ECAPACITY, "neighbour entries past 2^31");
   if ((rc = h->We.ensure(sizeof(double) * want, core.st))) return rc;
   if ((rc = h->CE.ensure(sizeof(PairOut) * want, core.st))) return rc;
-  if (want / 2 + 1 > (int64_t)INT32_MAX) return fail(GCSPH_ECAPACITY, "neighbour entries past 2^31");
   if ((rc = h->PQ.ensure(sizeof(int4) * (want / 2 + 1), core.st))) return rc;
   for (int d = 0; d < D; ++d) {
     if ((rc = h->GWe[d].ensure(sizeof(double) * want, core.st))) return rc;
@@ -992,14 +992,17 @@ static int choose_lanes(const sph_handle* h) {
 }
 
 template <int D>
-static int finish_call(sph_handle* h, const StepConst& c, Scal* dsc) {
+static int finish_call(sph_handle* h, const StepConst& c, Scal* dsc, bool stepped) {
   CellCore& core = h->cl->core;
   cudaStream_t st = core.st;
   int rc;
   const bool own = h->in_cell_order;
   const int L = choose_lanes(h);
-  // the split rows' sums write the state back to the caller's order as well
-  const bool fold = own && L > 1 && core.built;
+  // the split rows' sums write the state back to the caller's order as well,
+  // and add up the pairs' slots.  Those and the pair list are whole after a
+  // step of this call; the state of a call that failed between its rows and
+  // them is still in cell order, and rows are all that such a list has.
+  const bool fold = stepped && own && L > 1 && core.built;
   if (fold) h->in_cell_order = false;
   else if (own && (rc = scatter_state<D>(h))) return rc;
   if (core.built && core.rows_upper) {
@@ -1238,7 +1241,7 @@ static int step_eager(sph_handle* h, StepConst c, int32_t n, int64_t* updaten_ou
     if (mc > c.reb_thr) skip = false;
     if (mc > maxout) maxout = mc;
   }
-  if ((rc = finish_call<D>(h, c, dsc))) return rc;
+  if ((rc = finish_call<D>(h, c, dsc, n > 0))) return rc;
   GC_CUDA(cudaMemcpyAsync(h->pin, dsc, sizeof(Scal), cudaMemcpyDeviceToHost, st));
   const bool nup = core.built && core.up_scanned && !core.up_valid;
   if (nup && (rc = core.enqueue_nup())) return rc;
@@ -1375,7 +1378,7 @@ static int graph_capture(sph_handle* h, StepConst c, int32_t n, StepGraph& g) {
     if ((rc = rebuild<D>(h, c, &dsc->ovf))) break;
     rc = enqueue_stages<D>(h, c, dsc, cspmcnt, it + 1 < n);
   }
-  if (rc == GCSPH_OK) rc = finish_call<D>(h, c, dsc);
+  if (rc == GCSPH_OK) rc = finish_call<D>(h, c, dsc, true);
   h->keys_ready = false;
   timer_capture_to(nullptr);
   core.st = run_st;

@@ -1,6 +1,5 @@
-"""Builds that fail for want of memory, and what a caller may do after them:
-every request here is larger than the device, so it is refused at once and the
-device keeps its memory."""
+"""Builds that fail, and what a caller may do after them.  Every allocation that
+is refused here is larger than the device, so the device keeps its memory."""
 import ctypes as C
 
 import numpy as np
@@ -57,3 +56,30 @@ def test_a_failed_partialupdate_leaves_no_list(gpu_pkg):
     back()
     c.update()
     assert torch.equal(c.neighborlistview(), before)
+
+
+def test_a_call_of_no_steps_after_a_failed_one(gpu_pkg):
+    """66,000 particles crowd into reach of each other: their rows fit, the
+    pair list (past 2^31) does not, and the step is refused between the two.  A
+    call of no steps then sums W over the rows."""
+    N, H = 66000, 0.01
+    rng = np.random.default_rng(8)
+    x = 0.05 + 0.9 * rng.random((2, N))
+    c = gpu_pkg.GPUCellList(tuple(x), (H, H), H, MIN=(0.0, 0.0), MAX=(1.0, 1.0))
+    h = H / 2
+    prob = gpu_pkg.SPHProblem(c, h / 1.5, h, H, gpu_pkg.WendlandC2(dim=2), np.full(N, 1000.0), np.full(N, 2, np.int32),
+                              1000.0, 1.0, 1e-6, 0.01, 40.0, 7, 0.1, 0.2)
+    prob.set_lanes(4)
+    y = 0.5005 + 0.2 * H * rng.random((2, N))  # one cell
+    for d in range(2):
+        c.points[d].copy_(torch.from_numpy(y[d]))
+    with pytest.raises(gpu_pkg.GcsphError) as e:
+        prob.stepsolve(1)
+    assert e.value.code == gpu_pkg._lib.GCSPH_ECAPACITY
+    assert prob.stepsolve(0)[0] == 0
+    got = prob.field("sumW").cpu().numpy()
+    for i in (0, 1234, N - 1):
+        u = np.delete(np.hypot(y[0] - y[0, i], y[1] - y[1, i]), i) / H
+        want = (7.0 / np.pi / H**2) * ((1.0 + 4.0 * u) * (1.0 - u) ** 4).sum()
+        # a sum of N positive terms: N roundings of it at the very most
+        assert abs(got[i] - want) <= N * 2.0**-52 * want
