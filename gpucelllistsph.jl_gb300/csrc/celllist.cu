@@ -1210,8 +1210,13 @@ int CellCore::build_pairs(const double* const* xs, int* ovf_dev, bool scan_up, b
   int S = 16;
   while (S < 256 && (double)S < 1.5 * mean + 8.0) S <<= 1;
   int32_t* sp = nullptr;
-  if (mean > 0 && (rc0 = stage.ensure(sizeof(int32_t) * (size_t)N * (size_t)S, st)) == GCSPH_OK) sp = stage.as<int32_t>();
-  if (rc0) return rc0;
+  if (mean > 0) {
+    const void* was = stage.p;
+    rc0 = stage.ensure(sizeof(int32_t) * (size_t)N * (size_t)S, st);
+    if (stage.p != was) gen += 1;  // a captured step graph holds the buffer that is gone
+    if (rc0) return rc0;
+    sp = stage.as<int32_t>();
+  }
   // small sets: the count pass's last block scans the row counts (both
   // arrays), so no scan launch follows
   const bool fold = sp && foldsum.p && N + 1 <= SCAN_FOLD_MAX && nblocks(N * (int64_t)L, TPB) <= ROWS_FOLD_MAX_BLOCKS;
