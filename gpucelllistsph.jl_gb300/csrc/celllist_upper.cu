@@ -23,6 +23,7 @@
 // 125 + 86 -> 202 + 100 us.
 //
 // Compiled without FMA contraction: r2_ref is the reference's expression.
+#include <algorithm>
 #include "celllist.cuh"
 
 namespace gcsph {
@@ -589,17 +590,23 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
   timer_end(T_SORT, st);
   timer_begin(T_PAIRS, st);
   // What a point keeps: as much as the last search's fullest point needed and
-  // a quarter more, up to about three times the mean (a crowded cell's points
+  // a quarter more, up to three times the mean, and in dense sets up to 256 past
+  // it, so that what is kept takes no more memory than the neighbours of all
+  // points in one array and a staged row of 256 each (a crowded cell's points
   // are searched again in the emit).  A search that finds its points in need
-  // of more, or of the other form, is run again.  The first one guesses from
-  // the grid-wide mean of candidates, of which about a third are pairs in 2-D
-  // and a sixth in 3-D.
+  // of more, or of the other form, is run again; the width stays while the form
+  // does.  The first search guesses from the grid-wide density: twice the
+  // pairs that it gives a dist-ball (a little more in 3-D).
+  auto room = [](double mean) { return std::min(3.0 * mean + 16.0, mean + 256.0); };
+  auto whole4 = [](double w) { return ((int)w + 3) / 4 * 4; };
   const bool fold = nb <= SCAN_FOLD_MAX;
   if (C.up_w == 0) {
-    const double cand = 0.5 * C.candidates_per_point(), top = 4096.0;
+    const double cand = 0.5 * C.candidates_per_point();
     C.up_rows = cand > 32.0 * UP_FEW;
-    const double need = C.up_rows ? cand * (D == 2 ? 0.7 : 0.35) : cand / 16.0;
-    C.up_w = ((int)(need < top ? need : top) + 8) / 4 * 4;
+    double pairs = cand * (D == 2 ? GCSPH_PI64 / 9.0 : 4.0 * GCSPH_PI64 / 81.0);
+    for (int d = 0; d < D; ++d) pairs *= C.dist / C.cs[d];
+    const double need = C.up_rows ? std::min((D == 2 ? 2.0 : 2.25) * pairs, room(pairs)) : cand / 16.0;
+    C.up_w = whole4(std::min(need, 4096.0) + 8.0);
   }
   for (;;) {
     if ((rc = C.upkept.ensure(sizeof(unsigned) * (size_t)N * (size_t)C.up_w, st))) {
@@ -630,13 +637,12 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
       C.up_rows = !C.up_rows;
       // the other form's need: at a first guess its mean
       const double other = C.up_rows ? (double)C.pin[0] / (double)N : words;
-      C.up_w = ((int)(1.5 * other) + 8 + 3) / 4 * 4;
+      C.up_w = whole4(std::min(1.5 * other + 8.0, room(other)));
       continue;
     }
-    const double bound = 3.0 * mean + 16.0;
-    const int most = (double)s.most < bound ? s.most : (int)bound;
-    if (most <= C.up_w) break;
-    C.up_w = (most + most / 4 + 3) / 4 * 4;
+    const double bound = room(mean), most = std::min((double)s.most, bound);
+    if (whole4(most) <= C.up_w) break;
+    C.up_w = whole4(std::min(1.25 * most, bound));
   }
   timer_end(T_PAIRS, st);
   timer_collect();
