@@ -72,12 +72,14 @@ int minmax_blocks() {
 }
 
 // the bounding box of the D coordinate arrays: one launch, one read-back of
-// the per-block partials (part_dev, part_host: 2 * D * nb doubles), one wait
+// the per-block partials (part_dev, part_host: 2 * D * nb doubles, and one
+// buffer where the GPU writes page-locked host memory), one wait
 int bounding_box(int D, const double* const* x, int64_t N, int nb, double* part_dev, double* part_host,
                  cudaStream_t st, double* mn, double* mx) {
   k_minmax<<<dim3(nb, D), TPB, 0, st>>>(x[0], x[1], D == 3 ? x[2] : x[0], N, part_dev);
   GC_LAUNCHED();
-  GC_CUDA(cudaMemcpyAsync(part_host, part_dev, sizeof(double) * 2 * D * nb, cudaMemcpyDeviceToHost, st));
+  if (part_host != part_dev)
+    GC_CUDA(cudaMemcpyAsync(part_host, part_dev, sizeof(double) * 2 * D * nb, cudaMemcpyDeviceToHost, st));
   GC_CUDA(cudaStreamSynchronize(st));
   for (int d = 0; d < D; ++d) {
     double a = INFINITY, b = -INFINITY;
@@ -463,19 +465,10 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
   GC_CUDA(cudaMallocHost((void**)&pin, 8 * sizeof(int64_t) + sizeof(double) * 2 * D * minmax_blocks()));
   const double seps = 1.4901161193847656e-08;  // sqrt(eps(Float64)) = 2^-26
   double mn[3], mx[3];
-  // the cell-ordered positions and the bounding box's partial extents, one allocation
-  const int nb = minmax_blocks();
-  const size_t xb = (sizeof(double) * (size_t)N + 255) / 256 * 256;
-  int rc = arena_x.ensure(D * xb + sizeof(double) * 2 * D * nb, st);
-  if (rc) return rc;
-  for (int d = 0; d < D; ++d) {
-    pos[d].p = arena_x.as<char>() + d * xb;
-    pos[d].bytes = sizeof(double) * (size_t)N;
-    pos[d].part = true;
-  }
+  int rc;
   if (!MIN || !MAX) {
-    double* part = reinterpret_cast<double*>(arena_x.as<char>() + D * xb);
-    if ((rc = bounding_box(D, xin, N, nb, part, (double*)(pin + 8), st, mn, mx))) return rc;
+    double* part = (double*)(pin + 8);
+    if ((rc = bounding_box(D, xin, N, minmax_blocks(), part, part, st, mn, mx))) return rc;
   }
   int64_t ncell = 1;
   for (int d = 0; d < D; ++d) {
@@ -497,15 +490,18 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
   g.D = D;
   g.ncell = ncell;
   g.dist2 = dist * dist;
-  // What the point count and the grid size is cut from one allocation: a
-  // cudaMalloc takes 11 to 35 us, and these were two thirds of what the
-  // construction of a small list took
+  // What the point count and the grid size is cut from one allocation.  A
+  // cudaMalloc that opens another 2 MB of the device takes about 50 us, one
+  // within them 3: a list of 6,000 points in 2-D took 427 us to construct from
+  // some thirty allocations, 512 from three, and 354 from one.
   int64_t sc = scan_scratch_elems((ncell > N ? ncell : N) + 1);
   const bool radix = N > RADIX_MIN_N, small = N + 1 <= SCAN_FOLD_MAX;
   const int64_t ntiles = (N + RADIX_TILE - 1) / RADIX_TILE;
   if (radix && scan_scratch_elems(256 * ntiles + 1) > sc) return fail(GCSPH_EINVAL, "radix scan scratch");
-  size_t upf_b, uptot_b, upbase_b, upstat_b, uprec_b;
-  upper_sizes(&upf_b, &uptot_b, &upbase_b, &upstat_b, &uprec_b);
+  size_t upf_b, uptot_b, upbase_b, upstat_b, upkept_b;
+  upper_sizes(&upf_b, &uptot_b, &upbase_b, &upstat_b, &upkept_b);
+  // (where that is much, it can grow and be freed by itself)
+  if (upkept_b > KEPT_IN_ARENA) upkept_b = 0;
   const size_t n4 = sizeof(int32_t) * (size_t)N, n8 = sizeof(int64_t) * (size_t)(N + 1);
   const struct Cut {
     DevBuf* b;
@@ -545,7 +541,10 @@ int CellCore::init(int D_, int64_t N_, const double* cellsize, double dist_, con
       {&uptot, uptot_b},
       {&upbase, upbase_b},
       {&upstat, upstat_b},
-      {&uprec, uprec_b},
+      {&upkept, upkept_b},
+      {&pos[0], sizeof(double) * (size_t)N},
+      {&pos[1], sizeof(double) * (size_t)N},
+      {&pos[D - 1], D == 3 ? sizeof(double) * (size_t)N : 0},
   };
   size_t total = 0, zero = 0;
   for (const Cut& c : cuts) {
@@ -573,7 +572,7 @@ void CellCore::release() {
   DevBuf* all[] = {&count, &cellstart, &key, &slot, &tmp, &tord, &perm, &skey, &orig, &cnt_full, &cnt_up, &rs_full,
                    &rs_up, &nbr, &scratch, &pf[0], &pf[1], &pf[2], &pfmax, &pfthr, &pfcnt, &orig_b, &stage,
                    &foldcnt, &foldsum, &rkey[0], &rkey[1], &rval[0], &rval[1], &rhist, &rhoff, &popmax,
-                   &upf, &upkept, &uptot, &upbase, &upstat, &uprec, &arena, &arena_x};
+                   &upf, &upkept, &uptot, &upbase, &upstat, &arena};
   for (DevBuf* b : all) b->release();
   if (ev_pop) cudaEventDestroy(ev_pop);
   ev_pop = nullptr;

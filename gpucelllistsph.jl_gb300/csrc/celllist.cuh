@@ -185,6 +185,8 @@ constexpr int RADIX_MIN_POP = 128;
 // search and its fill together with lanes and with a thread: 3-D 26k points 107
 // and 125 us, 46k 160 and 146, 390k 1277 and 764; 2-D 40k 61 and 49)
 constexpr int64_t ROWS_THREAD_MIN_N = 32768;
+// up to this many bytes of what a search keeps are cut from the cell list's allocation
+constexpr size_t KEPT_IN_ARENA = 8u << 20;
 // blocks of the count pass whose row-start scan it folds (rows_fold)
 constexpr int ROWS_FOLD_MAX_BLOCKS = 2048;
 
@@ -215,9 +217,9 @@ struct CellCore {
   bool up_scanned = false;  // rs_up holds the last build's offsets (nup may still be unread)
   bool rows_upper = false;  // the last build is the list's own (pairs k < m alone, as masks or rows)
   // their search: FP32 vectors, what each point keeps, block totals and starts, statistics
-  DevBuf upf, upkept, uptot, upbase, upstat, uprec;
+  DevBuf upf, upkept, uptot, upbase, upstat;
   // the buffers whose size the point count and the grid fix, and the cell list's positions (init)
-  DevBuf arena, arena_x;
+  DevBuf arena;
   double* up_xs[3] = {nullptr, nullptr, nullptr};  // the positions it was made on
   int up_w = 0;          // entries kept per point
   bool up_rows = false;  // neighbours rather than words
@@ -231,7 +233,9 @@ struct CellCore {
   // neighbour count, else from the grid-wide mean per cell
   double candidates_per_point() const;
 
-  void upper_sizes(size_t* upf_b, size_t* uptot_b, size_t* upbase_b, size_t* upstat_b, size_t* uprec_b) const;
+  void upper_sizes(size_t* upf_b, size_t* uptot_b, size_t* upbase_b, size_t* upstat_b, size_t* upkept_b);
+  // what the next search may keep, and before that the points' records of its binning
+  size_t kept_bytes() const;
   int init(int D_, int64_t N_, const double* cellsize, double dist_, const double* MIN, const double* MAX,
            const double* const* xin, DevBuf* pos, cudaStream_t s);
   void release();

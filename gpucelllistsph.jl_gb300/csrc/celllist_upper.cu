@@ -545,16 +545,40 @@ static Pos3 pos3(const double* const* in, double* const* out) {
   return P;
 }
 
+// A width: three times the mean, and in dense sets 256 past it, so that what is
+// kept takes no more memory than the neighbours of all points in one array
+// and a staged row of 256 each.
+static double kept_room(double mean) { return std::min(3.0 * mean + 16.0, mean + 256.0); }
+static int whole4(double w) { return ((int)w + 3) / 4 * 4; }
+
+// The first search's form and width, from the grid-wide density: rows where a
+// point has more than UP_FEW words of candidates (half a word of each point's
+// is padding), as wide as kept_room allows for the pairs that the density gives
+// a dist-ball.  A point at its cell's near edge has up to 2.7 times the mean of
+// a uniform set, and a guess that one point outgrows costs a second search and
+// another allocation (130 us of a small list's construction).
+static void first_width(CellCore& C) {
+  const double cand = 0.5 * C.candidates_per_point();
+  C.up_rows = cand + 16.0 > 32.0 * UP_FEW;
+  double pairs = cand * (C.D == 2 ? GCSPH_PI64 / 9.0 : 4.0 * GCSPH_PI64 / 81.0);
+  for (int d = 0; d < C.D; ++d) pairs *= C.dist / C.cs[d];
+  C.up_w = whole4(std::min(C.up_rows ? kept_room(pairs) : cand / 16.0 + 8.0, 4096.0));
+}
+
+size_t CellCore::kept_bytes() const {
+  return (size_t)N * std::max(sizeof(unsigned) * (size_t)up_w, sizeof(PointRec));
+}
+
 // bytes of the search's buffers (cut from the cell list's allocation)
-void CellCore::upper_sizes(size_t* upf_b, size_t* uptot_b, size_t* upbase_b, size_t* upstat_b,
-                           size_t* uprec_b) const {
+void CellCore::upper_sizes(size_t* upf_b, size_t* uptot_b, size_t* upbase_b, size_t* upstat_b, size_t* upkept_b) {
   const size_t nb = (size_t)nblocks(N, UTPB), n = (size_t)N;
   // (a group of padding, which a walk may read and cut off)
   *upf_b = D == 2 ? sizeof(PfVec<2>::T) * (n + UP_GROUP<2>) : sizeof(PfVec<3>::T) * (n + UP_GROUP<3>);
   *uptot_b = sizeof(int32_t) * (nb + 4);
   *upbase_b = sizeof(int64_t) * (nb + 1);
   *upstat_b = sizeof(UpStat);
-  *uprec_b = sizeof(PointRec) * n;
+  first_width(*this);
+  *upkept_b = kept_bytes();
 }
 
 template <int D>
@@ -571,13 +595,20 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
   float2* thr = C.pfthr.as<float2>();
   unsigned* cnt = C.pfcnt.as<unsigned>();
   bool deferred = false;
+  if (C.up_w == 0) first_width(C);
+  if ((rc = C.upkept.ensure(C.kept_bytes(), st))) {
+    C.up_w = 0;  // the next build guesses anew
+    return rc;
+  }
+  // the records of the binning's arrival lists lie where the search that
+  // follows keeps its words or rows
   if (rebin) {
-    if ((rc = C.sort(xin, nullptr, true, &deferred, false, C.uprec.as<PointRec>()))) return rc;
+    if ((rc = C.sort(xin, nullptr, true, &deferred, false, C.upkept.as<PointRec>()))) return rc;
   }
   if (!C.sorted && !deferred) return fail(GCSPH_ESTATE, "pair build before binning");
   timer_begin(T_SORT, st);
   if (deferred) {
-    k_rank_place<D><<<nb, UTPB, 0, st>>>(C.uprec.as<PointRec>(), C.cellstart.as<int32_t>(), N, C.g,
+    k_rank_place<D><<<nb, UTPB, 0, st>>>(C.upkept.as<PointRec>(), C.cellstart.as<int32_t>(), N, C.g,
                                          C.perm.as<int32_t>(), C.skey.as<int32_t>(), C.orig_b.as<int32_t>(), P, pf,
                                          bm, thr, cnt);
     GC_LAUNCHED();
@@ -590,26 +621,12 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
   timer_end(T_SORT, st);
   timer_begin(T_PAIRS, st);
   // What a point keeps: as much as the last search's fullest point needed and
-  // a quarter more, up to three times the mean, and in dense sets up to 256 past
-  // it, so that what is kept takes no more memory than the neighbours of all
-  // points in one array and a staged row of 256 each (a crowded cell's points
-  // are searched again in the emit).  A search that finds its points in need
-  // of more, or of the other form, is run again; the width stays while the form
-  // does.  The first search guesses from the grid-wide density: twice the
-  // pairs that it gives a dist-ball (a little more in 3-D).
-  auto room = [](double mean) { return std::min(3.0 * mean + 16.0, mean + 256.0); };
-  auto whole4 = [](double w) { return ((int)w + 3) / 4 * 4; };
+  // a quarter more, up to kept_room (a crowded cell's points are searched again
+  // in the emit).  A search that finds its points in need of more, or of the
+  // other form, is run again; the width stays while the form does.
   const bool fold = nb <= SCAN_FOLD_MAX;
-  if (C.up_w == 0) {
-    const double cand = 0.5 * C.candidates_per_point();
-    C.up_rows = cand > 32.0 * UP_FEW;
-    double pairs = cand * (D == 2 ? GCSPH_PI64 / 9.0 : 4.0 * GCSPH_PI64 / 81.0);
-    for (int d = 0; d < D; ++d) pairs *= C.dist / C.cs[d];
-    const double need = C.up_rows ? std::min((D == 2 ? 2.0 : 2.25) * pairs, room(pairs)) : cand / 16.0;
-    C.up_w = whole4(std::min(need, 4096.0) + 8.0);
-  }
   for (;;) {
-    if ((rc = C.upkept.ensure(sizeof(unsigned) * (size_t)N * (size_t)C.up_w, st))) {
+    if ((rc = C.upkept.ensure(C.kept_bytes(), st))) {
       C.up_w = 0;  // the next build guesses anew
       return rc;
     }
@@ -637,10 +654,10 @@ static int build_upper_impl(CellCore& C, const double* const* xin, double* const
       C.up_rows = !C.up_rows;
       // the other form's need: at a first guess its mean
       const double other = C.up_rows ? (double)C.pin[0] / (double)N : words;
-      C.up_w = whole4(std::min(1.5 * other + 8.0, room(other)));
+      C.up_w = whole4(std::min(1.5 * other + 8.0, kept_room(other)));
       continue;
     }
-    const double bound = room(mean), most = std::min((double)s.most, bound);
+    const double bound = kept_room(mean), most = std::min((double)s.most, bound);
     if (whole4(most) <= C.up_w) break;
     C.up_w = whole4(std::min(1.25 * most, bound));
   }

@@ -42,3 +42,18 @@ def test_cells_wider_than_the_reach(gpu_pkg):
     assert 0 < c.pairsn < N
     # next to the positions and indices that any list of N points holds
     assert _used() - before <= 4 * (c.pairsn + 256 * N) + SLACK
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("N", [6000, 60000])
+def test_a_uniform_set_is_searched_once(gpu_pkg, D, N):
+    """The first search's guess of what a point keeps holds: the construction
+    launches what an update! does, and no second search (20 pairs a point)."""
+    x = np.random.default_rng(N + D).random((D, N))
+    ball = np.pi if D == 2 else 4.0 * np.pi / 3.0
+    dist = (40.0 / (N * ball)) ** (1.0 / D)
+    n0 = gpu_pkg.launch_count()
+    c = gpu_pkg.GPUCellList(tuple(x), (dist,) * D, dist, MIN=(0.0,) * D, MAX=(1.0,) * D, mpairs=22 * N)
+    n1 = gpu_pkg.launch_count()
+    c.update()
+    assert n1 - n0 == gpu_pkg.launch_count() - n1
