@@ -653,6 +653,10 @@ __global__ void __launch_bounds__(STPB) k_dpc_rows(StepConst c, const Scal* __re
   }
 }
 
+// w / s of the corrections' sums: a density of 0 or infinity (rcp_nr gives NaN
+// for both) is divided by
+__device__ __forceinline__ double quot(double w, double s) { return mid_range(s) ? w * rcp_nr(s) : w / s; }
+
 // xsphcorr! + update_xsphcorr!  (:1757-1779, :1827-1838), stage-1 W
 template <int D, int L>
 __global__ void __launch_bounds__(STPB) k_xsph_rows(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S) {
@@ -689,7 +693,7 @@ __global__ void __launch_bounds__(STPB) k_xsph_rows(StepConst c, const Scal* __r
 #pragma unroll
       for (int j = 0; j < GATHER_U; ++j) {
         if (!(pt[j] > 1) || m[j] == k) continue;
-        const double xs = w[j] * rcp_nr(rk + rm[j]);
+        const double xs = quot(w[j], rk + rm[j]);
 #pragma unroll
         for (int d = 0; d < D; ++d) sum[d] += (vm[j][d] - vk[d]) * xs;
       }
@@ -737,7 +741,7 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
       for (int j = 0; j < GATHER_U; ++j) {
         if (!(pt[j] > 0) || m[j] == k) continue;
         s[0] += w[j];
-        s[1] += w[j] * rcp_nr(rm[j]);
+        s[1] += quot(w[j], rm[j]);
       }
     }
     lanes_sum4<L>(s, lane, group_mask<L>());

@@ -68,12 +68,6 @@ __device__ inline double dotf(const double* a, const double* b) {
   return s;
 }
 
-// whether x's exponent lies in a range where the corrected approximations
-// hold (2^-900 .. 2^900); zeros, denormals, infinities and NaN take the IEEE
-// operations
-__device__ inline bool mid_range(double x) {
-  return ((unsigned)(dbits(x) >> 32) & 0x7fffffffu) - 0x07b00000u < 0x70800000u;
-}
 __device__ inline double rcp_pair(double x) { return mid_range(x) ? rcp_nr(x) : 1.0 / x; }
 __device__ inline double sqrt_pair(double x) { return mid_range(x) ? sqrt_nr(x) : sqrt(x); }
 

@@ -339,6 +339,13 @@ __device__ inline double sqrt_nr(double x) {
   return fma(s, e * fma(0.375, e, 0.5), s);
 }
 
+// whether x's exponent lies in a range where the corrected approximations
+// hold (2^-900 .. 2^900); zeros, denormals, infinities and NaN take the IEEE
+// operations
+__device__ inline bool mid_range(double x) {
+  return ((unsigned)(dbits(x) >> 32) & 0x7fffffffu) - 0x07b00000u < 0x70800000u;
+}
+
 // sqrt(x) as above by two Newton steps on the reciprocal root, y <- y + y (1/2 -
 // (x/2) y^2), then x y.  fbmolforce! takes it: lattice walls hold pairs at
 // exactly r₀, where the last bit of r decides whether the pair has a force.
