@@ -765,6 +765,9 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
 // entries, each pair twice: 3-D full physics, 23.5M pairs, a call 23.96 ms
 // against 23.46; 3-D plain, 5.5M pairs, 7242 us against 7098; 2-D, 102k pairs,
 // a call of one step 224 against 213).
+// A pair at an infinite separation adds Δx 0 and one at a NaN NaN to ∑∇W (a
+// particle that diverged within the step): the factor of its Δx.
+__device__ __forceinline__ double no_pair(double r2) { return r2 == r2 ? 0.0 : NAN; }
 constexpr int PS_TPB = 256;
 template <int D>
 __global__ void __launch_bounds__(PS_TPB) k_pair_sums(StepConst c, SArr<D> S, PairBuf B) {
@@ -787,6 +790,9 @@ __global__ void __launch_bounds__(PS_TPB) k_pair_sums(StepConst c, SArr<D> S, Pa
         const double t3 = r2pos ? t2 * t : NAN;  // the reference's d𝒲(0)/0
 #pragma unroll
         for (int d = 0; d < D; ++d) g[d] = dx[d] * t3;
+      } else if (!(r2 < INFINITY)) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) g[d] = dx[d] * no_pair(r2);
       }
     }
     put_slot(B.ce + q.z, w, g[0], g[1], g[2]);
@@ -856,7 +862,13 @@ __global__ void __launch_bounds__(STPB) k_sums_rows(StepConst c, int64_t N, cons
         const double r2 = dotD<D>(dx, dx);
         const bool r2pos = dbits(r2) != 0;
         const double u = r2pos ? sqrt_nr(r2) * c.Hinv : 0.0;
-        if (!(dbits(u) < ONE_BITS)) continue;
+        if (!(u < 1.0)) {
+          if (!(r2 < INFINITY)) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) s[1 + d] += dx[d] * no_pair(r2);
+          }
+          continue;
+        }
         const double t = 1.0 - u, t2 = t * t;
         s[0] += fma(4.0, u, 1.0) * (t2 * t2);
         const double t3 = r2pos ? t2 * t : NAN;  // the reference's d𝒲(0)/0

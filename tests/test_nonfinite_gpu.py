@@ -74,3 +74,32 @@ def test_an_infinite_density_in_cspmcorr(gpu_pkg, D):
     assert near.sum() > 4 and np.isfinite(np.delete(want["rho"], i)).all()
     for lanes in (2, 4, 32):
         _same(_run(gpu_pkg, c, lanes, cspmn=1), want, ("rho", "P"))
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("val", [np.nan, np.inf])
+def test_sums_over_a_diverged_particle(gpu_pkg, D, val):
+    """A wall particle's velocity moves it out of the world within the step; the
+    closing sums still go over the pairs that it had.  Then a call of no steps
+    over the caller's points, one of them moved away by hand."""
+    c = _case(gpu_pkg, D)
+    i = _behind_the_walls(c)
+    c.v[0, i] = val
+    want = _run(gpu_pkg, c, 1)
+    bad = ~np.isfinite(want["sumgW"])
+    assert bad.any() and np.isfinite(want["sumW"]).all()
+    c2 = _case(gpu_pkg, D)
+    sums = {}
+    for lanes in (1, 2, 4, 32):
+        if lanes > 1:
+            _same(_run(gpu_pkg, c, lanes), want, ("sumW", "sumgW"))
+        system = gpu_pkg.GPUCellList(tuple(c2.x), c2.cellsize, c2.dist)
+        prob = gpu_pkg.SPHProblem(system, c2.dx, c2.h, c2.H, gpu_pkg.WendlandC2(dim=D), c2.rho, c2.ptype, c2.rho0,
+                                  c2.m0, c2.dt, c2.alpha, c2.c0, c2.gamma, c2.delta, c2.CFL)
+        prob.set_lanes(lanes)
+        system.points[1][i] = val
+        prob.stepsolve(0)
+        sums[lanes] = {"sumW": prob.field("sumW").cpu().numpy(),
+                       "sumgW": torch.stack(prob.field("sumgW")).cpu().numpy()}
+        assert not np.isfinite(sums[1]["sumgW"]).all()
+        _same(sums[lanes], sums[1], ("sumW", "sumgW"))
