@@ -653,10 +653,6 @@ __global__ void __launch_bounds__(STPB) k_dpc_rows(StepConst c, const Scal* __re
   }
 }
 
-// w / s of the corrections' sums: a density of 0 or infinity (rcp_nr gives NaN
-// for both) is divided by
-__device__ __forceinline__ double quot(double w, double s) { return mid_range(s) ? w * rcp_nr(s) : w / s; }
-
 // xsphcorr! + update_xsphcorr!  (:1757-1779, :1827-1838), stage-1 W
 template <int D, int L>
 __global__ void __launch_bounds__(STPB) k_xsph_rows(StepConst c, const Scal* __restrict__ sc, int64_t N, SArr<D> S) {
@@ -693,9 +689,27 @@ __global__ void __launch_bounds__(STPB) k_xsph_rows(StepConst c, const Scal* __r
 #pragma unroll
       for (int j = 0; j < GATHER_U; ++j) {
         if (!(pt[j] > 1) || m[j] == k) continue;
-        const double xs = quot(w[j], rk + rm[j]);
+        const double xs = w[j] * rcp_nr(rk + rm[j]);
 #pragma unroll
         for (int d = 0; d < D; ++d) sum[d] += (vm[j][d] - vk[d]) * xs;
+      }
+    }
+    // a sum of densities of 0 or infinity, where rcp_nr is NaN: again with the
+    // division (rcp_any for every entry cost 0.6% of a call with surface
+    // tension, 65k particles in 2-D)
+    unsigned top = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) top = max(top, exponent(sum[d]));
+    if (top == HI_INF) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) sum[d] = 0.0;
+#pragma unroll 1
+      for (int64_t e = S.rs[k] + lane; e < e1; e += L) {
+        const int32_t i = S.nbr[e];
+        if (!(S.pt[i] > 1)) continue;
+        const double xs = S.We[e] / (rk + S.rho[i]);
+#pragma unroll
+        for (int d = 0; d < D; ++d) sum[d] += (S.v[d][i] - vk[d]) * xs;
       }
     }
     lanes_sum4<L>(sum, lane, group_mask<L>());
@@ -741,7 +755,7 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
       for (int j = 0; j < GATHER_U; ++j) {
         if (!(pt[j] > 0) || m[j] == k) continue;
         s[0] += w[j];
-        s[1] += quot(w[j], rm[j]);
+        s[1] += w[j] * rcp_any(rm[j]);
       }
     }
     lanes_sum4<L>(s, lane, group_mask<L>());
@@ -790,7 +804,7 @@ __global__ void __launch_bounds__(PS_TPB) k_pair_sums(StepConst c, SArr<D> S, Pa
         const double t3 = r2pos ? t2 * t : NAN;  // the reference's d𝒲(0)/0
 #pragma unroll
         for (int d = 0; d < D; ++d) g[d] = dx[d] * t3;
-      } else if (!(r2 < INFINITY)) {
+      } else if (exponent(r2) == HI_INF) {
 #pragma unroll
         for (int d = 0; d < D; ++d) g[d] = dx[d] * no_pair(r2);
       }

@@ -129,6 +129,11 @@ __device__ inline void step_end_body(const StepConst& c, Scal* sc) {
   }
 }
 
+// the exponent of x in its high word's place; HI_INF for infinities and NaN
+__device__ __forceinline__ unsigned exponent(double x) {
+  return (unsigned)((unsigned long long)__double_as_longlong(x) >> 32) & HI_INF;
+}
+
 // ∂ρ∂tDDT! pair value seen from particle k (src/gpukernels_sph.jl:579-625)
 template <int D>
 __device__ inline double ddt_term(const StepConst& c, int ptk, int ptm, const double* dx, double r2, const double* gw,
@@ -325,6 +330,15 @@ __device__ inline double rcp_nr(double x) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x, y, 1.0);
   return fma(y, fma(e, e, e), y);
+}
+
+// the same where x may be 0 (or a denormal), infinite or NaN: there the
+// approximation is the answer and the correction is NaN
+__device__ inline double rcp_any(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0), r = fma(y, fma(e, e, e), y);
+  return exponent(e) == HI_INF ? y : r;
 }
 
 // sqrt(x), x normal and positive: s = x y from the approximate reciprocal
