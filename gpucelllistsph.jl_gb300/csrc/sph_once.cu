@@ -75,8 +75,17 @@ __device__ __forceinline__ double flip(double x) { return __longlong_as_double(d
 // a skin holds them: its slots, W and ∇W are zero.  Stage 2 takes stage 1's ∇W
 // and ∂v∂tpF! at xΔt½.  Such a pair then costs 2 D + 2 FP64 instructions instead
 // of 70 to 90, which every pair pays, so make_const sets far_r2 only for lists
-// that reach 3% past (break-even: 5% of the pairs).  No far pair is NaN or
-// infinite: those run through the terms.
+// that reach 3% past (break-even: 5% of the pairs).  At a NaN or an infinity in
+// what the terms read they are NaN at any distance: a pair at such a separation
+// is not far, and once a particle's other values are such (Scal::wild, kept by
+// the passes that write them) no pair is.  (Read pair by pair, those values
+// cost 1.6% of a call with surface tension, 65k particles in 2-D.)
+// (read where it is asked for: held over the loop it took a register more)
+__device__ __forceinline__ bool tame(const int* wild) {
+  int w;
+  asm volatile("ld.global.ca.b32 %0, [%1];" : "=r"(w) : "l"(wild));
+  return w == 0;
+}
 template <int D, int STAGE>
 __device__ __forceinline__ bool pair_far(const StepConst& c, const SArr<D>& S, int u, const int4 q) {
   if (STAGE == 2) {
@@ -84,14 +93,14 @@ __device__ __forceinline__ bool pair_far(const StepConst& c, const SArr<D>& S, i
 #pragma unroll
     for (int d = 0; d < D; ++d) any |= dbits(S.gWe[d][u]);
     if ((any << 1) != 0) return false;
-    if (!c.use_pF) return true;
+    if (!c.use_pF) return tame(S.wild);
   }
   const double* const* XP = STAGE == 1 ? S.x : S.xh;
   double dx[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) dx[d] = XP[d][q.x] - XP[d][q.y];
   const double r2 = dotD<D>(dx, dx);
-  return dbits(r2) > dbits(c.far_r2) && dbits(r2) < dbits((double)INFINITY);
+  return dbits(r2) > dbits(c.far_r2) && dbits(r2) < dbits((double)INFINITY) && tame(S.wild);
 }
 
 template <int D, int STAGE>
@@ -404,15 +413,19 @@ __global__ void __launch_bounds__(32 * L) k_pairB1(StepConst c, const Scal* __re
   double rv = rh0 + drho * hdt;
   if (rv < c.rho0 && ptk < 0) rv = c.rho0;
   S.rhoh[k] = rv;
+  unsigned top = 0;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     double vh = vh0[d];
     if (ptk > 1) vh = vh + a[d] * hdt;
     S.vh[d][k] = vh;
     S.xh[d][k] = xh0[d] + vh * hdt;
+    top = max(top, exponent(vh));
   }
-  S.P2[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
-  S.irh[k] = 1.0 / rv;
+  const double Pk = eos(rv, c.gamma, c.rho0, c.P0, ptk), irk = 1.0 / rv;
+  S.P2[k] = Pk;
+  S.irh[k] = irk;
+  note_wild(S.wild, max(max(top, exponent(rv)), max(exponent(Pk), exponent(irk))));
 }
 
 // pass B, stage 2: row sums + symplectic_update! + max |cΔx|; with nb.key
@@ -458,8 +471,10 @@ __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict
     if (rv < c.rho0 && ptk <= 1) rv = c.rho0;
     S.rho[k] = rv;
     S.rhoho[k] = rv;
-    S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
-    S.ir[k] = 1.0 / rv;
+    const double Pk = eos(rv, c.gamma, c.rho0, c.P0, ptk), irk = 1.0 / rv;
+    S.P1[k] = Pk;
+    S.ir[k] = irk;
+    unsigned top = max(exponent(rv), max(exponent(Pk), exponent(irk)));
     const double ml = ptk > 1 ? 1.0 : 0.0;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -468,6 +483,7 @@ __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict
       const double nv = vv + a[d] * dt * ml;
       S.vho[d][k] = nv;
       S.v[d][k] = nv;
+      top = max(top, exponent(nv));
       const double ddx = (vv + nv) * 0.5 * dt;
       const double cd = cd0[d] + ddx;
       S.cdx[d][k] = cd;
@@ -478,6 +494,7 @@ __global__ void __launch_bounds__(32 * L) k_pairB2(StepConst c, Scal* __restrict
       xn[d] = xv;
       if (pc.f[0]) pc.f[d][k] = (float)(xv - pc.off[d]);
     }
+    note_wild(S.wild, top);
     if (nb.key) {
       const int32_t ck = cell_key_v<D>(xn, nb.g);
       nb.key[k] = ck;
@@ -650,6 +667,7 @@ __global__ void __launch_bounds__(STPB) k_dpc_rows(StepConst c, const Scal* __re
     }
     S.vo[d][k] = nv;
     S.xo[d][k] = nx;
+    note_wild(S.wild, exponent(nv));
   }
 }
 
@@ -765,8 +783,10 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
   const double nr = s[0] / s[1];
   const double rv = isnan(nr) ? rk : nr;
   S.rhoo[k] = rv;
-  S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
-  S.ir[k] = 1.0 / rv;
+  const double Pk = eos(rv, c.gamma, c.rho0, c.P0, ptk), irk = 1.0 / rv;
+  S.P1[k] = Pk;
+  S.ir[k] = irk;
+  note_wild(S.wild, max(exponent(rv), max(exponent(Pk), exponent(irk))));
   const double mw = c.m0 * c.nW;
   S.buf2[0][k] = s[0] * mw;
   S.buf2[1][k] = s[1] * mw;

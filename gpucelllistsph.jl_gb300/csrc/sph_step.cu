@@ -126,8 +126,10 @@ __global__ void __launch_bounds__(STPB) k_stage2(StepConst c, Scal* __restrict__
     if (rv < c.rho0 && ptk <= 1) rv = c.rho0;
     S.rho[k] = rv;
     S.rhoho[k] = rv;
-    S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
-    S.ir[k] = 1.0 / rv;
+    const double Pn = eos(rv, c.gamma, c.rho0, c.P0, ptk), irn = 1.0 / rv;
+    S.P1[k] = Pn;
+    S.ir[k] = irn;
+    unsigned top = max(exponent(rv), max(exponent(Pn), exponent(irn)));
     const double ml = ptk > 1 ? 1.0 : 0.0;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(STPB) k_stage2(StepConst c, Scal* __restrict__
       const double nv = vv + a[d] * dt * ml;
       S.vho[d][k] = nv;
       S.v[d][k] = nv;
+      top = max(top, exponent(nv));
       const double ddx = (vv + nv) * 0.5 * dt;
       const double cd = S.cdx[d][k] + ddx;
       S.cdx[d][k] = cd;
@@ -144,6 +147,7 @@ __global__ void __launch_bounds__(STPB) k_stage2(StepConst c, Scal* __restrict__
       S.xho[d][k] = xv;
       S.xo[d][k] = xv;
     }
+    note_wild(S.wild, top);
   }
   // maximum(maximum.(abs, cΔx)), src/sphproblem.jl:325
   mc = warp_max(mc);
@@ -250,6 +254,7 @@ __global__ void __launch_bounds__(STPB) k_dpc(StepConst c, const Scal* __restric
     }
     S.vo[d][k] = nv;
     S.xo[d][k] = nx;
+    note_wild(S.wild, exponent(nv));
   }
 }
 
@@ -308,8 +313,10 @@ __global__ void __launch_bounds__(STPB) k_cspm(StepConst c, int64_t N, SArr<D> S
   double nr = s1 / s2;
   double rv = isnan(nr) ? rk : nr;
   S.rhoo[k] = rv;
-  S.P1[k] = eos(rv, c.gamma, c.rho0, c.P0, ptk);
-  S.ir[k] = 1.0 / rv;
+  const double Pk = eos(rv, c.gamma, c.rho0, c.P0, ptk), irk = 1.0 / rv;
+  S.P1[k] = Pk;
+  S.ir[k] = irk;
+  note_wild(S.wild, max(exponent(rv), max(exponent(Pk), exponent(irk))));
   S.buf2[0][k] = s1;
   S.buf2[1][k] = s2;
   if (D == 3) S.buf2[2][k] = 0.0;
@@ -411,19 +418,24 @@ __global__ void k_gather_state(StepConst c, int64_t N, const int32_t* __restrict
   const int pt = O.pt[o];
   ((int32_t*)S.pt)[k] = pt;
   const double r = O.rho[o];
+  const double Pk = eos(r, c.gamma, c.rho0, c.P0, pt), irk = 1.0 / r;
   S.rho[k] = r;
-  S.P1[k] = eos(r, c.gamma, c.rho0, c.P0, pt);
-  S.ir[k] = 1.0 / r;
+  S.P1[k] = Pk;
+  S.ir[k] = irk;
   S.rhoh[k] = O.rhoh[o];
+  unsigned top = max(exponent(r), max(exponent(Pk), exponent(irk)));
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     S.x[d][k] = O.x[d][o];
-    S.v[d][k] = O.v[d][o];
+    const double vk = O.v[d][o];
+    S.v[d][k] = vk;
+    top = max(top, exponent(vk));
     S.vh[d][k] = O.vh[d][o];
     S.xh[d][k] = O.xh[d][o];
     S.buf2[d][k] = O.buf2[d][o];
     S.cdx[d][k] = 0.0;  // cΔx reset after update!, src/sphproblem.jl:229
   }
+  note_wild(S.wild, top);
 }
 
 // destination buffers of an in-loop re-sort
@@ -563,10 +575,12 @@ __global__ void k_rank_gather(StepConst c, int64_t N, const int32_t* __restrict_
     }
     const int64_t k = rank_in_cell(tmp, key, cellstart, nullptr, q, perm, skey, orig, nullptr, tord);
     ((int32_t*)S.pt)[k] = pt;
+    const double Pk = eos(r, c.gamma, c.rho0, c.P0, pt), irk = 1.0 / r;
     S.rho[k] = r;
-    S.P1[k] = eos(r, c.gamma, c.rho0, c.P0, pt);
-    S.ir[k] = 1.0 / r;
+    S.P1[k] = Pk;
+    S.ir[k] = irk;
     S.rhoh[k] = rh;
+    unsigned top = max(exponent(r), max(exponent(Pk), exponent(irk)));
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       S.x[d][k] = x[d];
@@ -574,11 +588,13 @@ __global__ void k_rank_gather(StepConst c, int64_t N, const int32_t* __restrict_
       F.pf[d][k] = (float)rel;
       b = max(b, abs_hi(rel));
       S.v[d][k] = v[d];
+      top = max(top, exponent(v[d]));
       S.vh[d][k] = vh[d];
       S.xh[d][k] = xh[d];
       S.buf2[d][k] = bu[d];
       S.cdx[d][k] = 0.0;  // cΔx reset after update!, src/sphproblem.jl:229
     }
+    note_wild(S.wild, top);
   }
   atomic_max_hi(F.pfmax, b);
   pf_thresholds_last_block<D>(F.pfmax, F.dist2, F.thr, F.cnt);
@@ -771,6 +787,7 @@ static SArr<D> make_arr(sph_handle* h) {
   S.drho = h->DRHO.as<double>();
   S.Plast = h->PLAST.as<double>();
   S.ovf = &h->scal.as<Scal>()->ovf;
+  S.wild = &h->scal.as<Scal>()->wild;
   return S;
 }
 
@@ -1185,6 +1202,7 @@ static void init_scal(sph_handle* h, int32_t n) {
   h->pin->bdone = 0;
   h->pin->maxout = 0;
   h->pin->nreb = n > 0 ? 1 : 0;  // the first step always runs update!
+  h->pin->wild = h->in_cell_order ? 1 : 0;  // (the gather of the caller's state looks at it)
 }
 
 // _stepsolve!, one host round trip per step: the host reads the step's

@@ -58,6 +58,7 @@ struct Scal {
   unsigned bdone;             // blocks of pass B2 done this step (k_step_end's work in its last block)
   unsigned long long maxout;  // bits of the largest max |cΔx| of the call (stepsolve!'s second result)
   long long nreb;             // update! calls of the call (stepsolve!'s first result)
+  int wild;                   // a velocity, density, 1/density or pressure was NaN or infinite in this call
 };
 
 template <int D>
@@ -67,6 +68,7 @@ struct SArr {
   const int32_t* pt;
   const int32_t* orig;
   const int* ovf;  // set: the step's kernels skip (buffers outgrown, see rebuild)
+  int* wild;       // Scal::wild
   double* x[3];
   double* v[3];
   double* rho;
@@ -132,6 +134,9 @@ __device__ inline void step_end_body(const StepConst& c, Scal* sc) {
 // the exponent of x in its high word's place; HI_INF for infinities and NaN
 __device__ __forceinline__ unsigned exponent(double x) {
   return (unsigned)((unsigned long long)__double_as_longlong(x) >> 32) & HI_INF;
+}
+__device__ __forceinline__ void note_wild(int* wild, unsigned top) {
+  if (top == HI_INF) *wild = 1;
 }
 
 // ∂ρ∂tDDT! pair value seen from particle k (src/gpukernels_sph.jl:579-625)

@@ -103,3 +103,23 @@ def test_sums_over_a_diverged_particle(gpu_pkg, D, val):
                        "sumgW": torch.stack(prob.field("sumgW")).cpu().numpy()}
         assert not np.isfinite(sums[1]["sumgW"]).all()
         _same(sums[lanes], sums[1], ("sumW", "sumgW"))
+
+
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("field", ["rho", "v"])
+@pytest.mark.parametrize("val", [np.nan, np.inf])
+def test_pairs_in_the_skin(gpu_pkg, D, field, val):
+    """Pairs past every term's reach add 0 at any finite state, and NaN with a
+    particle that is not: the list's length picks how they are told apart."""
+    c = _case(gpu_pkg, D, big=True, skin=1.2)
+    fl = np.flatnonzero(c.ptype > 1)
+    i = fl[len(fl) // 2]
+    if field == "rho":
+        c.rho[i] = val
+    else:
+        c.v[0, i] = val
+    want = _run(gpu_pkg, c, 1, cspmn=15, nui=0.0)
+    r = np.sqrt(((c.x - c.x[:, i:i + 1]) ** 2).sum(0))
+    skin = (r > 1.02 * c.H) & (r < c.dist) & (c.ptype > 0)
+    assert skin.sum() > 4 and not np.isfinite(want["a"][:, skin]).all(0).any()
+    _same(_run(gpu_pkg, c, 4, cspmn=15, nui=0.0), want)
