@@ -9,10 +9,16 @@
 namespace gcsph {
 
 // fbmolforce!, :1891-1901, for a pair with exactly one real side, at
-// separation dx (r2 = |dx|², r = |dx|): adds Δx Fc to f
+// separation dx: adds Δx Fc to f.  Lattice walls hold pairs at exactly r₀, where
+// the last bits of r² and of its root decide: the sum is the reference's (left to
+// right, no contraction), and r < r₀ is r² <= fb_r2max.
 template <int D>
-__device__ inline void fb_pair(const StepConst& c, const double* dx, double r2, double r, double* f) {
-  if (dbits(r) < dbits(c.fb_r0)) {
+__device__ inline void fb_pair(const StepConst& c, const double* dx, double* f) {
+  double r2 = __dmul_rn(dx[0], dx[0]);
+#pragma unroll
+  for (int d = 1; d < D; ++d) r2 = __dadd_rn(r2, __dmul_rn(dx[d], dx[d]));
+  if (dbits(r2) <= dbits(c.fb_r2max)) {
+    const double r = dbits(r2) != 0 ? sqrt_nr(r2) : 0.0;
     const double q = c.fb_r0 * rcp_nr(r + c.fb_eta2);
     const double q2 = q * q, q4 = q2 * q2, q8 = q4 * q4, q12 = q8 * q4;
     const double Fc = c.fb_d * (q12 - q4) * rcp_nr(r2 + c.fb_eta2);
@@ -114,8 +120,7 @@ __device__ __forceinline__ void pairA_one(const StepConst& c, const SArr<D>& S, 
     double dx[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) dx[d] = S.x[d][k] - S.x[d][m];
-    const double r2 = dotD<D>(dx, dx);
-    if (!(dbits(r2) > dbits(c.fb_r2cut))) fb_pair<D>(c, dx, r2, dbits(r2) != 0 ? sqrt_nr2(r2) : 0.0, f);
+    fb_pair<D>(c, dx, f);
   } else {
     const double* const* XP = STAGE == 1 ? S.x : S.xh;
     const double* const* VP = STAGE == 1 ? S.v : S.vh;

@@ -695,6 +695,16 @@ struct sph_handle {
   cudaStream_t cap_stream = nullptr;  // records captures only; replays run on the cell list's stream
 };
 
+// the largest x with sqrt(x) < r, the root correctly rounded (a step or two from
+// r²); -1 where r is not positive
+static double largest_square_below(double r) {
+  if (!(r > 0.0)) return -1.0;
+  double x = r * r;
+  while (std::sqrt(x) >= r) x = std::nextafter(x, 0.0);
+  for (double up; std::sqrt(up = std::nextafter(x, (double)INFINITY)) < r;) x = up;
+  return x;
+}
+
 static StepConst make_const(const sph_handle* h) {
   const gcsph_params& p = h->prm;
   StepConst c{};
@@ -1077,7 +1087,7 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
   c.fb_d = 0.4;
   c.fb_r0 = 2.0 * p.dx;
   c.fb_eta2 = 0.01 * (c.fb_r0 * c.fb_r0);
-  c.fb_r2cut = c.fb_r0 * c.fb_r0 * (1.0 + 1e-6);
+  c.fb_r2max = largest_square_below(c.fb_r0);
   const int L = choose_lanes(h);
   const bool once = L > 1;  // pair-once passes; L = 1 keeps the serial gather (bit-identical to the oracle)
   // W of the pairs is read by xsphcorr! and by a CSPM step's cspmcorr! only
@@ -1104,7 +1114,7 @@ static int enqueue_stages(sph_handle* h, StepConst& c, Scal* dsc, int32_t& cspmc
   c.fb_d = p.bound_D;
   c.fb_r0 = p.bound_l;
   c.fb_eta2 = 0.01 * (c.fb_r0 * c.fb_r0);
-  c.fb_r2cut = c.fb_r0 * c.fb_r0 * (1.0 + 1e-6);
+  c.fb_r2max = largest_square_below(c.fb_r0);
   if (once) {
     timer_begin(T_STAGE2, st);
     PAIRA_LAUNCH(2, c, make_arr<D>(h), make_pairbuf<D>(h), core.nfull_est / 2);

@@ -24,7 +24,7 @@ inline void pf_cos_coef(double f, double* C) {
 struct StepConst {
   double h, eta2, m0, rho0, ginv, DDTkh, DDTgz, P0, alpha, c0, nu, g, s, Hinv, nW, nDW;
   double fb_d, fb_r0, fb_eta2;  // fbmolforce constants of the stage being run
-  double fb_r2cut;              // r₀² (1 + 1e-6): past it √r² >= r₀ whatever the rounding
+  double fb_r2max;              // the largest r² whose (correctly rounded) root is below r₀; negative: none
   // pair-once products of the constants: m₀ d𝒲/r = dWr (1 - u)^3 (u / r = H⁻¹),
   // ∂v∂t_av!'s 2 α c₀ h and ∂v∂t_visc!'s 4 ν
   double dWr, avK, visc4;
@@ -363,20 +363,6 @@ __device__ inline double sqrt_nr(double x) {
 // operations
 __device__ inline bool mid_range(double x) {
   return ((unsigned)(dbits(x) >> 32) & 0x7fffffffu) - 0x07b00000u < 0x70800000u;
-}
-
-// sqrt(x) as above by two Newton steps on the reciprocal root, y <- y + y (1/2 -
-// (x/2) y^2), then x y.  fbmolforce! takes it: lattice walls hold pairs at
-// exactly r₀, where the last bit of r decides whether the pair has a force.
-__device__ inline double sqrt_nr2(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double hx = 0.5 * x;
-  double e = fma(-hx, y * y, 0.5);
-  y = fma(y, e, y);
-  e = fma(-hx, y * y, 0.5);
-  y = fma(y, e, y);
-  return x * y;
 }
 
 // cos(1.5π r/2h) of ∂v∂tpF! inside 2h, from r²: with s = 2 (r/2h)² - 1 it is
