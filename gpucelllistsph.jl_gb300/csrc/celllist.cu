@@ -301,15 +301,13 @@ __global__ void k_gather_pos(const int32_t* __restrict__ idx, int64_t N, const d
 // ---------------------------------------------------------------------------
 // pair search over the 3^D stencil, as 3^(D-1) contiguous x-rows
 // ---------------------------------------------------------------------------
-// MODE 0: count (full, up); MODE 1: fill nbr.  L lanes share one particle:
-// the candidates of each x-row are tested L at a time, and the fill keeps the
-// row ascending by compacting each round's hits with a sub-warp ballot.
-template <int D, int MODE, int L>
+// The counts (full, and of the larger indices) in FP64 alone.  L lanes share
+// one particle: the candidates of each x-row are tested L at a time.
+template <int D, int L>
 __global__ void __launch_bounds__(TPB) k_pairs(const double* __restrict__ x0, const double* __restrict__ x1,
                                                const double* __restrict__ x2, const int32_t* __restrict__ skey,
                                                const int32_t* __restrict__ cellstart, int64_t N, Grid g,
-                                               int32_t* __restrict__ cnt_full, int32_t* __restrict__ cnt_up,
-                                               const int64_t* __restrict__ rs_full, int32_t* __restrict__ nbr) {
+                                               int32_t* __restrict__ cnt_full, int32_t* __restrict__ cnt_up) {
   const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t k = gt / L;
   const int lane = (int)(gt % L);
@@ -325,7 +323,6 @@ __global__ void __launch_bounds__(TPB) k_pairs(const double* __restrict__ x0, co
   int cz = t / ny;
   double ax = x0[k], ay = x1[k], az = D == 3 ? x2[k] : 0.0;
   int32_t nf = 0, nu = 0;
-  int64_t wpos = MODE == 1 ? rs_full[k] : 0;
   const int xlo = cx > 0 ? cx - 1 : 0;
   const int xhi = cx < nx - 1 ? cx + 1 : nx - 1;
   for (int dz = (D == 3 ? -1 : 0); dz <= (D == 3 ? 1 : 0); ++dz) {
@@ -343,27 +340,19 @@ __global__ void __launch_bounds__(TPB) k_pairs(const double* __restrict__ x0, co
           double r2 = r2_ref<D>(ax, ay, az, x0[m], x1[m], D == 3 ? x2[m] : 0.0);
           hit = r2 < g.dist2;
         }
-        if (MODE == 0) {
-          nf += hit;
-          nu += hit && (m > k);
-        } else {
-          const unsigned bal = (__ballot_sync(gm, hit) >> gbase) & (L == 32 ? 0xffffffffu : ((1u << L) - 1u));
-          if (hit) nbr[wpos + __popc(bal & ((1u << lane) - 1u))] = m;
-          wpos += __popc(bal);
-        }
+        nf += hit;
+        nu += hit && (m > k);
       }
     }
   }
-  if (MODE == 0) {
 #pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) {
-      nf += __shfl_xor_sync(gm, nf, o);
-      nu += __shfl_xor_sync(gm, nu, o);
-    }
-    if (lane == 0) {
-      cnt_full[k] = nf;
-      cnt_up[k] = nu;
-    }
+  for (int o = L / 2; o > 0; o >>= 1) {
+    nf += __shfl_xor_sync(gm, nf, o);
+    nu += __shfl_xor_sync(gm, nu, o);
+  }
+  if (lane == 0) {
+    cnt_full[k] = nf;
+    cnt_up[k] = nu;
   }
 }
 
@@ -1614,9 +1603,9 @@ template <int D>
 static int preload_dim() {
   cudaFuncAttributes a;
   const void* fns[] = {(const void*)k_cellkey<D>,           (const void*)k_gather_pos<D>,
-                       (const void*)k_pairs<D, 0, 1>,       (const void*)k_pairs<D, 0, 2>,
-                       (const void*)k_pairs<D, 0, 4>,       (const void*)k_pairs<D, 0, 8>,
-                       (const void*)k_pairs<D, 0, 16>,      (const void*)k_pairs<D, 0, 32>,
+                       (const void*)k_pairs<D, 1>,       (const void*)k_pairs<D, 2>,
+                       (const void*)k_pairs<D, 4>,       (const void*)k_pairs<D, 8>,
+                       (const void*)k_pairs<D, 16>,      (const void*)k_pairs<D, 32>,
                        (const void*)k_pairs_direct<D, 1>,   (const void*)k_pairs_direct<D, 2>,
                        (const void*)k_pairs_direct<D, 4>,   (const void*)k_pairs_direct<D, 8>,
                        (const void*)k_pairs_direct<D, 16>,  (const void*)k_pairs_direct<D, 32>};
@@ -1735,12 +1724,12 @@ static int run(int64_t N, const double* const* x, const double* cellsize, double
     default: KER<D, 32><<<gb, TPB, 0, st>>>(__VA_ARGS__); break;        \
   }
   switch (L) {
-    case 1: k_pairs<D, 0, 1><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup, nullptr, nullptr); break;
-    case 2: k_pairs<D, 0, 2><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup, nullptr, nullptr); break;
-    case 4: k_pairs<D, 0, 4><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup, nullptr, nullptr); break;
-    case 8: k_pairs<D, 0, 8><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup, nullptr, nullptr); break;
-    case 16: k_pairs<D, 0, 16><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup, nullptr, nullptr); break;
-    default: k_pairs<D, 0, 32><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup, nullptr, nullptr); break;
+    case 1: k_pairs<D, 1><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup); break;
+    case 2: k_pairs<D, 2><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup); break;
+    case 4: k_pairs<D, 4><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup); break;
+    case 8: k_pairs<D, 8><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup); break;
+    case 16: k_pairs<D, 16><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup); break;
+    default: k_pairs<D, 32><<<gb, TPB, 0, st>>>(xs[0], xs[1], xc2, skey, cstart, N, g, cfull, cup); break;
   }
   GC_LAUNCHED();
   if ((rc = exclusive_scan_i32_to_i64(cup, rsup, N, scan, st))) return rc;

@@ -55,17 +55,12 @@ struct EnsInst {
   int nc[3];
   int key_off;
   int gamma;
-  int use_visc, use_pF;
   int cspmn;
   int use_dpc, use_xsph;
-  float csf, H2, h, Hinv, nW, nDW, m0, rho0, c0, P0, alpha, DDTkh, DDTgz, eta2, g, nu, s, twoh, pfc, hp1;
-  float fb_d[2], fb_r0[2], fb_eta2[2];  // fbmolforce constants of stage 1 and stage 2
+  float csf, H2, Hinv, nW, m0, rho0, P0, g;
   float dpc_l0inv, dpc_nW, dpc_whinv, dpc_kernlim, dpc_eta2, dpc_pmin, dpc_pmax, dpc_lambda;
   float xsph_c;                          // 2 m0 ε
-  float rho0inv, m0inv;                  // 1/ρ₀, 1/m₀
-  float pfcr;                            // 1.5π / 2h: the cosine's argument per unit r in ∂v∂tpF!
-  // products of the above that the stage passes use as one factor
-  float kpf;                             // s / m₀ (∂v∂tpF!)
+  float rho0inv;                         // 1/ρ₀
   int p_off;                             // first particle of the instance (list entries are instance-local)
   int reuse;                             // the list is kept while the particles stay within the skin
   float LR2;                             // list radius², (H (1 + skin))² = cell edge²
@@ -310,7 +305,7 @@ __device__ __forceinline__ void cell_of(int key, const EnsInst& I, int& c0, int&
 // the order stays as it is and the binning's passes return at once, on small
 // grids -- they took a tenth of a 2-D step (69 of 545 us at 743k particles).
 constexpr int BIN_TPB = 256;
-inline int bin_grid(int64_t n) { return (int)std::min<int64_t>(nblocks(n, BIN_TPB), 152 * 8); }
+inline int bin_grid(int64_t n, int sms) { return (int)std::min<int64_t>(nblocks(n, BIN_TPB), sms * 8); }
 
 template <int D>
 __global__ void k_ens_key(int64_t N, const int32_t* __restrict__ inst, const double* __restrict__ x0,
@@ -1136,7 +1131,8 @@ __global__ void k_ens_dpc_apply(EnsArr A, const EnsInst* __restrict__ T) {
 // records are loaded at a time (390k particles in 3-D: a step took 654 us with
 // two, 678 with one, 686 with four), each as one 32-byte access, at 56
 // registers, which leaves nine blocks of 128 an SM (a step 575 us; 59 registers
-// 610, 48 581, 40 620; two 16-byte accesses 587)
+// 610, 48 581, 40 620; two 16-byte accesses 587).  In 2-D a step takes 281 us with
+// two records and 293 with one (400k fluid particles), 20 instances 321 and 329.
 constexpr int XSPH_U = 2, XSPH_REGS = 56;
 template <int D>
 __global__ void __maxnreg__(XSPH_REGS) k_ens_xsph(EnsArr A, const EnsInst* __restrict__ T) {
@@ -1896,7 +1892,7 @@ int ens_enqueue_step(gcsph_ens* e, cudaStream_t st, int tpb) {
   const EnsInst* T = e->TAB.as<EnsInst>();
   const int* any = e->ANY.as<int>();
   const double* x2 = D == 3 ? e->X[e->cur][2].as<double>() : e->X[e->cur][0].as<double>();
-  const int bg = bin_grid(N);
+  const int bg = bin_grid(N, e->sms);
   k_ens_key<D><<<bg, BIN_TPB, 0, st>>>(N, e->INST.as<int32_t>(), e->X[e->cur][0].as<double>(),
                                        e->X[e->cur][1].as<double>(), x2, T, e->RB.as<int>(), e->SKEY.as<int32_t>(),
                                        e->KEY.as<int32_t>(), e->SLOT.as<int32_t>(), e->COUNT.as<int32_t>(), any);
@@ -2245,10 +2241,10 @@ void ens_destroy(gcsph_ens* e) {
 int ens_bytes_per_particle(int32_t D, int64_t* bytes) {
   if (!bytes || (D != 2 && D != 3)) return fail(GCSPH_EINVAL, "bad argument");
   // 2 x (x f64, v f32, x and v base differences f32) per dim + 2 x (δρ,
-  // δρ base, ptype, id) + inst, key, slot, tmp, skey and 4 spare + (off, offh, vh,
+  // δρ base, ptype, id) + inst, key, slot, tmp, skey + (off, offh, vh,
   // offn) per dim + δρ½, plus about one cell per particle
   // + the step's neighbour list (64 entries in 2-D, 256 in 3-D, 4 B each) and its length
-  *bytes = 2 * D * (8 + 4 + 8) + 2 * 16 + 6 * 4 + D * 16 + 4 + 8 + (D == 2 ? 64 : 256) * 4 + 4 +
+  *bytes = 2 * D * (8 + 4 + 8) + 2 * 16 + 5 * 4 + D * 16 + 4 + 8 + (D == 2 ? 64 : 256) * 4 + 4 +
            16 * (D == 2 ? 4 : 5) +  // packed records of the stages
            64 +                     // and of the correction passes
            D * 4 +                  // offsets at the last list build
@@ -2298,34 +2294,13 @@ int ens_add(gcsph_ens* e, int64_t n, const double* x, const double* v, const dou
   I.dt = p->dt;
   I.gamma = p->gamma;
   I.cspmn = p->cspmn > 0 ? p->cspmn : 0;
-  I.use_visc = p->nu > 0;
-  I.use_pF = p->s > 0;
   I.H2 = (float)(p->H * p->H);
-  I.h = (float)p->h;
   I.Hinv = (float)(1.0 / p->H);
   I.nW = (float)(D == 2 ? wc2_norm_w<2>(1.0 / p->H) : wc2_norm_w<3>(1.0 / p->H));
-  I.nDW = (float)(D == 2 ? wc2_norm_dw<2>(1.0 / p->H) : wc2_norm_dw<3>(1.0 / p->H));
   I.m0 = (float)p->m0;
   I.rho0 = (float)p->rho0;
-  I.c0 = (float)p->c0;
   I.P0 = (float)(p->c0 * p->c0 * p->rho0 / (double)p->gamma);
-  I.alpha = (float)p->alpha;
-  I.DDTkh = (float)(2.0 * p->h * p->delta * p->c0);
-  I.DDTgz = (float)(p->rho0 * p->g / ((p->c0 * p->c0 * p->rho0) / (double)p->gamma));
-  I.eta2 = (float)((0.1 * p->h) * (0.1 * p->h));
   I.g = (float)p->g;
-  I.nu = (float)p->nu;
-  I.s = (float)p->s;
-  I.twoh = (float)(2.0 * p->h);
-  I.pfc = (float)(1.5 * GCSPH_PI64);
-  I.hp1 = (float)(0.1 * p->h);
-  const double r01 = 2.0 * p->dx;
-  I.fb_d[0] = 0.4f;
-  I.fb_r0[0] = (float)r01;
-  I.fb_eta2[0] = (float)(0.01 * r01 * r01);
-  I.fb_d[1] = (float)p->bound_D;
-  I.fb_r0[1] = (float)p->bound_l;
-  I.fb_eta2[1] = (float)(0.01 * p->bound_l * p->bound_l);
   I.use_dpc = p->dpc_l0 > 0;
   if (I.use_dpc) {
     const double l0inv = 1.0 / p->dpc_l0;
@@ -2347,11 +2322,8 @@ int ens_add(gcsph_ens* e, int64_t n, const double* x, const double* v, const dou
   const double a = 1.0 / (double)p->gamma;
   const double c1 = a, c2 = c1 * (a - 1.0) / 2.0, c3 = c2 * (a - 2.0) / 3.0, c4 = c3 * (a - 3.0) / 4.0;
   I.rho0inv = (float)(1.0 / p->rho0);
-  I.m0inv = (float)(1.0 / p->m0);
   // W'(r)/r = dwc (1 - r/H)^3
   const double dwc = -20.0 * (D == 2 ? wc2_norm_dw<2>(1.0 / p->H) : wc2_norm_dw<3>(1.0 / p->H)) / p->H;
-  I.pfcr = (float)(1.5 * GCSPH_PI64 / (2.0 * p->h));
-  I.kpf = (float)(p->s / p->m0);
   auto as_float = [](int v) {
     float f;
     memcpy(&f, &v, sizeof(f));
@@ -2362,14 +2334,18 @@ int ens_add(gcsph_ens* e, int64_t n, const double* x, const double* v, const dou
     // m₀ goes into ∇W, ρ₀ and DDTgz into the series of ∂ρ∂tDDT!
     const double gz = p->rho0 * p->g / ((p->c0 * p->c0 * p->rho0) / (double)p->gamma);
     K.A = make_float4(I.H2, I.Hinv, (float)(dwc * p->m0), I.csf);
-    K.B = make_float4(I.rho0, I.eta2, 0.f, I.DDTgz);
+    K.B = make_float4(I.rho0, (float)((0.1 * p->h) * (0.1 * p->h)), 0.f, (float)gz);
     K.C = make_float4((float)(2.0 * p->h * p->delta * p->c0), (float)(2.0 * p->alpha * p->c0 * p->h),
                       (float)(4.0 * p->nu), gz != 0.0 ? (float)(0.01 / std::fabs(gz)) : INFINITY);
-    K.D = make_float4(I.pfcr, I.hp1, I.twoh, I.kpf);
+    // the cosine's argument per unit r, 0.1h, 2h and s/m₀ of ∂v∂tpF!
+    K.D = make_float4((float)(1.5 * GCSPH_PI64 / (2.0 * p->h)), (float)(0.1 * p->h), (float)(2.0 * p->h),
+                      (float)(p->s / p->m0));
     K.E = make_float4((float)(p->rho0 * c1 * gz), (float)(p->rho0 * c2 * gz * gz),
                       (float)(p->rho0 * c3 * gz * gz * gz), (float)(p->rho0 * c4 * gz * gz * gz * gz));
-    K.F = make_float4(I.fb_d[st], I.fb_r0[st], I.fb_eta2[st], 0.f);  // .w: ens_relayout
-    K.G = make_float4(I.rho0inv, I.P0, as_float(I.gamma), as_float((I.use_visc ? 1 : 0) | (I.use_pF ? 2 : 0)));
+    // fbmolforce!'s strength, r₀ and η²
+    const double r0 = st == 0 ? 2.0 * p->dx : p->bound_l;
+    K.F = make_float4(st == 0 ? 0.4f : (float)p->bound_D, (float)r0, (float)(0.01 * r0 * r0), 0.f);  // .w: ens_relayout
+    K.G = make_float4(I.rho0inv, I.P0, as_float(I.gamma), as_float((p->nu > 0 ? 1 : 0) | (p->s > 0 ? 2 : 0)));
   }
   // host staging in the engine's types
   std::vector<float> vf((size_t)D * n, 0.f), drf((size_t)n);

@@ -803,7 +803,7 @@ __global__ void __launch_bounds__(STPB) k_cspm_rows(StepConst c, int64_t N, SArr
 // so once a pair; the row sums then read slots (rows that evaluated their
 // entries, each pair twice: 3-D full physics, 23.5M pairs, a call 23.96 ms
 // against 23.46; 3-D plain, 5.5M pairs, 7242 us against 7098; 2-D, 102k pairs,
-// a call of one step 224 against 213).
+// a call of one step 211 against 205).
 // A pair at an infinite separation adds Δx 0 and one at a NaN NaN to ∑∇W (a
 // particle that diverged within the step): the factor of its Δx.
 __device__ __forceinline__ double no_pair(double r2) { return r2 == r2 ? 0.0 : NAN; }
@@ -813,8 +813,7 @@ __global__ void __launch_bounds__(PS_TPB) k_pair_sums(StepConst c, SArr<D> S, Pa
   if (*S.ovf) return;
   const int64_t np = *B.npair, stride = (int64_t)gridDim.x * PS_TPB;
   for (int64_t u = (int64_t)blockIdx.x * PS_TPB + threadIdx.x; u < np; u += stride) {
-    // (the mirrors of a list that an update! at the last step's end rebuilt are open)
-    const int4 q = pair_load<D, 1>(S, B, (int)u);
+    const int4 q = B.pq[u];  // (the last step's first stage has closed every mirror)
     double w = 0.0, g[3] = {0.0, 0.0, 0.0};
     if ((S.pt[q.x] > 0) == (S.pt[q.y] > 0)) {
       double dx[D];
@@ -1040,7 +1039,13 @@ int launch_sums_post(int L, int64_t N, cudaStream_t st, const StepConst& c, cons
                      const PairBuf& B, int64_t pairs_est) {
   const PairOut* ce = B.ce;
   if (scatter) {
-    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(nblocks(pairs_est, PS_TPB), 152 * 16));
+    static int sms = 0;
+    if (sms == 0) {
+      int dev = 0;
+      GC_CUDA(cudaGetDevice(&dev));
+      GC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(nblocks(pairs_est, PS_TPB), sms * 16));
     k_pair_sums<D><<<g, PS_TPB, 0, st>>>(c, S, B);
     GC_LAUNCHED();
   }

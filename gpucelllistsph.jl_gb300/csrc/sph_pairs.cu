@@ -68,6 +68,12 @@ __device__ inline double dotf(const double* a, const double* b) {
   return s;
 }
 
+// whether x's exponent lies in a range where the corrected approximations
+// hold (2^-900 .. 2^900); zeros, denormals, infinities and NaN take the IEEE
+// operations
+__device__ inline bool mid_range(double x) {
+  return ((unsigned)(dbits(x) >> 32) & 0x7fffffffu) - 0x07b00000u < 0x70800000u;
+}
 __device__ inline double rcp_pair(double x) { return mid_range(x) ? rcp_nr(x) : 1.0 / x; }
 __device__ inline double sqrt_pair(double x) { return mid_range(x) ? sqrt_nr(x) : sqrt(x); }
 
@@ -131,19 +137,23 @@ __global__ void __launch_bounds__(PTPB) k_pair_term(int64_t P, const int32_t* __
 
 template <class F>
 static int launch_pair_term(int64_t P, const int32_t* pairs, const F& f, cudaStream_t st) {
-  // the queue form's blocks stay resident: as many as fit
-  static int64_t grid = 0;
-  if (grid == 0) {
-    int dev = 0, sms = 0, per = 0;
-    GC_CUDA(cudaGetDevice(&dev));
-    GC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_term<F, true>, PTPB, 0));
-    grid = (int64_t)sms * (per > 0 ? per : 1);
+  if constexpr (F::QUEUE) {
+    // the queue form's blocks stay resident: as many as fit
+    static int64_t grid = 0;
+    if (grid == 0) {
+      int dev = 0, sms = 0, per = 0;
+      GC_CUDA(cudaGetDevice(&dev));
+      GC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pair_term<F, true>, PTPB, 0));
+      grid = (int64_t)sms * (per > 0 ? per : 1);
+    }
+    if (P > 2 * grid * PTPB) {
+      k_pair_term<F, true><<<(unsigned)grid, PTPB, 0, st>>>(P, pairs, f);
+      GC_LAUNCHED();
+      return GCSPH_OK;
+    }
   }
-  if (!F::QUEUE || P <= 2 * grid * PTPB)
-    k_pair_term<F, false><<<nblocks(P, PTPB), PTPB, 0, st>>>(P, pairs, f);
-  else
-    k_pair_term<F, true><<<(unsigned)grid, PTPB, 0, st>>>(P, pairs, f);
+  k_pair_term<F, false><<<nblocks(P, PTPB), PTPB, 0, st>>>(P, pairs, f);
   GC_LAUNCHED();
   return GCSPH_OK;
 }
