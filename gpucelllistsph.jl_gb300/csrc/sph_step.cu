@@ -1007,7 +1007,11 @@ static int rebuild(sph_handle* h, const StepConst& c, int* ovf_dev) {
 // fill the GPU once there are a few thousand particles (one GB300, a call at
 // 4 / 8 / 16 / 32 lanes: 390k particles in 3-D 26.8 / 27.2 / 28.2 / 31.5 ms,
 // 65k in 2-D 7.0 / 7.4 / 8.0 / 9.8 ms, 6.5k in 2-D 1.39 / 1.40 / 1.41 / 1.60 ms,
-// 1.7k in 2-D 0.87 / 0.81 / 0.81 / 0.86 ms).
+// 1.7k in 2-D 0.87 / 0.81 / 0.81 / 0.86 ms).  The line between four and eight is
+// 2-D's (ten steps of full physics at 4 / 8 / 16 lanes: 5.3k 958 / 937 / 985 us,
+// 6.5k 1048 / 1046 / 1096, 8.7k 1218 / 1252 / 1307); small 3-D sets, whose rows are
+// longer, would gain from more (2.2k 1431 / 1299 / 1183, 6.7k 2144 / 2125 / 1972,
+// 30k 6077 / 5953 / 5989).
 static int choose_lanes(const sph_handle* h) {
   if (h->lanes > 0) return h->lanes;
   const CellCore& core = h->cl->core;
