@@ -10,9 +10,18 @@ arithmetic, reproduces that rational function -- including the iteration's own
 small bias against the true 7th root -- to far below one ulp for |eps| <=
 EPS_MAX, at the cost of one polynomial instead of two divisions per call.
 
+The root itself, t = 1 + series(eps), is to come out rounded once.  In the
+series about eps = 0 that takes an addition after the polynomial: with the 1 in
+its constant term, the constant is a double only to 8e-18, a fourteenth of t's
+last bit.  So t has a series of its own, about the double 1 + PF7_ROOT_E at which
+the iteration's real value is a double, PF7_ROOT_T, to a 500th of that bit
+on both sides of 1: the polynomial's last step, PF7_ROOT_T + r (x - (1 + E)),
+is the one rounding.
+
 Run:  python gen_pf7_series.py   (writes pf7_series.cuh beside this file)
 """
 from fractions import Fraction as F
+from math import comb
 import os
 import struct
 
@@ -75,13 +84,18 @@ def first_guess(upper):
     return [a, b] + [F(0)] * (K - 1)
 
 
-def series(upper):
+def exact_series(upper):
     x = [F(1), F(1)] + [F(0)] * (K - 1)
     t = first_guess(upper)
     t = halley(t, x)
     t = halley(t, x)
     s = list(t)
     s[0] -= 1  # s = t - 1
+    return s
+
+
+def series(upper):
+    s = exact_series(upper)
     n = K
     while n > 1 and abs(float(s[n])) * float(EPS_MAX) ** n < TOL:
         n -= 1
@@ -133,6 +147,58 @@ def sweep(up, lo, eps_max, n):
     return worst
 
 
+def about(s, e0):
+    """The series s about e0, its constant term with the 1: t's."""
+    out = [sum(s[i] * comb(i, j) * e0 ** (i - j) for i in range(j, K + 1)) for j in range(K + 1)]
+    out[0] += 1
+    return out
+
+
+def head(s, e0, sign):
+    """C[0..3] of the head on one side of e0: the fifth-order term, 1.9e-17 at its
+    edge D = EPS_SHORT, goes into them as d D^4 times the cubic nearest to x^4 on
+    [0, 1], (256 x^3 - 160 x^2 + 32 x - 1) / 128, x = |d| / D (Chebyshev): 1.5e-19 is left."""
+    c = about(s, e0)
+    top = [c[5] * EPS_SHORT ** 4 * k / 128 for k in (-1, 32, -160, 256)]
+    return [float(c[1 + i] + top[i] * (sign / EPS_SHORT) ** i) for i in range(4)]
+
+
+def root_series(n):
+    """e0 and t's series about it, above and below 1 (n terms after the constant)."""
+    up, lo = exact_series(True), exact_series(False)
+    bits = 200  # fixed point; the terms past the third are below 1e-30 at these e0
+    fix = [[round(c * 2 ** bits) for c in s[:4]] for s in (up, lo)]
+
+    def t_ulp(side, m):
+        """t - 1 at m units of 2^-52, in those units (2^bits of them)."""
+        a, b, c, d = fix[side]
+        return (a << 52) + m * (b + (m * (c + (m * d >> 52)) >> 52))
+
+    def off(m):
+        """How far from a double, in 2^bits."""
+        half = 1 << (bits - 1)
+        return (t_ulp(0, m) + half) % (1 << bits) - half
+
+    # The residue moves by almost a seventh a unit, so every seventh unit's moves
+    # slowly, with the series' curvature; from e0 = 1.5e-8 on it passes 0 (and far
+    # past that the two sides of 1 part by more than is allowed).
+    tol = 1 << (bits - 9)
+    step = 7 * 4096
+    for m in range(2 ** 26, 2 ** 27, step):
+        for r in range(7):
+            a, b = m + r, m + r + step
+            if abs(off(a)) < 1 << (bits - 5) and (off(a) < 0) != (off(b) < 0):
+                while b - a > 7:
+                    c = a + (b - a) // 14 * 7
+                    a, b = (a, c) if (off(a) < 0) != (off(c) < 0) else (c, b)
+                if abs(off(a)) < tol and abs(t_ulp(0, a) - t_ulp(1, a)) < tol:
+                    e0 = F(a, 2 ** 52)
+                    t0 = 1 + F(((t_ulp(0, a) >> (bits - 1)) + 1) >> 1, 2 ** 52)
+                    return (e0, t0, *([float(c) for c in about(s, e0)[1: n + 1]] for s in (up, lo)),
+                            head(up, e0, 1), head(lo, e0, -1))
+    raise AssertionError("no expansion point")
+
+
 def main():
     up, lo = series(True), series(False)
     worst = sweep(up, lo, EPS_MAX, max(len(up), len(lo)))
@@ -152,6 +218,15 @@ def main():
         f.write("#define PF7_SHORT_N %d\n" % nshort)
         for name, c in (("PF7_UP", up), ("PF7_LO", lo)):
             f.write("#define %s_N %d\n" % (name, len(c)))
+            f.write("#define %s_C {%s}\n" % (name, ", ".join(repr(v) for v in c)))
+        assert nshort == 5
+        e0, t0, rup, rlo, hup, hlo = root_series(max(len(up), len(lo)) - 1)
+        f.write("// powfancy7th(x) = PF7_ROOT_T + d (C[0] + d (C[1] + ...)), d = x - (1 + PF7_ROOT_E); |d| <=\n")
+        f.write("// PF7_EPS_SHORT: by the head alone\n")
+        f.write("#define PF7_ROOT_E %r\n" % float(e0))
+        f.write("#define PF7_ROOT_T %r\n" % float(t0))
+        for name, c in (("PF7_ROOT_UP", rup), ("PF7_ROOT_LO", rlo), ("PF7_ROOT_HEAD_UP", hup),
+                        ("PF7_ROOT_HEAD_LO", hlo)):
             f.write("#define %s_C {%s}\n" % (name, ", ".join(repr(v) for v in c)))
     print("pf7 series:", len(up), len(lo), "terms; worst gap", worst, "; short head", nshort, "terms, gap",
           worst_short)

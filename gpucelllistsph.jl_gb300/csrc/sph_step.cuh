@@ -369,49 +369,57 @@ __device__ inline double pf_cos(double r2, double k, const double* C) {
   return p;
 }
 
-// powfancy7th(1 + e) - 1, src/gpukernels_sph.jl:499-515.  Where |e| <=
-// PF7_EPS_MAX the exact Taylor series of that iteration's output
-// (gen_pf7_series.py, bias included) replaces its two divisions, and where
-// |e| <= PF7_EPS_SHORT its first PF7_SHORT_N terms do; elsewhere the iteration
-// itself runs.  ROOT: powfancy7th(1 + e) itself, rounded once.  (With the 1 in
-// the series' constant term, which 1 + a₀ holds to 8e-18, it takes an addition
-// less, 1% of a call with surface tension; 8% of the roots are then an ulp off,
-// and ∂ρ/∂t's error against extended precision is 1.4% larger in 2-D and 2.3%
-// in 3-D.)
-template <bool ROOT>
-__device__ inline double pf7_series(double e, double ginv, int gamma) {
-  const long long ae = dbits(e) & 0x7FFFFFFFFFFFFFFFLL;
-  static_assert(PF7_UP_N == PF7_LO_N, "series lengths");
-  constexpr double A0U[PF7_UP_N] = PF7_UP_C, A0L[PF7_LO_N] = PF7_LO_C;
-  static_assert(A0U[0] == A0L[0], "constant terms");  // cu[0] below
-  if (gamma == 7 && ae <= dbits(PF7_EPS_MAX)) {
-    const double cu[PF7_UP_N] = PF7_UP_C;
-    const double cl[PF7_LO_N] = PF7_LO_C;
-    const bool up = dbits(e) >= 0;
-    double r;
-    if (ae <= dbits(PF7_EPS_SHORT)) {
-      r = up ? cu[PF7_SHORT_N - 1] : cl[PF7_SHORT_N - 1];
+// The exact Taylor series of powfancy7th's output (src/gpukernels_sph.jl:499-515,
+// gen_pf7_series.py, bias included) in place of its two divisions: its terms past
+// the constant, over d, the distance from the expansion point, by N coefficients of
+// the side of 1 that d is on.
+template <int N>
+__device__ inline double pf7_poly(double d, const double* cu, const double* cl) {
+  const bool up = dbits(d) >= 0;
+  double r = up ? cu[N - 1] : cl[N - 1];
 #pragma unroll
-      for (int i = PF7_SHORT_N - 2; i >= 1; --i) r = fma(r, e, up ? cu[i] : cl[i]);
-    } else {
-      r = up ? cu[PF7_UP_N - 1] : cl[PF7_UP_N - 1];
-#pragma unroll
-      for (int i = PF7_UP_N - 2; i >= 1; --i) r = fma(r, e, up ? cu[i] : cl[i]);
-    }
-    const double m1 = fma(r, e, cu[0]);
-    return ROOT ? 1.0 + m1 : m1;
-  }
-  const double t = powfancy7th_1div(1.0 + e, ginv, gamma);
-  return ROOT ? t : t - 1.0;
+  for (int i = N - 2; i >= 0; --i) r = fma(r, d, up ? cu[i] : cl[i]);
+  return r;
+}
+__device__ inline bool pf7_within(double d, double bound) {
+  return (dbits(d) & 0x7FFFFFFFFFFFFFFFLL) <= dbits(bound);
 }
 // powfancy7th(1 + e) - 1, e taken as it is
-__device__ inline double pf7m1_fast(double e, double ginv, int gamma) { return pf7_series<false>(e, ginv, gamma); }
-// powfancy7th(1 + eps): with e = (1 + eps) - 1, the argument that the
-// reference's rounded x carries, and rounded as its t.  The step's passes take
-// this: near rest ρ0 t - ρ0 is of the size of these roundings (without them a
-// resting tank's largest ∂ρ/∂t, 1.9e-8, is 1.1e-12 of it off the oracle's).
+__device__ inline double pf7m1_fast(double e, double ginv, int gamma) {
+  static_assert(PF7_UP_N == PF7_LO_N, "series lengths");
+  constexpr double A0U[PF7_UP_N] = PF7_UP_C, A0L[PF7_LO_N] = PF7_LO_C;
+  static_assert(A0U[0] == A0L[0], "constant terms");
+  if (gamma == 7 && pf7_within(e, PF7_EPS_MAX)) {
+    const double cu[PF7_UP_N] = PF7_UP_C;
+    const double cl[PF7_LO_N] = PF7_LO_C;
+    const double r = pf7_within(e, PF7_EPS_SHORT) ? pf7_poly<PF7_SHORT_N - 1>(e, cu + 1, cl + 1)
+                                                  : pf7_poly<PF7_UP_N - 1>(e, cu + 1, cl + 1);
+    return fma(r, e, cu[0]);
+  }
+  return powfancy7th_1div(1.0 + e, ginv, gamma) - 1.0;
+}
+// powfancy7th(x) of the reference's rounded x = 1 + eps, and rounded once, as its
+// t.  The step's passes take this: near rest ρ0 t - ρ0 is of the size of these
+// roundings (without them a resting tank's largest ∂ρ/∂t, 1.9e-8, is 1.1e-12 of it
+// off the oracle's).  The expansion point is a double at which t is one to
+// a 500th of its last bit, so the polynomial's last step is the rounding.  (About
+// 1, with the 1 in a constant that holds 1 + a₀ to 8e-18, 8% of the roots are an
+// ulp off, and ∂ρ/∂t's error against extended precision is 1.4% larger in 2-D and
+// 2.3% in 3-D; with the 1 added last, ten steps of 2-D full physics take 6149 us,
+// about this point 6023; about it with the bounds asked of eps rather than of d, for
+// the code's layout, 6134.)
 __device__ inline double pf7_fast(double eps, double ginv, int gamma) {
-  return pf7_series<true>((1.0 + eps) - 1.0, ginv, gamma);
+  const double x = 1.0 + eps, d = x - (1.0 + PF7_ROOT_E);
+  if (gamma == 7 && pf7_within(d, PF7_EPS_MAX)) {
+    const double cu[PF7_UP_N - 1] = PF7_ROOT_UP_C;
+    const double cl[PF7_LO_N - 1] = PF7_ROOT_LO_C;
+    const double hu[PF7_SHORT_N - 1] = PF7_ROOT_HEAD_UP_C;
+    const double hl[PF7_SHORT_N - 1] = PF7_ROOT_HEAD_LO_C;
+    const double r = pf7_within(d, PF7_EPS_SHORT) ? pf7_poly<PF7_SHORT_N - 1>(d, hu, hl)
+                                                  : pf7_poly<PF7_UP_N - 1>(d, cu, cl);
+    return fma(r, d, PF7_ROOT_T);
+  }
+  return powfancy7th_1div(x, ginv, gamma);
 }
 
 // pair-once passes (sph_once.cu): pass A over the device-side pair count,
