@@ -81,6 +81,8 @@ int gcl_partialupdate(gcl_handle* h, int64_t* pairsn_out);
  * (2*cap int32).  If the set holds more than cap pairs the first cap are
  * written and GCSPH_ECAPACITY is returned with *pairsn_out = the full count
  * (the reference counts past capacity too, src/gpukernels_cls.jl:333-338).
+ * After a build that failed there is no pair set: GCSPH_ESTATE, until the next
+ * build that succeeds.
  * fillzero != 0 zero-fills pairs [pairsn, cap) (src/celllist.jl:112,142). */
 int gcl_emit_pairs(gcl_handle* h, int32_t* pairs_dev, int64_t cap, int fillzero, int64_t* pairsn_out);
 
